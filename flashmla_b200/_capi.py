@@ -115,7 +115,12 @@ SYMBOLS = {
     "mla_selftest_bounded_wait": (c_int, [c_longlong, c_int, c_void_p, c_void_p, c_void_p]),
 }
 
+# the functions csrc/host.cpp calls, in the order of its Api structure
+_HOST_SYMBOLS = ("mla_last_error", "mla_num_sm_parts", "mla_num_sm_parts_uniform", "mla_get_sched_meta", "mla_dense_decode_fwd",
+                 "mla_sparse_decode_fwd", "mla_combine", "mla_sparse_prefill_fwd", "mla_quantize_fp8_kvcache")
+
 _lib = None
+_host = None
 _lock = threading.Lock()
 
 
@@ -139,6 +144,23 @@ def lib():
                                        f"{ABI_VERSION}: rebuild it with `python -m flashmla_b200.build --force`")
                 _lib = handle
     return _lib
+
+
+def host():
+    """The host extension (csrc/host.cpp), bound to the loaded library; raises if it has not been built."""
+    global _host
+    if _host is None:
+        handle = lib()
+        with _lock:
+            if _host is None:
+                import torch  # noqa: F401  (its libraries have to be loaded first)
+                try:
+                    from . import _host as module
+                except ImportError as e:
+                    raise RuntimeError(f"flashmla_b200/_host.so cannot be loaded ({e}): build it with `python -m flashmla_b200.build`") from e
+                module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in _HOST_SYMBOLS))
+                _host = module
+    return _host
 
 
 def check(rc: int, what: str):

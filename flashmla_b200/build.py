@@ -3,18 +3,21 @@
     python -m flashmla_b200.build [--force] [--verbose]
 
 Each .cu file is compiled to an object (in parallel, skipped when up to date) and the
-objects are linked into flashmla_b200/libflashmla_b200.so.  No PyTorch headers are used.
+objects are linked into flashmla_b200/libflashmla_b200.so.  No PyTorch headers are used there.
+csrc/host.cpp, the host path of the Python API, is compiled against PyTorch's C++ headers into
+flashmla_b200/_host.so.
 """
 import argparse
 import os
 import subprocess
-import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "libflashmla_b200.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -57,6 +60,28 @@ def _compile_one(src, obj, verbose):
     return log
 
 
+def _build_host(force):
+    src = os.path.join(CSRC, "host.cpp")
+    newest = max(os.path.getmtime(src), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= newest:
+        return
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = os.path.join(root, "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
+           src, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    with open(os.path.join(OBJ_DIR, "host.log"), "w") as f:
+        f.write(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
+    if proc.returncode != 0:
+        raise RuntimeError(f"compiling {src} failed:\n" + proc.stdout + proc.stderr)
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ_DIR, exist_ok=True)
     hdr_mtime = _headers_mtime()
@@ -68,8 +93,10 @@ def build(force=False, verbose=False):
         stale = force or not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_mtime)
         if stale:
             jobs.append((src, obj))
-    with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(jobs) + 1)) as ex:
+        host = ex.submit(_build_host, force)
         list(ex.map(lambda so: _compile_one(so[0], so[1], verbose), jobs))
+        host.result()
     if jobs or not os.path.exists(LIB_PATH):
         cmd = [_nvcc(), "-shared", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"]
         proc = subprocess.run(cmd, capture_output=True, text=True)

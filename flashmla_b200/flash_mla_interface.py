@@ -2,8 +2,8 @@
 (flash_mla/flash_mla_interface.py:8-211 of deepseek-ai/FlashMLA): same function names, parameter
 order, keywords, assertion texts and return shapes, so existing call sites only change the import.
 
-PyTorch is used for device memory and the current stream; every kernel is launched through the
-C ABI of libflashmla_b200.so (include/flashmla_b200.h).  There is no CPU path.
+PyTorch is used for device memory and the current stream; csrc/host.cpp checks the arguments, allocates the outputs and
+launches every kernel through the C ABI of libflashmla_b200.so (include/flashmla_b200.h).  There is no CPU path.
 """
 import dataclasses
 from typing import Optional, Tuple
@@ -32,39 +32,22 @@ def set_kernel_timer(timer) -> None:
     _kernel_timer = timer
 
 
-def _launch(name: str, fn, args) -> None:
-    if _kernel_timer is None:
-        _capi.check(fn(args), name)
-    else:
-        _kernel_timer.start(name)
-        _capi.check(fn(args), name)
-        _kernel_timer.stop(name)
-
-
-# Per-device status words written by kernels whose bounded waits ran out: [first code, count, -, -].
-_status_buffers = {}
-
-
 def _status(device) -> torch.Tensor:
-    buf = _status_buffers.get(device)
-    if buf is None:
-        buf = torch.zeros(4, dtype=torch.int32, device=device)
-        _status_buffers[device] = buf
-    return buf
+    """The device's status words, written by kernels whose bounded waits ran out: [first code, count, -, -]."""
+    device = torch.device(device)
+    return _capi.host().status(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def check_status(device=None) -> None:
     """Synchronises and raises if a kernel reported that one of its bounded waits ran out (a pipeline
     error: the results of that launch are invalid).  The status words are cleared."""
-    devices = list(_status_buffers) if device is None else [torch.device(device)]
-    for dev in devices:
-        buf = _status_buffers.get(dev)
-        if buf is None:
+    for buf in _capi.host().known_status():
+        if device is not None and buf.device != torch.device(device):
             continue
         vals = buf.cpu().tolist()
         if vals[0] != 0:
             buf.zero_()
-            raise RuntimeError(f"flashmla_b200: a kernel on {dev} gave up a bounded wait (code {vals[0]}, {vals[1]} threads)")
+            raise RuntimeError(f"flashmla_b200: a kernel on {buf.device} gave up a bounded wait (code {vals[0]}, {vals[1]} threads)")
 
 
 def set_impl(impl: int) -> None:
@@ -109,6 +92,13 @@ class FlashMLASchedMeta:
     uniform_costs: Optional[bool] = None
 
 
+# the fields of a schedule's configuration and what the caller knows them as
+_CONFIG_NAMES = (("b", "batch_size"), ("s_q", "seq_len_q"), ("h_q", "num_heads_q"), ("page_block_size", "page_block_size"),
+                 ("h_k", "num_heads_k"), ("causal", "causal"), ("is_fp8_kvcache", "is_fp8_kvcache"),
+                 ("topk", "the last dim of indices_in_kvcache"), ("extra_page_block_size", "the page_block_size of extra_k_cache"),
+                 ("extra_topk", "the last dim of extra_indices_in_kvcache"))
+
+
 def get_mla_metadata(*args, **kwargs) -> Tuple[FlashMLASchedMeta, None]:
     """
     Returns an empty FlashMLASchedMeta; the scheduling metadata is generated by the first
@@ -118,243 +108,18 @@ def get_mla_metadata(*args, **kwargs) -> Tuple[FlashMLASchedMeta, None]:
     return FlashMLASchedMeta(), None
 
 
-def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
-
-
-def _require_cuda(name: str, t: Optional[torch.Tensor], device=None):
-    if t is None:
-        return
-    if not t.is_cuda:
-        raise RuntimeError(f"{name} must be a CUDA tensor (this library has no CPU path)")
-    if device is not None and t.device != device:
-        raise RuntimeError(f"{name} must be on {device}, got {t.device}")
-
-
 def _make_sched_meta(b, s_q, num_sm_parts, device, seqlens_k=None, topk=-1, extra_topk=0,
                      topk_length=None, extra_topk_length=None):
+    """A schedule for callers of the C ABI (the calls below make theirs on the way)."""
     meta = torch.empty((num_sm_parts, _META_INTS), dtype=torch.int32, device=device)
     num_splits = torch.empty((b + 1,), dtype=torch.int32, device=device)
     a = _capi.SchedMetaArgs(
         b=b, s_q=s_q, block_size_n=_BLOCK_SIZE_N, fixed_overhead_num_blocks=_FIXED_OVERHEAD_NUM_BLOCKS,
         topk=topk, extra_topk=extra_topk,
         topk_length=ptr(topk_length), extra_topk_length=ptr(extra_topk_length), seqlens_k=ptr(seqlens_k),
-        meta=ptr(meta), num_splits=ptr(num_splits), num_sm_parts=num_sm_parts, stream=_stream_ptr(device))
+        meta=ptr(meta), num_splits=ptr(num_splits), num_sm_parts=num_sm_parts, stream=torch.cuda.current_stream(device).cuda_stream)
     _capi.check(_capi.lib().mla_get_sched_meta(a), "mla_get_sched_meta")
     return meta, num_splits
-
-
-def _check_meta(meta, num_splits, num_sm_parts, b, device):
-    if meta.dtype != torch.int32 or num_splits.dtype != torch.int32:
-        raise RuntimeError("tile_scheduler_metadata and num_splits must have dtype int32")
-    if tuple(meta.shape) != (num_sm_parts, _META_INTS) or tuple(num_splits.shape) != (b + 1,):
-        raise RuntimeError(
-            f"tile_scheduler_metadata must have shape ({num_sm_parts}, {_META_INTS}) and num_splits ({b + 1},); "
-            f"got {tuple(meta.shape)} and {tuple(num_splits.shape)}")
-    if not (meta.is_contiguous() and num_splits.is_contiguous()):
-        raise RuntimeError("tile_scheduler_metadata and num_splits must be contiguous")
-    _require_cuda("tile_scheduler_metadata", meta, device)
-    _require_cuda("num_splits", num_splits, device)
-
-
-def _dense_decode_fwd(q, kcache, head_size_v, seqlens_k, block_table, softmax_scale, is_causal, meta, num_splits):
-    """Mirror of dense_attn_decode_interface (csrc/api/dense_decode.h:13-225)."""
-    if q.dtype not in (torch.bfloat16, torch.float16):
-        raise RuntimeError("q must have dtype bfloat16 or float16")
-    if kcache.dtype != q.dtype:
-        raise RuntimeError("query and key must have the same dtype")
-    dtype_code = _capi.MLA_DTYPE_FP16 if q.dtype == torch.float16 else _capi.MLA_DTYPE_BF16
-    if seqlens_k.dtype != torch.int32:
-        raise RuntimeError("seqlens_k must have dtype int32")
-    if block_table.dtype != torch.int32:
-        raise RuntimeError("block_table must have dtype torch.int32")
-    device = q.device
-    for n, t in (("q", q), ("kcache", kcache), ("seqlens_k", seqlens_k), ("block_table", block_table)):
-        _require_cuda(n, t, device)
-    if q.stride(-1) != 1:
-        raise RuntimeError("q must have contiguous last dimension")
-    if kcache.stride(-1) != 1:
-        raise RuntimeError("kcache must have contiguous last dimension")
-    if not seqlens_k.is_contiguous():
-        raise RuntimeError("seqlens_k must be contiguous")
-    if block_table.stride(-1) != 1:
-        raise RuntimeError("block_table must have contiguous last dimension")
-    if q.dim() != 4 or kcache.dim() != 4 or block_table.dim() != 2:
-        raise RuntimeError("q and kcache must be 4-D, block_table 2-D")
-    b, s_q, h_q, d = q.shape
-    num_blocks, page_block_size, h_kv, d_k = kcache.shape
-    if d != 576 or d_k != d:
-        raise RuntimeError("Only head_size_k == 576 is supported")
-    if head_size_v != 512:
-        raise RuntimeError("Only head_size_v == 512 is supported")
-    if page_block_size != 64:
-        raise RuntimeError("Currently page_block_size must be 64")
-    if b <= 0:
-        raise RuntimeError("batch size must be positive")
-    if h_q % h_kv != 0:
-        raise RuntimeError("Number of heads in key/value must divide number of heads in query")
-    if tuple(seqlens_k.shape) != (b,) or block_table.size(0) != b:
-        raise RuntimeError("seqlens_k must have shape (batch_size,) and block_table (batch_size, max_num_blocks_per_seq)")
-    if s_q == 1:
-        is_causal = False
-
-    lib = _capi.lib()
-    with torch.cuda.device(device):
-        num_sm_parts = lib.mla_num_sm_parts(device.index, _capi.MLA_MODE_DENSE_DECODE, h_q, h_kv, s_q)
-        if num_sm_parts <= 0:
-            _capi.check(1, "mla_num_sm_parts")
-        if meta is None:
-            meta, num_splits = _make_sched_meta(b, s_q, num_sm_parts, device, seqlens_k=seqlens_k)
-        else:
-            _check_meta(meta, num_splits, num_sm_parts, b, device)
-
-        out = torch.empty((b, s_q, h_q, head_size_v), dtype=q.dtype, device=device)
-        lse = torch.empty((b, h_q, s_q), dtype=torch.float32, device=device)
-        total_splits = b + num_sm_parts
-        lse_accum = torch.empty((total_splits, s_q, h_q), dtype=torch.float32, device=device)
-        o_accum = torch.empty((total_splits, s_q, h_q, head_size_v), dtype=torch.float32, device=device)
-        stream = _stream_ptr(device)
-        a = _capi.DenseDecodeArgs(
-            b=b, s_q=s_q, h_q=h_q, h_kv=h_kv, d_qk=d, d_v=head_size_v, num_blocks=num_blocks,
-            page_block_size=page_block_size, is_causal=int(bool(is_causal)), softmax_scale=float(softmax_scale),
-            q=ptr(q), q_stride_b=q.stride(0), q_stride_s=q.stride(1), q_stride_h=q.stride(2),
-            k_cache=ptr(kcache), k_stride_block=kcache.stride(0), k_stride_row=kcache.stride(1), k_stride_head=kcache.stride(2),
-            block_table=ptr(block_table), block_table_stride_b=block_table.stride(0), max_blocks_per_seq=block_table.size(1),
-            seqlens_k=ptr(seqlens_k),
-            out=ptr(out), o_stride_b=out.stride(0), o_stride_s=out.stride(1), o_stride_h=out.stride(2),
-            lse=ptr(lse), lse_stride_b=lse.stride(0), lse_stride_s=lse.stride(2), lse_stride_h=lse.stride(1),
-            meta=ptr(meta), num_splits=ptr(num_splits), num_sm_parts=num_sm_parts,
-            lse_accum=ptr(lse_accum), o_accum=ptr(o_accum), status=ptr(_status(device)), impl=_impl_override,
-            dtype=dtype_code, stream=stream)
-        _launch("mla_dense_decode_fwd", lib.mla_dense_decode_fwd, a)
-        c = _capi.CombineArgs(
-            b=b, s_q=s_q, h_q=h_q, d_v=head_size_v,
-            lse=ptr(lse), lse_stride_b=lse.stride(0), lse_stride_s=lse.stride(2), lse_stride_h=lse.stride(1),
-            out=ptr(out), o_stride_b=out.stride(0), o_stride_s=out.stride(1), o_stride_h=out.stride(2),
-            lse_accum=ptr(lse_accum), o_accum=ptr(o_accum), num_splits=ptr(num_splits), attn_sink=None,
-            dtype=dtype_code, stream=stream)
-        _launch("mla_combine", lib.mla_combine, c)
-    return out, lse, meta, num_splits
-
-
-def _fp8_cache_check(name, kv, d_qk):
-    if kv.dtype not in (torch.float8_e4m3fn, torch.int8, torch.uint8):
-        raise RuntimeError(f"{name} must have dtype fp8_e4m3fn, int8 or uint8")
-    if kv.dim() != 4:
-        raise RuntimeError(f"{name} must be 4-D (num_blocks, page_block_size, 1, bytes_per_token)")
-    if kv.stride(-1) != 1:
-        raise RuntimeError(f"{name} must have contiguous last dimension")
-    if kv.size(2) != 1:
-        raise RuntimeError("Currently only MQA (i.e. h_kv == 1) is supported for sparse decoding")
-    # bytes per token as the reference computes them (csrc/api/sparse_decode.h:289-299)
-    bytes_per_token = 512 + 64 * 2 + (512 // 128) * 4 if d_qk == 576 else 448 + 64 * 2 + (448 // 64) * 1 + 1
-    if kv.size(3) != bytes_per_token:
-        what = "512 fp8 + 4 fp32 scales + 64 bf16" if d_qk == 576 else "448 fp8 + 64 bf16 + 7 e8m0 scales + 1 pad"
-        raise RuntimeError(f"{name}: each token must take {bytes_per_token} bytes ({what}), got {kv.size(3)}")
-    if kv.stride(1) != bytes_per_token:
-        raise RuntimeError("The whole block must be contiguous when is_fp8_cache is True for kv cache")
-
-
-def _sparse_decode_fwd(q, kv, indices, topk_length, attn_sink, meta, num_splits, extra_kv, extra_indices,
-                       extra_topk_length, d_v, sm_scale):
-    """Mirror of sparse_attn_decode_interface (csrc/api/sparse_decode.h:183-495)."""
-    if q.dim() != 4 or indices.dim() != 3:
-        raise RuntimeError("q must be 4-D and indices 3-D")
-    device = q.device
-    b, s_q, h_q, d_qk = q.shape
-    topk = indices.size(2)
-    if q.dtype != torch.bfloat16:
-        raise RuntimeError("q must have dtype bfloat16")
-    if d_qk not in (576, 512):
-        raise RuntimeError("Only head_size_k == 576 or 512 is supported for sparse decoding")
-    if d_v != 512:
-        raise RuntimeError("Only head_size_v == 512 is supported for sparse decoding")
-    if topk <= 0:
-        raise RuntimeError("topk must be positive")
-    _fp8_cache_check("key", kv, d_qk)
-    if extra_kv is not None:
-        if extra_indices is None:
-            raise RuntimeError("extra_indices_in_kvcache must be provided when extra_kcache is provided for sparse attention")
-        _fp8_cache_check("extra k cache", extra_kv, d_qk)
-    else:
-        if extra_indices is not None:
-            raise RuntimeError("extra_indices_in_kvcache must not be provided when extra_k_cache is not provided")
-        if extra_topk_length is not None:
-            raise RuntimeError("extra_topk_length must not be provided when extra_k_cache is not provided")
-    for n, t in (("q", q), ("kv", kv), ("indices", indices), ("topk_length", topk_length), ("attn_sink", attn_sink),
-                 ("extra_kv", extra_kv), ("extra_indices", extra_indices), ("extra_topk_length", extra_topk_length)):
-        _require_cuda(n, t, device)
-    for n, t in (("indices", indices), ("extra_indices", extra_indices), ("topk_length", topk_length),
-                 ("extra_topk_length", extra_topk_length)):
-        if t is not None and t.dtype != torch.int32:
-            raise RuntimeError(f"{n} must have dtype int32")
-    if attn_sink is not None and (attn_sink.dtype != torch.float32 or tuple(attn_sink.shape) != (h_q,) or not attn_sink.is_contiguous()):
-        raise RuntimeError("attn_sink must be a contiguous float32 tensor of shape (h_q,)")
-    if q.stride(-1) != 1 or indices.stride(-1) != 1 or (extra_indices is not None and extra_indices.stride(-1) != 1):
-        raise RuntimeError("q and indices must have contiguous last dimension")
-    if tuple(indices.shape[:2]) != (b, s_q):
-        raise RuntimeError("indices must have shape (b, s_q, topk)")
-    for n, t in (("topk_length", topk_length), ("extra_topk_length", extra_topk_length)):
-        if t is not None and (tuple(t.shape) != (b,) or not t.is_contiguous()):
-            raise RuntimeError(f"{n} must be contiguous with shape (b,)")
-    extra_topk = extra_indices.size(-1) if extra_indices is not None else 0
-    if extra_indices is not None and tuple(extra_indices.shape[:2]) != (b, s_q):
-        raise RuntimeError("extra_indices must have shape (b, s_q, extra_topk)")
-
-    lib = _capi.lib()
-    with torch.cuda.device(device):
-        uniform = topk_length is None and extra_topk_length is None
-        if uniform:
-            # every request costs the same number of KV blocks: let the partition count follow the batch size
-            blocks = (topk + 63) // 64 + (extra_topk + 63) // 64
-            num_sm_parts = lib.mla_num_sm_parts_uniform(device.index, _capi.MLA_MODE_SPARSE_DECODE, h_q, 1, s_q, b, blocks)
-        else:
-            num_sm_parts = lib.mla_num_sm_parts(device.index, _capi.MLA_MODE_SPARSE_DECODE, h_q, 1, s_q)
-        if num_sm_parts <= 0:
-            _capi.check(1, "mla_num_sm_parts")
-        if meta is None:
-            meta, num_splits = _make_sched_meta(b, s_q, num_sm_parts, device, topk=topk, extra_topk=extra_topk,
-                                                topk_length=topk_length, extra_topk_length=extra_topk_length)
-        else:
-            _check_meta(meta, num_splits, num_sm_parts, b, device)
-        out = torch.empty((b, s_q, h_q, d_v), dtype=q.dtype, device=device)
-        lse = torch.empty((b, s_q, h_q), dtype=torch.float32, device=device)
-        total_splits = b + num_sm_parts
-        lse_accum = torch.empty((total_splits, s_q, h_q), dtype=torch.float32, device=device)
-        o_accum = torch.empty((total_splits, s_q, h_q, d_v), dtype=torch.float32, device=device)
-        stream = _stream_ptr(device)
-        a = _capi.SparseDecodeArgs(
-            b=b, s_q=s_q, h_q=h_q, d_qk=d_qk, d_v=d_v, sm_scale=float(sm_scale),
-            q=ptr(q), q_stride_b=q.stride(0), q_stride_s=q.stride(1), q_stride_h=q.stride(2),
-            kv=ptr(kv), kv_stride_block_bytes=kv.stride(0) * kv.element_size(), num_blocks=kv.size(0), page_block_size=kv.size(1),
-            indices=ptr(indices), indices_stride_b=indices.stride(0), indices_stride_s=indices.stride(1), topk=topk,
-            topk_length=ptr(topk_length),
-            extra_kv=ptr(extra_kv),
-            extra_kv_stride_block_bytes=(extra_kv.stride(0) * extra_kv.element_size()) if extra_kv is not None else 0,
-            extra_num_blocks=extra_kv.size(0) if extra_kv is not None else 0,
-            extra_page_block_size=extra_kv.size(1) if extra_kv is not None else 0,
-            extra_indices=ptr(extra_indices),
-            extra_indices_stride_b=extra_indices.stride(0) if extra_indices is not None else 0,
-            extra_indices_stride_s=extra_indices.stride(1) if extra_indices is not None else 0,
-            extra_topk=extra_topk, extra_topk_length=ptr(extra_topk_length),
-            attn_sink=ptr(attn_sink),
-            out=ptr(out), o_stride_b=out.stride(0), o_stride_s=out.stride(1), o_stride_h=out.stride(2),
-            lse=ptr(lse), lse_stride_b=lse.stride(0), lse_stride_s=lse.stride(1), lse_stride_h=lse.stride(2),
-            meta=ptr(meta), num_splits=ptr(num_splits), num_sm_parts=num_sm_parts,
-            lse_accum=ptr(lse_accum), o_accum=ptr(o_accum), status=ptr(_status(device)), impl=_impl_override, stream=stream)
-        _launch("mla_sparse_decode_fwd", lib.mla_sparse_decode_fwd, a)
-        if uniform and num_sm_parts == b:
-            # equal costs and one partition per request: the scheduler cuts at every request boundary, no request is
-            # split and the decode kernel has already written `out` and `lse`
-            return out, lse.transpose(1, 2), meta, num_splits
-        c = _capi.CombineArgs(
-            b=b, s_q=s_q, h_q=h_q, d_v=d_v,
-            lse=ptr(lse), lse_stride_b=lse.stride(0), lse_stride_s=lse.stride(1), lse_stride_h=lse.stride(2),
-            out=ptr(out), o_stride_b=out.stride(0), o_stride_s=out.stride(1), o_stride_h=out.stride(2),
-            lse_accum=ptr(lse_accum), o_accum=ptr(o_accum), num_splits=ptr(num_splits), attn_sink=ptr(attn_sink),
-            stream=stream)
-        _launch("mla_combine", lib.mla_combine, c)
-    return out, lse.transpose(1, 2), meta, num_splits
 
 
 def flash_mla_with_kvcache(
@@ -407,34 +172,32 @@ def flash_mla_with_kvcache(
     assert isinstance(sched_meta, FlashMLASchedMeta), "tile_scheduler_metadata must be of type FlashMLASchedMeta"
     assert num_splits is None, "num_splits must be None"
 
+    q_shape, k_shape = q.shape, k_cache.shape
     topk = indices_in_kvcache.shape[-1] if indices_in_kvcache is not None else None
     extra_k_page_block_size = extra_k_cache.shape[1] if extra_k_cache is not None else None
     extra_topk = extra_indices_in_kvcache.shape[-1] if extra_indices_in_kvcache is not None else None
     if softmax_scale is None:
-        softmax_scale = q.shape[-1] ** (-0.5)
+        softmax_scale = q_shape[-1] ** (-0.5)
 
     if not sched_meta.have_initialized:
         if indices_in_kvcache is not None:
             assert not causal, "causal must be False when indices_in_kvcache is not None (i.e. sparse attention is enabled)"
         sched_meta.have_initialized = True
         sched_meta.config = FlashMLASchedMeta.Config(
-            q.shape[0], q.shape[1], q.shape[2], k_cache.shape[1], k_cache.shape[2],
+            q_shape[0], q_shape[1], q_shape[2], k_shape[1], k_shape[2],
             causal, is_fp8_kvcache, topk, extra_k_page_block_size, extra_topk)
     else:
-        helper_msg = " Your input arguments are inconsistent with sched_meta. Please make sure the input arguments are consistent across different invocations of flash_mla_with_kvcache on the same sched_meta."
         cfg = sched_meta.config
         assert cfg is not None
-        assert cfg.b == q.shape[0], "sched_meta.config.b must be equal to batch_size." + helper_msg
-        assert cfg.s_q == q.shape[1], "sched_meta.config.s_q must be equal to seq_len_q." + helper_msg
-        assert cfg.h_q == q.shape[2], "sched_meta.config.h_q must be equal to num_heads_q." + helper_msg
-        assert cfg.page_block_size == k_cache.shape[1], "sched_meta.config.page_block_size must be equal to page_block_size." + helper_msg
-        assert cfg.h_k == k_cache.shape[2], "sched_meta.config.h_k must be equal to num_heads_k." + helper_msg
-        assert cfg.causal == causal, "sched_meta.config.causal must be equal to causal." + helper_msg
-        assert cfg.is_fp8_kvcache == is_fp8_kvcache, "sched_meta.config.is_fp8_kvcache must be equal to is_fp8_kvcache." + helper_msg
-        assert cfg.topk == topk, "sched_meta.config.topk must be equal to the last dim of indices_in_kvcache." + helper_msg
-        assert cfg.extra_page_block_size == extra_k_page_block_size, "sched_meta.config.extra_page_block_size must be equal to the page_block_size of extra_k_cache." + helper_msg
-        assert cfg.extra_topk == extra_topk, "sched_meta.config.extra_topk must be equal to the last dim of extra_indices_in_kvcache." + helper_msg
+        given = (q_shape[0], q_shape[1], q_shape[2], k_shape[1], k_shape[2], causal, is_fp8_kvcache, topk, extra_k_page_block_size, extra_topk)
+        if given != (cfg.b, cfg.s_q, cfg.h_q, cfg.page_block_size, cfg.h_k, cfg.causal, cfg.is_fp8_kvcache, cfg.topk,
+                     cfg.extra_page_block_size, cfg.extra_topk):
+            for (name, what), value in zip(_CONFIG_NAMES, given):
+                assert getattr(cfg, name) == value, (
+                    f"sched_meta.config.{name} must be equal to {what}. Your input arguments are inconsistent with sched_meta. "
+                    "Please make sure the input arguments are consistent across different invocations of flash_mla_with_kvcache on the same sched_meta.")
 
+    host = _capi.host()
     if topk is not None:
         assert not causal, "causal must be False when sparse attention is enabled"
         assert is_fp8_kvcache, "is_fp8_kvcache must be True when sparse attention is enabled"
@@ -442,18 +205,16 @@ def flash_mla_with_kvcache(
         if sched_meta.tile_scheduler_metadata is not None and sched_meta.uniform_costs != uniform:
             sched_meta.tile_scheduler_metadata = sched_meta.num_splits = None      # made under the other partition rule
         sched_meta.uniform_costs = uniform
-        out, lse, new_meta, new_num_splits = _sparse_decode_fwd(
+        out, lse, sched_meta.tile_scheduler_metadata, sched_meta.num_splits = host.sparse_decode(
             q, k_cache, indices_in_kvcache, topk_length, attn_sink,
             sched_meta.tile_scheduler_metadata, sched_meta.num_splits,
-            extra_k_cache, extra_indices_in_kvcache, extra_topk_length, head_dim_v, softmax_scale)
+            extra_k_cache, extra_indices_in_kvcache, extra_topk_length, head_dim_v, softmax_scale, _impl_override, _kernel_timer)
     else:
         assert indices_in_kvcache is None and attn_sink is None and extra_k_cache is None and extra_indices_in_kvcache is None and topk_length is None and extra_topk_length is None, "indices_in_kvcache, attn_sink, extra_k_cache, extra_indices_in_kvcache, topk_length and extra_topk_length must be None when dense attention is used."
         assert block_table is not None and cache_seqlens is not None, "block_table and cache_seqlens must be provided when dense attention is used."
-        out, lse, new_meta, new_num_splits = _dense_decode_fwd(
+        out, lse, sched_meta.tile_scheduler_metadata, sched_meta.num_splits = host.dense_decode(
             q, k_cache, head_dim_v, cache_seqlens, block_table, softmax_scale, causal,
-            sched_meta.tile_scheduler_metadata, sched_meta.num_splits)
-    sched_meta.tile_scheduler_metadata = new_meta
-    sched_meta.num_splits = new_num_splits
+            sched_meta.tile_scheduler_metadata, sched_meta.num_splits, _impl_override, _kernel_timer)
     return out, lse
 
 
@@ -474,45 +235,4 @@ def flash_mla_sparse_fwd(
         attn_sink [h_q] fp32 (optional); topk_length [s_q] int32 (optional)
     Returns (out [s_q, h_q, 512] bf16, max_logits [s_q, h_q] fp32, lse [s_q, h_q] fp32).
     """
-    if q.dim() != 3 or kv.dim() != 3 or indices.dim() != 3:
-        raise RuntimeError("q, kv and indices must be 3-D")
-    device = q.device
-    for n, t in (("q", q), ("kv", kv), ("indices", indices), ("attn_sink", attn_sink), ("topk_length", topk_length)):
-        _require_cuda(n, t, device)
-    s_q, h_q, d_qk = q.shape
-    s_kv, h_kv, _ = kv.shape
-    topk = indices.size(2)
-    if q.dtype != torch.bfloat16 or kv.dtype != torch.bfloat16:
-        raise RuntimeError("q and kv must have dtype bfloat16")
-    if indices.dtype != torch.int32:
-        raise RuntimeError("indices must have dtype int32")
-    if d_qk not in (576, 512) or kv.size(2) != d_qk:
-        raise RuntimeError("Only d_qk == 576 or 512 is supported")
-    if d_v != 512:
-        raise RuntimeError("Only d_v == 512 is supported")
-    if h_kv != 1:
-        raise RuntimeError("Only h_kv == 1 is supported")
-    if tuple(indices.shape[:2]) != (s_q, h_kv):
-        raise RuntimeError("indices must have shape (s_q, h_kv, topk)")
-    if q.stride(-1) != 1 or kv.stride(-1) != 1 or indices.stride(-1) != 1:
-        raise RuntimeError("q, kv and indices must have contiguous last dimension")
-    if attn_sink is not None and (attn_sink.dtype != torch.float32 or tuple(attn_sink.shape) != (h_q,) or not attn_sink.is_contiguous()):
-        raise RuntimeError("attn_sink must be a contiguous float32 tensor of shape (h_q,)")
-    if topk_length is not None and (topk_length.dtype != torch.int32 or tuple(topk_length.shape) != (s_q,) or not topk_length.is_contiguous()):
-        raise RuntimeError("topk_length must be a contiguous int32 tensor of shape (s_q,)")
-
-    lib = _capi.lib()
-    with torch.cuda.device(device):
-        out = torch.empty((s_q, h_q, d_v), dtype=q.dtype, device=device)
-        max_logits = torch.empty((s_q, h_q), dtype=torch.float32, device=device)
-        lse = torch.empty((s_q, h_q), dtype=torch.float32, device=device)
-        a = _capi.SparsePrefillArgs(
-            s_q=s_q, s_kv=s_kv, h_q=h_q, h_kv=h_kv, d_qk=d_qk, d_v=d_v, topk=topk, sm_scale=float(sm_scale),
-            q=ptr(q), q_stride_s=q.stride(0), q_stride_h=q.stride(1),
-            kv=ptr(kv), kv_stride_s=kv.stride(0), kv_stride_h=kv.stride(1),
-            indices=ptr(indices), indices_stride_s=indices.stride(0), indices_stride_h=indices.stride(1),
-            attn_sink=ptr(attn_sink), topk_length=ptr(topk_length),
-            out=ptr(out), max_logits=ptr(max_logits), lse=ptr(lse),
-            status=ptr(_status(device)), impl=_impl_override, stream=_stream_ptr(device))
-        _launch("mla_sparse_prefill_fwd", lib.mla_sparse_prefill_fwd, a)
-    return out, max_logits, lse
+    return _capi.host().sparse_prefill(q, kv, indices, sm_scale, d_v, attn_sink, topk_length, _impl_override, _kernel_timer)

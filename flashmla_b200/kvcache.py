@@ -30,12 +30,7 @@ def quantize_fp8_kvcache(blocked_k: torch.Tensor, pow2_scale: bool = False, pad_
     buf = torch.empty((nb, bs + pad_rows, BYTES_PER_TOKEN), dtype=torch.float8_e4m3fn, device=blocked_k.device)
     res = buf[:, :bs, :]
     assert x.stride(-1) == 1, "the last dimension of blocked_k must be contiguous"
-    with torch.cuda.device(blocked_k.device):
-        args = _capi.QuantizeArgs(
-            x=_capi.ptr(x), x_stride_block=x.stride(0), x_stride_row=x.stride(1), num_blocks=nb, block_size=bs,
-            out=_capi.ptr(buf), out_stride_block_bytes=buf.stride(0), pow2_scale=1 if pow2_scale else 0,
-            stream=torch.cuda.current_stream().cuda_stream)
-        _capi.check(_capi.lib().mla_quantize_fp8_kvcache(args), "mla_quantize_fp8_kvcache")
+    _capi.host().quantize(x, buf, buf.stride(0), pow2_scale, 0)
     return res.view(nb, bs, 1, BYTES_PER_TOKEN)
 
 
@@ -59,10 +54,5 @@ def quantize_fp8_kvcache_model1(blocked_k: torch.Tensor) -> torch.Tensor:
     x = blocked_k.squeeze(2)
     assert x.stride(-1) == 1, "the last dimension of blocked_k must be contiguous"
     buf = torch.zeros((nb, model1_block_bytes(bs)), dtype=torch.uint8, device=blocked_k.device).view(torch.float8_e4m3fn)
-    with torch.cuda.device(blocked_k.device):
-        args = _capi.QuantizeArgs(
-            x=_capi.ptr(x), x_stride_block=x.stride(0), x_stride_row=x.stride(1), num_blocks=nb, block_size=bs,
-            out=_capi.ptr(buf), out_stride_block_bytes=buf.stride(0), pow2_scale=1, layout=1,
-            stream=torch.cuda.current_stream().cuda_stream)
-        _capi.check(_capi.lib().mla_quantize_fp8_kvcache(args), "mla_quantize_fp8_kvcache")
+    _capi.host().quantize(x, buf, buf.stride(0), True, 1)
     return buf[:, :bs * M1_BYTES_PER_TOKEN].view(nb, bs, 1, M1_BYTES_PER_TOKEN)
