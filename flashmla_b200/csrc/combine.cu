@@ -5,44 +5,71 @@
 // where g' additionally absorbs the attention sink: g' = g + log2(1 + 2^{sink*log2e - g}).
 // Semantics follow csrc/smxx/decode/combine/combine.cu:72-160 of the reference.
 //
-// HBM-bound: per (request, query token, head) it reads n_splits * 2 KiB and writes 1 KiB.
-// One warp per row; every lane keeps 16 output columns in registers (4 x float4 loads per split,
-// fully coalesced 512 B per warp instruction), split weights are computed once per 32 splits and
-// broadcast by shuffle, so there is no limit on the number of splits.
+// Per (request, query token, head) it reads n_splits * 2 KiB and writes 1 KiB: HBM-bound where there are many rows, bound
+// by its chain of memory latencies (split counts -> log-sum-exps -> partials -> output) where there are few.  A row is served
+// by WPR warps of a CTA, each taking every WPR-th split with 16 output columns per lane (4 x float4 per split: 512 coalesced
+// bytes per warp instruction); with WPR > 1 their sums meet in shared memory.  The first partials are requested together
+// with the log-sum-exps, so that a row of up to WPR * UNROLL splits costs two round trips instead of three.  There is no
+// limit on the number of splits.
 #include "common.cuh"
 #include <cuda_fp16.h>
+#include <algorithm>
 
 namespace mla {
 
 constexpr int COMBINE_WARPS = 8;
 
-__global__ void __launch_bounds__(COMBINE_WARPS * 32)
+template <int WPR>
+__global__ void __launch_bounds__(COMBINE_WARPS * 32, WPR == 8 ? 2 : WPR == 1 ? 4 : 3)
 combine_kernel(const mla_combine_args_t a) {
-    // launched with programmatic stream serialization: the decode kernel before it may still be running
+    // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
+    // kernel set itself up from here on costs more than it hides: its CTAs take whole SMs while this grid still needs them;
+    // dense decode with 2 query tokens 346 -> 351 us a step.)
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int ROWS = COMBINE_WARPS / WPR;            // heads per CTA
+    constexpr int UNROLL = WPR == 8 ? 4 : 2;             // splits in flight per warp
+    __shared__ float part[WPR > 1 ? COMBINE_WARPS * 512 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sub = warp % WPR;
     const int bs_idx = blockIdx.x;                       // request * s_q + query token
     const int req = bs_idx / a.s_q, t = bs_idx - req * a.s_q;
-    const int head = blockIdx.y * COMBINE_WARPS + warp;
-    if (head >= a.h_q) return;
+    const int head = min((int)blockIdx.y * ROWS + warp / WPR, a.h_q - 1);
+    const bool head_ok = blockIdx.y * ROWS + warp / WPR < a.h_q;
     const int s0 = a.num_splits[req], s1 = a.num_splits[req + 1];
     const int n = s1 - s0;
-    if (n <= 1) return;                                  // the decode kernel wrote the final result
+    if (n <= 1) return;                                  // the decode kernel wrote the final result (whole CTA)
 
     const int64_t row_stride = (int64_t)a.s_q * a.h_q;   // rows per split slot
     const float* lse_acc = a.lse_accum + (int64_t)s0 * row_stride + (int64_t)t * a.h_q + head;
-    const float* o_acc = a.o_accum + ((int64_t)s0 * row_stride + (int64_t)t * a.h_q + head) * a.d_v;
+    const float4* o_acc = reinterpret_cast<const float4*>(a.o_accum + ((int64_t)s0 * row_stride + (int64_t)t * a.h_q + head) * 512) + lane;
+    const int64_t o_step = row_stride * 128;             // float4s from one split to the next
+
+    // the first partials of this warp; their weights are not known yet
+    float4 v[UNROLL][4];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+        const int s = sub + u * WPR;
+        if (s < n) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
+        }
+    }
 
     // pass 1: global log-sum-exp over the splits
-    float mx = -INFINITY;
-    for (int s = lane; s < n; s += 32) mx = fmaxf(mx, lse_acc[(int64_t)s * row_stride]);
+    const float l_first = lane < n ? lse_acc[lane * row_stride] : -INFINITY;
+    float mx = l_first;
+#pragma unroll 1
+    for (int s = lane + 32; s < n; s += 32) mx = fmaxf(mx, lse_acc[(int64_t)s * row_stride]);
+#pragma unroll
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (mx == -INFINITY) mx = 0.f;
-    float sum = 0.f;
-    for (int s = lane; s < n; s += 32) sum += exp2f(lse_acc[(int64_t)s * row_stride] - mx);
+    float sum = exp2f(l_first - mx);
+#pragma unroll 1
+    for (int s = lane + 32; s < n; s += 32) sum += exp2f(lse_acc[(int64_t)s * row_stride] - mx);
+#pragma unroll
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     float g = (sum == 0.f || sum != sum) ? INFINITY : log2f(sum) + mx;
-    if (lane == 0)
+    if (lane == 0 && sub == 0 && head_ok)
         a.lse[req * a.lse_stride_b + t * a.lse_stride_s + head * a.lse_stride_h] = g * kLn2;
     if (a.attn_sink) {
         const float sink = a.attn_sink[head];
@@ -50,41 +77,78 @@ combine_kernel(const mla_combine_args_t a) {
         else g = sink == -INFINITY ? INFINITY : sink * kLog2e;
     }
 
-    // pass 2: weighted sum.  d_v = 512 = 32 lanes x 4 float4.
+    // pass 2: weighted sum of this warp's splits.  Lane l holds columns 4 l .. 4 l + 3 of every 128.
     float4 acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int sb = 0; sb < n; sb += 32) {
-        const int s_mine = sb + lane;
-        const float w_mine = s_mine < n ? exp2f(lse_acc[(int64_t)s_mine * row_stride] - g) : 0.f;
-        const int cnt = min(32, n - sb);
-        for (int j = 0; j < cnt; ++j) {
-            const float w = __shfl_sync(0xffffffffu, w_mine, j);
-            const float4* src = reinterpret_cast<const float4*>(o_acc + (int64_t)(sb + j) * row_stride * a.d_v);
+    float w_block = exp2f(l_first - g);                  // weights of splits block .. block + 31, one per lane
+    int block = 0;
+#pragma unroll 1
+    for (int base = sub; base < n; base += UNROLL * WPR) {
+        if (base >= UNROLL * WPR) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 v = src[lane + i * 32];
-                acc[i].x += w * v.x; acc[i].y += w * v.y; acc[i].z += w * v.z; acc[i].w += w * v.w;
+            for (int u = 0; u < UNROLL; ++u) {
+                const int s = base + u * WPR;
+                if (s < n) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int s = base + u * WPR;
+            if (s < n) {
+                if ((s & ~31) != block) {                // (splits of a warp ascend)
+                    block = s & ~31;
+                    w_block = block + lane < n ? exp2f(lse_acc[(int64_t)(block + lane) * row_stride] - g) : 0.f;
+                }
+                const float w = __shfl_sync(0xffffffffu, w_block, s & 31);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[i].x += w * v[u][i].x; acc[i].y += w * v[u][i].y; acc[i].z += w * v[u][i].z; acc[i].w += w * v[u][i].w;
+                }
             }
         }
     }
     // out is bf16 or fp16: both are 2 bytes wide
     __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + req * a.o_stride_b + t * a.o_stride_s + head * a.o_stride_h;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    auto store4 = [&](int col, float4 x) {
         uint2 packed;
         if (a.dtype == MLA_DTYPE_FP16) {
-            __half2 lo = __floats2half2_rn(acc[i].x, acc[i].y);
-            __half2 hi = __floats2half2_rn(acc[i].z, acc[i].w);
+            __half2 lo = __floats2half2_rn(x.x, x.y);
+            __half2 hi = __floats2half2_rn(x.z, x.w);
             packed.x = *reinterpret_cast<uint32_t*>(&lo);
             packed.y = *reinterpret_cast<uint32_t*>(&hi);
         } else {
-            __nv_bfloat162 lo = __floats2bfloat162_rn(acc[i].x, acc[i].y);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(acc[i].z, acc[i].w);
+            __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y);
+            __nv_bfloat162 hi = __floats2bfloat162_rn(x.z, x.w);
             packed.x = *reinterpret_cast<uint32_t*>(&lo);
             packed.y = *reinterpret_cast<uint32_t*>(&hi);
         }
-        *reinterpret_cast<uint2*>(o + (lane + i * 32) * 4) = packed;
+        *reinterpret_cast<uint2*>(o + col) = packed;
+    };
+    if (WPR == 1) {
+        if (!head_ok) return;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) store4((lane + i * 32) * 4, acc[i]);
+    } else {
+        float4* mine = reinterpret_cast<float4*>(part) + warp * 128 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mine[i * 32] = acc[i];
+        __syncthreads();
+        // every warp of the row adds up and writes 512 / WPR columns
+        if (!head_ok) return;
+        const float4* row = reinterpret_cast<const float4*>(part) + (warp - sub) * 128;
+        for (int c = sub * (128 / WPR) + lane; c < (sub + 1) * (128 / WPR); c += 32) {
+            float4 x = row[c];
+#pragma unroll
+            for (int k = 1; k < WPR; ++k) {
+                const float4 y = row[k * 128 + c];
+                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+            }
+            store4(c * 4, x);
+        }
     }
 }
 
@@ -96,8 +160,22 @@ int launch_combine(const mla_combine_args_t& a) {
     MLA_CHECK_ARG(is_aligned16(a.o_accum), "combine: o_accum must be 16-byte aligned");
     MLA_CHECK_ARG(((uintptr_t)a.out & 7u) == 0 && a.o_stride_b % 4 == 0 && a.o_stride_s % 4 == 0 && a.o_stride_h % 4 == 0,
                   "combine: out must be 8-byte aligned with strides that are multiples of 4 elements");
-    dim3 grid(a.b * a.s_q, (a.h_q + COMBINE_WARPS - 1) / COMBINE_WARPS);
-    MLA_CHECK_CUDA(launch_dependent(combine_kernel, grid, dim3(COMBINE_WARPS * 32), 0, (cudaStream_t)a.stream, a));
+    // Warps per row: about one for every two splits a row can be expected to have (the partitions of a decode launch shared
+    // out over the batch), as long as all CTAs run in one wave (2 per SM with the deeper unrolling of WPR = 8, else 3).  With
+    // few rows the time is one row's chain of loads: 128 rows of 74 splits took 42 us with one warp per row, 10 us with eight;
+    // 976 rows of 2 splits are 3 us slower with two warps per row than with one.
+    const int64_t rows = (int64_t)a.b * a.s_q * a.h_q;
+    const int sms = current_device_num_sms() > 0 ? current_device_num_sms() : 148;
+    const int splits = 1 + sms / 2 / std::max(1, (a.s_q * a.h_q + 127) / 128) / a.b;
+    const int64_t wave = (int64_t)sms * 3 * COMBINE_WARPS;         // warps
+    const int wpr = splits >= 16 && rows <= 2 * sms ? 8 : splits >= 8 && rows * 4 <= wave ? 4 : splits >= 4 && rows * 2 <= wave ? 2 : 1;
+    const int rows_per_cta = COMBINE_WARPS / wpr;
+    const dim3 grid(a.b * a.s_q, (a.h_q + rows_per_cta - 1) / rows_per_cta), block(COMBINE_WARPS * 32);
+    const cudaStream_t stream = (cudaStream_t)a.stream;
+    MLA_CHECK_CUDA(wpr == 8   ? launch_dependent(combine_kernel<8>, grid, block, 0, stream, a)
+                   : wpr == 4 ? launch_dependent(combine_kernel<4>, grid, block, 0, stream, a)
+                   : wpr == 2 ? launch_dependent(combine_kernel<2>, grid, block, 0, stream, a)
+                              : launch_dependent(combine_kernel<1>, grid, block, 0, stream, a));
     return MLA_OK;
 }
 
