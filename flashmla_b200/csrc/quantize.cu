@@ -3,8 +3,11 @@
 // (tests/quant.py:20-53 of the reference: scale = amax / 448 per group of 128, optionally rounded up to a power of
 // two; q = e4m3(x / scale), round to nearest even).
 //
-// One warp per token: lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is
-// one coalesced 512-byte store.  HBM-bound: 1152 bytes read + 656 bytes written per token.
+// One warp per token: lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is one
+// coalesced 512-byte store.  HBM-bound: 1152 bytes read + 656 bytes written per token.  Every warp takes two tokens, whose
+// loads are in flight together.  With one IEEE division per value (__fdiv_rn, a dozen instructions and a branch) the kernel
+// was bound by instructions instead: 34 us for 66 K tokens (3.5 TB/s).  The quotients x / s only need the correctly rounded
+// reciprocal of s, once per group, and three instructions each (Markstein's theorem; quotient16 below).
 //
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
@@ -16,11 +19,65 @@
 
 namespace mla {
 
+constexpr int TOKENS = 2;             // per warp, in flight together
+
 __device__ __forceinline__ float pow2_ceil(float s) {
     // smallest power of two >= s (s > 0, normal)
     const uint32_t bits = __float_as_uint(s);
     const uint32_t mant = bits & 0x007fffffu;
     return __uint_as_float((bits & 0x7f800000u) + (mant ? 0x00800000u : 0u));
+}
+
+__device__ __forceinline__ void unpack16(const uint4& v0, const uint4& v1, float (&f)[16], float& amax) {
+    const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        amax = fmaxf(amax, fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1])));
+    }
+}
+
+// e4m3(x / s) of a lane's 16 values, x / s rounded to fp32 first.  With r = RN(1 / s) and q = RN(x r), q + r (x - q s)
+// is RN(x / s) (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990; here checked for every bf16 significand against every fp32 significand of s).  The remainder has to be exact: the
+// group's largest magnitude `amax` keeps clear of overflow and underflow, and values so far below it that the remainder
+// could be subnormal (below 2^-20 amax) have quotients under 2^-11, which are zeros in e4m3 whatever their last bit.
+// Groups outside that range (warp-uniform choice) divide.
+__device__ __forceinline__ uint4 quotient16(const float (&f)[16], float s, float amax) {
+    const bool plain = (amax >= 0x1p-60f && amax <= 0x1p100f) || amax == 0.f;
+    uint32_t q[4];
+    if (__all_sync(0xffffffffu, plain)) {
+        const float r = __frcp_rn(s);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float2 d[2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float x = f[4 * i + k], q0 = x * r;
+                reinterpret_cast<float*>(d)[k] = fmaf(fmaf(-q0, s, x), r, q0);
+            }
+            q[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(d[0], __NV_SATFINITE, __NV_E4M3) |
+                   (uint32_t)__nv_cvt_float2_to_fp8x2(d[1], __NV_SATFINITE, __NV_E4M3) << 16;
+        }
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+            uint32_t word = 0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (k >> 2 == i) word |= (uint32_t)__nv_cvt_float_to_fp8(__fdiv_rn(f[k], s), __NV_SATFINITE, __NV_E4M3) << (8 * (k & 3));
+            if (i == 0) q[0] = word; else if (i == 1) q[1] = word; else if (i == 2) q[2] = word; else q[3] = word;
+        }
+    }
+    return make_uint4(q[0], q[1], q[2], q[3]);
+}
+
+// 32-bit division where the token count allows
+__device__ __forceinline__ void block_of(int64_t tok, int64_t ntok, int block_size, int64_t& blk, int64_t& row) {
+    blk = ntok <= 0x7fffffff ? (int64_t)((uint32_t)tok / (uint32_t)block_size) : tok / block_size;
+    row = tok - blk * block_size;
 }
 
 __global__ void __launch_bounds__(256)
@@ -29,39 +86,35 @@ quantize_fp8_kernel(const mla_quantize_args_t a) {
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    for (int64_t tok = warp; tok < ntok; tok += nwarps) {
-        const int64_t blk = tok / a.block_size, row = tok - blk * a.block_size;
-        const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk * a.x_stride_block + row * a.x_stride_row;
-        uint8_t* out = (uint8_t*)a.out + blk * a.out_stride_block_bytes + row * 656;
-        const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(x + lane * 16));
-        const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
-        const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        float f[16];
-        float amax = 0.f;
+    for (int64_t tok0 = warp * TOKENS; tok0 < ntok; tok0 += nwarps * TOKENS) {
+        uint4 v0[TOKENS], v1[TOKENS], rope[TOKENS];
+        uint8_t* out[TOKENS];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            f[2 * i] = __uint_as_float(w[i] << 16);
-            f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-            amax = fmaxf(amax, fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1])));
+        for (int k = 0; k < TOKENS; ++k) {
+            if (tok0 + k >= ntok) break;
+            int64_t blk, row;
+            block_of(tok0 + k, ntok, a.block_size, blk, row);
+            const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk * a.x_stride_block + row * a.x_stride_row;
+            out[k] = (uint8_t*)a.out + blk * a.out_stride_block_bytes + row * 656;
+            v0[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16));
+            v1[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
+            if (lane < 8) rope[k] = __ldcs(reinterpret_cast<const uint4*>(x + 512 + lane * 8));
         }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        float s = __fdiv_rn(amax, 448.f);
-        s = a.pow2_scale ? pow2_ceil(fmaxf(s, 1e-4f)) : fmaxf(s, 1e-30f);
-        uint32_t q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t word = 0;
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                word |= (uint32_t)__nv_cvt_float_to_fp8(__fdiv_rn(f[4 * i + b], s), __NV_SATFINITE, __NV_E4M3) << (8 * b);
-            q[i] = word;
+        for (int k = 0; k < TOKENS; ++k) {
+            if (tok0 + k >= ntok) break;
+            float f[16], amax;
+            unpack16(v0[k], v1[k], f, amax);
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+            float s = __fdiv_rn(amax, 448.f);
+            s = a.pow2_scale ? pow2_ceil(fmaxf(s, 1e-4f)) : fmaxf(s, 1e-30f);
+            *reinterpret_cast<uint4*>(out[k] + lane * 16) = quotient16(f, s, amax);
+            const float sg = __shfl_sync(0xffffffffu, s, (lane & 3) * 8);          // lanes 0-3: scale of group `lane`
+            if (lane < 4) reinterpret_cast<float*>(out[k] + 512)[lane] = sg;
+            if (lane < 8) *reinterpret_cast<uint4*>(out[k] + 528 + lane * 16) = rope[k];
         }
-        *reinterpret_cast<uint4*>(out + lane * 16) = make_uint4(q[0], q[1], q[2], q[3]);
-        const float sg = __shfl_sync(0xffffffffu, s, (lane & 3) * 8);          // lanes 0-3: scale of group `lane`
-        if (lane < 4) reinterpret_cast<float*>(out + 512)[lane] = sg;
-        if (lane < 8) *reinterpret_cast<uint4*>(out + 528 + lane * 16) = __ldg(reinterpret_cast<const uint4*>(x + 512 + lane * 8));
     }
 }
 
@@ -71,43 +124,39 @@ quantize_fp8_model1_kernel(const mla_quantize_args_t a) {
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    for (int64_t tok = warp; tok < ntok; tok += nwarps) {
-        const int64_t blk = tok / a.block_size, row = tok - blk * a.block_size;
-        const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk * a.x_stride_block + row * a.x_stride_row;
-        uint8_t* block = (uint8_t*)a.out + blk * a.out_stride_block_bytes;
-        uint8_t* out = block + row * 576;
-        const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(x + lane * 16));
-        const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
-        const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        float f[16];
-        float amax = 0.f;
+    for (int64_t tok0 = warp * TOKENS; tok0 < ntok; tok0 += nwarps * TOKENS) {
+        uint4 v0[TOKENS], v1[TOKENS];
+        int64_t blk[TOKENS], row[TOKENS];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            f[2 * i] = __uint_as_float(w[i] << 16);
-            f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-            amax = fmaxf(amax, fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1])));
+        for (int k = 0; k < TOKENS; ++k) {
+            if (tok0 + k >= ntok) break;
+            block_of(tok0 + k, ntok, a.block_size, blk[k], row[k]);
+            const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk[k] * a.x_stride_block + row[k] * a.x_stride_row;
+            v0[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16));
+            v1[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
         }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float s = pow2_ceil(fmaxf(__fdiv_rn(amax, 448.f), 1e-4f));
-        if (lane < 28) {
-            uint32_t q[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t word = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-                    word |= (uint32_t)__nv_cvt_float_to_fp8(__fdiv_rn(f[4 * i + b], s), __NV_SATFINITE, __NV_E4M3) << (8 * b);
-                q[i] = word;
+        for (int k = 0; k < TOKENS; ++k) {
+            if (tok0 + k >= ntok) break;
+            uint8_t* block = (uint8_t*)a.out + blk[k] * a.out_stride_block_bytes;
+            uint8_t* out = block + row[k] * 576;
+            float f[16], amax;
+            unpack16(v0[k], v1[k], f, amax);
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            const float s = pow2_ceil(fmaxf(__fdiv_rn(amax, 448.f), 1e-4f));
+            const uint4 q = quotient16(f, s, lane < 28 ? amax : 0.f);
+            if (lane < 28) {
+                *reinterpret_cast<uint4*>(out + lane * 16) = q;
+            } else {
+                *reinterpret_cast<uint4*>(out + 448 + (lane - 28) * 32) = v0[k];
+                *reinterpret_cast<uint4*>(out + 448 + (lane - 28) * 32 + 16) = v1[k];
             }
-            *reinterpret_cast<uint4*>(out + lane * 16) = make_uint4(q[0], q[1], q[2], q[3]);
-        } else {
-            *reinterpret_cast<uint4*>(out + 448 + (lane - 28) * 32) = v0;
-            *reinterpret_cast<uint4*>(out + 448 + (lane - 28) * 32 + 16) = v1;
+            // lane g < 7 writes the scale of group g (held by lanes 4g .. 4g+3) as its exponent byte; lane 7 the pad byte
+            const float sg = __shfl_sync(0xffffffffu, s, (lane & 7) * 4);
+            uint8_t* scales = block + (int64_t)a.block_size * 576;
+            if (lane < 8) scales[row[k] * 8 + lane] = lane < 7 ? (uint8_t)(__float_as_uint(sg) >> 23) : 0;
         }
-        // lane g < 7 writes the scale of group g (held by lanes 4g .. 4g+3) as its exponent byte; lane 7 the pad byte
-        const float sg = __shfl_sync(0xffffffffu, s, (lane & 7) * 4);
-        if (lane < 8) block[(int64_t)a.block_size * 576 + row * 8 + lane] = lane < 7 ? (uint8_t)(__float_as_uint(sg) >> 23) : 0;
     }
 }
 
@@ -121,10 +170,7 @@ int launch_quantize_fp8(const mla_quantize_args_t& a) {
     MLA_CHECK_ARG(is_aligned16(a.out) && a.out_stride_block_bytes % 16 == 0 && a.out_stride_block_bytes >= (int64_t)a.block_size * rec,
                   "mla_quantize_fp8_kvcache: out must be 16-byte aligned, block stride a multiple of 16 bytes and >= block_size * %d", rec);
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    const int sms = current_device_num_sms();
-    int64_t blocks = (ntok + 7) / 8;
-    const int64_t cap = (int64_t)(sms > 0 ? sms : 148) * 32;
-    if (blocks > cap) blocks = cap;
+    const int64_t blocks = min((ntok + 8 * TOKENS - 1) / (8 * TOKENS), (int64_t)1 << 24);
     if (a.layout) quantize_fp8_model1_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
     else quantize_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
     MLA_CHECK_CUDA(cudaGetLastError());

@@ -53,6 +53,6 @@ def quantize_fp8_kvcache_model1(blocked_k: torch.Tensor) -> torch.Tensor:
         raise RuntimeError("blocked_k must be a CUDA tensor (this library has no CPU path)")
     x = blocked_k.squeeze(2)
     assert x.stride(-1) == 1, "the last dimension of blocked_k must be contiguous"
-    buf = torch.zeros((nb, model1_block_bytes(bs)), dtype=torch.uint8, device=blocked_k.device).view(torch.float8_e4m3fn)
+    buf = torch.empty((nb, model1_block_bytes(bs)), dtype=torch.float8_e4m3fn, device=blocked_k.device)
     _capi.host().quantize(x, buf, buf.stride(0), True, 1)
     return buf[:, :bs * M1_BYTES_PER_TOKEN].view(nb, bs, 1, M1_BYTES_PER_TOKEN)
