@@ -36,8 +36,8 @@
 // up to rounding.
 //
 // Every mbarrier wait is bounded (Params::wait_limit SM cycles, about a second by default).  A thread whose
-// wait ran out records a code in the status words, raises the `aborted` flag of both CTAs and LEAVES its role:
-// it issues no further arrival, MMA or copy.  Single-thread roles leave at once; warps leave together (a vote
+// wait ran out LEAVES its role - it issues no further arrival, MMA or copy -, records a code in the status words and raises
+// the `aborted` flag of both CTAs.  Single-thread roles leave at once; warps leave together (a vote
 // after every wait, because tcgen05.ld/st are warp-collective); the two softmax warpgroups, which meet at a
 // named barrier every tile, carry the flag through that barrier (bar.red.or) and leave together behind it.
 // Threads that depend on the one that left run into their own limit.  The wind-down then waits - again
@@ -72,19 +72,32 @@ constexpr int NPB = 4;                        // P buffers in the value CTA: (ti
 constexpr int NRING = 5;                      // ring barriers: K groups (score CTA, 3 or 4) / V slots (value CTA, 5)
 constexpr int SIDE_BYTES = 144;               // per warp and tile: 32 rescale factors + flag (+ pad)
 constexpr int NTHREADS = 384;                 // dense mode: control warpgroup + two softmax / correction warpgroups
-constexpr int NTHREADS_GATHER = 512;          // sparse modes: one more warpgroup that gathers KV rows by index
 constexpr long long WAIT_LIMIT_DEFAULT = 2000000000LL;    // SM cycles (about one second)
 constexpr long long DRAIN_LIMIT = 4000000LL;              // wind-down after an expired wait: per tracked operation
 constexpr long long SETTLE_CYCLES = 400000LL;             // ... and for copies between the two CTAs
 #ifndef MLA_TAIL_BULK
 #define MLA_TAIL_BULK 1
 #endif
-#ifndef MLA_SLEEP_NS
-#define MLA_SLEEP_NS 200u
-#endif
 constexpr float RESCALE_THRESHOLD = 6.0f;         // log2 units
 
 enum { MODE_DENSE = 0, MODE_PREFILL = 1, MODE_SPARSE_DECODE = 2 };
+
+// Warps behind the control warpgroup and the two softmax / correction warpgroups: GATHER warps copy KV rows by index,
+// CONVERT warps de-quantise FP8 records.  A kernel starts with its registers shared out evenly (launch bound) and every
+// warpgroup re-sizes its share as the first thing in its branch; the shares add up to no more than the launch had.
+//   prefill     640 threads x 96 registers: control 64, softmax 144, gather 64.  EIGHT gather warps: an SM's copy rate is
+//               bound by what its warps can issue, 77 GB/s with four warps, 102 with eight (stand-alone probe).
+//   FP8 decode  768 threads x 80 registers: control 48, softmax 112, gather 80, convert 64.  The conversion has warps of its
+//               own: on the softmax warps it was serial with the softmax (5.2 us a tile).
+template <int MODE>
+struct Warps {
+    static constexpr int GATHER = MODE == MODE_DENSE ? 0 : MODE == MODE_PREFILL ? 8 : 4;
+    static constexpr int CONVERT = MODE == MODE_SPARSE_DECODE ? 8 : 0;
+    static constexpr int FIRST_GATHER = 12, FIRST_CONVERT = 12 + GATHER;
+    static constexpr int THREADS = (12 + GATHER + CONVERT) * 32;
+};
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // Shared-memory and tensor-memory plan of the score CTA, per mode (byte offsets inside Smem::data).
 template <int MODE>
@@ -142,7 +155,7 @@ struct Params {
     int head_chunks;                       // dense mode: 64-column chunks between two kv heads of a cache row
     int max_blocks;                        // dense mode: width of the block table
     float scale_log2;
-    long long wait_limit;                  // SM cycles after which a barrier wait gives up
+    uint32_t wait_limit;                   // SM cycles after which a barrier wait gives up
     const __nv_bfloat16* q; int64_t q_sb, q_ss, q_sh;
     int q_tma, q_box_bytes;                // a request's Q comes as 9 TMA boxes of q_box_bytes through the empty K ring
     __nv_bfloat16* out; int64_t o_sb, o_ss, o_sh;
@@ -247,54 +260,47 @@ struct Walker<MODE_PREFILL> {
     __device__ void next() { req += gridDim.z; }
 };
 
-#ifndef MLA_PRESPIN_DENSE
-#define MLA_PRESPIN_DENSE 0
-#endif
-#ifndef MLA_PRESPIN_GATHER
-#define MLA_PRESPIN_GATHER 64
-#endif
-
-// What a thread does when one of its bounded waits runs out: first code and a count in the global status words,
-// the `aborted` flag of this CTA and of its peer.  Shared with the self-test kernel at the end of this file.
-// (Out of line on purpose: inlined at every wait site it cost the dense kernel 10 % - 0.176 against 0.160 ms - although
-// it never runs: the hot loops of all roles have to share the instruction cache.)
+// ---- bounded waits -------------------------------------------------------------------------------------------
+// A wait is a loop of probes (the hardware holds a thread for a while before it answers one) and 32-bit clock reads: eight
+// instructions.  All roles of a CTA share one instruction cache, and there are some thirty wait sites in their loops: with
+// 64-bit clocks, unrolled probes and the reporting at every site the gather modes spent most of their time fetching
+// instructions (4096-token prefill 3440 -> 3010 us, FP8 decode of 64 requests 143 -> 102 us, dense serving 200 -> 186 us for kernels otherwise equal).
+// A thread whose wait ran out only keeps the site's code; it reports when it has left its role.
+//
+// wait() / wait_warp() return false when the wait ran out now or earlier: the caller leaves its role.  CLUSTER: the
+// arrivals come from the other CTA of the pair.
+struct Waiter {
+    uint32_t limit;                      // SM cycles (below 2^32)
+    int code = 0;
+    __device__ explicit Waiter(uint32_t limit_) : limit(limit_) {}
+    template <bool CLUSTER>
+    __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int site) {
+        if (code) return false;
+        const uint32_t t0 = clock_lo();
+#pragma unroll 1
+        while (!(CLUSTER ? mbar_try_wait_cluster(smem_addr(bar), parity) : mbar_try_wait(smem_addr(bar), parity)))
+            if (clock_lo() - t0 > limit) { code = site; break; }
+        return code == 0;
+    }
+    // whole warps (all 32 lanes execute this): the same answer for every lane
+    template <bool CLUSTER>
+    __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, int site) {
+        wait<CLUSTER>(bar, parity, site);
+        return !__any_sync(0xffffffffu, code != 0);
+    }
+};
+// First code and a count in the global status words, the `aborted` flag of this CTA and of its peer.
 __device__ __noinline__ void report_expired_wait(int* status, uint32_t* flag, uint32_t peer_flag, int code) {
     *reinterpret_cast<volatile uint32_t*>(flag) = 1;
     if (peer_flag) st_cluster_u32(peer_flag, 1u);
     if (status) { atomicCAS(status, 0, code); atomicAdd(status + 1, 1); }
 }
 
-// Bounded wait helper.  wait() returns false when the wait ran out now or earlier: the caller leaves its role.
-// LEAN: no unrolled probes before the timed loop (dense mode).
-template <bool LEAN>
-struct Waiter {
-    bool aborted = false;
-    bool parked;                         // park the thread between probes instead of spinning
-    uint32_t sleep_ns;                   // ... and sleep this long between probes
-    long long limit;
-    int* status;
-    uint32_t* flag;
-    uint32_t peer_flag;
-    __device__ Waiter(int* st, uint32_t* flag_, uint32_t peer_flag_, long long limit_, bool park = false, uint32_t sleep = 0)
-        : parked(park), sleep_ns(sleep), limit(limit_), status(st), flag(flag_), peer_flag(peer_flag_) {}
-    template <bool CLUSTER>
-    __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int code) {
-        if (aborted) return false;
-        const bool ok = parked ? mbar_wait_bounded_parked<CLUSTER>(smem_addr(bar), parity, limit, sleep_ns)
-                               : mbar_wait_bounded<CLUSTER, LEAN ? MLA_PRESPIN_DENSE : MLA_PRESPIN_GATHER>(smem_addr(bar), parity, limit);
-        if (!ok) {
-            aborted = true;
-            report_expired_wait(status, flag, peer_flag, code);
-        }
-        return ok;
-    }
-};
-
 // single-thread roles: leave at once
 #define WAIT_OR_LEAVE(W, CL, bar, par, code) do { if (!(W).template wait<CL>(bar, par, code)) goto wind_down; } while (0)
 // whole warps (all 32 lanes execute this): leave together, tcgen05.ld/st and shuffles are warp-collective
 #define WAIT_WARP_OR_LEAVE(W, CL, bar, par, code) \
-    do { (W).template wait<CL>(bar, par, code); if (__any_sync(0xffffffffu, (W).aborted)) goto wind_down; } while (0)
+    do { if (!(W).template wait_warp<CL>(bar, par, code)) goto wind_down; } while (0)
 // the two softmax warpgroups of the score CTA: their named barrier carries the flag
 #define BAR_OR_LEAVE(flag) do { if (named_bar_red_or(1, 256, flag)) goto wind_down; } while (0)
 
@@ -405,11 +411,12 @@ __device__ __noinline__ void load_q_by_threads(Smem& sm, const __nv_bfloat16* qr
 // Sparse prefill: 512-wide rows; the ninth 64-column chunk of Q and K is zeros.  (A compile-time switch in every mode: the
 // same choice read from the parameters inside the gather loop cost the 576-wide prefill 8 %.)
 template <int MODE, bool ALT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MODE == MODE_DENSE ? NTHREADS : NTHREADS_GATHER, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Warps<MODE>::THREADS, 1)
 attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                   const __grid_constant__ CUtensorMap qmap, const Params p) {
     using WalkerT = Walker<MODE>;
     using L = Lay<MODE>;
+    using W = Warps<MODE>;
     constexpr int NKS = L::NKS;
     constexpr bool DENSE = MODE == MODE_DENSE;
     constexpr bool FP16 = ALT && MODE == MODE_DENSE;
@@ -430,11 +437,11 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     }
 
     if (threadIdx.x == 0) {
-        // a ring slot is filled by TMA (one arrive.expect_tx + bytes) in dense mode, by the 128 gather threads otherwise
-        // ... except the K groups of FP8 decode, which the 256 softmax threads of the score CTA hand over after de-quantising them
-        const uint32_t full_count = DENSE ? 1 : (MODE == MODE_SPARSE_DECODE && cta_rank == 0) ? 256 : 128;
+        // a ring slot is filled by TMA (one arrive.expect_tx + bytes) in dense mode, by the gather threads in prefill, and
+        // handed over by the converting threads in FP8 decode
+        const uint32_t full_count = DENSE ? 1 : 32 * (MODE == MODE_SPARSE_DECODE ? W::CONVERT : W::GATHER);
         for (int i = 0; i < NRING; ++i) { mbar_init(smem_addr(&sm.kv_full[i]), full_count); mbar_init(smem_addr(&sm.kv_empty[i]), 1); }
-        for (int i = 0; i < NRING; ++i) mbar_init(smem_addr(&sm.raw_full[i]), 128);
+        for (int i = 0; i < NRING; ++i) mbar_init(smem_addr(&sm.raw_full[i]), DENSE ? 1 : 32 * W::GATHER);
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_addr(&sm.s_full[i]), 1);
             mbar_init(smem_addr(&sm.s_empty[i]), 256);
@@ -472,18 +479,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t tmem = sm.tmem_base;
-    // gather modes: the gather warps need the issue slots that waiting warps would otherwise spin on
-    // (FP8 decode, where a tile takes several microseconds, also sleeps between probes)
-    using WaiterT = Waiter<DENSE>;
-    const uint32_t peer_flag = map_to_cta(smem_addr(&sm.aborted), cta_rank ^ 1u);
-#ifndef MLA_DENSE_PARK_WARPS
-#define MLA_DENSE_PARK_WARPS 99          // dense mode: warps from this index on park between barrier probes
-#endif
-#ifndef MLA_DENSE_PARK_SLEEP
-#define MLA_DENSE_PARK_SLEEP 0u
-#endif
-    WaiterT wt(p.status, &sm.aborted, peer_flag, p.wait_limit, DENSE ? warp >= MLA_DENSE_PARK_WARPS : warp < 12,
-               MODE == MODE_SPARSE_DECODE ? MLA_SLEEP_NS : (DENSE ? MLA_DENSE_PARK_SLEEP : 0u));
+    Waiter wt(p.wait_limit);
     const int oob_page = p.num_blocks;                     // a page coordinate outside the cache: TMA fills zeros
     // what the wind-down has to wait for after an expired wait (thread 0: ring fills and Q boxes it armed)
     uint32_t fills_armed = 0, q_armed = 0;
@@ -509,10 +505,10 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     };
 
     // =====================================================================================================
-    // In the sparse modes the CTA has 512 threads that start with 128 registers each; every warpgroup re-sizes its
-    // share as the first thing in its own branch (the compiler budgets registers per branch from this).
+    // (the compiler budgets registers per branch from the share each takes first)
     if (warp < 4) {
-    if (!DENSE) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    if (MODE == MODE_PREFILL) regs_dec<64>();
+    if (MODE == MODE_SPARSE_DECODE) regs_dec<48>();
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ---------------------------------------------------------
         if (!DENSE) {
@@ -726,14 +722,15 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
             }
         }
     }
-    } else if (!DENSE && warp >= 12) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    } else if (!DENSE && warp >= W::FIRST_GATHER && warp < W::FIRST_CONVERT) {
+        if (MODE == MODE_PREFILL) regs_dec<64>();          // (FP8 decode: keeps the 80 it started with)
         // ---------------- gather warpgroup (sparse modes): fills the K ring (score CTA) / V ring (value CTA) by index ----
         // Every warp owns a block of tokens; one cp.async instruction of the warp copies consecutive 16-byte pieces of
         // ONE token row (coalesced 128-byte lines, no registers held, as many copies in flight as the ring has room
         // for) into the 128-byte-swizzled operand layout; invalid tokens get zeros (zero-size source).  The ring
         // barrier counts one arrival per thread, made by the copy engine when that thread's copies have landed.
-        const int gw = warp - 12;                                 // warp inside the gather warpgroup
+        const int gw = warp - W::FIRST_GATHER;
+        constexpr int TPW = 128 / (W::GATHER ? W::GATHER : 1), VPW = TPW / 2;      // tokens per warp: of a tile (score CTA) / of a page (value CTA)
         uint32_t ks = 0, g = 0, nreq_p = 0;
         uint32_t* kmask = reinterpret_cast<uint32_t*>(sm.data + L::SC_MASK);
         if (MODE == MODE_SPARSE_DECODE) {
@@ -892,26 +889,28 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
             const int* idx = p.indices + (int64_t)w.req * p.idx_ss;
             // the index of a tile's token is loaded one tile ahead (a load that is used at once costs its latency)
             int id_next = -1;
-            if (cta_rank == 0) { const int pos0 = gw * 32 + lane; id_next = pos0 < w.seqlen ? __ldg(idx + pos0) : -1; }
+            const int tok = gw * TPW + lane % TPW, vtok = gw * VPW + lane % VPW;      // token this lane looks up
+            if (cta_rank == 0) id_next = tok < w.seqlen ? __ldg(idx + tok) : -1;
             int vid_next = -1;                       // value CTA: index of this lane's token of the next page
-            if (cta_rank == 1) { const int pos0 = gw * 16 + (lane & 15); vid_next = pos0 < w.seqlen ? __ldg(idx + pos0) : -1; }
+            if (cta_rank == 1) vid_next = vtok < w.seqlen ? __ldg(idx + vtok) : -1;
             for (int i = 0; i < w.ntiles; ++i, ++g) {
                 if (cta_rank == 0) {
-                    // warp gw owns tokens 32*gw .. 32*gw+31 of the tile; lane l looks up token 32*gw + l
+                    // warp gw owns tokens TPW*gw .. TPW*gw + TPW-1 of the tile
                     const int id = id_next;
                     const bool ok = id >= 0 && id < p.s_kv;
                     const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-                    if (lane == 0) { kmask[(g & 3) * 4 + gw] = bal; __threadfence_block(); }   // token 32w + l of the tile is bit l of word w
+                    // token 32w + l of the tile is bit l of word w; a warp of 16 tokens writes half a word
+                    if (lane == 0) { reinterpret_cast<uint16_t*>(kmask)[(g & 3) * 8 + gw] = (uint16_t)bal; __threadfence_block(); }
                     // (issued after the fence, which would otherwise wait for it)
-                    { const int posn = (i + 1) * 128 + gw * 32 + lane; id_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
+                    { const int posn = (i + 1) * 128 + tok; id_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
                     const int row_id = ok ? id : -1;
                     // A copy instruction costs the warp the same whatever its active lanes, so a token row (72 pieces of
                     // 16 bytes) is copied by two full-warp instructions (chunks 0-3, chunks 4-7) and the RoPE chunk of
-                    // four rows by a third: 72 instructions per 32 rows.  The ring barriers still count per group of 3
+                    // four rows by a third: 36 instructions per 16 rows.  The ring barriers still count per group of 3
                     // chunks: every group's arrival is issued once all copies that touch it have been issued.
                     // the tile's three groups are fills ks, ks + 1, ks + 2 of the ring; chunk c of the tile lives in the slot of
                     // group c / 3, at chunk position c % 3
-                    const uint32_t ring0 = smem_addr(sm.data + L::SC_KRING) + gw * 32 * 128;
+                    const uint32_t ring0 = smem_addr(sm.data + L::SC_KRING) + gw * TPW * 128;
                     // (three slots: group j sits in slot j and every address below is a compile-time offset)
                     const uint32_t slot0 = L::WIDE ? ks % NKS : 0u, slot1 = L::WIDE ? (ks + 1) % NKS : 1u, slot2 = L::WIDE ? (ks + 2) % NKS : 2u;
                     const int c = lane & 7;
@@ -922,7 +921,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                         const int ch = lane >> 3;                     // chunks 0-3: 0, 1, 2 in group 0, chunk 3 in group 1
                         const uint32_t dst0 = ring0 + (ch < 3 ? slot0 * K_GROUP_BYTES + ch * K_CHUNK_BYTES : slot1 * K_GROUP_BYTES);
 #pragma unroll 8
-                        for (int rr = 0; rr < 32; ++rr) {
+                        for (int rr = 0; rr < TPW; ++rr) {
                             const int rid = __shfl_sync(0xffffffffu, row_id, rr);
                             const __nv_bfloat16* src = p.kv + (int64_t)(rid < 0 ? 0 : rid) * p.kv_ss + lane * 8;
                             cp_async16_zfill(dst0 + rr * 128 + ((c ^ (rr & 7)) << 4), src, rid < 0 ? 0u : 16u);
@@ -935,7 +934,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                         const uint32_t dst0 = ring0 + (ch < 6 ? slot1 * K_GROUP_BYTES + (ch - 3) * K_CHUNK_BYTES
                                                               : slot2 * K_GROUP_BYTES + (ch - 6) * K_CHUNK_BYTES);
 #pragma unroll 8
-                        for (int rr = 0; rr < 32; ++rr) {
+                        for (int rr = 0; rr < TPW; ++rr) {
                             const int rid = __shfl_sync(0xffffffffu, row_id, rr);
                             const __nv_bfloat16* src = p.kv + (int64_t)(rid < 0 ? 0 : rid) * p.kv_ss + (32 + lane) * 8;
                             cp_async16_zfill(dst0 + rr * 128 + ((c ^ (rr & 7)) << 4), src, rid < 0 ? 0u : 16u);
@@ -945,7 +944,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     {
                         const uint32_t dst0 = ring0 + slot2 * K_GROUP_BYTES + 2 * K_CHUNK_BYTES;      // chunk 8
 #pragma unroll
-                        for (int q4 = 0; q4 < 8; ++q4) {
+                        for (int q4 = 0; q4 < TPW / 4; ++q4) {
                             const int rr = 4 * q4 + (lane >> 3);
                             const int rid = __shfl_sync(0xffffffffu, row_id, rr);
                             // (rows of 512 columns have no ninth chunk: zeros, as for an invalid token)
@@ -956,18 +955,18 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     cp_async_arrive_noinc(smem_addr(&sm.kv_full[slot2]));
                     ks += 3;
                 } else {
-                    // warp gw owns tokens 16*gw .. 16*gw+15 of each page; one instruction copies 512 bytes of one row
+                    // warp gw owns tokens VPW*gw .. VPW*gw + VPW-1 of each page; one instruction copies 512 bytes of one row
                     for (int h = 0; h < 2; ++h) {
                         const int id = vid_next;
-                        { const int posn = i * 128 + (h + 1) * 64 + gw * 16 + (lane & 15); vid_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
+                        { const int posn = i * 128 + (h + 1) * 64 + vtok; vid_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
                         const int row_id = (id >= 0 && id < p.s_kv) ? id : -1;
                         for (int nh = 0; nh < 2; ++nh, ++ks) {
                             const uint32_t slot = ks % NVS;
                             WAIT_WARP_OR_LEAVE(wt, false, &sm.kv_empty[slot], ((ks / NVS) & 1) ^ 1, 202);
                             const int box = lane >> 3, c = lane & 7;
-                            const uint32_t dst0 = smem_addr(sm.data + VA_VRING + slot * V_SLOT_BYTES) + box * BOX_BYTES + gw * 16 * 128;
+                            const uint32_t dst0 = smem_addr(sm.data + VA_VRING + slot * V_SLOT_BYTES) + box * BOX_BYTES + gw * VPW * 128;
 #pragma unroll 8
-                            for (int rr = 0; rr < 16; ++rr) {
+                            for (int rr = 0; rr < VPW; ++rr) {
                                 const int rid = __shfl_sync(0xffffffffu, row_id, rr);
                                 const __nv_bfloat16* src = p.kv + (int64_t)(rid < 0 ? 0 : rid) * p.kv_ss + (nh * 32 + lane) * 8;
                                 cp_async16_zfill(dst0 + rr * 128 + ((c ^ (rr & 7)) << 4), src, rid < 0 ? 0u : 16u);
@@ -978,8 +977,120 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 }
             }
         }
+    } else if (MODE == MODE_SPARSE_DECODE && warp >= W::FIRST_CONVERT) {
+        regs_dec<64>();
+        // ---------------- FP8 decode: these 256 threads de-quantise the raw records in place ---------------------------
+        const int ct = threadIdx.x - W::FIRST_CONVERT * 32;
+        uint32_t g = 0, ks = 0;
+        if (cta_rank == 0) {
+            // K groups: two threads per token row, every other 16-value piece each
+            const int r = ct & 127, half = ct >> 7, sw = r & 7;
+            for (WalkerT wk(p, part); wk.valid(); wk.next()) {
+                const Work w = wk.get();
+                for (int i = 0; i < w.ntiles; ++i, ++g) {
+                    float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+                    for (int grp = 0; grp < 3; ++grp) {
+                        WAIT_WARP_OR_LEAVE(wt, false, &sm.raw_full[grp], g & 1, 205);
+                        // the tile's scales were stored (and fenced) by the gather warps before they issued its first copies
+                        if (grp == 0) sc = reinterpret_cast<const float4*>(sm.data + L::SC_SCALES)[(g & 1) * ROWS + r];
+                        // group 2: chunks 6, 7 and the RoPE chunk (copied as it is); 512-wide form: chunk 6, the RoPE chunk and zeros
+                        const int nconv = grp < 2 ? 3 : (M1 ? 1 : 2);
+#pragma unroll 1
+                        for (int cj = 0; cj < nconv; ++cj) {
+                            const int j = grp * 3 + cj, sg = j >> 1;
+                            uint8_t* rowp = sm.data + L::SC_KRING + j * K_CHUNK_BYTES + r * 128;
+                            // one fp32 scale per two chunks, or one e8m0 exponent byte per chunk (byte j of the first two words)
+                            const float scale = M1 ? e8m0_to_float((__float_as_uint(j < 4 ? sc.x : sc.y) >> (8 * (j & 3))) & 0xffu)
+                                                   : (sg == 0 ? sc.x : sg == 1 ? sc.y : sg == 2 ? sc.z : sc.w);
+                            uint4 raw[2];
+#pragma unroll
+                            for (int k2 = 0; k2 < 2; ++k2) raw[k2] = *reinterpret_cast<const uint4*>(rowp + (((2 * (half + 2 * k2) + 1) ^ sw) << 4));
+#pragma unroll
+                            for (int k2 = 0; k2 < 2; ++k2) {
+                                const int k = half + 2 * k2;
+                                uint4 lo, hi;
+                                dequant16(raw[k2], scale, lo, hi);
+                                *reinterpret_cast<uint4*>(rowp + (((2 * k) ^ sw) << 4)) = lo;
+                                *reinterpret_cast<uint4*>(rowp + (((2 * k + 1) ^ sw) << 4)) = hi;
+                            }
+                        }
+                        if (M1 && grp == 2) {
+                            // the ninth chunk of a 512-wide row does not exist: zeros (this thread's half of the token's row)
+                            uint8_t* row8 = sm.data + L::SC_KRING + 8 * K_CHUNK_BYTES + r * 128;
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(row8 + (((half * 4 + k) ^ sw) << 4)) = make_uint4(0, 0, 0, 0);
+                        }
+                        fence_proxy_async_smem();          // generic-proxy stores -> visible to the tensor core's reads
+                        mbar_arrive(smem_addr(&sm.kv_full[grp]));
+                    }
+                }
+            }
+        } else {
+            // V slots: thread = (token row of the page, chunk of the slot).  It looks up its token's record by itself, one
+            // page ahead, for the scales it needs; the raw pieces were copied by the gather warpgroup.
+            const int trow = ct & 63, box = ct >> 6, sw = trow & 7;
+            const int tq = blockIdx.y;
+            for (WalkerT wk(p, part); wk.valid(); wk.next()) {
+                const Work w = wk.get();
+                const int* idx0 = p.sidx[0] + (int64_t)w.req * p.sidx_sb[0] + (int64_t)tq * p.sidx_ss[0];
+                const int* idx1 = p.stopk[1] ? p.sidx[1] + (int64_t)w.req * p.sidx_sb[1] + (int64_t)tq * p.sidx_ss[1] : nullptr;
+                auto load_id = [&](int blk) -> int {
+                    if (blk >= w.blk_end) return -1;
+                    const int scope = blk >= w.nblk0 ? 1 : 0;
+                    const int pos = (scope ? blk - w.nblk0 : blk) * PAGE + trow;
+                    if (pos >= (scope ? w.len1 : w.len0)) return -1;
+                    return __ldg((scope ? idx1 : idx0) + pos);
+                };
+                // the scales of this thread's chunk in the two halves of the page: x of dims 0..255, y of dims 256..511 (512-wide
+                // form: the record's eight exponent bytes)
+                auto scales_of_id = [&](int blk, int id) -> float2 {
+                    const int scope = blk >= w.nblk0 ? 1 : 0;
+                    const int pbs = p.pbs[scope];
+                    if (id < 0 || (int64_t)id >= (int64_t)p.nblocks[scope] * pbs) return make_float2(0.f, 0.f);
+                    const uint8_t* block = p.kvb[scope] + (int64_t)(id / pbs) * p.kvb_sblock[scope];
+                    if (M1) return __ldg(reinterpret_cast<const float2*>(block + (int64_t)pbs * 576 + (int64_t)(id % pbs) * 8));
+                    const float* sc = reinterpret_cast<const float*>(block + (int64_t)(id % pbs) * 656 + 512);
+                    return make_float2(__ldg(sc + (box >> 1)), __ldg(sc + 2 + (box >> 1)));
+                };
+                float2 sc_next = scales_of_id(w.blk_begin, load_id(w.blk_begin));
+                int id_next = load_id(w.blk_begin + 1);
+                for (int i = 0; i < w.ntiles; ++i) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 sc = sc_next;
+                        const int nblk = w.blk_begin + 2 * i + h + 1;
+                        sc_next = scales_of_id(nblk, id_next);
+                        id_next = load_id(nblk + 1);
+#pragma unroll 1
+                        for (int nh = 0; nh < 2; ++nh, ++ks) {
+                            const uint32_t slot = ks % NVS;
+                            WAIT_WARP_OR_LEAVE(wt, false, &sm.raw_full[slot], (ks / NVS) & 1, 206);
+                            // (512-wide form: one exponent byte per chunk; chunk 7 is the RoPE part, copied as it is)
+                            if (!(M1 && nh == 1 && box == 3)) {
+                                const float scale = M1 ? e8m0_to_float((__float_as_uint(nh ? sc.y : sc.x) >> (8 * box)) & 0xffu) : (nh ? sc.y : sc.x);
+                                uint8_t* rowp = sm.data + VA_VRING + slot * V_SLOT_BYTES + box * BOX_BYTES + trow * 128;
+                                uint4 raw[4];
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) raw[k] = *reinterpret_cast<const uint4*>(rowp + (((2 * k + 1) ^ sw) << 4));
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    uint4 lo, hi;
+                                    dequant16(raw[k], scale, lo, hi);
+                                    *reinterpret_cast<uint4*>(rowp + (((2 * k) ^ sw) << 4)) = lo;
+                                    *reinterpret_cast<uint4*>(rowp + (((2 * k + 1) ^ sw) << 4)) = hi;
+                                }
+                            }
+                            fence_proxy_async_smem();              // generic-proxy stores -> visible to the tensor core's reads
+                            mbar_arrive(smem_addr(&sm.kv_full[slot]));
+                        }
+                    }
+                }
+            }
+        }
     } else {
-        if (!DENSE) asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+        if (MODE == MODE_PREFILL) regs_inc<144>();
+        if (MODE == MODE_SPARSE_DECODE) regs_inc<112>();
         const int wq = warp & 3;                                  // TMEM lane quarter of this warp
         const int half = (warp - 4) >> 2;                         // score CTA: page of the tile this warpgroup owns
         const int r = wq * 32 + lane;                             // row inside the block = TMEM lane
@@ -1002,50 +1113,6 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
             float* xmax = reinterpret_cast<float*>(sm.data + L::SC_XMAX);
             const uint32_t remote_fin = map_to_cta(smem_addr(sm.data + VA_FIN), 1) + (uint32_t)r * 4u;
             const uint32_t remote_fin_full = map_to_cta(smem_addr(&sm.fin_full), 1);
-            // FP8 decode: these 256 threads also de-quantise the K tiles in place (two threads per token row, every other
-            // 16-value piece each), one tile ahead of the softmax they compute: tile g + 1 is converted before the scores
-            // of tile g are awaited, so the MMA warp has the next tile while this warpgroup is busy with the softmax.
-            uint32_t conv_tile = 0;
-            WaiterT wt_fast(p.status, &sm.aborted, peer_flag, p.wait_limit);     // conversion sits on the MMA warp's critical path: no sleeping
-            auto convert_tile = [&](const uint32_t tile) {
-                const int sw = r & 7;
-                float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-                for (int grp = 0; grp < 3; ++grp) {
-                    if (!wt_fast.template wait<false>(&sm.raw_full[grp], tile & 1, 205)) { wt.aborted = true; return; }
-                    // the tile's scales were stored (and fenced) by the gather warps before they issued its first copies
-                    if (grp == 0) sc = reinterpret_cast<const float4*>(sm.data + L::SC_SCALES)[(tile & 1) * ROWS + r];
-                    // group 2: chunks 6, 7 and the RoPE chunk (copied as it is); 512-wide form: chunk 6, the RoPE chunk and zeros
-                    const int nconv = grp < 2 ? 3 : (M1 ? 1 : 2);
-#pragma unroll 1
-                    for (int cj = 0; cj < nconv; ++cj) {
-                        const int j = grp * 3 + cj, sg = j >> 1;
-                        uint8_t* rowp = sm.data + L::SC_KRING + j * K_CHUNK_BYTES + r * 128;
-                        // one fp32 scale per two chunks, or one e8m0 exponent byte per chunk (byte j of the first two words)
-                        const float scale = M1 ? e8m0_to_float((__float_as_uint(j < 4 ? sc.x : sc.y) >> (8 * (j & 3))) & 0xffu)
-                                               : (sg == 0 ? sc.x : sg == 1 ? sc.y : sg == 2 ? sc.z : sc.w);
-                        uint4 raw[2];
-#pragma unroll
-                        for (int k2 = 0; k2 < 2; ++k2) raw[k2] = *reinterpret_cast<const uint4*>(rowp + (((2 * (half + 2 * k2) + 1) ^ sw) << 4));
-#pragma unroll
-                        for (int k2 = 0; k2 < 2; ++k2) {
-                            const int k = half + 2 * k2;
-                            uint4 lo, hi;
-                            dequant16(raw[k2], scale, lo, hi);
-                            *reinterpret_cast<uint4*>(rowp + (((2 * k) ^ sw) << 4)) = lo;
-                            *reinterpret_cast<uint4*>(rowp + (((2 * k + 1) ^ sw) << 4)) = hi;
-                        }
-                    }
-                    if (M1 && grp == 2) {
-                        // the ninth chunk of a 512-wide row does not exist: zeros (this thread's half of the token's row)
-                        uint8_t* row8 = sm.data + L::SC_KRING + 8 * K_CHUNK_BYTES + r * 128;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(row8 + (((half * 4 + k) ^ sw) << 4)) = make_uint4(0, 0, 0, 0);
-                    }
-                    fence_proxy_async_smem();          // generic-proxy stores -> visible to the tensor core's reads
-                    mbar_arrive(smem_addr(&sm.kv_full[grp]));
-                }
-            };
             for (WalkerT wk(p, part); wk.valid(); wk.next(), ++nreq) {
                 const Work w = wk.get();
                 // ---- Q row -> A operand: chunks [0, Q_TMEM_CHUNKS) to tensor memory (2 x 16 bit per 32-bit column), in the
@@ -1073,14 +1140,14 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                             tmem_st32(tlane + L::TM_Q + c * 32, v);
                         }
                         tmem_wait_st();
-                        if (!wt.aborted) mbar_arrive(smem_addr(&sm.ring_released));        // the producers may fill the ring with K now
+                        if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.ring_released));        // the producers may fill the ring with K now
                     } else {
                         load_q_by_threads<MODE>(sm, qrow, row_ok, half, r, tlane, NO_CHUNK8);
                     }
                     tmem_wait_st();
                     fence_proxy_async_smem();
                     tc_fence_before();
-                    if (!wt.aborted) mbar_arrive(smem_addr(&sm.q_ready));
+                    if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.q_ready));
                 }
                 // first key position this row must NOT see (causal limit, and the end of this partition's range)
                 const int limit = min(p.causal ? w.seqlen - (p.s_q - 1 - t) : w.seqlen, w.blk_end * PAGE);
@@ -1088,10 +1155,6 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 for (int i = 0; i < w.ntiles; ++i, ++g) {
                     const uint32_t sb = L::S_BUFS == 2 ? (g & 1) : 0;
                     const uint32_t ph = L::S_BUFS == 2 ? ((g >> 1) & 1) : (g & 1);
-                    if (MODE == MODE_SPARSE_DECODE)
-                        // one tile ahead, but never into the next request: its first tile can only be gathered after
-                        // these threads have moved that request's Q out of the K ring
-                        while (!wt.aborted && conv_tile <= g + 1 && conv_tile < g + (uint32_t)(w.ntiles - i)) convert_tile(conv_tile++);
                     wt.template wait<false>(&sm.s_full[sb], ph, 5);
                     tc_fence_after();
                     uint32_t s[64];
@@ -1103,7 +1166,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     }
                     tmem_wait_ld();
                     tc_fence_before();
-                    if (!wt.aborted) mbar_arrive(smem_addr(&sm.s_empty[sb]));          // the MMA warp may overwrite this S accumulator
+                    if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.s_empty[sb]));          // the MMA warp may overwrite this S accumulator
 
                     if (!DENSE) {
                         // validity bits of the gathered tokens: token 32w + l of the tile is bit l of word w
@@ -1131,7 +1194,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     float mx = fmaxf(mx0, mx1);
                     // the row maximum over both pages of the tile; the barrier also carries the abort flag
                     xmax[((g & 1) * 2 + half) * ROWS + r] = mx;
-                    BAR_OR_LEAVE(wt.aborted);
+                    BAR_OR_LEAVE((wt.code != 0));
                     mx = fmaxf(mx, xmax[((g & 1) * 2 + (half ^ 1)) * ROWS + r]);
                     mx *= p.scale_log2;                                // scale > 0: max commutes with scaling
                     m_true = fmaxf(m_true, mx);
@@ -1160,7 +1223,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
 
                     // staging of this warp is free once the previous tile's copy has landed in the value CTA
                     wt.template wait<true>(&sm.stage_free[half], (g & 1) ^ 1, 8);
-                    if (!wt.aborted) {
+                    if (!(wt.code != 0)) {
                         uint8_t* prow = stage + (lane >> 3) * 1024 + (lane & 7) * 128;
 #pragma unroll
                         for (int ch = 0; ch < 8; ++ch)
@@ -1179,13 +1242,13 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 {
                     float* lsum = L::WIDE ? xmax + ((g & 1) * 2) * ROWS : reinterpret_cast<float*>(sm.data + L::SC_LSUM);
                     if (half == 1) lsum[r] = l_run;
-                    BAR_OR_LEAVE(wt.aborted);
+                    BAR_OR_LEAVE((wt.code != 0));
                     if (half == 0) l_run += lsum[r];
-                    BAR_OR_LEAVE(wt.aborted);
+                    BAR_OR_LEAVE((wt.code != 0));
                 }
                 if (half == 0) {
                     wt.template wait<true>(&sm.fin_empty, (nreq & 1) ^ 1, 7);
-                    if (!wt.aborted) {
+                    if (!(wt.code != 0)) {
                         st_cluster_f32(remote_fin, l_run);
                         st_cluster_f32(remote_fin + ROWS * 4, m_run);
                         st_cluster_f32(remote_fin + 2 * ROWS * 4, m_true);
@@ -1336,81 +1399,11 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 tc_fence_before();
                 mbar_arrive_remote(remote_fin_empty);        // the final statistics may be rewritten
             }
-        } else if (MODE == MODE_SPARSE_DECODE) {
-            // ---------------- value CTA, FP8 decode: warps 8-11 de-quantise the V slots in place ------------------
-            // Thread = (token row of the page, half of the slot's four chunks).  It looks up its token's record by
-            // itself, one page ahead, for the two scales it needs; the raw pieces were copied by the gather warpgroup.
-            const int trow = r & 63, hb = r >> 6, sw = trow & 7;
-            const int tq = blockIdx.y;
-            uint32_t ks = 0;
-            WaiterT wt_fast(p.status, &sm.aborted, peer_flag, p.wait_limit);   // this sits on the MMA warp's critical path: no sleeping
-            for (WalkerT wk(p, part); wk.valid(); wk.next()) {
-                const Work w = wk.get();
-                const int* idx0 = p.sidx[0] + (int64_t)w.req * p.sidx_sb[0] + (int64_t)tq * p.sidx_ss[0];
-                const int* idx1 = p.stopk[1] ? p.sidx[1] + (int64_t)w.req * p.sidx_sb[1] + (int64_t)tq * p.sidx_ss[1] : nullptr;
-                auto load_id = [&](int blk) -> int {
-                    if (blk >= w.blk_end) return -1;
-                    const int scope = blk >= w.nblk0 ? 1 : 0;
-                    const int pos = (scope ? blk - w.nblk0 : blk) * PAGE + trow;
-                    if (pos >= (scope ? w.len1 : w.len0)) return -1;
-                    return __ldg((scope ? idx1 : idx0) + pos);
-                };
-                auto scales_of_id = [&](int blk, int id) -> float4 {
-                    const int scope = blk >= w.nblk0 ? 1 : 0;
-                    const int pbs = p.pbs[scope];
-                    if (id < 0 || (int64_t)id >= (int64_t)p.nblocks[scope] * pbs) return make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (M1) {
-                        const uint2 e = __ldg(reinterpret_cast<const uint2*>(p.kvb[scope] + (int64_t)(id / pbs) * p.kvb_sblock[scope] +
-                                                                             (int64_t)pbs * 576 + (int64_t)(id % pbs) * 8));
-                        return make_float4(__uint_as_float(e.x), __uint_as_float(e.y), 0.f, 0.f);
-                    }
-                    return __ldg(reinterpret_cast<const float4*>(p.kvb[scope] + (int64_t)(id / pbs) * p.kvb_sblock[scope] +
-                                                                 (int64_t)(id % pbs) * 656 + 512));
-                };
-                float4 sc_next = scales_of_id(w.blk_begin, load_id(w.blk_begin));
-                int id_next = load_id(w.blk_begin + 1);
-                for (int i = 0; i < w.ntiles; ++i) {
-#pragma unroll 1
-                    for (int h = 0; h < 2; ++h) {
-                        const float4 sc = sc_next;
-                        const int nblk = w.blk_begin + 2 * i + h + 1;
-                        sc_next = scales_of_id(nblk, id_next);
-                        id_next = load_id(nblk + 1);
-#pragma unroll 1
-                        for (int nh = 0; nh < 2; ++nh, ++ks) {
-                            const uint32_t slot = ks % NVS;
-                            WAIT_WARP_OR_LEAVE(wt_fast, false, &sm.raw_full[slot], (ks / NVS) & 1, 206);
-                            float scale = hb ? (nh ? sc.w : sc.y) : (nh ? sc.z : sc.x);
-                            // (512-wide form: one exponent byte per chunk; chunk 7 is the RoPE part, copied as it is)
-                            const int nconv = (M1 && nh == 1 && hb == 1) ? 1 : 2;
-#pragma unroll 1
-                            for (int cj = 0; cj < nconv; ++cj) {
-                                if (M1) {
-                                    const int c = nh * 4 + hb * 2 + cj;
-                                    scale = e8m0_to_float((__float_as_uint(c < 4 ? sc.x : sc.y) >> (8 * (c & 3))) & 0xffu);
-                                }
-                                uint8_t* rowp = sm.data + VA_VRING + slot * V_SLOT_BYTES + (hb * 2 + cj) * BOX_BYTES + trow * 128;
-                                uint4 raw[4];
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) raw[k] = *reinterpret_cast<const uint4*>(rowp + (((2 * k + 1) ^ sw) << 4));
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    uint4 lo, hi;
-                                    dequant16(raw[k], scale, lo, hi);
-                                    *reinterpret_cast<uint4*>(rowp + (((2 * k) ^ sw) << 4)) = lo;
-                                    *reinterpret_cast<uint4*>(rowp + (((2 * k + 1) ^ sw) << 4)) = hi;
-                                }
-                            }
-                            fence_proxy_async_smem();              // generic-proxy stores -> visible to the tensor core's reads
-                            mbar_arrive(smem_addr(&sm.kv_full[slot]));
-                        }
-                    }
-                }
-            }
         }
     }
 
 wind_down:
+    if (wt.code) report_expired_wait(p.status, &sm.aborted, map_to_cta(smem_addr(&sm.aborted), cta_rank ^ 1u), wt.code);
     // ---- wind down: both CTAs leave together, tensor memory is released -----------------------------------
     if (!DENSE && warp >= 12) cp_async_wait_all();          // this thread's own row copies have landed
     tc_fence_before();
@@ -1420,17 +1413,17 @@ wind_down:
         // and write tensor memory) and the TMA loads into its rings.
         if (warp == 1 && lane == 0) {
             tc_commit(smem_addr(&sm.drain));
-            mbar_wait_bounded<false, 0>(smem_addr(&sm.drain), 0, DRAIN_LIMIT);
+            mbar_wait_bounded(smem_addr(&sm.drain), 0, DRAIN_LIMIT);
         }
         if (threadIdx.x == 0) {
             if (DENSE) {
                 const uint32_t nslots = cta_rank == 0 ? (uint32_t)NKS : (uint32_t)NVS;
                 for (uint32_t back = 1; back <= nslots && back <= fills_armed; ++back) {
                     const uint32_t f = fills_armed - back;     // one of the last fills this thread armed: its slot has seen no later phase
-                    mbar_wait_bounded<false, 0>(smem_addr(&sm.kv_full[f % nslots]), (f / nslots) & 1, DRAIN_LIMIT);
+                    mbar_wait_bounded(smem_addr(&sm.kv_full[f % nslots]), (f / nslots) & 1, DRAIN_LIMIT);
                 }
             }
-            if (q_armed) mbar_wait_bounded<false, 0>(smem_addr(&sm.q_landed), (q_armed - 1) & 1, DRAIN_LIMIT);
+            if (q_armed) mbar_wait_bounded(smem_addr(&sm.q_landed), (q_armed - 1) & 1, DRAIN_LIMIT);
         }
     }
     cluster_sync();                                            // from here on neither CTA starts anything
@@ -1451,13 +1444,11 @@ __global__ void bounded_wait_selftest_kernel(int* status, long long limit_cycles
     __shared__ uint32_t flag;
     if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); flag = 0; fence_mbar_init(); }
     __syncthreads();
-    Waiter<true> lean(status, &flag, 0u, limit_cycles);
-    Waiter<false> spin(status, &flag, 0u, limit_cycles);
-    bool ok = true;
-    if (threadIdx.x < 32) ok = lean.wait<false>(&bar, 0, code);
-    else ok = spin.wait<false>(&bar, 0, code);
+    Waiter w((uint32_t)limit_cycles);
+    bool ok = threadIdx.x < 32 ? w.wait<false>(&bar, 0, code) : w.wait_warp<false>(&bar, 0, code);
     // a second wait by the same thread returns at once
-    if (threadIdx.x < 32) ok = lean.wait<false>(&bar, 0, code + 1) || ok;
+    if (threadIdx.x < 32) ok = w.wait<false>(&bar, 0, code + 1) || ok;
+    if (w.code) report_expired_wait(status, &flag, 0u, w.code);
     __syncthreads();
     if (threadIdx.x == 0 && flag_out) { flag_out[0] = (int)flag; flag_out[1] = ok ? 1 : 0; }
 }
@@ -1479,11 +1470,11 @@ static EncodeTiledFn get_encode_fn() {
 }
 
 // Barrier-wait limit in SM cycles: the default, or MLA_WAIT_LIMIT_CYCLES from the environment (read once).
-static long long wait_limit_cycles() {
-    static const long long v = [] {
+static uint32_t wait_limit_cycles() {
+    static const uint32_t v = [] {
         const char* e = getenv("MLA_WAIT_LIMIT_CYCLES");
         const long long x = e ? atoll(e) : 0;
-        return x > 0 ? x : WAIT_LIMIT_DEFAULT;
+        return (uint32_t)(x > 0 ? (x < 4000000000LL ? x : 4000000000LL) : WAIT_LIMIT_DEFAULT);
     }();
     return v;
 }
@@ -1677,9 +1668,9 @@ int launch_sparse_prefill_sm100(const mla_sparse_prefill_args_t& a) {
     p.q_tma = encode_q_map(&qmap, a.q, 1, a.s_q, a.h_q, 0, a.q_stride_s, a.q_stride_h, a.h_q < ROWS ? a.h_q : ROWS, 1,
                            &p.q_box_bytes, false, a.d_qk) ? 1 : 0;
     if (d512)
-        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_PREFILL, true>, grid, dim3(NTHREADS_GATHER), sizeof(Smem), (cudaStream_t)a.stream, kmap, kmap, qmap, p));
+        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_PREFILL, true>, grid, dim3(Warps<MODE_PREFILL>::THREADS), sizeof(Smem), (cudaStream_t)a.stream, kmap, kmap, qmap, p));
     else
-        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_PREFILL, false>, grid, dim3(NTHREADS_GATHER), sizeof(Smem), (cudaStream_t)a.stream, kmap, kmap, qmap, p));
+        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_PREFILL, false>, grid, dim3(Warps<MODE_PREFILL>::THREADS), sizeof(Smem), (cudaStream_t)a.stream, kmap, kmap, qmap, p));
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;
 }
@@ -1725,9 +1716,9 @@ int launch_sparse_decode_sm100(const mla_sparse_decode_args_t& a) {
                            a.h_q < ROWS ? a.h_q : ROWS, 1, &p.q_box_bytes, false, a.d_qk) ? 1 : 0;
     dim3 grid(2, a.s_q, a.num_sm_parts);
     if (m1)
-        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_SPARSE_DECODE, true>, grid, dim3(NTHREADS_GATHER), sizeof(Smem), (cudaStream_t)a.stream, unused_map, unused_map, qmap, p));
+        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_SPARSE_DECODE, true>, grid, dim3(Warps<MODE_SPARSE_DECODE>::THREADS), sizeof(Smem), (cudaStream_t)a.stream, unused_map, unused_map, qmap, p));
     else
-        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_SPARSE_DECODE, false>, grid, dim3(NTHREADS_GATHER), sizeof(Smem), (cudaStream_t)a.stream, unused_map, unused_map, qmap, p));
+        MLA_CHECK_CUDA(launch_dependent(attn_sm100_kernel<MODE_SPARSE_DECODE, false>, grid, dim3(Warps<MODE_SPARSE_DECODE>::THREADS), sizeof(Smem), (cudaStream_t)a.stream, unused_map, unused_map, qmap, p));
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;
 }

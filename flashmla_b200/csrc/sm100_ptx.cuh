@@ -61,16 +61,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Non-blocking probe (try_wait may suspend the thread for a while when the phase is still open).
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
 // Same, with acquire semantics at cluster scope (the arrival came from the other CTA of the pair).
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -82,72 +72,18 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
     return ok != 0;
 }
 
-// try_wait with a suspend-time hint (ns): the thread is parked by the hardware until the phase completes or the time is
-// up, instead of spinning on the issue slots that the other warps of its scheduler need.
-template <bool CLUSTER_SCOPE>
-__device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-    uint32_t ok;
-    if (CLUSTER_SCOPE)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity), "r"(hint_ns) : "memory");
-    else
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity), "r"(hint_ns) : "memory");
-    return ok != 0;
-}
-// Bounded wait that sleeps between probes: a warp that spins on try_wait takes issue slots from the other warps of
-// its scheduler (measured: a de-quantisation loop ran 4-6 times slower next to three spinning warps).
-template <bool CLUSTER_SCOPE>
-__device__ __forceinline__ bool mbar_wait_bounded_parked(uint32_t bar, uint32_t parity, long long limit_cycles, uint32_t sleep_ns) {
-    if (CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-#pragma unroll 1
-    while (true) {
-        if (sleep_ns) __nanosleep(sleep_ns);
-        if (mbar_try_wait_hint<CLUSTER_SCOPE>(bar, parity, 1000u)) return true;
-        if (clock64() - t0 > limit_cycles) return false;
-    }
+__device__ __forceinline__ uint32_t clock_lo() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    return t;
 }
 
-// Bounded wait: gives up after `limit_cycles` SM clock cycles and returns false.  PRESPIN probes come first without
-// looking at the clock, fully unrolled.  How a waiting thread spins is worth several percent of the attention kernels
-// either way, and the two families want opposite things (measured): the TMA-fed dense kernel is 3.5 % faster without
-// them (they are a third of its code, copied to every wait site), the gather-fed kernels are 25 % slower without them
-// or with the same probes in a rolled loop.
-// The timed loop of a bounded wait, out of line (build option MLA_OUTLINE_TIMED_WAIT; measured 3 % slower for the dense
-// kernel than the inlined loop: a wait that is not served at once is the common case there, and the call costs more
-// than the copy of the loop).
-template <bool CLUSTER_SCOPE>
-__device__ __noinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, long long limit_cycles) {
-    const long long t0 = clock64();
-#pragma unroll 1
-    while (true) {
-        if (CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
-        if (clock64() - t0 > limit_cycles) return false;
-    }
-}
-template <bool CLUSTER_SCOPE, int PRESPIN = 64>
+// Bounded wait: gives up after `limit_cycles` SM clock cycles and returns false.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, long long limit_cycles) {
-#pragma unroll
-    for (int i = 0; i < PRESPIN; ++i) {
-        if (CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
-    }
-    if (PRESPIN == 0) {
-        if (CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
-#ifdef MLA_OUTLINE_TIMED_WAIT
-        return mbar_wait_timed<CLUSTER_SCOPE>(bar, parity, limit_cycles);
-#endif
-    }
     const long long t0 = clock64();
 #pragma unroll 1
     while (true) {
-        if (CLUSTER_SCOPE ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if (clock64() - t0 > limit_cycles) return false;
     }
 }
