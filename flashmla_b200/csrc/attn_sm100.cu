@@ -85,8 +85,10 @@ enum { MODE_DENSE = 0, MODE_PREFILL = 1, MODE_SPARSE_DECODE = 2 };
 // Warps behind the control warpgroup and the two softmax / correction warpgroups: GATHER warps copy KV rows by index,
 // CONVERT warps de-quantise FP8 records.  A kernel starts with its registers shared out evenly (launch bound) and every
 // warpgroup re-sizes its share as the first thing in its branch; the shares add up to no more than the launch had.
-//   prefill     640 threads x 96 registers: control 64, softmax 144, gather 64.  EIGHT gather warps: an SM's copy rate is
-//               bound by what its warps can issue, 77 GB/s with four warps, 102 with eight (stand-alone probe).
+//   prefill     640 threads x 96 registers: control 96, softmax 136, gather 56.  EIGHT gather warps: an SM's copy rate is
+//               bound by what its warps can issue, 77 GB/s with four warps, 102 with eight (stand-alone probe).  The control
+//               warps' share is what the issuing thread of the MMAs needs: with 64 it spilled the descriptors of its unrolled
+//               loop (4096 tokens: 2590 us with control 64, 2450 with 80, 2410 with 96).
 //   FP8 decode  768 threads x 80 registers: control 48, softmax 112, gather 80, convert 64.  The conversion has warps of its
 //               own: on the softmax warps it was serial with the softmax (5.2 us a tile).
 template <int MODE>
@@ -421,6 +423,12 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     constexpr bool DENSE = MODE == MODE_DENSE;
     constexpr bool FP16 = ALT && MODE == MODE_DENSE;
     constexpr bool M1 = ALT && MODE == MODE_SPARSE_DECODE;
+    // How far the MMA issue loops are unrolled (turns of one loop body).  Unrolled, an MMA's descriptor is a compile-time
+    // offset and issuing is fastest; rolled, the roles of an SM share less code.  FP8 decode has issue time to spare and six
+    // roles per SM (rolled by groups 102 -> 93 us for 64 requests); prefill and dense decode have not (rolled 2760 -> 2940 us
+    // for 4096 tokens, 165 -> 172 us for the serving batch).  The pages of P V stay rolled everywhere (unrolled: prefill
+    // 2590 -> 2765 us, dense decode the same).
+    constexpr int MMA_GROUPS = MODE == MODE_SPARSE_DECODE ? 1 : 3;
     constexpr bool NO_CHUNK8 = ALT && MODE != MODE_DENSE;  // 512-wide rows
     constexpr int REC_BYTES = M1 ? 576 : 656;              // bytes between two tokens' values inside a block
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -507,7 +515,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     // =====================================================================================================
     // (the compiler budgets registers per branch from the share each takes first)
     if (warp < 4) {
-    if (MODE == MODE_PREFILL) regs_dec<64>();
+    // (prefill: keeps the 96 it started with)
     if (MODE == MODE_SPARSE_DECODE) regs_dec<48>();
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ---------------------------------------------------------
@@ -619,7 +627,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                         // every address below is a compile-time offset)
                         if (!L::WIDE) { slot = 0; par = g & 1; }
                         bool ready = mbar_try_wait(kv_full0 + slot * 8, par);
-#pragma unroll
+#pragma unroll MMA_GROUPS
                         for (int grp = 0; grp < 3; ++grp) {
                             const uint32_t cur = L::WIDE ? slot : (uint32_t)grp;
                             if (!ready) WAIT_OR_LEAVE(wt, false, &sm.kv_full[cur], par, 3);
@@ -654,6 +662,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 for (WalkerT wk(p, part); wk.valid(); wk.next(), ++nreq) {
                     const Work w = wk.get();
                     for (int i = 0; i < w.ntiles; ++i, ++g) {
+#pragma unroll 1
                         for (int h = 0; h < 2; ++h) {
                             const uint32_t pb = (g & 1) * 2 + h, pph = (g >> 1) & 1;
                             WAIT_OR_LEAVE(wt, true, &sm.p_full[pb], pph, 104);
@@ -723,7 +732,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
         }
     }
     } else if (!DENSE && warp >= W::FIRST_GATHER && warp < W::FIRST_CONVERT) {
-        if (MODE == MODE_PREFILL) regs_dec<64>();          // (FP8 decode: keeps the 80 it started with)
+        if (MODE == MODE_PREFILL) regs_dec<56>();          // (FP8 decode: keeps the 80 it started with)
         // ---------------- gather warpgroup (sparse modes): fills the K ring (score CTA) / V ring (value CTA) by index ----
         // Every warp owns a block of tokens; one cp.async instruction of the warp copies consecutive 16-byte pieces of
         // ONE token row (coalesced 128-byte lines, no registers held, as many copies in flight as the ring has room
@@ -824,7 +833,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                             const int srcoff = is_rope ? (M1 ? 448 : 528) + (ql - N_RAW2) * 16 : q * 16;
                             const int dslot = is_rope ? ql - N_RAW2 : 2 * (q & 3) + 1;
                             const uint32_t dst0 = kring + (is_rope ? (M1 ? 7 : 8) : (q >> 2)) * K_CHUNK_BYTES + gw * 32 * 128;
-#pragma unroll 8
+#pragma unroll 4
                             for (int u = 0; u < 16; ++u) {
                                 const int rr = 2 * u + (active ? sub : 0);
                                 const uint8_t* r = shfl_ptr(rec, rr);
@@ -858,7 +867,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                                 const int dslot = 2 * (ql & 3) + 1;
                                 // (512-wide form, second half: 12 raw pieces - chunks 4, 5, 6 - and, below, the RoPE part as chunk 7)
                                 const bool piece_ok = !M1 || nh == 0 || ql < 12;
-#pragma unroll
+#pragma unroll 4
                                 for (int u = 0; u < 8; ++u) {
                                     const int rr = 2 * u + sub;
                                     const uint8_t* r = shfl_ptr(rec, rr);
@@ -1089,7 +1098,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
             }
         }
     } else {
-        if (MODE == MODE_PREFILL) regs_inc<144>();
+        if (MODE == MODE_PREFILL) regs_inc<136>();
         if (MODE == MODE_SPARSE_DECODE) regs_inc<112>();
         const int wq = warp & 3;                                  // TMEM lane quarter of this warp
         const int half = (warp - 4) >> 2;                         // score CTA: page of the tile this warpgroup owns
