@@ -750,8 +750,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
             //   copy:    this warpgroup brings every raw piece with cp.async straight into the UPPER of its own two
             //            destination slots (lanes = pieces of two token rows: coalesced, no registers held), RoPE pieces
             //            into their final place, and counts the landing on the element's raw_full barrier;
-            //   convert: warps that are idle most of a tile's time in this mode - the softmax warpgroups of the score
-            //            CTA, warps 8-11 of the value CTA - expand the pieces of their token row in place (a thread reads
+            //   convert: eight warps of its own expand the pieces of their token row in place (a thread reads
             //            a slot only it will overwrite; 16-byte accesses, conflict-free thanks to the swizzle) and hand
             //            the element to the MMA warp.
             // Copying and converting run side by side on different warps; record pointers (and, in the score CTA, the
@@ -840,7 +839,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                                 if (active)
                                     cp_async16_zfill(dst0 + rr * 128 + ((dslot ^ (rr & 7)) << 4), (r ? r : p.kvb[0]) + srcoff, r ? 16u : 0u);
                             }
-                            // the softmax warpgroups expand the pieces in place once they have landed
+                            // the converting warps expand the pieces in place once they have landed
                             cp_async_arrive_noinc(smem_addr(&sm.raw_full[grp]));
                         }
                     }
@@ -884,7 +883,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                                         cp_async16_zfill(dst7 + rr * 128 + ((piece ^ (rr & 7)) << 4), (r ? r : p.kvb[0]) + 448 + piece * 16, r ? 16u : 0u);
                                     }
                                 }
-                                cp_async_arrive_noinc(smem_addr(&sm.raw_full[slot]));      // warps 8-11 expand the pieces
+                                cp_async_arrive_noinc(smem_addr(&sm.raw_full[slot]));      // the converting warps expand the pieces
                             }
                         }
                     }
