@@ -41,7 +41,9 @@ __device__ __forceinline__ void unpack16(const uint4& v0, const uint4& v1, float
 
 // e4m3(x / s) of a lane's 16 values, x / s rounded to fp32 first.  With r = RN(1 / s) and q = RN(x r), q + r (x - q s)
 // is RN(x / s) (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 1990; here checked for every bf16 significand against every fp32 significand of s).  The remainder has to be exact: the
+// Dev. 34, 1990; here checked for every bf16 significand against every fp32 significand of s).  It is computed as
+// q + (-r) (q s - x): for x = -0 the remainder q s - x is -0 + 0 = +0 and the sum -0 + -0 keeps the sign, where
+// x - q s = +0 would give +0 + -0 = +0.  The remainder has to be exact: the
 // group's largest magnitude `amax` keeps clear of overflow and underflow, and values so far below it that the remainder
 // could be subnormal (below 2^-20 amax) have quotients under 2^-11, which are zeros in e4m3 whatever their last bit.
 // Groups outside that range (warp-uniform choice) divide.
@@ -56,7 +58,7 @@ __device__ __forceinline__ uint4 quotient16(const float (&f)[16], float s, float
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float x = f[4 * i + k], q0 = x * r;
-                reinterpret_cast<float*>(d)[k] = fmaf(fmaf(-q0, s, x), r, q0);
+                reinterpret_cast<float*>(d)[k] = fmaf(fmaf(q0, s, -x), -r, q0);
             }
             q[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(d[0], __NV_SATFINITE, __NV_E4M3) |
                    (uint32_t)__nv_cvt_float2_to_fp8x2(d[1], __NV_SATFINITE, __NV_E4M3) << 16;

@@ -64,3 +64,62 @@ def test_written_records_over_the_exponent_range(tokens, pow2):
     x = x.to(torch.bfloat16)
     got = quantize_fp8_kvcache(x.to(DEV), pow2).view(torch.uint8).cpu()
     assert torch.equal(got, quant.quantize_v32(x, pow2_scale=pow2).view(torch.uint8))
+
+
+def _records_by_division(x, width, pow2):
+    """(value bytes [..., 512 or 448], scales [..., groups] fp32) of x [blocks, tokens, 1, width], by plain fp32 division.
+    NaNs do not count towards a group's largest magnitude."""
+    group, values = (128, 512) if width == 576 else (64, 448)
+    f = x.squeeze(2)[..., :values].float().unflatten(-1, (-1, group))
+    s = torch.where(f.isnan(), 0.0, f.abs()).amax(-1, keepdim=True) / 448
+    s = torch.exp2(s.clamp_min(1e-4).log2().ceil()) if pow2 or width == 512 else s.clamp_min(1e-30)
+    return (f / s).to(torch.float8_e4m3fn).view(torch.uint8).flatten(-2), s.squeeze(-1)
+
+
+def _signed_zero_rows(width):
+    """A block of token rows: ordinary groups, all-zero groups, and rows whose groups force the division (warps choose
+    between quotient and division by all groups of their token), all with zeros of both signs."""
+    gen = torch.Generator().manual_seed(width)
+    group = 128 if width == 576 else 64
+    x = torch.randn(3, 9, 1, width, generator=gen)
+    x[:, 1, ..., :group] = 0                       # an all-zero group beside ordinary ones
+    x[:, 2] = 0                                    # nothing but zeros
+    x[:, 3, ..., group:2 * group] *= 2.0 ** -100   # this row divides
+    x[:, 4, ..., :group] *= 2.0 ** 110
+    x[:, 5, ..., :group] *= 2.0 ** -55             # the smallest of the quotient's range
+    x[..., 3::7] = 0.0
+    x[..., 5::11] = -0.0
+    return x.to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("width,pow2", [(576, False), (576, True), (512, True)])
+@pytest.mark.parametrize("special", [None, "nan", "inf"])
+def test_written_records_signed_zeros_and_specials(width, pow2, special):
+    """Byte for byte against the division: zeros keep their sign (0x80 for -0) wherever they stand, NaN stays NaN, and a group
+    with an infinity has NaN in its place and signed zeros elsewhere."""
+    from flashmla_b200.kvcache import quantize_fp8_kvcache, quantize_fp8_kvcache_model1
+    x = _signed_zero_rows(width)
+    if special == "nan":
+        x[:, 6:, ..., 9:200:50] = float("nan")     # in ordinary groups, beside zeros
+        x[:, 2, ..., 4] = float("nan")             # in an all-zero group
+    elif special == "inf":
+        x[:, 6:, ..., 9] = float("inf")
+        x[:, 7, ..., 200] = float("-inf")
+    got = (quantize_fp8_kvcache(x.to(DEV), pow2) if width == 576 else quantize_fp8_kvcache_model1(x.to(DEV))).view(torch.uint8).cpu()
+    want, scale = _records_by_division(x, width, pow2)
+    blocks, tokens = x.shape[:2]
+    if width == 576:
+        rows = got.squeeze(2)
+        assert torch.equal(rows[..., 512:528].contiguous().view(torch.int32), scale.contiguous().view(torch.int32))
+    else:
+        flat = got.reshape(blocks, -1)
+        rows = flat[:, :tokens * 576].view(blocks, tokens, 576)
+        assert torch.equal(flat[:, tokens * 576:].view(blocks, tokens, 8)[..., :7], (scale.view(torch.int32) >> 23).to(torch.uint8))
+    rows = rows[..., :want.shape[-1]]
+    is_nan = (want & 0x7f) == 0x7f
+    assert torch.equal((rows & 0x7f) == 0x7f, is_nan)
+    assert torch.equal(rows[~is_nan], want[~is_nan])
+    assert (want == 0x80).sum() > 500              # the case is not empty
+    if special is None:                            # and the repository's restatement of the reference says the same
+        full = quant.quantize_v32(x, pow2_scale=pow2) if width == 576 else quant.quantize_model1(x)
+        assert torch.equal(got, full.view(torch.uint8).contiguous())
