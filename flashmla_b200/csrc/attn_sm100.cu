@@ -1172,14 +1172,20 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                         tmem_ld32(tlane + L::TM_S + sb * 128 + half * 64, lo);
                         tmem_ld32(tlane + L::TM_S + sb * 128 + half * 64 + 32, hi);
                     }
+                    // Validity bits of the gathered tokens: token 32w + l of the tile is bit l of word w.  They are read before the
+                    // arrival below: through the MMAs of tile g + 2, which wait for it, it is all that keeps the copy warps
+                    // from writing tile g + 4's bits over these.
+                    uint32_t m0 = 0xffffffffu, m1 = 0xffffffffu;
+                    if (!DENSE) {
+                        const uint32_t* km = reinterpret_cast<const uint32_t*>(sm.data + L::SC_MASK) + (g & 3) * 4 + half * 2;
+                        m0 = km[0];
+                        m1 = km[1];
+                    }
                     tmem_wait_ld();
                     tc_fence_before();
                     if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.s_empty[sb]));          // the MMA warp may overwrite this S accumulator
 
                     if (!DENSE) {
-                        // validity bits of the gathered tokens: token 32w + l of the tile is bit l of word w
-                        const uint32_t* km = reinterpret_cast<const uint32_t*>(sm.data + L::SC_MASK) + (g & 3) * 4 + half * 2;
-                        const uint32_t m0 = km[0], m1 = km[1];
                         if ((m0 & m1) != 0xffffffffu) {
 #pragma unroll
                             for (int c = 0; c < 64; ++c)
