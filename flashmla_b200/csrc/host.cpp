@@ -11,7 +11,10 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ops/empty.h>
-#include <ATen/ops/zeros.h>
+#include <ATen/ops/from_blob.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -111,11 +114,32 @@ void launch(PyObject* timer, const char* name, F&& f) {
 // ---- per-device status words written by kernels whose bounded waits ran out: [first code, count, -, -] --------
 at::Tensor status_words[64];
 
+// Kernels on any stream write these words, so they are zero before the first of them is launched: a fill queued on the
+// first caller's stream would run behind that stream's work, over the report of another stream's kernel, or be captured
+// and run with every replay.  For the same reason the memory is none of a capture's: it is allocated once per device,
+// zeroed on a stream of its own, and lives as long as the process.
+at::Tensor make_status_words(const at::Device& device) {
+    const c10::cuda::CUDAGuard guard(device);
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // another stream may be capturing
+    constexpr size_t bytes = 4 * sizeof(int32_t);
+    void* words = nullptr;
+    if (cudaMalloc(&words, bytes) != cudaSuccess) {                        // all memory is in the caching allocator's hands
+        (void)cudaGetLastError();
+        c10::cuda::CUDACachingAllocator::emptyCache();
+        C10_CUDA_CHECK(cudaMalloc(&words, bytes));
+    }
+    cudaStream_t stream;
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    C10_CUDA_CHECK(cudaMemsetAsync(words, 0, bytes, stream));
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    C10_CUDA_CHECK(cudaStreamDestroy(stream));
+    return at::from_blob(words, {4}, at::TensorOptions().dtype(at::kInt).device(device));
+}
+
 const at::Tensor& status(const at::Device& device) {
     const int i = device.index();
     require(i >= 0 && i < 64, "device index out of range");
-    if (!status_words[i].defined())          // under the GIL
-        status_words[i] = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(device));
+    if (!status_words[i].defined()) status_words[i] = make_status_words(device);          // under the GIL
     return status_words[i];
 }
 
