@@ -341,13 +341,15 @@ PyObject* sparse_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         if (all[i].t && all[i].t->scalar_type() != at::kInt) refuse(std::string(all[i].name) + " must have dtype int32");
     require(!sink || (sink->scalar_type() == at::kFloat && has_shape(*sink, {h_q}) && sink->is_contiguous()),
             "attn_sink must be a contiguous float32 tensor of shape (h_q,)");
-    require(!extra_indices || extra_indices->dim() == 3, "extra_indices must have shape (b, s_q, extra_topk)");
-    require(q.stride(3) == 1 && indices.stride(2) == 1 && (!extra_indices || extra_indices->stride(2) == 1),
+    // (the list is the last dimension; one more in front of it, as prefill's lists have for the kv head, is accepted.  A missing
+    // dimension is not: with several query tokens their rows would be read as one.)
+    require(!extra_indices || extra_indices->dim() >= (s_q > 1 ? 3 : 2), "extra_indices must have shape (b, s_q, extra_topk)");
+    require(q.stride(3) == 1 && indices.stride(2) == 1 && (!extra_indices || extra_indices->stride(-1) == 1),
             "q and indices must have contiguous last dimension");
     require(indices.size(0) == b && indices.size(1) == s_q, "indices must have shape (b, s_q, topk)");
     for (int i : {3, 7})
         if (all[i].t && !(has_shape(*all[i].t, {b}) && all[i].t->is_contiguous())) refuse(std::string(all[i].name) + " must be contiguous with shape (b,)");
-    const int64_t extra_topk = extra_indices ? extra_indices->size(2) : 0;
+    const int64_t extra_topk = extra_indices ? extra_indices->size(-1) : 0;
     require(!extra_indices || (extra_indices->size(0) == b && extra_indices->size(1) == s_q), "extra_indices must have shape (b, s_q, extra_topk)");
 
     const c10::cuda::CUDAGuard guard(device);

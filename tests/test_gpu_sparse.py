@@ -315,3 +315,14 @@ def test_sparse_prefill_many_query_tokens_per_cta_pair():
     assert_out_close("out", out, ref[0])
     assert_lse_close("max_logits", mx, ref[1])
     assert_lse_close("lse", lse, ref[2])
+
+
+def test_sparse_decode_extra_indices_with_a_unit_dimension():
+    """Lists for the extra cache may carry a dimension of one in front of the keys, as prefill's lists do."""
+    from tests import workloads as W
+    d = W.sparse_decode_inputs(3, 2, 64, 512, 128, seed=5, device="cpu", pad_rows=0)
+    e = W.sparse_decode_inputs(3, 2, 64, 300, 64, seed=6, device="cpu", pad_rows=0)
+    args = [d["q"].to(DEV), d["kv_fp8"].to(DEV), d["indices"].to(DEV), 576 ** -0.5, None, None, e["kv_fp8"].to(DEV)]
+    out, lse = _decode(*args, e["indices"].to(DEV))
+    out4, lse4 = _decode(*args, e["indices"].to(DEV).unsqueeze(2))
+    assert torch.equal(out, out4) and torch.equal(lse, lse4)
