@@ -111,13 +111,14 @@ SYMBOLS = {
     "mla_sparse_prefill_fwd": (c_int, [POINTER(SparsePrefillArgs)]),
     "mla_dense_decode_noalloc": (c_int, [POINTER(DenseDecodeArgs)]),
     "mla_quantize_fp8_kvcache": (c_int, [POINTER(QuantizeArgs)]),
+    "mla_quantize_fp8_kvcache_padded": (c_int, [POINTER(QuantizeArgs)]),
     "mla_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int, POINTER(c_size_t)]),
     "mla_selftest_bounded_wait": (c_int, [c_longlong, c_int, c_void_p, c_void_p, c_void_p]),
 }
 
 # the functions csrc/host.cpp calls, in the order of its Api structure
 _HOST_SYMBOLS = ("mla_last_error", "mla_num_sm_parts", "mla_num_sm_parts_uniform", "mla_get_sched_meta", "mla_dense_decode_fwd",
-                 "mla_sparse_decode_fwd", "mla_combine", "mla_sparse_prefill_fwd", "mla_quantize_fp8_kvcache")
+                 "mla_sparse_decode_fwd", "mla_combine", "mla_sparse_prefill_fwd", "mla_quantize_fp8_kvcache_padded")
 
 _lib = None
 _host = None

@@ -218,7 +218,12 @@ int mla_selftest_bounded_wait(long long limit_cycles, int code, int32_t* status,
 
 int mla_quantize_fp8_kvcache(const mla_quantize_args_t* a) {
     MLA_CHECK_ARG(a != nullptr, "mla_quantize_fp8_kvcache: null argument struct");
-    return launch_quantize_fp8(*a);
+    return launch_quantize_fp8(*a, false);
+}
+
+int mla_quantize_fp8_kvcache_padded(const mla_quantize_args_t* a) {
+    MLA_CHECK_ARG(a != nullptr, "mla_quantize_fp8_kvcache_padded: null argument struct");
+    return launch_quantize_fp8(*a, true);
 }
 
 }  // extern "C"

@@ -37,7 +37,7 @@ struct Api {
     decltype(&mla_sparse_decode_fwd) sparse_decode_fwd;
     decltype(&mla_combine) combine;
     decltype(&mla_sparse_prefill_fwd) sparse_prefill_fwd;
-    decltype(&mla_quantize_fp8_kvcache) quantize;
+    decltype(&mla_quantize_fp8_kvcache_padded) quantize;
 } api;
 
 // tile-scheduler arguments (csrc/api/dense_decode.h:104-105, csrc/api/sparse_decode.h:92-99)
@@ -462,7 +462,7 @@ PyObject* sparse_prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 // ---- FP8 cache writer -----------------------------------------------------------------------------------------------------
-// quantize(x [blocks, block_size, d], out, out_stride_block_bytes, pow2_scale, layout)
+// quantize(x [blocks, block_size, d], out, out_stride_block_bytes, pow2_scale, layout): `out` is the writer's own buffer
 PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     HOST_TRY
     require(nargs == 5, "quantize takes 5 arguments");

@@ -12,7 +12,8 @@
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
 // block_size x 8 scale bytes (7 scales + 1 pad).  Lanes 0-27 hold the quantised values (4 lanes per group), lanes 28-31
-// the RoPE part.
+// the RoPE part.  The first warps also zero the `pad_bytes` behind every block, where the caller owns
+// them (one warp a block; with the last token's stores, inside the loop, 66 K tokens took 36.9 us instead of 34.9).
 #include "common.cuh"
 
 #include <cuda_fp8.h>
@@ -121,11 +122,16 @@ quantize_fp8_kernel(const mla_quantize_args_t a) {
 }
 
 __global__ void __launch_bounds__(256)
-quantize_fp8_model1_kernel(const mla_quantize_args_t a) {
+quantize_fp8_model1_kernel(const mla_quantize_args_t a, const int pad_bytes) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
+    if (pad_bytes)
+#pragma unroll 1
+        for (int64_t blk = warp; blk < a.num_blocks; blk += nwarps)
+            for (int i = lane * 8; i < pad_bytes; i += 256)
+                *reinterpret_cast<uint2*>((uint8_t*)a.out + blk * a.out_stride_block_bytes + (int64_t)a.block_size * 584 + i) = make_uint2(0, 0);
     for (int64_t tok0 = warp * TOKENS; tok0 < ntok; tok0 += nwarps * TOKENS) {
         uint4 v0[TOKENS], v1[TOKENS];
         int64_t blk[TOKENS], row[TOKENS];
@@ -162,7 +168,7 @@ quantize_fp8_model1_kernel(const mla_quantize_args_t a) {
     }
 }
 
-int launch_quantize_fp8(const mla_quantize_args_t& a) {
+int launch_quantize_fp8(const mla_quantize_args_t& a, bool zero_padding) {
     MLA_CHECK_ARG(a.x && a.out, "mla_quantize_fp8_kvcache: x and out must not be null");
     MLA_CHECK_ARG(a.num_blocks > 0 && a.block_size > 0, "mla_quantize_fp8_kvcache: num_blocks and block_size must be positive");
     MLA_CHECK_ARG(a.layout == 0 || a.layout == 1, "mla_quantize_fp8_kvcache: layout must be 0 (656-byte records) or 1 (MODEL1)");
@@ -171,9 +177,12 @@ int launch_quantize_fp8(const mla_quantize_args_t& a) {
                   "mla_quantize_fp8_kvcache: x must be 16-byte aligned with strides that are multiples of 8 elements");
     MLA_CHECK_ARG(is_aligned16(a.out) && a.out_stride_block_bytes % 16 == 0 && a.out_stride_block_bytes >= (int64_t)a.block_size * rec,
                   "mla_quantize_fp8_kvcache: out must be 16-byte aligned, block stride a multiple of 16 bytes and >= block_size * %d", rec);
+    // (records and stride are multiples of 8 bytes, so the padding is too)
+    const int64_t pad_bytes = zero_padding && a.layout ? a.out_stride_block_bytes - (int64_t)a.block_size * rec : 0;
+    MLA_CHECK_ARG(pad_bytes <= 0x7fffff00, "mla_quantize_fp8_kvcache_padded: more than 2 GB of padding behind a block");
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
     const int64_t blocks = min((ntok + 8 * TOKENS - 1) / (8 * TOKENS), (int64_t)1 << 24);
-    if (a.layout) quantize_fp8_model1_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
+    if (a.layout) quantize_fp8_model1_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
     else quantize_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;

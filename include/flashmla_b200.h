@@ -273,6 +273,10 @@ typedef struct {
 } mla_quantize_args_t;
 int mla_quantize_fp8_kvcache(const mla_quantize_args_t* args);
 
+/* Same, for a caller that owns the whole output buffer: with layout 1 the bytes behind a block's records, from
+ * block_size * 584 up to the next block, are written as zeros (the function above leaves them alone). */
+int mla_quantize_fp8_kvcache_padded(const mla_quantize_args_t* args);
+
 /* Self-test of the kernels' bounded barrier wait: launches one small CTA that waits, with the same helper the
  * attention kernels use, on a barrier nobody arrives on, with nothing else in flight.  After `limit_cycles` SM
  * cycles (at most 2e9) every one of its 64 threads gives up, the kernel returns normally and status[0] == code,

@@ -196,3 +196,19 @@ def test_model1_rejects_wrong_record_size():
     meta, _ = fm.get_mla_metadata()
     with pytest.raises(RuntimeError, match="584"):
         fm.flash_mla_with_kvcache(q, kv, None, None, 512, meta, None, None, False, True, idx)
+
+
+@pytest.mark.parametrize("block_size", [64, 1, 61, 72])
+def test_model1_block_padding_is_zero(block_size):
+    """The bytes behind a block's records (blocks are padded to a multiple of 576 bytes) are part of what is saved or sent
+    with the storage: zeros, whatever the memory held before."""
+    from flashmla_b200.kvcache import model1_block_bytes, quantize_fp8_kvcache_model1
+    blocks, n = 7, model1_block_bytes(block_size)
+    x = torch.randn(blocks, block_size, 1, 512, generator=torch.Generator().manual_seed(block_size)).to(torch.bfloat16).to("cuda:0")
+    dirty = torch.full((blocks * n,), 0xa5, dtype=torch.uint8, device="cuda:0")
+    del dirty                                      # the allocator hands the same memory out again
+    got = quantize_fp8_kvcache_model1(x)
+    assert got.stride(0) == n
+    whole = got.view(torch.uint8).as_strided((blocks, n), (n, 1))
+    assert not whole[:, block_size * 584:].any()
+    assert torch.equal(got.view(torch.uint8).cpu(), quant.quantize_model1(x.cpu()).view(torch.uint8))
