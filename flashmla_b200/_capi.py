@@ -5,6 +5,7 @@ or unloadable library raises.
 """
 import ctypes
 import os
+import sys
 import threading
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_longlong, c_size_t, c_void_p
 
@@ -117,8 +118,8 @@ SYMBOLS = {
 }
 
 # the functions csrc/host.cpp calls, in the order of its Api structure
-_HOST_SYMBOLS = ("mla_last_error", "mla_num_sm_parts", "mla_num_sm_parts_uniform", "mla_get_sched_meta", "mla_dense_decode_fwd",
-                 "mla_sparse_decode_fwd", "mla_combine", "mla_sparse_prefill_fwd", "mla_quantize_fp8_kvcache_padded")
+_HOST_SYMBOLS = ("mla_abi_version", "mla_last_error", "mla_num_sm_parts", "mla_num_sm_parts_uniform", "mla_get_sched_meta",
+                 "mla_dense_decode_fwd", "mla_sparse_decode_fwd", "mla_combine", "mla_sparse_prefill_fwd", "mla_quantize_fp8_kvcache_padded")
 
 _lib = None
 _host = None
@@ -147,8 +148,17 @@ def lib():
     return _lib
 
 
+def _check_built_for(module):
+    """The host extension uses torch's C++ objects directly: another torch or Python than it was compiled against is refused."""
+    import torch
+    running = "torch %s, Python %d.%d" % (torch.__version__, *sys.version_info[:2])
+    if module.built_for != running:
+        raise RuntimeError(f"flashmla_b200/_host.so was built for {module.built_for}, running is {running}: "
+                           "rebuild it with `python -m flashmla_b200.build`")
+
+
 def host():
-    """The host extension (csrc/host.cpp), bound to the loaded library; raises if it has not been built."""
+    """The host extension (csrc/host.cpp), bound to the loaded library; raises if it has not been built, or for something else."""
     global _host
     if _host is None:
         handle = lib()
@@ -159,6 +169,7 @@ def host():
                     from . import _host as module
                 except ImportError as e:
                     raise RuntimeError(f"flashmla_b200/_host.so cannot be loaded ({e}): build it with `python -m flashmla_b200.build`") from e
+                _check_built_for(module)
                 module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in _HOST_SYMBOLS))
                 _host = module
     return _host

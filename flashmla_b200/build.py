@@ -60,24 +60,39 @@ def _compile_one(src, obj, verbose):
     return log
 
 
-def _build_host(force):
-    src = os.path.join(CSRC, "host.cpp")
-    newest = max(os.path.getmtime(src), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= newest:
-        return
+HOST_LOG = os.path.join(OBJ_DIR, "host.log")          # the command that built the host extension, and what it printed
+
+
+def _host_command(src):
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     inc = os.path.join(root, "include")
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
-           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
-           src, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
-           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DFLASHMLA_TORCH_VERSION="{torch.__version__}"',
+            "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+            "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
+            src, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def _host_is_stale(src):
+    """Sources newer than the extension, or another command (which names the torch and Python it is compiled against)."""
+    newest = max(os.path.getmtime(src), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
+    if not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < newest or not os.path.exists(HOST_LOG):
+        return True
+    with open(HOST_LOG) as f:
+        return f.readline().rstrip("\n") != " ".join(_host_command(src))
+
+
+def _build_host(force):
+    src = os.path.join(CSRC, "host.cpp")
+    if not force and not _host_is_stale(src):
+        return
+    cmd = _host_command(src)
     proc = subprocess.run(cmd, capture_output=True, text=True)
-    with open(os.path.join(OBJ_DIR, "host.log"), "w") as f:
-        f.write(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
+    with open(HOST_LOG, "w") as f:
+        f.write(("" if proc.returncode == 0 else "failed: ") + " ".join(cmd) + "\n" + proc.stdout + proc.stderr)
     if proc.returncode != 0:
         raise RuntimeError(f"compiling {src} failed:\n" + proc.stdout + proc.stderr)
 

@@ -67,7 +67,7 @@ extern "C" {
 
 const char* mla_last_error(void) { return last_error_buffer(); }
 
-int mla_abi_version(void) { return 2; }
+int mla_abi_version(void) { return MLA_ABI_VERSION; }
 
 int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q) {
     const int sms = device_num_sms(device);

@@ -29,6 +29,7 @@ namespace {
 
 // ---- the C ABI, bound by address ---------------------------------------------------------------------------
 struct Api {
+    decltype(&mla_abi_version) abi_version;
     decltype(&mla_last_error) last_error;
     decltype(&mla_num_sm_parts) num_sm_parts;
     decltype(&mla_num_sm_parts_uniform) num_sm_parts_uniform;
@@ -505,12 +506,19 @@ PyObject* known_status(PyObject*, PyObject*) {
     HOST_END
 }
 
-// bind(addresses of the C functions in the order of Api's members)
+// bind(addresses of the C functions in the order of Api's members): refuses a library whose structures are not the ones this
+// file was compiled with
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     HOST_TRY
     require(nargs == (Py_ssize_t)(sizeof(Api) / sizeof(void*)), "bind: one address for every function is needed");
-    for (Py_ssize_t i = 0; i < nargs; ++i) reinterpret_cast<void**>(&api)[i] = PyLong_AsVoidPtr(args[i]);
+    Api given;
+    for (Py_ssize_t i = 0; i < nargs; ++i) reinterpret_cast<void**>(&given)[i] = PyLong_AsVoidPtr(args[i]);
     if (PyErr_Occurred()) throw python_error();
+    const int version = given.abi_version();
+    if (version != MLA_ABI_VERSION)
+        refuse("the host extension was compiled for ABI version " + std::to_string(MLA_ABI_VERSION) + " of the library, which has " +
+               std::to_string(version) + ": rebuild both with `python -m flashmla_b200.build --force`");
+    api = given;
     Py_RETURN_NONE;
     HOST_END
 }
@@ -529,4 +537,12 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module_def); }
+#define TEXT_(x) #x
+#define TEXT(x) TEXT_(x)
+PyMODINIT_FUNC PyInit__host() {
+    PyObject* m = PyModule_Create(&module_def);
+    // what the file was compiled against; _capi.py compares it with what is running
+    if (m && PyModule_AddStringConstant(m, "built_for", "torch " FLASHMLA_TORCH_VERSION ", Python " TEXT(PY_MAJOR_VERSION) "." TEXT(PY_MINOR_VERSION)))
+        Py_CLEAR(m);
+    return m;
+}

@@ -55,7 +55,8 @@ typedef struct {
 /* Message of the last failing call on this thread ("" if none). */
 const char* mla_last_error(void);
 
-/* Library ABI version (bumped when a struct below changes). */
+/* Library ABI version (bumped when a struct below changes): what a caller was compiled with, and what the library is. */
+#define MLA_ABI_VERSION 2
 int mla_abi_version(void);
 
 /* Number of SM partitions the decode kernels of `mode` use on `device` for a

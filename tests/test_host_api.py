@@ -119,3 +119,32 @@ def test_workspace_bytes():
     rows = (3 + 7) * 2 * 5
     assert off.value >= rows * 512 * 4 and off.value % 256 == 0 and total == off.value + rows * 4
     assert lib.mla_workspace_bytes(0, 1, 128, 512, 74, None) == 0 and b"positive" in lib.mla_last_error()
+
+
+def test_host_extension_refuses_a_library_of_another_abi_version():
+    from flashmla_b200 import _capi
+    host, lib = _capi.host(), _capi.lib()
+    addresses = [ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _capi._HOST_SYMBOLS]
+    other = ctypes.CFUNCTYPE(ctypes.c_int)(lambda: _capi.ABI_VERSION + 1)
+    with pytest.raises(RuntimeError, match="ABI version"):
+        host.bind(ctypes.cast(other, ctypes.c_void_p).value, *addresses[1:])
+    host.bind(*addresses)
+
+
+def test_host_extension_belongs_to_the_running_torch(monkeypatch, tmp_path):
+    from flashmla_b200 import _capi, build
+    host = _capi.host()
+    source = os.path.join(build.CSRC, "host.cpp")
+    for name in ("HOST_PATH", "HOST_LOG"):
+        monkeypatch.setattr(build, name, str(tmp_path / name))
+    assert build._host_is_stale(source)                          # not there
+    (tmp_path / "HOST_PATH").touch()
+    (tmp_path / "HOST_LOG").write_text("failed: " + " ".join(build._host_command(source)) + "\n")
+    assert build._host_is_stale(source)
+    (tmp_path / "HOST_LOG").write_text(" ".join(build._host_command(source)) + "\n")
+    assert not build._host_is_stale(source)
+    _capi._check_built_for(host)
+    monkeypatch.setattr(torch, "__version__", "0.1")
+    assert build._host_is_stale(source)
+    with pytest.raises(RuntimeError, match="was built for torch"):
+        _capi._check_built_for(host)
