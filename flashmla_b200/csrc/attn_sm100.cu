@@ -49,6 +49,7 @@
 // csrc/sm100/prefill/sparse/fwd/head128/phase1.cuh:65-614 (prefill outputs) of deepseek-ai/FlashMLA.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "wait_limit.h"
 #include <cuda_fp16.h>
 #include <string.h>
 #include <stdlib.h>
@@ -72,7 +73,6 @@ constexpr int NPB = 4;                        // P buffers in the value CTA: (ti
 constexpr int NRING = 5;                      // ring barriers: K groups (score CTA, 3 or 4) / V slots (value CTA, 5)
 constexpr int SIDE_BYTES = 144;               // per warp and tile: 32 rescale factors + flag (+ pad)
 constexpr int NTHREADS = 384;                 // dense mode: control warpgroup + two softmax / correction warpgroups
-constexpr long long WAIT_LIMIT_DEFAULT = 2000000000LL;    // SM cycles (about one second)
 constexpr long long DRAIN_LIMIT = 4000000LL;              // wind-down after an expired wait: per tracked operation
 constexpr long long SETTLE_CYCLES = 400000LL;             // ... and for copies between the two CTAs
 #ifndef MLA_TAIL_BULK
@@ -157,7 +157,7 @@ struct Params {
     int head_chunks;                       // dense mode: 64-column chunks between two kv heads of a cache row
     int max_blocks;                        // dense mode: width of the block table
     float scale_log2;
-    uint32_t wait_limit;                   // SM cycles after which a barrier wait gives up
+    uint32_t wait_limit;                   // units of 2^WAIT_UNIT_LOG2 SM cycles after which a barrier wait gives up
     const __nv_bfloat16* q; int64_t q_sb, q_ss, q_sh;
     int q_tma, q_box_bytes;                // a request's Q comes as 9 TMA boxes of q_box_bytes through the empty K ring
     __nv_bfloat16* out; int64_t o_sb, o_ss, o_sh;
@@ -263,25 +263,27 @@ struct Walker<MODE_PREFILL> {
 };
 
 // ---- bounded waits -------------------------------------------------------------------------------------------
-// A wait is a loop of probes (the hardware holds a thread for a while before it answers one) and 32-bit clock reads: eight
-// instructions.  All roles of a CTA share one instruction cache, and there are some thirty wait sites in their loops: with
-// 64-bit clocks, unrolled probes and the reporting at every site the gather modes spent most of their time fetching
+// A wait is a loop of probes (the hardware holds a thread for a while before it answers one) and clock reads, compared in 32
+// bits and units of 2^8 cycles.  (Counted in cycles, prefill is 0.5 % faster - 2774 against 2790 us for 4096 tokens, back to
+// back - but limits above 2^32 cycles are lost; waiting for those in rounds of a 32-bit limit costs every site a few
+// instructions more: 2920 us, and FP8 decode of 64 requests 93.6 -> 105.2.)  All roles of a CTA share one instruction
+// cache, and there are some thirty wait sites in their loops: with 64-bit comparisons, unrolled probes and the reporting at every site the gather modes spent most of their time fetching
 // instructions (4096-token prefill 3440 -> 3010 us, FP8 decode of 64 requests 143 -> 102 us, dense serving 200 -> 186 us for kernels otherwise equal).
 // A thread whose wait ran out only keeps the site's code; it reports when it has left its role.
 //
 // wait() / wait_warp() return false when the wait ran out now or earlier: the caller leaves its role.  CLUSTER: the
 // arrivals come from the other CTA of the pair.
 struct Waiter {
-    uint32_t limit;                      // SM cycles (below 2^32)
+    uint32_t limit;                      // units of 2^WAIT_UNIT_LOG2 SM cycles
     int code = 0;
     __device__ explicit Waiter(uint32_t limit_) : limit(limit_) {}
     template <bool CLUSTER>
     __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int site) {
         if (code) return false;
-        const uint32_t t0 = clock_lo();
+        const uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
         while (!(CLUSTER ? mbar_try_wait_cluster(smem_addr(bar), parity) : mbar_try_wait(smem_addr(bar), parity)))
-            if (clock_lo() - t0 > limit) { code = site; break; }
+            if (clock_units<WAIT_UNIT_LOG2>() - t0 > limit) { code = site; break; }
         return code == 0;
     }
     // whole warps (all 32 lanes execute this): the same answer for every lane
@@ -1452,13 +1454,13 @@ wind_down:
 
 // ---- self-test of the bounded wait: one CTA, one barrier nobody arrives on ---------------------------------
 // Uses the same Waiter and the same reporting as the attention kernels, with nothing in flight (no TMA, no MMA, no
-// cluster): the wait runs into `limit_cycles`, the status words are written, the kernel returns normally.
-__global__ void bounded_wait_selftest_kernel(int* status, long long limit_cycles, int code, int* flag_out) {
+// cluster): the wait runs into its limit, the status words are written, the kernel returns normally.
+__global__ void bounded_wait_selftest_kernel(int* status, uint32_t limit, int code, int* flag_out) {
     __shared__ uint64_t bar;
     __shared__ uint32_t flag;
     if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); flag = 0; fence_mbar_init(); }
     __syncthreads();
-    Waiter w((uint32_t)limit_cycles);
+    Waiter w(limit);
     bool ok = threadIdx.x < 32 ? w.wait<false>(&bar, 0, code) : w.wait_warp<false>(&bar, 0, code);
     // a second wait by the same thread returns at once
     if (threadIdx.x < 32) ok = w.wait<false>(&bar, 0, code + 1) || ok;
@@ -1483,13 +1485,9 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-// Barrier-wait limit in SM cycles: the default, or MLA_WAIT_LIMIT_CYCLES from the environment (read once).
-static uint32_t wait_limit_cycles() {
-    static const uint32_t v = [] {
-        const char* e = getenv("MLA_WAIT_LIMIT_CYCLES");
-        const long long x = e ? atoll(e) : 0;
-        return (uint32_t)(x > 0 ? (x < 4000000000LL ? x : 4000000000LL) : WAIT_LIMIT_DEFAULT);
-    }();
+// Barrier-wait limit of the attention kernels (MLA_WAIT_LIMIT_CYCLES is read once).
+static uint32_t wait_limit() {
+    static const uint32_t v = wait_units_from(getenv("MLA_WAIT_LIMIT_CYCLES"));
     return v;
 }
 
@@ -1512,7 +1510,7 @@ static int configure_once(K kernel, bool (&done)[64]) {
 int launch_bounded_wait_selftest(long long limit_cycles, int code, int* status, int* flag_out, void* stream) {
     MLA_CHECK_ARG(limit_cycles > 0 && limit_cycles <= 2000000000LL, "mla_selftest_bounded_wait: limit_cycles must be in (0, 2e9]");
     MLA_CHECK_ARG(status != nullptr, "mla_selftest_bounded_wait: status must not be null");
-    sm100::bounded_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status, limit_cycles, code, flag_out);
+    sm100::bounded_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status, wait_units(limit_cycles), code, flag_out);
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;
 }
@@ -1611,7 +1609,7 @@ int launch_dense_decode_sm100(const mla_dense_decode_args_t& a) {
     p.rows = a.s_q * p.g;
     p.causal = (a.is_causal && a.s_q > 1) ? 1 : 0;
     p.scale_log2 = a.softmax_scale * kLog2e;
-    p.wait_limit = wait_limit_cycles();
+    p.wait_limit = wait_limit();
     p.q = (const __nv_bfloat16*)a.q; p.q_sb = a.q_stride_b; p.q_ss = a.q_stride_s; p.q_sh = a.q_stride_h;
     p.out = (__nv_bfloat16*)a.out; p.o_sb = a.o_stride_b; p.o_ss = a.o_stride_s; p.o_sh = a.o_stride_h;
     p.lse = a.lse; p.l_sb = a.lse_stride_b; p.l_ss = a.lse_stride_s; p.l_sh = a.lse_stride_h;
@@ -1659,7 +1657,7 @@ int launch_sparse_prefill_sm100(const mla_sparse_prefill_args_t& a) {
     p.b = a.s_q; p.s_q = 1; p.h_q = a.h_q; p.h_kv = 1; p.g = a.h_q; p.rows = a.h_q;
     p.causal = 0;
     p.scale_log2 = a.sm_scale * kLog2e;
-    p.wait_limit = wait_limit_cycles();
+    p.wait_limit = wait_limit();
     p.q = (const __nv_bfloat16*)a.q; p.q_ss = a.q_stride_s; p.q_sh = a.q_stride_h;
     p.out = (__nv_bfloat16*)a.out; p.lse = a.lse; p.max_logits = a.max_logits;
     p.attn_sink = a.attn_sink;
@@ -1703,7 +1701,7 @@ int launch_sparse_decode_sm100(const mla_sparse_decode_args_t& a) {
     p.b = a.b; p.s_q = a.s_q; p.h_q = a.h_q; p.h_kv = 1; p.g = a.h_q; p.rows = a.h_q;
     p.causal = 0;
     p.scale_log2 = a.sm_scale * kLog2e;
-    p.wait_limit = wait_limit_cycles();
+    p.wait_limit = wait_limit();
     p.q = (const __nv_bfloat16*)a.q; p.q_sb = a.q_stride_b; p.q_ss = a.q_stride_s; p.q_sh = a.q_stride_h;
     p.out = (__nv_bfloat16*)a.out; p.o_sb = a.o_stride_b; p.o_ss = a.o_stride_s; p.o_sh = a.o_stride_h;
     p.lse = a.lse; p.l_sb = a.lse_stride_b; p.l_ss = a.lse_stride_s; p.l_sh = a.lse_stride_h;

@@ -72,10 +72,12 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
     return ok != 0;
 }
 
-__device__ __forceinline__ uint32_t clock_lo() {
-    uint32_t t;
-    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
-    return t;
+// SM clock in units of 2^SHIFT cycles
+template <int SHIFT>
+__device__ __forceinline__ uint32_t clock_units() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%clock64;" : "=l"(t));
+    return (uint32_t)(t >> SHIFT);
 }
 
 // Bounded wait: gives up after `limit_cycles` SM clock cycles and returns false.

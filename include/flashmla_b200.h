@@ -284,7 +284,7 @@ int mla_quantize_fp8_kvcache_padded(const mla_quantize_args_t* args);
  * status[1] == 64 (status: device int32[4], zeroed by the caller); flag_out (device int32[2], optional) receives
  * {1, 0}: the CTA's abort flag, and the result of the wait.  This is how an expired wait looks to a caller of the
  * entry points above, which all take the same `status` words.  The default limit of the attention kernels is 2e9
- * cycles; the environment variable MLA_WAIT_LIMIT_CYCLES, read once, overrides it.
+ * cycles; the environment variable MLA_WAIT_LIMIT_CYCLES, read once, overrides it (up to 1.1e12, about nine minutes).
  * No counterpart in the reference (its kernels wait without a limit). */
 int mla_selftest_bounded_wait(long long limit_cycles, int code, int32_t* status, int32_t* flag_out, void* stream);
 

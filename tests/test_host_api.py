@@ -3,6 +3,7 @@ structures agree, and the host-side API mirror enforces the reference's misuse c
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 import torch
@@ -148,3 +149,18 @@ def test_host_extension_belongs_to_the_running_torch(monkeypatch, tmp_path):
     assert build._host_is_stale(source)
     with pytest.raises(RuntimeError, match="was built for torch"):
         _capi._check_built_for(host)
+
+
+@pytest.mark.parametrize("text,cycles", [(None, 2e9), ("", 2e9), ("0", 2e9), ("-5", 2e9), ("1", 1), ("257", 257), ("4000000000", 4e9),
+                                         ("6000000000", 6e9), ("1000000000000", 1e12)])
+def test_wait_limit_from_the_environment(tmp_path, text, cycles):
+    """Waits count in units of 256 cycles: a limit is never shortened, and prolonged by less than one unit."""
+    exe = tmp_path / "limit"
+    source = """#include "wait_limit.h"
+                #include <stdio.h>
+                int main() { printf("%u", mla::wait_units_from(getenv("LIMIT"))); }"""
+    csrc = os.path.join(ROOT, "flashmla_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-I", csrc, "-x", "c++", "-", "-o", str(exe)], input=source, text=True, check=True)
+    env = {"LIMIT": text} if text is not None else {}
+    units = int(subprocess.run([str(exe)], env=env, capture_output=True, text=True, check=True).stdout)
+    assert 0 <= units * 256 - cycles < 256
