@@ -123,3 +123,41 @@ def test_written_records_signed_zeros_and_specials(width, pow2, special):
     if special is None:                            # and the repository's restatement of the reference says the same
         full = quant.quantize_v32(x, pow2_scale=pow2) if width == 576 else quant.quantize_model1(x)
         assert torch.equal(got, full.view(torch.uint8).contiguous())
+
+
+@pytest.mark.parametrize("h_q,counts", [
+    (64, [41]),                                   # 8 warps per row
+    (64, [2, 1, 9]),                              # 4
+    (50, [3, 1, 34] * 4),                         # 2
+    (50, [2, 1, 5, 9] * 5),                       # 1
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_combine_variants_two_query_tokens(h_q, counts, dtype, with_sink):
+    """Every number of warps per row with two query tokens, both output types, attention sinks (infinite ones too) and a row
+    without keys."""
+    from flashmla_b200 import _capi
+    gen = torch.Generator().manual_seed(h_q + len(counts))
+    b, s_q, total = len(counts), 2, sum(counts)
+    ns = torch.tensor([0] + list(np.cumsum(counts)), dtype=torch.int32)
+    lse_acc = torch.randn(total, s_q, h_q, generator=gen) * 3
+    o_acc = torch.randn(total, s_q, h_q, 512, generator=gen)
+    lse_acc[0, 1, 2] = float("-inf")                                       # an empty split
+    lse_acc[:counts[0], 0, 3], o_acc[:counts[0], 0, 3] = float("-inf"), 0  # a row of request 0 without keys
+    sink = torch.randn(h_q, generator=gen) if with_sink else None
+    if with_sink:
+        sink[0], sink[1], sink[3] = float("inf"), float("-inf"), float("inf")
+    out0, lse0 = torch.randn(b, s_q, h_q, 512, generator=gen).to(dtype), torch.randn(b, h_q, s_q, generator=gen)
+    ref_out, ref_lse = _combine_ref(lse_acc, o_acc, ns, b, s_q, h_q, sink, out0, lse0)
+    out, lse, la, oa, nd = out0.to(DEV), lse0.to(DEV), lse_acc.to(DEV), o_acc.to(DEV), ns.to(DEV)
+    sink_d = sink.to(DEV) if with_sink else None
+    c = _capi.CombineArgs(b=b, s_q=s_q, h_q=h_q, d_v=512, lse=_capi.ptr(lse), lse_stride_b=lse.stride(0), lse_stride_s=lse.stride(2),
+                          lse_stride_h=lse.stride(1), out=_capi.ptr(out), o_stride_b=out.stride(0), o_stride_s=out.stride(1),
+                          o_stride_h=out.stride(2), lse_accum=_capi.ptr(la), o_accum=_capi.ptr(oa), num_splits=_capi.ptr(nd),
+                          attn_sink=_capi.ptr(sink_d), dtype=_capi.MLA_DTYPE_FP16 if dtype == torch.float16 else _capi.MLA_DTYPE_BF16,
+                          stream=torch.cuda.current_stream().cuda_stream)
+    _capi.check(_capi.lib().mla_combine(c), "mla_combine")
+    # fp32 sums in another order, then one rounding: at most one step of the output type (2^-7 / 2^-10 of the value)
+    step = 2 ** -7 if dtype == torch.bfloat16 else 2 ** -10
+    assert torch.allclose(out.cpu().float(), ref_out.to(dtype).float(), rtol=step, atol=1e-5, equal_nan=True)
+    assert torch.allclose(lse.cpu(), ref_lse, rtol=1e-5, atol=1e-5)
