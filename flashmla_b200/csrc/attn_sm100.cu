@@ -277,20 +277,21 @@ struct Waiter {
     uint32_t limit;                      // units of 2^WAIT_UNIT_LOG2 SM cycles
     int code = 0;
     __device__ explicit Waiter(uint32_t limit_) : limit(limit_) {}
+    __device__ __forceinline__ bool expired() const { return code != 0; }
     template <bool CLUSTER>
     __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int site) {
-        if (code) return false;
+        if (expired()) return false;
         const uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
         while (!(CLUSTER ? mbar_try_wait_cluster(smem_addr(bar), parity) : mbar_try_wait(smem_addr(bar), parity)))
             if (clock_units<WAIT_UNIT_LOG2>() - t0 > limit) { code = site; break; }
-        return code == 0;
+        return !expired();
     }
     // whole warps (all 32 lanes execute this): the same answer for every lane
     template <bool CLUSTER>
     __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, int site) {
         wait<CLUSTER>(bar, parity, site);
-        return !__any_sync(0xffffffffu, code != 0);
+        return !__any_sync(0xffffffffu, expired());
     }
 };
 // First code and a count in the global status words, the `aborted` flag of this CTA and of its peer.
@@ -1150,14 +1151,14 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                             tmem_st32(tlane + L::TM_Q + c * 32, v);
                         }
                         tmem_wait_st();
-                        if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.ring_released));        // the producers may fill the ring with K now
+                        if (!wt.expired()) mbar_arrive(smem_addr(&sm.ring_released));        // the producers may fill the ring with K now
                     } else {
                         load_q_by_threads<MODE>(sm, qrow, row_ok, half, r, tlane, NO_CHUNK8);
                     }
                     tmem_wait_st();
                     fence_proxy_async_smem();
                     tc_fence_before();
-                    if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.q_ready));
+                    if (!wt.expired()) mbar_arrive(smem_addr(&sm.q_ready));
                 }
                 // first key position this row must NOT see (causal limit, and the end of this partition's range)
                 const int limit = min(p.causal ? w.seqlen - (p.s_q - 1 - t) : w.seqlen, w.blk_end * PAGE);
@@ -1185,7 +1186,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     }
                     tmem_wait_ld();
                     tc_fence_before();
-                    if (!(wt.code != 0)) mbar_arrive(smem_addr(&sm.s_empty[sb]));          // the MMA warp may overwrite this S accumulator
+                    if (!wt.expired()) mbar_arrive(smem_addr(&sm.s_empty[sb]));            // the MMA warp may overwrite this S accumulator
 
                     if (!DENSE) {
                         if ((m0 & m1) != 0xffffffffu) {
@@ -1210,7 +1211,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                     float mx = fmaxf(mx0, mx1);
                     // the row maximum over both pages of the tile; the barrier also carries the abort flag
                     xmax[((g & 1) * 2 + half) * ROWS + r] = mx;
-                    BAR_OR_LEAVE((wt.code != 0));
+                    BAR_OR_LEAVE(wt.expired());
                     mx = fmaxf(mx, xmax[((g & 1) * 2 + (half ^ 1)) * ROWS + r]);
                     mx *= p.scale_log2;                                // scale > 0: max commutes with scaling
                     m_true = fmaxf(m_true, mx);
@@ -1239,7 +1240,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
 
                     // staging of this warp is free once the previous tile's copy has landed in the value CTA
                     wt.template wait<true>(&sm.stage_free[half], (g & 1) ^ 1, 8);
-                    if (!(wt.code != 0)) {
+                    if (!wt.expired()) {
                         uint8_t* prow = stage + (lane >> 3) * 1024 + (lane & 7) * 128;
 #pragma unroll
                         for (int ch = 0; ch < 8; ++ch)
@@ -1258,13 +1259,13 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
                 {
                     float* lsum = L::WIDE ? xmax + ((g & 1) * 2) * ROWS : reinterpret_cast<float*>(sm.data + L::SC_LSUM);
                     if (half == 1) lsum[r] = l_run;
-                    BAR_OR_LEAVE((wt.code != 0));
+                    BAR_OR_LEAVE(wt.expired());
                     if (half == 0) l_run += lsum[r];
-                    BAR_OR_LEAVE((wt.code != 0));
+                    BAR_OR_LEAVE(wt.expired());
                 }
                 if (half == 0) {
                     wt.template wait<true>(&sm.fin_empty, (nreq & 1) ^ 1, 7);
-                    if (!(wt.code != 0)) {
+                    if (!wt.expired()) {
                         st_cluster_f32(remote_fin, l_run);
                         st_cluster_f32(remote_fin + ROWS * 4, m_run);
                         st_cluster_f32(remote_fin + 2 * ROWS * 4, m_true);
@@ -1419,7 +1420,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     }
 
 wind_down:
-    if (wt.code) report_expired_wait(p.status, &sm.aborted, map_to_cta(smem_addr(&sm.aborted), cta_rank ^ 1u), wt.code);
+    if (wt.expired()) report_expired_wait(p.status, &sm.aborted, map_to_cta(smem_addr(&sm.aborted), cta_rank ^ 1u), wt.code);
     // ---- wind down: both CTAs leave together, tensor memory is released -----------------------------------
     if (!DENSE && warp >= 12) cp_async_wait_all();          // this thread's own row copies have landed
     tc_fence_before();
@@ -1464,7 +1465,7 @@ __global__ void bounded_wait_selftest_kernel(int* status, uint32_t limit, int co
     bool ok = threadIdx.x < 32 ? w.wait<false>(&bar, 0, code) : w.wait_warp<false>(&bar, 0, code);
     // a second wait by the same thread returns at once
     if (threadIdx.x < 32) ok = w.wait<false>(&bar, 0, code + 1) || ok;
-    if (w.code) report_expired_wait(status, &flag, 0u, w.code);
+    if (w.expired()) report_expired_wait(status, &flag, 0u, w.code);
     __syncthreads();
     if (threadIdx.x == 0 && flag_out) { flag_out[0] = (int)flag; flag_out[1] = ok ? 1 : 0; }
 }

@@ -541,6 +541,10 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, 
 #define TEXT(x) TEXT_(x)
 PyMODINIT_FUNC PyInit__host() {
     PyObject* m = PyModule_Create(&module_def);
+    // the tile scheduler's arguments, for callers that make a schedule through the C ABI
+    if (m && (PyModule_AddIntConstant(m, "BLOCK_SIZE_N", BLOCK_SIZE_N) || PyModule_AddIntConstant(m, "META_INTS", META_INTS) ||
+              PyModule_AddIntConstant(m, "FIXED_OVERHEAD_NUM_BLOCKS", FIXED_OVERHEAD_NUM_BLOCKS)))
+        Py_CLEAR(m);
     // what the file was compiled against; _capi.py compares it with what is running
     if (m && PyModule_AddStringConstant(m, "built_for", "torch " FLASHMLA_TORCH_VERSION ", Python " TEXT(PY_MAJOR_VERSION) "." TEXT(PY_MINOR_VERSION)))
         Py_CLEAR(m);

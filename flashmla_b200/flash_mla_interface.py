@@ -13,11 +13,6 @@ import torch
 from . import _capi
 from ._capi import ptr
 
-# Arguments of the tile scheduler (csrc/api/dense_decode.h:104-105, csrc/api/sparse_decode.h:92-99)
-_BLOCK_SIZE_N = 64
-_FIXED_OVERHEAD_NUM_BLOCKS = 5
-_META_INTS = 8
-
 # Kernel selection for tests / benchmarks: 0 = fastest supporting kernel, 1 = portable, 2 = tcgen05
 _impl_override = 0
 
@@ -111,10 +106,11 @@ def get_mla_metadata(*args, **kwargs) -> Tuple[FlashMLASchedMeta, None]:
 def _make_sched_meta(b, s_q, num_sm_parts, device, seqlens_k=None, topk=-1, extra_topk=0,
                      topk_length=None, extra_topk_length=None):
     """A schedule for callers of the C ABI (the calls below make theirs on the way)."""
-    meta = torch.empty((num_sm_parts, _META_INTS), dtype=torch.int32, device=device)
+    host = _capi.host()
+    meta = torch.empty((num_sm_parts, host.META_INTS), dtype=torch.int32, device=device)
     num_splits = torch.empty((b + 1,), dtype=torch.int32, device=device)
     a = _capi.SchedMetaArgs(
-        b=b, s_q=s_q, block_size_n=_BLOCK_SIZE_N, fixed_overhead_num_blocks=_FIXED_OVERHEAD_NUM_BLOCKS,
+        b=b, s_q=s_q, block_size_n=host.BLOCK_SIZE_N, fixed_overhead_num_blocks=host.FIXED_OVERHEAD_NUM_BLOCKS,
         topk=topk, extra_topk=extra_topk,
         topk_length=ptr(topk_length), extra_topk_length=ptr(extra_topk_length), seqlens_k=ptr(seqlens_k),
         meta=ptr(meta), num_splits=ptr(num_splits), num_sm_parts=num_sm_parts, stream=torch.cuda.current_stream(device).cuda_stream)
