@@ -87,8 +87,10 @@ enum { MODE_DENSE = 0, MODE_PREFILL = 1, MODE_SPARSE_DECODE = 2 };
 // warpgroup re-sizes its share as the first thing in its branch; the shares add up to no more than the launch had.
 //   prefill     640 threads x 96 registers: control 96, softmax 136, gather 56.  EIGHT gather warps: an SM's copy rate is
 //               bound by what its warps can issue, 77 GB/s with four warps, 102 with eight (stand-alone probe).  The control
-//               warps' share is what the issuing thread of the MMAs needs: with 64 it spilled the descriptors of its unrolled
-//               loop (4096 tokens: 2590 us with control 64, 2450 with 80, 2410 with 96).
+//               warps' share is what the issuing thread of the MMAs needs: with less it spills the descriptors of its unrolled
+//               loop (4096 tokens: 2526 us with control 64, 2428 with 80, 2421 with 96 in short runs; 2894, 2812 and 2800
+//               back to back under the power limit).  Warps 8-11 of the value CTA have no work in the gather modes, and
+//               their registers none either: the shares are the same in both CTAs.
 //   FP8 decode  768 threads x 80 registers: control 48, softmax 112, gather 80, convert 64.  The conversion has warps of its
 //               own: on the softmax warps it was serial with the softmax (5.2 us a tile).
 template <int MODE>
@@ -108,8 +110,8 @@ struct Lay {
     // WIDE plan (dense decode): all 576 dims of Q in tensor memory (288 columns) next to ONE S accumulator, which frees
     // the shared memory for a K ring of FOUR groups.  The gather modes keep the narrow plan (dims 0..447 of Q in tensor
     // memory, 448..575 in shared memory, two S accumulators, three groups): prefill is paced by the copy instructions of
-    // its gather warps, not by the ring (measured with the wide plan: 3.49 against 3.41 ms), and FP8 decode needs 4 KB for
-    // the tokens' scales.
+    // its gather warps, not by the ring (the wide plan, measured when four warps copied: 3.49 against 3.41 ms), and FP8 decode
+    // needs 4 KB for the tokens' scales.
     static constexpr bool WIDE = MODE == MODE_DENSE;
     static constexpr int NKS = WIDE ? 4 : 3;              // K ring slots; group j of tile g is fill 3 g + j and uses slot (3 g + j) mod NKS
     static constexpr int S_BUFS = WIDE ? 1 : 2;           // S accumulators in tensor memory
@@ -264,11 +266,11 @@ struct Walker<MODE_PREFILL> {
 
 // ---- bounded waits -------------------------------------------------------------------------------------------
 // A wait is a loop of probes (the hardware holds a thread for a while before it answers one) and clock reads, compared in 32
-// bits and units of 2^8 cycles.  (Counted in cycles, prefill is 0.5 % faster - 2774 against 2790 us for 4096 tokens, back to
-// back - but limits above 2^32 cycles are lost; waiting for those in rounds of a 32-bit limit costs every site a few
-// instructions more: 2920 us, and FP8 decode of 64 requests 93.6 -> 105.2.)  All roles of a CTA share one instruction
-// cache, and there are some thirty wait sites in their loops: with 64-bit comparisons, unrolled probes and the reporting at every site the gather modes spent most of their time fetching
-// instructions (4096-token prefill 3440 -> 3010 us, FP8 decode of 64 requests 143 -> 102 us, dense serving 200 -> 186 us for kernels otherwise equal).
+// bits and units of 2^8 cycles.  All roles of a CTA share one instruction cache, and there are some thirty wait sites in
+// their loops: with 64-bit comparisons and the report at every site, 4096-token prefill takes 2870 us in the place of 2800,
+// FP8 decode of 64 requests 95.7 (94.4), of 512-wide records 84.7 (81.6), dense decode the same (back to back, kernels
+// otherwise equal).  Counted in cycles, prefill is 0.5 % faster (2774 against 2790), but limits above 2^32 cycles are lost;
+// waiting for those in several 32-bit spans costs every site a few instructions more: 2920, and FP8 decode 93.6 -> 105.2.
 // A thread whose wait ran out only keeps the site's code; it reports when it has left its role.
 //
 // wait() / wait_warp() return false when the wait ran out now or earlier: the caller leaves its role.  CLUSTER: the
@@ -428,9 +430,9 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
     constexpr bool M1 = ALT && MODE == MODE_SPARSE_DECODE;
     // How far the MMA issue loops are unrolled (turns of one loop body).  Unrolled, an MMA's descriptor is a compile-time
     // offset and issuing is fastest; rolled, the roles of an SM share less code.  FP8 decode has issue time to spare and six
-    // roles per SM (rolled by groups 102 -> 93 us for 64 requests); prefill and dense decode have not (rolled 2760 -> 2940 us
-    // for 4096 tokens, 165 -> 172 us for the serving batch).  The pages of P V stay rolled everywhere (unrolled: prefill
-    // 2590 -> 2765 us, dense decode the same).
+    // roles per SM (64 requests: unrolled 102.2 us, rolled by groups 94.4); prefill and dense decode have not (4096 tokens:
+    // 2800 unrolled, 3393 rolled; the serving batch 196.3 and 202.5).  The pages of P V stay rolled everywhere (unrolled:
+    // prefill 2918, FP8 decode 99.2, dense decode the same).  All back to back.
     constexpr int MMA_GROUPS = MODE == MODE_SPARSE_DECODE ? 1 : 3;
     constexpr bool NO_CHUNK8 = ALT && MODE != MODE_DENSE;  // 512-wide rows
     constexpr int REC_BYTES = M1 ? 576 : 656;              // bytes between two tokens' values inside a block

@@ -160,10 +160,17 @@ int launch_combine(const mla_combine_args_t& a) {
     MLA_CHECK_ARG(is_aligned16(a.o_accum), "combine: o_accum must be 16-byte aligned");
     MLA_CHECK_ARG(((uintptr_t)a.out & 7u) == 0 && a.o_stride_b % 4 == 0 && a.o_stride_s % 4 == 0 && a.o_stride_h % 4 == 0,
                   "combine: out must be 8-byte aligned with strides that are multiples of 4 elements");
-    // Warps per row: about one for every two splits a row can be expected to have (the partitions of a decode launch shared
-    // out over the batch), as long as all CTAs run in one wave (2 per SM with the deeper unrolling of WPR = 8, else 3).  With
-    // few rows the time is one row's chain of loads: 128 rows of 74 splits took 42 us with one warp per row, 10 us with eight;
-    // 976 rows of 2 splits are 3 us slower with two warps per row than with one.
+    // Warps per row, from an estimate of the splits a request has: the SM pairs shared out over row blocks of 128 and the batch.
+    // This kernel knows neither the partition count nor h_kv: the estimate is high for several kv heads and, in sparse decode,
+    // for several query tokens of at most 64 heads.  The bounds on the rows (all CTAs in one wave: 2 per SM with the deeper
+    // unrolling of WPR = 8, else 3) keep that harmless.  us alone, behind a 256 MB scrub, with
+    // 1 / 2 / 4 / 8 warps per row, and the rule's choice (event resolution 2 us):
+    //    rows  splits                            rows  splits
+    //     128    74    35 / 23 / 16 / 14   8      1024    10    12 / 12 / 12 / 14   2
+    //     128    16    12 / 10 /  8 /  8   8      1536     7    12 / 12 / 12 / 16   2
+    //     256    37    23 / 16 / 12 / 12   8      1536     2     8 /  8 / 10 / 16   2
+    //     512    19    14 / 12 / 12 / 12   4       976     2     8 /  8 / 10 / 12   1 or 2
+    //     768    13    14 / 12 / 12 / 14   4     16384     2    20 / 27 / 45 /100   1
     const int64_t rows = (int64_t)a.b * a.s_q * a.h_q;
     const int sms = current_device_num_sms() > 0 ? current_device_num_sms() : 148;
     const int splits = 1 + sms / 2 / std::max(1, (a.s_q * a.h_q + 127) / 128) / a.b;

@@ -3,17 +3,17 @@
 // (tests/quant.py:20-53 of the reference: scale = amax / 448 per group of 128, optionally rounded up to a power of
 // two; q = e4m3(x / scale), round to nearest even).
 //
-// One warp per token: lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is one
-// coalesced 512-byte store.  HBM-bound: 1152 bytes read + 656 bytes written per token.  Every warp takes two tokens, whose
-// loads are in flight together.  With one IEEE division per value (__fdiv_rn, a dozen instructions and a branch) the kernel
-// was bound by instructions instead: 34 us for 66 K tokens (3.5 TB/s).  The quotients x / s only need the correctly rounded
-// reciprocal of s, once per group, and three instructions each (Markstein's theorem; quotient16 below).
+// A warp takes two tokens, whose loads are in flight together; lane l holds values 16l .. 16l+15 of a token (8 lanes per
+// scale group), so the record's e4m3 part is one coalesced 512-byte store.  1152 bytes read + 656 bytes written per token.
+// With one IEEE division per value (__fdiv_rn, a dozen instructions and a branch) 66 K tokens took 34 us (3.5 TB/s).  The
+// quotients x / s only need the correctly rounded reciprocal of s, once per group, and three instructions each (Markstein's
+// theorem; quotient16 below): 28.7 us (4.2 TB/s).  What bounds it is still the instructions, not memory.
 //
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
 // block_size x 8 scale bytes (7 scales + 1 pad).  Lanes 0-27 hold the quantised values (4 lanes per group), lanes 28-31
-// the RoPE part.  The first warps also zero the `pad_bytes` behind every block, where the caller owns
-// them (one warp a block; with the last token's stores, inside the loop, 66 K tokens took 36.9 us instead of 34.9).
+// the RoPE part.  The first warps also zero the `pad_bytes` behind every block, where the caller owns them (one warp a
+// block; with the last token's stores, inside the loop, 66 K tokens took 36.9 us instead of 34.9).
 #include "common.cuh"
 
 #include <cuda_fp8.h>

@@ -138,7 +138,7 @@ int mla_dense_decode_fwd(const mla_dense_decode_args_t* args);
  *   d_qk 576: 656 bytes per token = 512 e4m3 | 4 fp32 scales (one per 128 values) | 64 bf16 RoPE; V = the first 512 dims.
  *   d_qk 512 ("MODEL1"): a block holds page_block_size x [448 e4m3 | 64 bf16 RoPE] (576 bytes per token) followed by
  *            page_block_size x [7 e8m0 scales (one per 64 values) | 1 pad byte]; the tensor is the
- *            [num_blocks, page_block_size, 1, 584] view of it and V = all 512 dims.  Served by the all-shape kernel.
+ *            [num_blocks, page_block_size, 1, 584] view of it and V = all 512 dims.
  * Replaces
  * DecodeImplBase::run as driven by sparse_attn_decode_interface
  * (csrc/api/sparse_decode.h:183-495); arguments mirror SparseAttnDecodeParams
