@@ -13,9 +13,11 @@
 // starts at cost position x (request r, block x - C[r]) may spend up to X = x + budget: it finishes every request e' with
 // C[e' + 1] <= X, and cuts the next one, e, if blocks are left after that request's overhead (X - F > C[e]).  So the next
 // partition starts at X - F or at C[e], and only this position is serial: one warp walks the partitions, comparing 32
-// prefix sums at a time (a vote instead of a walk over the requests, about 60 cycles a partition).  Prefix sums, metadata
-// rows and split counts are made by all threads.  A serial walk of one thread over requests and partitions took 14 us for
-// 128 requests on 74 partitions.
+// prefix sums at a time (a vote instead of a walk over the requests).  Nothing else stands in that chain: lane l keeps the
+// start of partition l, and 32 metadata rows are finished and written side by side, each ending where the next one starts.
+// What bounds it is the chain, about 130 cycles a partition.  us a schedule, one after the other in a graph: one thread that
+// walks requests and partitions / rows written and cuts counted by one lane inside the chain / now:
+//    b 1, 74 partitions  9 / 13 / 5.3;   b 32  12 / 15.5 / 6.6;   b 128  17 / 16 / 6.9;   b 1000  60 / 20 / 10.6
 #include "common.cuh"
 
 #include <limits.h>
@@ -91,62 +93,65 @@ sched_meta_kernel(const mla_sched_meta_args_t a) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         const int budget = (C[b] + P - 1) / P + F;
+        auto blocks = [&](int r) { const int n = C[r + 1] - C[r] - F; return (zero_len[r >> 5] >> (r & 31)) & 1u ? -1 : n; };
         // window: lane l holds C[base + l + 1] (past the end: never reached)
         int base = 0, window = lane < b ? C[lane + 1] : INT_MAX;
         int x = 0, r = 0, split = 0, at_r = 0;                      // at_r = C[r]
-        for (int p = 0; p < P; ++p) {
-            // (completed below: the end as request e, `end_block` blocks of it)
-            mla_sched_meta_t m;
-            m.begin_req_idx = r;
-            m.begin_block_idx = x - at_r;
-            m.begin_split_idx = split;
-            m.end_req_idx = r;
-            m.end_block_idx = 0;
-            m.is_first_req_splitted = m.is_last_req_splitted = m._pad = 0;
-            if (r < b) {
+        for (int p0 = 0; p0 < P; p0 += 32) {
+            // lane l keeps where partition p0 + l begins: request, block, split
+            int begin_r = r, begin_block = x - at_r, begin_split = split;
+            const int n_parts = min(32, P - p0);
+#pragma unroll 1
+            for (int i = 1; i <= n_parts && r < b; ++i) {          // (behind the last request every partition begins where this one ends)
                 const int X = x + budget;
                 int n = __popc(__ballot_sync(0xffffffffu, window <= X));
-                int e = base + n, at_e = n ? __shfl_sync(0xffffffffu, window, n - 1) : at_r;
+                int at_e = __shfl_sync(0xffffffffu, window, n - 1);
                 while (n == 32) {                                  // the window lies wholly inside the budget: the next one
                     base += 32;
                     at_r = at_e;
                     window = base + lane < b ? C[base + lane + 1] : INT_MAX;
                     n = __popc(__ballot_sync(0xffffffffu, window <= X));
-                    e = base + n;
-                    if (n) at_e = __shfl_sync(0xffffffffu, window, n - 1);
+                    at_e = __shfl_sync(0xffffffffu, window, n - 1);
                 }
+                const int e = base + n;
+                at_e = n ? at_e : at_r;
                 const bool cut = e < b && X - F > at_e;
                 split = cut ? (e == r ? split + 1 : 1) : 0;
-                if (cut && lane == 0) ++cuts[e];
                 x = cut ? X - F : at_e;
                 r = e;
                 at_r = at_e;
-                m.end_req_idx = e;
-                m.end_block_idx = x - at_e;
+                if (lane >= i) { begin_r = r; begin_block = x - at_r; begin_split = split; }
             }
-            if (lane == 0) a.meta[p] = m;
+            // ... and ends where the next one begins
+            mla_sched_meta_t m;
+            m.end_req_idx = __shfl_down_sync(0xffffffffu, begin_r, 1);
+            m.end_block_idx = __shfl_down_sync(0xffffffffu, begin_block, 1);
+            if (lane == n_parts - 1) { m.end_req_idx = r; m.end_block_idx = x - at_r; }
+            if (lane < n_parts) {
+                m.begin_req_idx = begin_r;
+                // A partition that starts after the last request reports the last block index of request 0
+                // here: the reference reads one element past its first-block array, which is the first
+                // element of its last-block array.  Consumers skip such partitions (begin_req_idx >= b).
+                m.begin_block_idx = begin_r < b ? begin_block : abs(blocks(0)) - 1;
+                m.begin_split_idx = begin_split;
+                m.is_first_req_splitted = begin_block != 0;
+                if (m.end_block_idx == 0) {
+                    --m.end_req_idx;
+                    m.end_block_idx = max(blocks(m.end_req_idx), 0);
+                } else {
+                    atomicAdd(&cuts[m.end_req_idx], 1);
+                }
+                const int n_end = blocks(m.end_req_idx);
+                m.is_last_req_splitted = n_end > 0 && m.end_block_idx != n_end;
+                if (m.begin_req_idx == m.end_req_idx)
+                    m.is_first_req_splitted = m.is_last_req_splitted = (m.is_first_req_splitted || m.is_last_req_splitted);
+                m._pad = 0;
+                a.meta[p0 + lane] = m;
+            }
         }
     }
     __syncthreads();
 
-    for (int p = threadIdx.x; p < P; p += SCHED_THREADS) {
-        auto blocks = [&](int r) { const int n = C[r + 1] - C[r] - F; return (zero_len[r >> 5] >> (r & 31)) & 1u ? -1 : n; };
-        mla_sched_meta_t m = a.meta[p];
-        m.is_first_req_splitted = m.begin_block_idx != 0;
-        // A partition that starts after the last request reports the last block index of request 0
-        // here: the reference reads one element past its first-block array, which is the first
-        // element of its last-block array.  Consumers skip such partitions (begin_req_idx >= b).
-        if (m.begin_req_idx >= b) m.begin_block_idx = abs(blocks(0)) - 1;
-        if (m.end_block_idx == 0) {
-            --m.end_req_idx;
-            m.end_block_idx = max(blocks(m.end_req_idx), 0);
-        }
-        const int n_end = blocks(m.end_req_idx);
-        m.is_last_req_splitted = n_end > 0 && m.end_block_idx != n_end;
-        if (m.begin_req_idx == m.end_req_idx)
-            m.is_first_req_splitted = m.is_last_req_splitted = (m.is_first_req_splitted || m.is_last_req_splitted);
-        a.meta[p] = m;
-    }
     // a request has one piece more than cuts
     carry = 0;
     if (threadIdx.x == 0) a.num_splits[0] = 0;
