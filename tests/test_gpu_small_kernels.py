@@ -161,3 +161,17 @@ def test_combine_variants_two_query_tokens(h_q, counts, dtype, with_sink):
     step = 2 ** -7 if dtype == torch.bfloat16 else 2 ** -10
     assert torch.allclose(out.cpu().float(), ref_out.to(dtype).float(), rtol=step, atol=1e-5, equal_nan=True)
     assert torch.allclose(lse.cpu(), ref_lse, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("b", [1, 2, 33, 128])
+@pytest.mark.parametrize("parts", [1, 31, 32, 33, 64, 65])
+def test_schedule_rows_in_groups_of_32_partitions(b, parts):
+    """The walk finishes 32 metadata rows at a time: the last row of a group ends where the next group starts, and the work may
+    end inside a group or with it."""
+    for longest in (0, 64, 5000, 90000):
+        gen = np.random.default_rng(b * 100 + parts + longest)
+        seq = [int(x) for x in gen.integers(0, longest + 1, b)]
+        seq[-1] = longest
+        meta, ns = _run_meta(b, parts, 64, 5, seqlens=seq)
+        want_meta, want_ns = sched_meta.get_sched_meta(b, parts, 64, 5, seqlens_k=seq)
+        assert np.array_equal(np.asarray(meta)[:, :7], want_meta[:, :7]) and np.array_equal(np.asarray(ns), want_ns)
