@@ -269,7 +269,8 @@ struct Walker<MODE_PREFILL> {
 // bits and units of 2^8 cycles.  All roles of a CTA share one instruction cache, and there are some thirty wait sites in
 // their loops: with 64-bit comparisons and the report at every site, 4096-token prefill takes 2870 us in the place of 2800,
 // FP8 decode of 64 requests 95.7 (94.4), of 512-wide records 84.7 (81.6), dense decode the same (back to back, kernels
-// otherwise equal).  Counted in cycles, prefill is 0.5 % faster (2774 against 2790), but limits above 2^32 cycles are lost;
+// otherwise equal).  Counted in cycles, prefill (2774 against 2790) and dense decode (192.2 against 193.1 for the serving
+// batch) are 0.5 % faster, but limits above 2^32 cycles are lost;
 // waiting for those in several 32-bit spans costs every site a few instructions more: 2920, and FP8 decode 93.6 -> 105.2.
 // A thread whose wait ran out only keeps the site's code; it reports when it has left its role.
 //

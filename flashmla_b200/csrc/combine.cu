@@ -169,7 +169,7 @@ int launch_combine(const mla_combine_args_t& a) {
     //     128    74    35 / 23 / 16 / 14   8      1024    10    12 / 12 / 12 / 14   2
     //     128    16    12 / 10 /  8 /  8   8      1536     7    12 / 12 / 12 / 16   2
     //     256    37    23 / 16 / 12 / 12   8      1536     2     8 /  8 / 10 / 16   2
-    //     512    19    14 / 12 / 12 / 12   4       976     2     8 /  8 / 10 / 12   1 or 2
+    //     512    19    14 / 12 / 12 / 12   4       976     2     8 /  8 / 10 / 12   1
     //     768    13    14 / 12 / 12 / 14   4     16384     2    20 / 27 / 45 /100   1
     const int64_t rows = (int64_t)a.b * a.s_q * a.h_q;
     const int sms = current_device_num_sms() > 0 ? current_device_num_sms() : 148;
