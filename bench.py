@@ -399,7 +399,7 @@ def bind_to_gpu_numa_node(gpu_index):
 
 
 # ------------------------------------------------------------------------------------------------------
-# CPU arm: the reference's torch attention on the host cores, bounded sample.  Returns the checker's outputs too, so
+# CPU arm: the reference's torch attention on the host cores, bounded sample.  Returns the oracle's outputs too, so
 # that the timed GPU result can be compared with them.
 # ------------------------------------------------------------------------------------------------------
 def _reference_dense_fn():
@@ -489,7 +489,7 @@ def cpu_baseline(w, budget_s=15.0, keep_outputs=False):
 
 
 def check_against_oracle(w, out, lse, oracle_outputs):
-    """Compares the TIMED result (the output of the replayed graph) with the checker's outputs, unit by unit (request /
+    """Compares the TIMED result (the output of the replayed graph) with the oracle's outputs, unit by unit (request /
     query row); raises on the first unit outside the acceptance bounds.  Returns the number of units checked."""
     from oracle.compare import cos_diff, max_abs_err
     out_c, lse_c = out.detach().cpu(), lse.detach().cpu()
@@ -839,7 +839,7 @@ def main():
         r = cpu_baseline(w, budget_s=12.0, keep_outputs=True)
         line["cpu_baseline"] = {"value": units_per_step * r["frac"] / r["seconds"], "unit": unit, "cores": r["cores"],
                                 "kind": r["kind"], "sample": r["sample"]}
-        # the result that was timed (the replayed graph's output) against the checker, unit by unit
+        # the result that was timed (the replayed graph's output) against the oracle, unit by unit
         line["parity_checked"] = check_against_oracle(w, g_out, g_lse, r["outputs"])
         line["parity_bounds"] = {"out_cos_deficit": OUT_COS_TOL, "out_max_abs": OUT_ABS_TOL, "lse_abs": LSE_TOL}
     # (not with a forced replay count: that is how profiler captures keep the run short)

@@ -1,7 +1,7 @@
 """CPU restatement of the reference's MLA decode / sparse-prefill algorithms.
 
 TEST INFRASTRUCTURE ONLY.  Nothing in the shipped package may import this
-directory: it is the checker for the CUDA path (tests, the smoke check and the
+directory: it is what the CUDA path is checked against (tests, the smoke check and the
 CPU-baseline leg of the benchmark), never the thing that is measured or
 shipped.
 
