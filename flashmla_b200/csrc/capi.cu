@@ -63,6 +63,10 @@ static int check_decode_common(const char* who, bool allow_512, int b, int s_q, 
 
 using namespace mla;
 
+// Query rows (query tokens x heads of a kv head) that one SM serves by itself (attn_rows64.cu, with what it measured on both sides
+// of this line): O^T of more rows and the scores do not fit its tensor memory, Q and a tile not its shared memory.
+constexpr int ROWS64 = 64;
+
 extern "C" {
 
 const char* mla_last_error(void) { return last_error_buffer(); }
@@ -78,15 +82,15 @@ int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q) {
     }
     if (mode == MLA_MODE_DENSE_DECODE) {
         // A partition is walked, for every block of 128 query rows of every kv head, by a pair of CTAs on two
-        // SMs (the tcgen05 kernel's score / value CTAs, or two 64-row CTAs of the portable kernel).
+        // SMs (the tcgen05 kernel's score / value CTAs, or two 64-row CTAs of the portable kernel); up to 64 rows take one CTA.
         const int rows = s_q * (h_q / h_kv);
         const int row_blocks = (rows + 127) / 128;
-        int p = sms / 2 / h_kv / row_blocks;
+        int p = (rows <= ROWS64 ? sms : sms / 2) / h_kv / row_blocks;
         return p > 0 ? p : 1;
     } else if (mode == MLA_MODE_SPARSE_DECODE) {
-        // up to 128 heads: one CTA pair of the tcgen05 kernel per partition and query token; more heads run on the
-        // portable kernel, one CTA per 64 heads
-        int p = h_q <= 128 ? sms / 2 / s_q : sms / s_q / ((h_q + 63) / 64);
+        // per partition and query token: up to 64 heads one CTA, up to 128 a pair of CTAs on two SMs (the tcgen05 kernels), more
+        // heads one CTA per 64 of them (the portable kernel)
+        int p = sms / s_q / ((h_q + 63) / 64);
         return p > 0 ? p : 1;
     }
     set_error(MLA_ERR_INVALID_ARG, "mla_num_sm_parts: unknown mode %d", mode);
@@ -135,12 +139,13 @@ int mla_dense_decode_fwd(const mla_dense_decode_args_t* a) {
     MLA_CHECK_ARG(a->num_blocks > 0, "mla_dense_decode_fwd: num_blocks must be positive");
     MLA_CHECK_ARG(is_aligned16(a->k_cache) && a->k_stride_block % 8 == 0 && a->k_stride_row % 8 == 0 && a->k_stride_head % 8 == 0,
                   "mla_dense_decode_fwd: k_cache must be 16-byte aligned with strides that are multiples of 8 elements");
+    const bool rows64 = a->s_q * (a->h_q / a->h_kv) <= ROWS64;
     if (a->impl == 2) {
         if (!dense_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: the tcgen05 kernel does not support this shape");
-        return launch_dense_decode_sm100(*a);
+        return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_sm100(*a);
     }
-    if (a->impl == 0 && dense_decode_sm100_supports(*a)) return launch_dense_decode_sm100(*a);
+    if (a->impl == 0 && dense_decode_sm100_supports(*a)) return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_sm100(*a);
     if (a->dtype != MLA_DTYPE_BF16)
         return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: fp16 is served by the tcgen05 kernel only, which does not support this shape");
     return launch_dense_decode_portable(*a);
@@ -170,14 +175,13 @@ int mla_sparse_decode_fwd(const mla_sparse_decode_args_t* a) {
     } else {
         MLA_CHECK_ARG(!a->extra_indices && !a->extra_topk_length, "mla_sparse_decode_fwd: extra_indices / extra_topk_length need extra_kv");
     }
+    const bool rows64 = a->h_q <= ROWS64;
     if (a->impl == 2) {
         if (!sparse_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_decode_fwd: the tcgen05 kernel does not support this shape");
-        return launch_sparse_decode_sm100(*a);
+        return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_sm100(*a);
     }
-    // (also with few heads: the work is dominated by gathering and de-quantising the records, which the tcgen05
-    // kernel does 2x faster than the portable one even when most of its 128 rows are padding)
-    if (a->impl == 0 && sparse_decode_sm100_supports(*a)) return launch_sparse_decode_sm100(*a);
+    if (a->impl == 0 && sparse_decode_sm100_supports(*a)) return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_sm100(*a);
     return launch_sparse_decode_portable(*a);
 }
 
@@ -192,12 +196,13 @@ int mla_sparse_prefill_fwd(const mla_sparse_prefill_args_t* a) {
     MLA_CHECK_ARG(is_aligned16(a->kv) && a->kv_stride_s % 8 == 0,
                   "mla_sparse_prefill_fwd: kv must be 16-byte aligned with a row stride that is a multiple of 8 elements");
     MLA_CHECK_ARG(is_aligned16(a->out), "mla_sparse_prefill_fwd: out must be 16-byte aligned");
+    const bool rows64 = a->h_q <= ROWS64;
     if (a->impl == 2) {
         if (!sparse_prefill_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_prefill_fwd: the tcgen05 kernel does not support this shape");
-        return launch_sparse_prefill_sm100(*a);
+        return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_sm100(*a);
     }
-    if (a->impl == 0 && sparse_prefill_sm100_supports(*a)) return launch_sparse_prefill_sm100(*a);
+    if (a->impl == 0 && sparse_prefill_sm100_supports(*a)) return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_sm100(*a);
     return launch_sparse_prefill_portable(*a);
 }
 

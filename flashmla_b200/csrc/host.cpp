@@ -145,7 +145,7 @@ const at::Tensor& status(const at::Device& device) {
 }
 
 // ---- pieces shared by the decode calls ----------------------------------------------------------------------------
-struct Sched { at::Tensor meta, num_splits; bool made = false; };
+struct Sched { at::Tensor meta, num_splits; int parts = 0; bool made = false; };
 
 void check_sched(const Sched& s, int num_sm_parts, int64_t b, const at::Device& device) {
     require(s.meta.scalar_type() == at::kInt && s.num_splits.scalar_type() == at::kInt,
@@ -164,15 +164,19 @@ void check_sched(const Sched& s, int num_sm_parts, int64_t b, const at::Device& 
     require_cuda("num_splits", s.num_splits, &device);
 }
 
-// The stored schedule, or a new one.
-Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, const at::Device& device) {
+// The stored schedule, or a new one.  A stored one may also have `pair_parts` partitions: a schedule made when every shape ran
+// on pairs of SMs stays usable (the kernels take any number of partitions).
+Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, int pair_parts, const at::Device& device) {
     Sched s;
     if (meta != Py_None) {
         s.meta = tensor(meta, "tile_scheduler_metadata");
         s.num_splits = tensor(num_splits, "num_splits");
+        if (has_shape(s.meta, {pair_parts, META_INTS})) a.num_sm_parts = pair_parts;
         check_sched(s, a.num_sm_parts, a.b, device);
+        s.parts = a.num_sm_parts;
         return s;
     }
+    s.parts = a.num_sm_parts;
     s.made = true;
     s.meta = empty({a.num_sm_parts, META_INTS}, at::kInt, device);
     s.num_splits = empty({a.b + 1}, at::kInt, device);
@@ -249,12 +253,14 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
     const c10::cuda::CUDAGuard guard(device);
     void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
-    const int parts = api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_q, (int)h_kv, (int)s_q);
-    if (parts <= 0) check(1, "mla_num_sm_parts");
     mla_sched_meta_args_t sa = {};
     sa.b = (int32_t)b; sa.s_q = (int32_t)s_q; sa.topk = -1;
-    sa.seqlens_k = ptr<int32_t>(seqlens); sa.num_sm_parts = parts; sa.stream = stream;
-    const Sched sched = schedule(args[7], args[8], sa, device);
+    sa.num_sm_parts = api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_q, (int)h_kv, (int)s_q);
+    if (sa.num_sm_parts <= 0) check(1, "mla_num_sm_parts");
+    sa.seqlens_k = ptr<int32_t>(seqlens); sa.stream = stream;
+    const int pair_parts = s_q * (h_q / h_kv) <= 64 ? api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_kv * 128, (int)h_kv, 1) : sa.num_sm_parts;
+    const Sched sched = schedule(args[7], args[8], sa, pair_parts, device);
+    const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);
     const at::Tensor lse = empty({b, h_q, s_q}, at::kFloat, device);
@@ -356,20 +362,20 @@ PyObject* sparse_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const c10::cuda::CUDAGuard guard(device);
     void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     const bool uniform = !topk_length && !extra_topk_length;
-    int parts;
-    if (uniform) {
+    const auto count_parts = [&](int64_t heads) {
         // every request costs the same number of KV blocks: let the partition count follow the batch size
         const int64_t blocks = (topk + 63) / 64 + (extra_topk + 63) / 64;
-        parts = api.num_sm_parts_uniform(device.index(), MLA_MODE_SPARSE_DECODE, (int)h_q, 1, (int)s_q, (int)b, (int)blocks);
-    } else {
-        parts = api.num_sm_parts(device.index(), MLA_MODE_SPARSE_DECODE, (int)h_q, 1, (int)s_q);
-    }
-    if (parts <= 0) check(1, "mla_num_sm_parts");
+        const int n = uniform ? api.num_sm_parts_uniform(device.index(), MLA_MODE_SPARSE_DECODE, (int)heads, 1, (int)s_q, (int)b, (int)blocks)
+                              : api.num_sm_parts(device.index(), MLA_MODE_SPARSE_DECODE, (int)heads, 1, (int)s_q);
+        if (n <= 0) check(1, "mla_num_sm_parts");
+        return n;
+    };
     mla_sched_meta_args_t sa = {};
     sa.b = (int32_t)b; sa.s_q = (int32_t)s_q; sa.topk = (int32_t)topk; sa.extra_topk = (int32_t)extra_topk;
     sa.topk_length = ptr<int32_t>(topk_length); sa.extra_topk_length = ptr<int32_t>(extra_topk_length);
-    sa.num_sm_parts = parts; sa.stream = stream;
-    const Sched sched = schedule(args[5], args[6], sa, device);
+    sa.num_sm_parts = count_parts(h_q); sa.stream = stream;
+    const Sched sched = schedule(args[5], args[6], sa, h_q <= 64 ? count_parts(128) : sa.num_sm_parts, device);
+    const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);
     const at::Tensor lse = empty({b, s_q, h_q}, at::kFloat, device);

@@ -243,14 +243,14 @@ int mla_sparse_prefill_fwd(const mla_sparse_prefill_args_t* args);
  * decode loop runs on a memory plan fixed at start-up, where a cudaMalloc would stall the device or fail;
  * host runtimes that bind this ABI without a device allocator).  Same arguments as mla_dense_decode_fwd, but
  * args->lse_accum and args->o_accum are ignored: the split-KV scratch is a fixed array inside the library,
- * about 64 MiB per GPU that loads it, held until the process exits (enough for batch 128 with 128 heads on a 148-SM part:
+ * about 73 MiB per GPU that loads it, held until the process exits (enough for batch 128 with 128 heads on a 148-SM part:
  * (128 + 74) * 128 = 25856 rows).  Limit: (b + num_sm_parts) * s_q * h_q
  * must not exceed MLA_NOALLOC_MAX_ROWS, otherwise MLA_ERR_INVALID_ARG is returned.  The first call on each
  * device looks up the array's device address (make that call with the device current and before any stream
  * capture).  All calls on a GPU share the array: calls that may overlap on the GPU race and must be
  * serialised by the caller.  Nothing in the array needs clearing between calls.  Calls no allocation routine.
  * This entry point has no counterpart in the reference. */
-#define MLA_NOALLOC_MAX_ROWS 32768
+#define MLA_NOALLOC_MAX_ROWS 37504
 int mla_dense_decode_noalloc(const mla_dense_decode_args_t* args);
 
 /* FP8 KV-cache writer (the step before sparse decode): bf16 token rows -> 656-byte records.  Replaces the torch
