@@ -67,6 +67,16 @@ using namespace mla;
 // of this line): O^T of more rows and the scores do not fit its tensor memory, Q and a tile not its shared memory.
 constexpr int ROWS64 = 64;
 
+// Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens (one per SM, or one per pair) takes
+// 9 : 5 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 330, 444 tokens: 56 / 81, 98 / 82,
+// 141 / 159, 189 / 158, 230 / 234, 283 / 235; with 512 keys 24 / 28, 37 / 29, 51 / 52, 66 / 53, 79 / 76, 93 / 77.
+static bool prefill_rows64(const mla_sparse_prefill_args_t& a) {
+    const int sms = current_device_num_sms();
+    if (a.h_q > ROWS64 || sms < 2) return false;
+    const int64_t waves = (a.s_q + sms - 1) / sms, pair_waves = (a.s_q + sms / 2 - 1) / (sms / 2);
+    return 9 * waves <= 5 * pair_waves;
+}
+
 extern "C" {
 
 const char* mla_last_error(void) { return last_error_buffer(); }
@@ -196,7 +206,7 @@ int mla_sparse_prefill_fwd(const mla_sparse_prefill_args_t* a) {
     MLA_CHECK_ARG(is_aligned16(a->kv) && a->kv_stride_s % 8 == 0,
                   "mla_sparse_prefill_fwd: kv must be 16-byte aligned with a row stride that is a multiple of 8 elements");
     MLA_CHECK_ARG(is_aligned16(a->out), "mla_sparse_prefill_fwd: out must be 16-byte aligned");
-    const bool rows64 = a->h_q <= ROWS64;
+    const bool rows64 = prefill_rows64(*a);
     if (a->impl == 2) {
         if (!sparse_prefill_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_prefill_fwd: the tcgen05 kernel does not support this shape");
