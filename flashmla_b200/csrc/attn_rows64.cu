@@ -16,6 +16,8 @@
 // Order of the MMAs: Q K^T over the pairs as they arrive, then P V block by block; block m reads pair m only, so the next
 // tile's pairs move in while P V still runs.
 //
+// Where the ring holds more than a tile (dense, up to 32 rows), the next tile's first pair is multiplied during the softmax.
+//
 // Softmax: warps 4..11, a thread = one token (tensor-memory lane) and NH / 2 rows (columns).  A row's running maximum is shared
 // by all threads and only has to bound the scores: it moves when a score exceeds it by 2^6 (always on a request's first
 // tile), which is what the threads vote on once per tile; P, the row sums and O always refer to the same maximum, so results
@@ -73,8 +75,9 @@ struct Lay {
     static constexpr int Q_CHUNK = NH * 128;
     // 64 rows of 576: Q, four pairs, RoPE and P together are 5 KB more than there is.  P moves into the RoPE slot, which Q K^T has
     // read by then (the next tile's RoPE chunk waits for P V, like its last pair).
-    static constexpr bool P_IN_ROPE = NH == 64 && WIDE;
-    static constexpr int NP = NH == 16 ? 5 : 4;
+    // (With 32 rows the same buys a fifth pair.)
+    static constexpr bool P_IN_ROPE = NH >= 32 && WIDE;
+    static constexpr int NP = NH <= 32 ? 5 : 4;
     static constexpr int Q = 0;
     static constexpr int RING = Q + CHUNKS * Q_CHUNK;
     static constexpr int ROPE = RING + NP * PAIR_BYTES;
@@ -83,7 +86,7 @@ struct Lay {
     static_assert(RING % 1024 == 0, "swizzle atoms");
 };
 constexpr int DATA_BYTES = Lay<64, true>::END > Lay<16, true>::END ? Lay<64, true>::END : Lay<16, true>::END;
-static_assert(Lay<32, true>::END <= DATA_BYTES && Lay<64, false>::END <= DATA_BYTES, "shared memory plan");
+static_assert(Lay<32, true>::END <= DATA_BYTES && Lay<32, false>::END <= DATA_BYTES && Lay<64, false>::END <= DATA_BYTES, "shared memory plan");
 
 struct Smem {
     uint8_t data[DATA_BYTES];
@@ -151,7 +154,8 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
     using W = Warps<MODE>;
     using WalkerT = Walker<MODE>;
     constexpr int NP = L::NP, HC = NH / 2;
-    constexpr uint32_t TM_O = 0, TM_S = 4 * NH;
+    constexpr bool EARLY = DENSE && NP > 4;                // Q K^T of the next tile begins before P V of this one
+    constexpr uint32_t TM_O = 0, TM_S = 4 * NH;            // tensor memory: O^T, S^T (EARLY: of two tiles)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -277,26 +281,32 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
             const uint32_t q_lo = sw128_desc_lo(smem_addr(sm.data + L::Q), 16), p_lo = sw128_desc_lo(smem_addr(sm.data + L::P), 1024);
             RingPos<NP> ring;
             uint32_t g = 0, nq = 0;
+            // Q K^T over pair q of a tile, which is in `slot`
+            auto scores_of_pair = [&](uint32_t d_tmem, int q, uint32_t slot) {
+                if (!DENSE) fence_proxy_async_smem();      // the feeding warps' stores and copies -> visible to the tensor core
+                tc_fence_after();
+                const uint32_t a_lo = ring_k + slot * (PAIR_BYTES >> 4), b_lo = q_lo + q * (2 * L::Q_CHUNK >> 4);
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        mma_ss_lohi(d_tmem, a_lo + c * (1024 >> 4) + k4 * 2, hi_pair, b_lo + c * (L::Q_CHUNK >> 4) + k4 * 2, hi_row,
+                                    idesc_s, (q | c | k4) ? 1u : 0u);
+            };
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
                 const Work w = wk.get();
                 if (w.ntiles == 0) continue;
                 WAIT_OR_LEAVE(wt, false, &sm.q_full, nq & 1, 3);
                 ++nq;
+                bool begun = false;                        // the tile's first pair has been done already
                 for (int i = 0; i < w.ntiles; ++i, ++g) {
+                    const uint32_t s_tmem = tmem + TM_S + (EARLY ? (g & 1) * NH : 0);
                     RingPos<NP> pv = ring;
-                    // (S is free: the softmax warps read the previous tile's before they arrived on p_full)
+                    if (begun) ring.next();
 #pragma unroll 1
-                    for (int q = 0; q < 4; ++q, ring.next()) {
+                    for (int q = begun ? 1 : 0; q < 4; ++q, ring.next()) {
                         WAIT_OR_LEAVE(wt, false, &sm.k_full[ring.slot], ring.par, 4);
-                        if (!DENSE) fence_proxy_async_smem();      // the feeding warps' stores and copies -> visible to the tensor core
-                        tc_fence_after();
-                        const uint32_t a_lo = ring_k + ring.slot * (PAIR_BYTES >> 4), b_lo = q_lo + q * (2 * L::Q_CHUNK >> 4);
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-#pragma unroll
-                            for (int k4 = 0; k4 < 4; ++k4)
-                                mma_ss_lohi(tmem + TM_S, a_lo + c * (1024 >> 4) + k4 * 2, hi_pair, b_lo + c * (L::Q_CHUNK >> 4) + k4 * 2, hi_row,
-                                            idesc_s, (q | c | k4) ? 1u : 0u);
+                        scores_of_pair(s_tmem, q, ring.slot);
                     }
                     if (WIDE) {
                         WAIT_OR_LEAVE(wt, false, &sm.r_full, g & 1, 5);
@@ -304,11 +314,14 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                         tc_fence_after();
 #pragma unroll
                         for (int k4 = 0; k4 < 4; ++k4)
-                            mma_ss_lohi(tmem + TM_S, rope_lo + k4 * 2, hi_row, q_lo + 8 * (L::Q_CHUNK >> 4) + k4 * 2, hi_row, idesc_s, 1u);
+                            mma_ss_lohi(s_tmem, rope_lo + k4 * 2, hi_row, q_lo + 8 * (L::Q_CHUNK >> 4) + k4 * 2, hi_row, idesc_s, 1u);
                         if (!L::P_IN_ROPE) tc_commit(smem_addr(&sm.r_empty));
                     }
                     if (i + 1 == w.ntiles) tc_commit(smem_addr(&sm.q_empty));
                     tc_commit(smem_addr(&sm.s_full));
+                    // While the softmax runs: the next tile's first pair, where the ring holds one more than a tile and it is there.
+                    begun = EARLY && i + 1 < w.ntiles && mbar_try_wait(smem_addr(&sm.k_full[ring.slot]), ring.par);
+                    if (begun) scores_of_pair(tmem + TM_S + ((g + 1) & 1) * NH, 0, ring.slot);
                     WAIT_OR_LEAVE(wt, false, &sm.p_full, g & 1, 6);
                     tc_fence_after();
 #pragma unroll 1
@@ -521,7 +534,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                 // Scores of CW rows at a time, -inf where masked.  Dense mode keeps all of them in registers; the gather modes, whose
                 // registers hold the sums and little else, read tensor memory again for every pass.
                 auto scores = [&](int c0, uint32_t (&s)[CW]) {
-                    tmem_ld(tlane + TM_S + col0 + c0, s);
+                    tmem_ld(tlane + TM_S + (EARLY ? (g & 1) * NH : 0) + col0 + c0, s);
                     tmem_wait_ld();
                     if (!ok) {
 #pragma unroll
@@ -684,7 +697,10 @@ each([&](int c0, uint32_t (&s)[CW]) {
                 }
             }
             named_bar_sync(1, 256);
-            constexpr int WC = NH < 32 ? NH : 32;
+            // (Short loops: a kernel runs this once or twice, and the time of an unrolled body is that of fetching its instructions.
+            // Prefill with rows 16 at a time 306 us, 32 at a time 314 (512 x 2048).  Partials of 64 rows, 128 KB a CTA, are
+            // bound by the stores: 32 at a time 78 us, 16 at a time 80 (dense, 61 x 4096).)
+            constexpr int WC = PREFILL || NH < 32 || (DENSE && NH == 32) ? 16 : 32;
 #pragma unroll 1
             for (int c0 = 0; c0 < 2 * NH; c0 += WC) {                 // this half's two blocks of dims, WC rows at a time
                 const int d = (2 * half + c0 / NH) * 128 + tok, r0 = c0 % NH;
