@@ -3,24 +3,27 @@
 // (tests/quant.py:20-53 of the reference: scale = amax / 448 per group of 128, optionally rounded up to a power of
 // two; q = e4m3(x / scale), round to nearest even).
 //
-// A warp takes two tokens, whose loads are in flight together; lane l holds values 16l .. 16l+15 of a token (8 lanes per
-// scale group), so the record's e4m3 part is one coalesced 512-byte store.  1152 bytes read + 656 bytes written per token.
-// With one IEEE division per value (__fdiv_rn, a dozen instructions and a branch) 66 K tokens took 34 us (3.5 TB/s).  The
-// quotients x / s only need the correctly rounded reciprocal of s, once per group, and three instructions each (Markstein's
-// theorem; quotient16 below): 28.7 us (4.2 TB/s).  What bounds it is still the instructions, not memory.
+// A warp takes a token; lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is one coalesced
+// 512-byte store.  1152 bytes read + 656 bytes written per token.  The quotients x / s only need the correctly rounded reciprocal
+// of s, once per group, and three instructions each (Markstein's theorem; quotient16 below), two values per instruction.  66 K
+// tokens take 23.3 us (5.1 TB/s), 256 K 87 us (5.3 TB/s).  Registers count: with two tokens per warp (75 of them in the place of 47)
+// 26.6 and 96.7 us; with the scalar instructions, two / one token per warp, 27.3 / 26.8 and 98.2 / 99.2.  A persistent grid that
+// loads a token ahead is no faster (27.3).
 //
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
 // block_size x 8 scale bytes (7 scales + 1 pad).  Lanes 0-27 hold the quantised values (4 lanes per group), lanes 28-31
-// the RoPE part.  The first warps also zero the `pad_bytes` behind every block, where the caller owns them (one warp a
-// block; with the last token's stores, inside the loop, 66 K tokens took 36.9 us instead of 34.9).
+// the RoPE part.  A warp takes two tokens here, whose loads are in flight together, with registers for four blocks per SM: 66 K
+// tokens 27.2 us, 256 K 92.9 (one token per warp 27.2 and 101, scalar instructions 35.5 and 131.7).  The first warps also zero
+// the `pad_bytes` behind every block, where the caller owns them (one warp a block; with the last token's stores, inside the
+// loop, 66 K tokens took 36.9 us instead of 34.9, on the scalar kernel).
 #include "common.cuh"
 
 #include <cuda_fp8.h>
 
 namespace mla {
 
-constexpr int TOKENS = 2;             // per warp, in flight together
+constexpr int TOKENS = 2;             // layout 1: tokens per warp, in flight together
 
 __device__ __forceinline__ float pow2_ceil(float s) {
     // smallest power of two >= s (s > 0, normal)
@@ -29,18 +32,33 @@ __device__ __forceinline__ float pow2_ceil(float s) {
     return __uint_as_float((bits & 0x7f800000u) + (mant ? 0x00800000u : 0u));
 }
 
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+// A lane's 16 values, NEGATED (what the quotients below start from), and their largest magnitude.
 __device__ __forceinline__ void unpack16(const uint4& v0, const uint4& v1, float (&f)[16], float& amax) {
     const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        f[2 * i] = __uint_as_float(w[i] << 16 ^ 0x80000000u);
+        f[2 * i + 1] = __uint_as_float((w[i] & 0xffff0000u) ^ 0x80000000u);
         amax = fmaxf(amax, fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1])));
     }
 }
 
-// e4m3(x / s) of a lane's 16 values, x / s rounded to fp32 first.  With r = RN(1 / s) and q = RN(x r), q + r (x - q s)
+// e4m3(x / s) of a lane's 16 values (f holds -x), x / s rounded to fp32 first.  With r = RN(1 / s) and q = RN(x r), q + r (x - q s)
 // is RN(x / s) (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34, 1990; here checked for every bf16 significand against every fp32 significand of s).  It is computed as
 // q + (-r) (q s - x): for x = -0 the remainder q s - x is -0 + 0 = +0 and the sum -0 + -0 keeps the sign, where
@@ -52,14 +70,15 @@ __device__ __forceinline__ uint4 quotient16(const float (&f)[16], float s, float
     const bool plain = (amax >= 0x1p-60f && amax <= 0x1p100f) || amax == 0.f;
     uint32_t q[4];
     if (__all_sync(0xffffffffu, plain)) {
-        const float r = __frcp_rn(s);
+        const float r = -__frcp_rn(s);
+        const float2 r2 = make_float2(r, r), s2 = make_float2(s, s);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             float2 d[2];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float x = f[4 * i + k], q0 = x * r;
-                reinterpret_cast<float*>(d)[k] = fmaf(fmaf(q0, s, -x), -r, q0);
+            for (int k = 0; k < 2; ++k) {
+                const float2 nx = make_float2(f[4 * i + 2 * k], f[4 * i + 2 * k + 1]), q0 = mul2(nx, r2);
+                d[k] = fma2(fma2(q0, s2, nx), r2, q0);
             }
             q[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(d[0], __NV_SATFINITE, __NV_E4M3) |
                    (uint32_t)__nv_cvt_float2_to_fp8x2(d[1], __NV_SATFINITE, __NV_E4M3) << 16;
@@ -70,7 +89,7 @@ __device__ __forceinline__ uint4 quotient16(const float (&f)[16], float s, float
             uint32_t word = 0;
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                if (k >> 2 == i) word |= (uint32_t)__nv_cvt_float_to_fp8(__fdiv_rn(f[k], s), __NV_SATFINITE, __NV_E4M3) << (8 * (k & 3));
+                if (k >> 2 == i) word |= (uint32_t)__nv_cvt_float_to_fp8(__fdiv_rn(-f[k], s), __NV_SATFINITE, __NV_E4M3) << (8 * (k & 3));
             if (i == 0) q[0] = word; else if (i == 1) q[1] = word; else if (i == 2) q[2] = word; else q[3] = word;
         }
     }
@@ -89,39 +108,30 @@ quantize_fp8_kernel(const mla_quantize_args_t a) {
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    for (int64_t tok0 = warp * TOKENS; tok0 < ntok; tok0 += nwarps * TOKENS) {
-        uint4 v0[TOKENS], v1[TOKENS], rope[TOKENS];
-        uint8_t* out[TOKENS];
-#pragma unroll
-        for (int k = 0; k < TOKENS; ++k) {
-            if (tok0 + k >= ntok) break;
-            int64_t blk, row;
-            block_of(tok0 + k, ntok, a.block_size, blk, row);
-            const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk * a.x_stride_block + row * a.x_stride_row;
-            out[k] = (uint8_t*)a.out + blk * a.out_stride_block_bytes + row * 656;
-            v0[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16));
-            v1[k] = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
-            if (lane < 8) rope[k] = __ldcs(reinterpret_cast<const uint4*>(x + 512 + lane * 8));
-        }
-#pragma unroll
-        for (int k = 0; k < TOKENS; ++k) {
-            if (tok0 + k >= ntok) break;
-            float f[16], amax;
-            unpack16(v0[k], v1[k], f, amax);
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-            float s = __fdiv_rn(amax, 448.f);
-            s = a.pow2_scale ? pow2_ceil(fmaxf(s, 1e-4f)) : fmaxf(s, 1e-30f);
-            *reinterpret_cast<uint4*>(out[k] + lane * 16) = quotient16(f, s, amax);
-            const float sg = __shfl_sync(0xffffffffu, s, (lane & 3) * 8);          // lanes 0-3: scale of group `lane`
-            if (lane < 4) reinterpret_cast<float*>(out[k] + 512)[lane] = sg;
-            if (lane < 8) *reinterpret_cast<uint4*>(out[k] + 528 + lane * 16) = rope[k];
-        }
+    for (int64_t tok = warp; tok < ntok; tok += nwarps) {
+        int64_t blk, row;
+        block_of(tok, ntok, a.block_size, blk, row);
+        const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + blk * a.x_stride_block + row * a.x_stride_row;
+        uint8_t* out = (uint8_t*)a.out + blk * a.out_stride_block_bytes + row * 656;
+        const uint4 v0 = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16));
+        const uint4 v1 = __ldcs(reinterpret_cast<const uint4*>(x + lane * 16 + 8));
+        uint4 rope;
+        if (lane < 8) rope = __ldcs(reinterpret_cast<const uint4*>(x + 512 + lane * 8));
+        float f[16], amax;
+        unpack16(v0, v1, f, amax);
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+        float s = __fdiv_rn(amax, 448.f);
+        s = a.pow2_scale ? pow2_ceil(fmaxf(s, 1e-4f)) : fmaxf(s, 1e-30f);
+        *reinterpret_cast<uint4*>(out + lane * 16) = quotient16(f, s, amax);
+        const float sg = __shfl_sync(0xffffffffu, s, (lane & 3) * 8);          // lanes 0-3: scale of group `lane`
+        if (lane < 4) reinterpret_cast<float*>(out + 512)[lane] = sg;
+        if (lane < 8) *reinterpret_cast<uint4*>(out + 528 + lane * 16) = rope;
     }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 quantize_fp8_model1_kernel(const mla_quantize_args_t a, const int pad_bytes) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -181,7 +191,8 @@ int launch_quantize_fp8(const mla_quantize_args_t& a, bool zero_padding) {
     const int64_t pad_bytes = zero_padding && a.layout ? a.out_stride_block_bytes - (int64_t)a.block_size * rec : 0;
     MLA_CHECK_ARG(pad_bytes <= 0x7fffff00, "mla_quantize_fp8_kvcache_padded: more than 2 GB of padding behind a block");
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    const int64_t blocks = min((ntok + 8 * TOKENS - 1) / (8 * TOKENS), (int64_t)1 << 24);
+    const int per_block = a.layout ? 8 * TOKENS : 8;             // tokens
+    const int64_t blocks = min((ntok + per_block - 1) / per_block, (int64_t)1 << 24);
     if (a.layout) quantize_fp8_model1_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
     else quantize_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
     MLA_CHECK_CUDA(cudaGetLastError());
