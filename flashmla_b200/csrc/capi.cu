@@ -68,13 +68,14 @@ using namespace mla;
 constexpr int ROWS64 = 64;
 
 // Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens (one per SM, or one per pair) takes
-// 9 : 5 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 330, 444 tokens: 56 / 81, 98 / 82,
-// 141 / 159, 189 / 158, 230 / 234, 283 / 235; with 512 keys 24 / 28, 37 / 29, 51 / 52, 66 / 53, 79 / 76, 93 / 77.
+// about 5 : 3 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 330, 444, 512 tokens: 56 / 81,
+// 98 / 82, 141 / 159, 189 / 158, 230 / 234, 283 / 235, 336 / 314; with 512 keys, up to 444 tokens: 24 / 28, 37 / 29, 51 / 52,
+// 66 / 53, 79 / 76, 93 / 77.
 static bool prefill_rows64(const mla_sparse_prefill_args_t& a) {
     const int sms = current_device_num_sms();
     if (a.h_q > ROWS64 || sms < 2) return false;
     const int64_t waves = (a.s_q + sms - 1) / sms, pair_waves = (a.s_q + sms / 2 - 1) / (sms / 2);
-    return 9 * waves <= 5 * pair_waves;
+    return 5 * waves <= 3 * pair_waves;
 }
 
 extern "C" {
