@@ -24,15 +24,17 @@
 // are exact up to rounding.  Sums stay per thread until the end of a request.
 //
 // What bounds it: one tile is in flight, so a tile's period is the chain  fill -> Q K^T (36 MMAs) -> softmax -> P V (32 MMAs); an
-// MMA of 128 x NH x 16 takes 56 SM cycles for every NH up to 64.  Dense decode with 16 / 64 rows: 5800 / 6600 cycles a tile, the
+// MMA of 128 x NH x 16 takes 56 SM cycles for every NH up to 64.  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
 // fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
 // Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
 // and its loads 4500-6000 of them.  us a call, before (pairs of SMs for every shape) and now, back to back in short runs:
-//   dense, 4 requests of 64..512, 16 heads     18.7 ->  13.9    dense fp16, 61 x 4096, 16 heads     77   ->  63.5
-//   dense, 30 x 2048, 8 heads                  32.8 ->  24.5    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 72.3 / 77.7
+//   dense, 4 requests of 64..512, 16 heads     18.7 ->  13.9    dense fp16, 61 x 4096, 16 heads     77   ->  63.4
+//   dense, 30 x 2048, 8 heads                  32.8 ->  23.7    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 68.7 / 78.0
 //   FP8, 64 x 2048, 16 heads                   93.3 ->  54.7    FP8, 74 x 2048, 64 heads            95.9 ->  82.2
-//   FP8, 2 x 2 x 2048, 64 heads                27.2 ->  23.3    prefill 512-wide, 117 tokens, ragged 42.3 ->  32.2
-//   prefill, 512 x 2048, 64 heads               333 ->   312    prefill, 2000 x 1024, 64 heads       677 ->   584
+//   FP8, 2 x 2 x 2048, 64 heads                27.2 ->  23.3    prefill 512-wide, 117 tokens, ragged 42.3 ->  31.0
+//   prefill, 512 x 2048, 64 heads               333 ->   308    prefill, 2000 x 1024, 64 heads       677 ->   564
+// (The shortest dense requests with 64 heads lose: 15 of about 68 tokens 15.8 -> 17.1, since twice the partitions split requests of
+// two blocks; with 100 tokens and more they gain.)
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert
 // every record.
 //
@@ -698,8 +700,8 @@ each([&](int c0, uint32_t (&s)[CW]) {
             }
             named_bar_sync(1, 256);
             // (Short loops: a kernel runs this once or twice, and the time of an unrolled body is that of fetching its instructions.
-            // Prefill with rows 16 at a time 306 us, 32 at a time 314 (512 x 2048).  Partials of 64 rows, 128 KB a CTA, are
-            // bound by the stores: 32 at a time 78 us, 16 at a time 80 (dense, 61 x 4096).)
+            // Prefill, 700 x 640 keys, 512-wide: 142.3 us with 32 rows at a time and a branch per two rows, 136.5 with 16 and none.
+            // Partials of 64 rows, 128 KB a CTA, are bound by the stores: FP8, 74 x 2048: 81.4 us with 32, 83 with 16.)
             constexpr int WC = PREFILL || NH < 32 || (DENSE && NH == 32) ? 16 : 32;
 #pragma unroll 1
             for (int c0 = 0; c0 < 2 * NH; c0 += WC) {                 // this half's two blocks of dims, WC rows at a time
@@ -718,16 +720,14 @@ each([&](int c0, uint32_t (&s)[CW]) {
                     // two rows at a time: the even lane of a pair takes both dims of the first row, the odd lane those of the second
 #pragma unroll
                     for (int c = 0; c < WC; c += 2) {
-                        if (r0 + c < rows) {
-                            const float f0 = sm.inv[r0 + c], f1 = sm.inv[min(r0 + c + 1, rows - 1)];
-                            const float x0 = f0 < 0.f ? 0.f : __uint_as_float(v[c]) * f0, x1 = f1 < 0.f ? 0.f : __uint_as_float(v[c + 1]) * f1;
-                            const bool odd = lane & 1;
-                            const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
-                            const int r = r0 + c + odd;
-                            if (r < rows)
-                                *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(sm.optr[r]) + (d & ~1)) =
-                                    odd ? pack16<FP16>(other, x1) : pack16<FP16>(x0, other);
-                        }
+                        const float f0 = sm.inv[r0 + c], f1 = sm.inv[r0 + c + 1];
+                        const float x0 = f0 < 0.f ? 0.f : __uint_as_float(v[c]) * f0, x1 = f1 < 0.f ? 0.f : __uint_as_float(v[c + 1]) * f1;
+                        const bool odd = lane & 1;
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+                        const int r = r0 + c + odd;
+                        if (r < rows)
+                            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(sm.optr[r]) + (d & ~1)) =
+                                odd ? pack16<FP16>(other, x1) : pack16<FP16>(x0, other);
                     }
                 }
             }
