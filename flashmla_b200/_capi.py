@@ -16,7 +16,7 @@ MLA_MODE_DENSE_DECODE = 0
 MLA_MODE_SPARSE_DECODE = 1
 
 IMPL_AUTO, IMPL_PORTABLE, IMPL_TCGEN05 = 0, 1, 2
-NOALLOC_MAX_ROWS = 37504
+NOALLOC_MAX_ROWS = 38720
 MLA_DTYPE_BF16, MLA_DTYPE_FP16 = 0, 1
 ABI_VERSION = 2
 

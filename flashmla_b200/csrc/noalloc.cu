@@ -6,7 +6,7 @@
 // owning a device allocator at all.  For them the split-KV scratch that mla_dense_decode_fwd expects from
 // the caller lives here, in a fixed array inside the library image.
 //
-// Cost and limits: every GPU that loads the library keeps MLA_NOALLOC_MAX_ROWS * 513 floats (about 73 MiB)
+// Cost and limits: every GPU that loads the library keeps MLA_NOALLOC_MAX_ROWS * 513 floats (about 76 MiB)
 // resident until the process exits.  The array is shared by all calls on a device and keeps the previous
 // call's contents; no part of it has to start at zero (each split slot a request uses is written in full
 // before the combine step reads it), so nothing is cleared.  Two calls whose kernels can overlap on the

@@ -243,14 +243,16 @@ int mla_sparse_prefill_fwd(const mla_sparse_prefill_args_t* args);
  * decode loop runs on a memory plan fixed at start-up, where a cudaMalloc would stall the device or fail;
  * host runtimes that bind this ABI without a device allocator).  Same arguments as mla_dense_decode_fwd, but
  * args->lse_accum and args->o_accum are ignored: the split-KV scratch is a fixed array inside the library,
- * about 73 MiB per GPU that loads it, held until the process exits (enough for batch 128 with 128 heads on a 148-SM part:
+ * about 76 MiB per GPU that loads it, held until the process exits (enough for batch 128 with 128 heads on a 148-SM part:
  * (128 + 74) * 128 = 25856 rows).  Limit: (b + num_sm_parts) * s_q * h_q
  * must not exceed MLA_NOALLOC_MAX_ROWS, otherwise MLA_ERR_INVALID_ARG is returned.  The first call on each
  * device looks up the array's device address (make that call with the device current and before any stream
  * capture).  All calls on a GPU share the array: calls that may overlap on the GPU race and must be
  * serialised by the caller.  Nothing in the array needs clearing between calls.  Calls no allocation routine.
+ * (32768 rows with a partition per pair of SMs; with one per SM, up to 64 query rows per kv head, the same batches need up to
+ * 38688 on 148 SMs: 48 kv heads of 62 rows, whose division of the SMs rounds from 1 to 3 partitions.)
  * This entry point has no counterpart in the reference. */
-#define MLA_NOALLOC_MAX_ROWS 37504
+#define MLA_NOALLOC_MAX_ROWS 38720
 int mla_dense_decode_noalloc(const mla_dense_decode_args_t* args);
 
 /* FP8 KV-cache writer (the step before sparse decode): bf16 token rows -> 656-byte records.  Replaces the torch

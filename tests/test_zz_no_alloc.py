@@ -14,27 +14,27 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-def _run_pair(b, s_q, h_q, seqlens, seed, check_oracle=False):
+def _run_pair(b, s_q, h_q, seqlens, seed, check_oracle=False, h_kv=1):
     import flashmla_b200 as fm
     from flashmla_b200 import _capi
     from tests import workloads as W
     from flashmla_b200.flash_mla_interface import _make_sched_meta
     lib = _capi.lib()
     seq = torch.tensor(seqlens, dtype=torch.int32)
-    d = W.dense_decode_inputs(seq, s_q, h_q, 1, seed=seed, device=DEV, poison_unused=True)
+    d = W.dense_decode_inputs(seq, s_q, h_q, h_kv, seed=seed, device=DEV, poison_unused=True)
     q, kc, bt, sl = d["q"], d["blocked_k"], d["block_table"], d["cache_seqlens"]
     # regular path through the public API (caller-side scratch)
     meta = fm.get_mla_metadata()[0]
     ref_out, ref_lse = fm.flash_mla_with_kvcache(q, kc, bt, sl, 512, meta, None, causal=True)
     # allocation-free path through the C ABI: outputs, metadata and status words are passed in, scratch is not
-    P = lib.mla_num_sm_parts(0, _capi.MLA_MODE_DENSE_DECODE, h_q, 1, s_q)
+    P = lib.mla_num_sm_parts(0, _capi.MLA_MODE_DENSE_DECODE, h_q, h_kv, s_q)
     assert (b + P) * s_q * h_q <= _capi.NOALLOC_MAX_ROWS
     sched, num_splits = _make_sched_meta(b, s_q, P, torch.device(DEV), seqlens_k=sl)
     out = torch.full((b, s_q, h_q, 512), float("nan"), dtype=torch.bfloat16, device=DEV)
     lse = torch.full((b, h_q, s_q), float("nan"), dtype=torch.float32, device=DEV)
     status = torch.zeros(4, dtype=torch.int32, device=DEV)
     a = _capi.DenseDecodeArgs(
-        b=b, s_q=s_q, h_q=h_q, h_kv=1, d_qk=576, d_v=512, num_blocks=kc.size(0), page_block_size=64,
+        b=b, s_q=s_q, h_q=h_q, h_kv=h_kv, d_qk=576, d_v=512, num_blocks=kc.size(0), page_block_size=64,
         is_causal=int(s_q > 1), softmax_scale=576 ** -0.5,
         q=_capi.ptr(q), q_stride_b=q.stride(0), q_stride_s=q.stride(1), q_stride_h=q.stride(2),
         k_cache=_capi.ptr(kc), k_stride_block=kc.stride(0), k_stride_row=kc.stride(1), k_stride_head=kc.stride(2),
@@ -84,6 +84,18 @@ def test_no_alloc_admits_the_serving_shape():
     from tests import workloads as W
     seq = W.seqlens_normal(128, 512, 64, 1, 1024, True, seed=3).tolist()
     _run_pair(128, 1, 128, seq, seed=23)
+
+
+def test_no_alloc_admits_what_one_partition_per_pair_of_sms_did():
+    """Up to 64 rows per kv head have a partition per SM.  Every batch whose scratch fitted 32768 rows with one per pair of SMs
+    fits the array with them too, also where the division by the kv heads rounds."""
+    from flashmla_b200 import _capi
+    parts = lambda h_q, h_kv: _capi.lib().mla_num_sm_parts(0, _capi.MLA_MODE_DENSE_DECODE, h_q, h_kv, 1)
+    for h_kv in range(1, 301):
+        for g in (1, 16, 63, 64):
+            b = 32768 // (h_kv * g) - parts(128 * h_kv, h_kv)
+            assert (b + parts(g * h_kv, h_kv)) * h_kv * g <= _capi.NOALLOC_MAX_ROWS, (h_kv, g, b)
+    _run_pair(110, 1, 256, [1 + 37 * i % 200 for i in range(110)], seed=24, h_kv=4)
 
 
 def test_no_alloc_rejects_oversized_requests():
