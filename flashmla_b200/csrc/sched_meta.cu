@@ -12,12 +12,18 @@
 // One CTA.  In terms of the prefix sums C[i] = cost of requests 0 .. i - 1 (blocks plus overhead each), a partition that
 // starts at cost position x (request r, block x - C[r]) may spend up to X = x + budget: it finishes every request e' with
 // C[e' + 1] <= X, and cuts the next one, e, if blocks are left after that request's overhead (X - F > C[e]).  So the next
-// partition starts at X - F or at C[e], and only this position is serial: one warp walks the partitions, comparing 32
-// prefix sums at a time (a vote instead of a walk over the requests).  Nothing else stands in that chain: lane l keeps the
-// start of partition l, and 32 metadata rows are finished and written side by side, each ending where the next one starts.
-// What bounds it is the chain, about 130 cycles a partition.  us a schedule, one after the other in a graph: one thread that
-// walks requests and partitions / rows written and cuts counted by one lane inside the chain / now:
-//    b 1, 74 partitions  9 / 13 / 5.3;   b 32  12 / 15.5 / 6.6;   b 128  17 / 16 / 6.9;   b 1000  60 / 20 / 10.6
+// partition starts at the larger of X - F and C[e] (at the end of all costs if X reaches that), and only this position is
+// serial: one warp walks the partitions, 32 prefix sums at a time, whose largest one within X is one reduction.  Everything
+// else follows from two neighbouring positions - requests by binary search, splits because starts inside a request lie
+// budget - F apart - and is done with a thread per partition afterwards.
+// What bounds it is the chain, about 78 cycles a partition; up to 64 query rows have a partition per SM, and with votes and
+// shuffles in the chain (118 cycles) their schedules took 4 to 5 us longer than with one per pair of SMs.  us a schedule of
+// lengths up to 8000, one after the other in a graph, votes and shuffles / now:
+//                     b 4          b 32         b 64         b 128        b 1000
+//    74 partitions    6.6 / 5.3    7.0 / 5.8    7.0 / 5.9    7.2 / 6.1    10.8 / 9.3
+//   148 partitions   11.1 / 8.2   11.4 / 8.7   11.8 / 9.0   12.1 / 9.3    15.7 / 12.6
+// (A serial walk over the requests by one thread: 6.9, 8.4, 9.8, 12.2, 32 with 148 partitions.  A branch that steps inside a
+// request without the reduction: 6.4, 7.7, 8.8, 10.2, 15.4, but slower than votes and shuffles where requests are short.)
 #include "common.cuh"
 
 #include <limits.h>
@@ -59,7 +65,7 @@ sched_meta_kernel(const mla_sched_meta_args_t a) {
     int* C = smem_i;                              // [b + 1]  prefix sums of the requests' costs
     int* cuts = C + b + 1;                        // [b]      partitions that end inside a request
     uint32_t* zero_len = reinterpret_cast<uint32_t*>(cuts + b);      // a bit per request without keys
-    __shared__ int warp_sums[SCHED_THREADS / 32];
+    __shared__ int warp_sums[SCHED_THREADS / 32], starts[SCHED_THREADS + 1];
 
     int carry = 0;
     for (int i0 = 0; i0 < b; i0 += SCHED_THREADS) {
@@ -90,67 +96,74 @@ sched_meta_kernel(const mla_sched_meta_args_t a) {
     if (threadIdx.x == 0) C[0] = 0;
     __syncthreads();
 
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        const int budget = (C[b] + P - 1) / P + F;
-        auto blocks = [&](int r) { const int n = C[r + 1] - C[r] - F; return (zero_len[r >> 5] >> (r & 31)) & 1u ? -1 : n; };
-        // window: lane l holds C[base + l + 1] (past the end: never reached)
-        int base = 0, window = lane < b ? C[lane + 1] : INT_MAX;
-        int x = 0, r = 0, split = 0, at_r = 0;                      // at_r = C[r]
-        for (int p0 = 0; p0 < P; p0 += 32) {
-            // lane l keeps where partition p0 + l begins: request, block, split
-            int begin_r = r, begin_block = x - at_r, begin_split = split;
-            const int n_parts = min(32, P - p0);
-#pragma unroll 1
-            for (int i = 1; i <= n_parts && r < b; ++i) {          // (behind the last request every partition begins where this one ends)
-                const int X = x + budget;
-                int n = __popc(__ballot_sync(0xffffffffu, window <= X));
-                int at_e = __shfl_sync(0xffffffffu, window, n - 1);
-                while (n == 32) {                                  // the window lies wholly inside the budget: the next one
-                    base += 32;
-                    at_r = at_e;
-                    window = base + lane < b ? C[base + lane + 1] : INT_MAX;
-                    n = __popc(__ballot_sync(0xffffffffu, window <= X));
-                    at_e = __shfl_sync(0xffffffffu, window, n - 1);
-                }
-                const int e = base + n;
-                at_e = n ? at_e : at_r;
-                const bool cut = e < b && X - F > at_e;
-                split = cut ? (e == r ? split + 1 : 1) : 0;
-                x = cut ? X - F : at_e;
-                r = e;
-                at_r = at_e;
-                if (lane >= i) { begin_r = r; begin_block = x - at_r; begin_split = split; }
-            }
-            // ... and ends where the next one begins
-            mla_sched_meta_t m;
-            m.end_req_idx = __shfl_down_sync(0xffffffffu, begin_r, 1);
-            m.end_block_idx = __shfl_down_sync(0xffffffffu, begin_block, 1);
-            if (lane == n_parts - 1) { m.end_req_idx = r; m.end_block_idx = x - at_r; }
-            if (lane < n_parts) {
-                m.begin_req_idx = begin_r;
-                // A partition that starts after the last request reports the last block index of request 0
-                // here: the reference reads one element past its first-block array, which is the first
-                // element of its last-block array.  Consumers skip such partitions (begin_req_idx >= b).
-                m.begin_block_idx = begin_r < b ? begin_block : abs(blocks(0)) - 1;
-                m.begin_split_idx = begin_split;
-                m.is_first_req_splitted = begin_block != 0;
-                if (m.end_block_idx == 0) {
-                    --m.end_req_idx;
-                    m.end_block_idx = max(blocks(m.end_req_idx), 0);
-                } else {
-                    atomicAdd(&cuts[m.end_req_idx], 1);
-                }
-                const int n_end = blocks(m.end_req_idx);
-                m.is_last_req_splitted = n_end > 0 && m.end_block_idx != n_end;
-                if (m.begin_req_idx == m.end_req_idx)
-                    m.is_first_req_splitted = m.is_last_req_splitted = (m.is_first_req_splitted || m.is_last_req_splitted);
-                m._pad = 0;
-                a.meta[p0 + lane] = m;
-            }
+    const int total = C[b], budget = (total + P - 1) / P + F, own = budget - F;
+    const int lane = threadIdx.x & 31;
+    // (first warp) window: lane l holds C[base + l + 1] (past the end: never reached); floor and top: C[base], C[base + 32]
+    int base = 0, window = lane < b ? C[lane + 1] : INT_MAX, floor = 0, top = b >= 32 ? C[32] : INT_MAX;
+    int x = 0;
+    auto blocks = [&](int r) { const int n = C[r + 1] - C[r] - F; return (zero_len[r >> 5] >> (r & 31)) & 1u ? -1 : n; };
+    auto request_at = [&](int pos, int lo) {                        // the request a position lies in (b: behind the last one), lo or a later one
+        int hi = b;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (C[mid + 1] <= pos) lo = mid + 1; else hi = mid;
         }
+        return lo;
+    };
+    for (int p0 = 0; p0 < P; p0 += SCHED_THREADS) {
+        // the serial chain: where partitions p0 .. begin, and where the last of them ends
+        if (threadIdx.x < 32) {
+            const int n_all = min(SCHED_THREADS, P - p0);
+            for (int g0 = 0; g0 < n_all; g0 += 32) {
+                int begin = x;                                      // lane l: where partition p0 + g0 + l begins
+                const int n = min(32, n_all - g0);
+#pragma unroll 1
+                for (int i = 1; i <= n && x < total; ++i) {         // (behind the last request every partition begins where this one ends)
+                    const int X = x + budget;
+                    while (X >= top) {                              // the window lies wholly inside the budget: the next one
+                        base += 32;
+                        floor = top;
+                        window = base + lane < b ? C[base + lane + 1] : INT_MAX;
+                        top = base + 32 <= b ? C[base + 32] : INT_MAX;
+                    }
+                    x = min(max(__reduce_max_sync(0xffffffffu, window <= X ? window : floor), x + own), total);
+                    if (lane >= i) begin = x;
+                }
+                if (g0 + lane < n_all) starts[g0 + lane] = begin;
+            }
+            if (lane == 0) starts[n_all] = x;
+        }
+        __syncthreads();
+        // the rows, a thread each: every partition ends where the next one begins
+        if (p0 + threadIdx.x < P) {
+            const int begin = starts[threadIdx.x], end = starts[threadIdx.x + 1];
+            mla_sched_meta_t m;
+            m.begin_req_idx = request_at(begin, 0);
+            m.end_req_idx = request_at(end, m.begin_req_idx);
+            const int begin_block = begin - C[m.begin_req_idx];
+            m.end_block_idx = end - C[m.end_req_idx];
+            // A partition that starts after the last request reports the last block index of request 0
+            // here: the reference reads one element past its first-block array, which is the first
+            // element of its last-block array.  Consumers skip such partitions (begin_req_idx >= b).
+            m.begin_block_idx = m.begin_req_idx < b ? begin_block : abs(blocks(0)) - 1;
+            // Inside a request the starts lie budget - F apart, the first at most that far from the request's beginning.
+            m.begin_split_idx = (begin_block + own - 1) / own;
+            m.is_first_req_splitted = begin_block != 0;
+            if (m.end_block_idx == 0) {
+                --m.end_req_idx;
+                m.end_block_idx = max(blocks(m.end_req_idx), 0);
+            } else {
+                atomicAdd(&cuts[m.end_req_idx], 1);
+            }
+            const int n_end = blocks(m.end_req_idx);
+            m.is_last_req_splitted = n_end > 0 && m.end_block_idx != n_end;
+            if (m.begin_req_idx == m.end_req_idx)
+                m.is_first_req_splitted = m.is_last_req_splitted = (m.is_first_req_splitted || m.is_last_req_splitted);
+            m._pad = 0;
+            a.meta[p0 + threadIdx.x] = m;
+        }
+        __syncthreads();
     }
-    __syncthreads();
 
     // a request has one piece more than cuts
     carry = 0;

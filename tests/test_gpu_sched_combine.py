@@ -79,6 +79,21 @@ def test_sched_meta_bit_exact_sparse():
         check_schedule_properties(meta, ns, eff, P, 64, 5)
 
 
+@pytest.mark.parametrize("P", [1, 31, 32, 33, 255, 256, 257, 600])
+def test_sched_meta_at_the_edges_of_its_groups(P):
+    """Requests come in windows of 32, starts in groups of 32 partitions, rows in groups of 256."""
+    rng = random.Random(P)
+    for b in (1, 31, 32, 33, 64, 65, 300):
+        for top in (1, 64, 1000, 40000):
+            for F in (0, 5):
+                seq = [0 if rng.random() < 0.1 else rng.randint(1, top) for _ in range(b)]
+                ref_meta, ref_ns = osm.get_sched_meta(b, P, 64, F, seqlens_k=seq)
+                meta, ns = _run_meta(b, P, 64, F, seqlens=seq)
+                assert np.array_equal(meta[:, :7], ref_meta[:, :7]), (b, top, F)
+                assert np.array_equal(ns, ref_ns), (b, top, F)
+                assert not meta[:, 7].any()
+
+
 def _combine_ref(lse_acc, o_acc, num_splits, b, s_q, h_q, sink, out_init, lse_init):
     """torch restatement of csrc/smxx/decode/combine/combine.cu:72-160."""
     LOG2E = 1.4426950408889634
