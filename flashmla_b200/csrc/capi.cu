@@ -68,14 +68,26 @@ using namespace mla;
 constexpr int ROWS64 = 64;
 
 // Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens (one per SM, or one per pair) takes
-// about 5 : 3 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 330, 444, 512 tokens: 56 / 81,
-// 98 / 82, 141 / 159, 189 / 158, 230 / 234, 283 / 235, 336 / 314; with 512 keys, up to 444 tokens: 24 / 28, 37 / 29, 51 / 52,
-// 66 / 53, 79 / 76, 93 / 77.
+// about 5 : 3 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 444, 512 tokens: 56 / 81,
+// 98 / 82, 141 / 159, 189 / 158, 283 / 235, 336 / 314; with 512 keys, up to 444 tokens: 24 / 28, 37 / 29, 51 / 52, 66 / 53, 93 / 77.
+//   Even counts (three waves against five, 297 to 370 tokens): 80 / 72 with 512 keys, 135 / 125 with 1024; with more keys the fuller
+// SMs lose, 2048 keys 220 / 231 for 297 tokens, 229.5 / 230.8 for 326, 235 / 231 for 370, 4096 keys 416 to 432 / 441.
+//   Lists with lengths of their own: the fullest CTA sets the time, and a pair, with two lists for one, varies less.  us, lists from
+// a quarter full to full, pair / one SM, up to three seeds: 75 tokens x 2048 keys 59 / 80, 223 x 2048 125 / 156, 310 to 350 x 2048 3 to
+// 20 % longer on single SMs, 520 x 2048 8 to 14 %, 75 and 223 x 1024 1 to 23 %; but 90 x 2048 up to 15 % shorter, 240 x 1024
+// 6 to 12 %, 76 to 84 x 640 3 to 14 %, 256 keys 7 to 25 % everywhere.  Lists that are full after all gain as above, so single SMs are given up
+// only where their last wave is less than 60 % full (more than 1024 keys, fewer than eight waves) or hardly more than half (more than
+// 512 keys, one or two waves).  Left: up to 8 % on some seeds, 740 x 2048 for one, and 12 % at 310 x 1024.
 static bool prefill_rows64(const mla_sparse_prefill_args_t& a) {
     const int sms = current_device_num_sms();
     if (a.h_q > ROWS64 || sms < 2) return false;
     const int64_t waves = (a.s_q + sms - 1) / sms, pair_waves = (a.s_q + sms / 2 - 1) / (sms / 2);
-    return 5 * waves <= 3 * pair_waves;
+    if (5 * waves > 3 * pair_waves) return false;
+    const int64_t last = a.s_q - (waves - 1) * sms;                // tokens of the last wave
+    if (a.topk_length && a.topk > 1024) return waves >= 8 || 5 * last >= 3 * sms;
+    if (a.topk_length) return a.topk <= 512 || waves > 2 || last >= sms / 2 + 2;
+    if (5 * waves == 3 * pair_waves) return a.topk <= 1024 || (a.topk <= 2048 && 6 * last >= sms);
+    return true;
 }
 
 extern "C" {

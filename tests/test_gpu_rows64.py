@@ -116,9 +116,10 @@ def test_sparse_decode(width, s_q, h_q, topk):
 
 
 @pytest.mark.parametrize("width", [576, 512])
-@pytest.mark.parametrize("s_q,h_q,topk", [(1, 1, 64), (80, 1, 64), (90, 33, 128), (230, 64, 192), (20, 64, 704), (75, 64, 704)])
+@pytest.mark.parametrize("s_q,h_q,topk", [(1, 1, 64), (80, 1, 64), (90, 33, 128), (230, 64, 192), (20, 64, 704), (75, 64, 704), (100, 64, 704)])
 def test_sparse_prefill(width, s_q, h_q, topk):
-    """(On 148 SMs the kernel for 64 rows takes 75 to 148 and 223 to 296 tokens, the one for pairs of SMs the other counts here.)"""
+    """(On 148 SMs the kernel for 64 rows takes 75 to 148 and 223 to 296 tokens here, 704 keys from 76 tokens on; the one for pairs of
+    SMs the others.)"""
     import flashmla_b200 as fm
     from tests import workloads as W
     d = W.sparse_prefill_inputs(s_q, h_q, 900, topk, seed=s_q)
