@@ -13,8 +13,9 @@
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
 // block_size x 8 scale bytes (7 scales + 1 pad).  Lanes 0-27 hold the quantised values (4 lanes per group), lanes 28-31
-// the RoPE part.  A warp takes two tokens here, whose loads are in flight together, with registers for four blocks per SM: 66 K
-// tokens 27.2 us, 256 K 92.9 (one token per warp 27.2 and 101, scalar instructions 35.5 and 131.7).  The first warps also zero
+// the RoPE part.  A warp of a long call takes two tokens, whose loads are in flight together, with registers for four blocks per SM
+// (20 bytes of them spilled): 66 K tokens 27.2 us, 256 K 92.9 (one token per warp 27.2 and 101, scalar instructions 35.5 and
+// 131.7).  A short call is bound by its own latency and takes one (MODEL1_TWO_FROM).  The first warps also zero
 // the `pad_bytes` behind every block, where the caller owns them (one warp a block; with the last token's stores, inside the
 // loop, 66 K tokens took 36.9 us instead of 34.9, on the scalar kernel).
 #include "common.cuh"
@@ -23,7 +24,9 @@
 
 namespace mla {
 
-constexpr int TOKENS = 2;             // layout 1: tokens per warp, in flight together
+// Layout 1, more tokens than this: two per warp, up to it one.  us, one / two tokens per warp: 64 tokens 1.9 / 2.7, 4 K 2.9 / 3.7,
+// 33 K 12.0 / 12.5, 66 K 24.7 / 24.3, 131 K 51.5 / 48.0.
+constexpr int64_t MODEL1_TWO_FROM = 40000;
 
 __device__ __forceinline__ float pow2_ceil(float s) {
     // smallest power of two >= s (s > 0, normal)
@@ -131,6 +134,8 @@ quantize_fp8_kernel(const mla_quantize_args_t a) {
     }
 }
 
+// TOKENS: tokens per warp, in flight together
+template <int TOKENS>
 __global__ void __launch_bounds__(256, 4)
 quantize_fp8_model1_kernel(const mla_quantize_args_t a, const int pad_bytes) {
     const int lane = threadIdx.x & 31;
@@ -191,9 +196,10 @@ int launch_quantize_fp8(const mla_quantize_args_t& a, bool zero_padding) {
     const int64_t pad_bytes = zero_padding && a.layout ? a.out_stride_block_bytes - (int64_t)a.block_size * rec : 0;
     MLA_CHECK_ARG(pad_bytes <= 0x7fffff00, "mla_quantize_fp8_kvcache_padded: more than 2 GB of padding behind a block");
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    const int per_block = a.layout ? 8 * TOKENS : 8;             // tokens
+    const int per_warp = a.layout && ntok > MODEL1_TWO_FROM ? 2 : 1, per_block = 8 * per_warp;         // tokens
     const int64_t blocks = min((ntok + per_block - 1) / per_block, (int64_t)1 << 24);
-    if (a.layout) quantize_fp8_model1_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
+    if (a.layout && per_warp == 2) quantize_fp8_model1_kernel<2><<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
+    else if (a.layout) quantize_fp8_model1_kernel<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
     else quantize_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;
