@@ -165,8 +165,8 @@ void check_sched(const Sched& s, int num_sm_parts, int64_t b, const at::Device& 
 }
 
 // The stored schedule, or a new one.  A stored one may also have `pair_parts` partitions: a schedule made when every shape ran
-// on pairs of SMs stays usable (the kernels take any number of partitions).
-Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, int pair_parts, const at::Device& device) {
+// on pairs of SMs stays usable (the kernels take any number of partitions).  `new_with_pair_parts`: a new one has that many.
+Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, int pair_parts, bool new_with_pair_parts, const at::Device& device) {
     Sched s;
     if (meta != Py_None) {
         s.meta = tensor(meta, "tile_scheduler_metadata");
@@ -176,6 +176,7 @@ Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, in
         s.parts = a.num_sm_parts;
         return s;
     }
+    if (new_with_pair_parts) a.num_sm_parts = pair_parts;
     s.parts = a.num_sm_parts;
     s.made = true;
     s.meta = empty({a.num_sm_parts, META_INTS}, at::kInt, device);
@@ -259,7 +260,12 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (sa.num_sm_parts <= 0) check(1, "mla_num_sm_parts");
     sa.seqlens_k = ptr<int32_t>(seqlens); sa.stream = stream;
     const int pair_parts = s_q * (h_q / h_kv) <= 64 ? api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_kv * 128, (int)h_kv, 1) : sa.num_sm_parts;
-    const Sched sched = schedule(args[7], args[8], sa, pair_parts, device);
+    // A table of two blocks a request: as many partitions as there are SMs cut requests of two blocks in two when b of them cost
+    // less than that many (two blocks and the overhead each), half as many leave them whole from half that cost on, and nothing is
+    // left to combine.  us, 15 requests of 68 / 100 tokens: 33 to 64 rows 16.6 / 15.9 -> 15.7 / 14.9; up to 32 rows lose nothing.
+    const int64_t cost = b * (2 + FIXED_OVERHEAD_NUM_BLOCKS);
+    const bool whole = s_q * (h_q / h_kv) > 32 && table.size(1) == 2 && pair_parts <= cost && cost < sa.num_sm_parts;
+    const Sched sched = schedule(args[7], args[8], sa, pair_parts, whole, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);
@@ -374,7 +380,7 @@ PyObject* sparse_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     sa.b = (int32_t)b; sa.s_q = (int32_t)s_q; sa.topk = (int32_t)topk; sa.extra_topk = (int32_t)extra_topk;
     sa.topk_length = ptr<int32_t>(topk_length); sa.extra_topk_length = ptr<int32_t>(extra_topk_length);
     sa.num_sm_parts = count_parts(h_q); sa.stream = stream;
-    const Sched sched = schedule(args[5], args[6], sa, h_q <= 64 ? count_parts(128) : sa.num_sm_parts, device);
+    const Sched sched = schedule(args[5], args[6], sa, h_q <= 64 ? count_parts(128) : sa.num_sm_parts, false, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);

@@ -84,6 +84,26 @@ def test_schedule_made_for_pairs_of_sms():
                 _dense(q, k, bt, sl, False, meta)
 
 
+@pytest.mark.parametrize("b,longest,whole", [(10, 128, False), (11, 128, True), (21, 128, True), (22, 128, False), (15, 64, False), (15, 129, False)])
+@pytest.mark.parametrize("h_q", [32, 33, 64])
+def test_requests_of_two_blocks_stay_whole(b, longest, whole, h_q):
+    """33 to 64 rows and a table of two blocks a request (148 SMs): a new schedule has a partition per pair of SMs where that leaves the
+    requests whole and one per SM does not.  A schedule with either count is taken, the table as wide as it may be."""
+    import flashmla_b200 as fm
+    lengths = [longest - 7 * i % 60 for i in range(b)]
+    q, k, bt, sl = _dense_inputs(1, h_q, 1, lengths, seed=b)
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, False)
+    meta = fm.get_mla_metadata()[0]
+    assert bt.size(1) > 3
+    for width in ((longest + 63) // 64, bt.size(1)):
+        out, lse = _dense(q, k, bt[:, :width].contiguous(), sl, False, meta)
+        assert meta.tile_scheduler_metadata.size(0) == (74 if whole and h_q > 32 else 148)
+        assert_out_close("out", out, ref_out)
+        assert_lse_close("lse", lse, ref_lse)
+    if whole and h_q > 32:
+        assert torch.equal(meta.num_splits.cpu(), torch.arange(b + 1, dtype=torch.int32))
+
+
 def _cache(width, b, s_kv, topk, s_q, h_q, seed):
     from tests import workloads as W
     d = W.sparse_decode_inputs(b, s_q, h_q, s_kv, topk, seed=seed, device="cpu")
