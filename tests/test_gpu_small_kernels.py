@@ -125,6 +125,15 @@ def test_written_records_signed_zeros_and_specials(width, pow2, special):
         assert torch.equal(got, full.view(torch.uint8).contiguous())
 
 
+@pytest.mark.parametrize("blocks,page", [(39999, 1), (625, 64), (3077, 13), (40003, 1)])
+def test_512_wide_writer_around_forty_thousand_tokens(blocks, page):
+    """Up to 40000 tokens a warp takes one, above two (the last warp of an odd count one): 39999, 40000, 40001, 40003 tokens."""
+    from flashmla_b200.kvcache import quantize_fp8_kvcache_model1
+    x = (torch.randn(blocks, page, 1, 512, generator=torch.Generator().manual_seed(blocks)) * 3).to(torch.bfloat16)
+    got = quantize_fp8_kvcache_model1(x.to(DEV))
+    assert torch.equal(got.view(torch.uint8).cpu(), quant.quantize_model1(x).view(torch.uint8))
+
+
 @pytest.mark.parametrize("h_q,counts", [
     (64, [41]),                                   # 8 warps per row
     (64, [2, 1, 9]),                              # 4
