@@ -78,7 +78,8 @@ def _model1_prefill_golden(golden_dir):
     (3, 2, 128, 1024, 320, 64, True),
     (5, 1, 64, 960, 192, 48, False),       # a block size that is not a power of two: 48 * 584 bytes padded to 49 * 576
     (2, 1, 200, 512, 128, 64, False),      # more heads than one row block
-    (80, 1, 16, 256, 128, 64, True),       # more requests than SM partitions
+    (80, 1, 16, 256, 128, 64, True),       # more requests than pairs of SMs
+    (200, 1, 16, 256, 128, 64, True),      # more requests than SM partitions
     (9, 2, 128, 4096, 2048, 64, False),    # the serving top-k: 16 tiles per request
 ])
 @pytest.mark.parametrize("impl", [1, 2])
