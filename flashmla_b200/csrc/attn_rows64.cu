@@ -27,14 +27,20 @@
 // MMA of 128 x NH x 16 takes 56 SM cycles for every NH up to 64.  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
 // fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
 // Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
-// and its loads 4500-6000 of them.  us a call, before (pairs of SMs for every shape) and now, back to back in short runs:
-//   dense, 4 requests of 64..512, 16 heads     18.7 ->  13.9    dense fp16, 61 x 4096, 16 heads     77   ->  63.4
+// and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape -> now, inputs changing from call to call, clocks settled:
+//   dense, 4 requests of 64..512, 16 heads     18.3 ->  13.1    dense fp16, 61 x 4096, 16 heads     95.9 ->  64.4
+//   FP8, 2 x 2 x 2048, 64 heads, schedule too  26.2 ->  21.7    prefill 512-wide, 117 tokens, ragged 38.8 ->  30.6
+// and one input in short runs:
 //   dense, 30 x 2048, 8 heads                  32.8 ->  23.7    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 68.7 / 78.0
 //   FP8, 64 x 2048, 16 heads                   93.3 ->  54.7    FP8, 74 x 2048, 64 heads            95.9 ->  82.2
-//   FP8, 2 x 2 x 2048, 64 heads                27.2 ->  23.3    prefill 512-wide, 117 tokens, ragged 42.3 ->  31.0
 //   prefill, 512 x 2048, 64 heads               333 ->   308    prefill, 2000 x 1024, 64 heads       677 ->   564
-// (The shortest dense requests with 64 heads lose: 15 of about 68 tokens 15.8 -> 17.1, since twice the partitions split requests of
-// two blocks; with 100 tokens and more they gain.)
+// What loses: dense decode with 33 to 64 rows where as many pairs of SMs as requests left every request whole - 37 to 74 requests of
+// nearly the same, short length.  One input, us, pairs -> now, with 64 heads: 45 x 200 tokens 17.5 -> 21.2, 64 x 300 20.0 -> 24.7,
+// 64 x 400 21.9 -> 24.7, 56 x 800 26.8 -> 28.8, 70 x 1000 32.3 -> 35.4, 64 x 2048 56.0 -> 54.5.  With lengths spread by 30 % pairs cut
+// requests as well (64 x 200 27.8 -> 21.4), and the lengths are known on the device only, so no rule of the host tells them apart.
+// (Two blocks at most: see csrc/host.cpp.)
+// Registers: at the launch bound of the FP8 variants 36 to 76 bytes are spilled (576-wide 64 / 16 heads 76 / 56, 512-wide 64 heads 36,
+// 16 none), of prefill 8 (576-wide); where they are reloaded has not been established.  Dense: none.
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert
 // every record.
 //
@@ -849,6 +855,7 @@ int launch_sparse_decode_rows64(const mla_sparse_decode_args_t& a) {
     const dim3 grid((a.h_q + 63) / 64, a.s_q, a.num_sm_parts);
 #define MLA_SPARSE(NH) (a.d_qk == 512 ? rows64::launch<MODE_SPARSE_DECODE, true, NH>(grid, unused, unused, qmap, p, a.stream) \
                                       : rows64::launch<MODE_SPARSE_DECODE, false, NH>(grid, unused, unused, qmap, p, a.stream))
+    // (17 to 32 heads: a variant of 32, with a fifth pair as in dense decode, has not been measured)
     return a.h_q <= 16 ? MLA_SPARSE(16) : MLA_SPARSE(64);
 #undef MLA_SPARSE
 }

@@ -29,7 +29,7 @@ struct Params {
     float scale_log2;
     uint32_t wait_limit;                   // units of 2^WAIT_UNIT_LOG2 SM cycles after which a barrier wait gives up
     const __nv_bfloat16* q; int64_t q_sb, q_ss, q_sh;
-    int q_tma, q_box_bytes;                // a request's Q comes as 9 TMA boxes of q_box_bytes through the empty K ring
+    int q_tma, q_box_bytes;                // a request's Q comes as TMA boxes of q_box_bytes: 9 through the empty K ring (128 rows), 8 or 9 into a buffer of its own (64)
     __nv_bfloat16* out; int64_t o_sb, o_ss, o_sh;
     float* lse; int64_t l_sb, l_ss, l_sh;
     const int* block_table; int64_t bt_sb; const int* seqlens;

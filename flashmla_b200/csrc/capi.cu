@@ -63,9 +63,8 @@ static int check_decode_common(const char* who, bool allow_512, int b, int s_q, 
 
 using namespace mla;
 
-// Query rows (query tokens x heads of a kv head) that one SM serves by itself (attn_rows64.cu, with what it measured on both sides
-// of this line): O^T of more rows and the scores do not fit its tensor memory, Q and a tile not its shared memory.
-constexpr int ROWS64 = 64;
+// MLA_SINGLE_SM_ROWS: the kernel for that many rows on one SM (attn_rows64.cu) has measured both sides of the line.  Q of 96 rows
+// and a tile would not fit shared memory (108 + 144 KB), O^T and the scores tensor memory from 103 rows on.
 
 // Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens (one per SM, or one per pair) takes
 // about 5 : 3 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 444, 512 tokens: 56 / 81,
@@ -80,7 +79,7 @@ constexpr int ROWS64 = 64;
 // 512 keys, one or two waves).  Left: up to 8 % on some seeds, 740 x 2048 for one, and 12 % at 310 x 1024.
 static bool prefill_rows64(const mla_sparse_prefill_args_t& a) {
     const int sms = current_device_num_sms();
-    if (a.h_q > ROWS64 || sms < 2) return false;
+    if (a.h_q > MLA_SINGLE_SM_ROWS || sms < 2) return false;
     const int64_t waves = (a.s_q + sms - 1) / sms, pair_waves = (a.s_q + sms / 2 - 1) / (sms / 2);
     if (5 * waves > 3 * pair_waves) return false;
     const int64_t last = a.s_q - (waves - 1) * sms;                // tokens of the last wave
@@ -108,7 +107,7 @@ int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q) {
         // SMs (the tcgen05 kernel's score / value CTAs, or two 64-row CTAs of the portable kernel); up to 64 rows take one CTA.
         const int rows = s_q * (h_q / h_kv);
         const int row_blocks = (rows + 127) / 128;
-        int p = (rows <= ROWS64 ? sms : sms / 2) / h_kv / row_blocks;
+        int p = (rows <= MLA_SINGLE_SM_ROWS ? sms : sms / 2) / h_kv / row_blocks;
         return p > 0 ? p : 1;
     } else if (mode == MLA_MODE_SPARSE_DECODE) {
         // per partition and query token: up to 64 heads one CTA, up to 128 a pair of CTAs on two SMs (the tcgen05 kernels), more
@@ -131,8 +130,9 @@ int mla_num_sm_parts_uniform(int device, int mode, int h_q, int h_kv, int s_q, i
     // Every request costs the same, so with exactly b partitions the greedy scheduler cuts at every request boundary
     // (budget = blocks + 2 * overhead per partition, a request costs blocks + overhead: one fits, two do not): no
     // partition walks two requests (one Q load and one epilogue each instead of two), no request is split and nothing
-    // is left to combine.  That leaves p - b CTA pairs idle; take it when the extra blocks per partition cost less
-    // than the boundary they save (about 8 blocks of 64 tokens, measured).  (For a multiple k > 1 of b the cuts
+    // is left to combine.  That leaves p - b partitions idle; take it when the extra blocks per partition cost less
+    // than the boundary they save (about 8 blocks of 64 tokens, measured on pairs of SMs, not again with up to 64 heads on single
+    // SMs: lists of at most 512 keys are never split there either).  (For a multiple k > 1 of b the cuts
     // drift off the request boundaries - the scheduler's budget rounds up - so only k = 1 is offered.)
     const double blocks_greedy = (double)blocks_per_request * b / p;
     return ((double)blocks_per_request - blocks_greedy) < 8.0 ? b : p;
@@ -162,7 +162,7 @@ int mla_dense_decode_fwd(const mla_dense_decode_args_t* a) {
     MLA_CHECK_ARG(a->num_blocks > 0, "mla_dense_decode_fwd: num_blocks must be positive");
     MLA_CHECK_ARG(is_aligned16(a->k_cache) && a->k_stride_block % 8 == 0 && a->k_stride_row % 8 == 0 && a->k_stride_head % 8 == 0,
                   "mla_dense_decode_fwd: k_cache must be 16-byte aligned with strides that are multiples of 8 elements");
-    const bool rows64 = a->s_q * (a->h_q / a->h_kv) <= ROWS64;
+    const bool rows64 = a->s_q * (a->h_q / a->h_kv) <= MLA_SINGLE_SM_ROWS;
     if (a->impl == 2) {
         if (!dense_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: the tcgen05 kernel does not support this shape");
@@ -198,7 +198,7 @@ int mla_sparse_decode_fwd(const mla_sparse_decode_args_t* a) {
     } else {
         MLA_CHECK_ARG(!a->extra_indices && !a->extra_topk_length, "mla_sparse_decode_fwd: extra_indices / extra_topk_length need extra_kv");
     }
-    const bool rows64 = a->h_q <= ROWS64;
+    const bool rows64 = a->h_q <= MLA_SINGLE_SM_ROWS;
     if (a->impl == 2) {
         if (!sparse_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_decode_fwd: the tcgen05 kernel does not support this shape");

@@ -162,8 +162,8 @@ int launch_combine(const mla_combine_args_t& a) {
                   "combine: out must be 8-byte aligned with strides that are multiples of 4 elements");
     // Warps per row, from an estimate of the splits a request has: the SM pairs shared out over row blocks of 128 and the batch
     // (up to 64 rows: the SMs over the batch).
-    // This kernel knows neither the partition count nor h_kv: the estimate is high for several kv heads and, in sparse decode,
-    // for several query tokens of at most 64 heads.  The bounds on the rows (all CTAs in one wave: 2 per SM with the deeper
+    // This kernel knows neither the partition count nor h_kv: the estimate is high for several kv heads and low, in sparse decode,
+    // for several query tokens of at most 64 heads (3 x 64, one request: 38, of 49 partitions).  The bounds on the rows (all CTAs in one wave: 2 per SM with the deeper
     // unrolling of WPR = 8, else 3) keep that harmless.  us alone, behind a 256 MB scrub, with
     // 1 / 2 / 4 / 8 warps per row, and the rule's choice (event resolution 2 us):
     //    rows  splits                            rows  splits
@@ -175,7 +175,7 @@ int launch_combine(const mla_combine_args_t& a) {
     const int64_t rows = (int64_t)a.b * a.s_q * a.h_q;
     const int sms = current_device_num_sms() > 0 ? current_device_num_sms() : 148;
     const int rows_each = a.s_q * a.h_q;
-    const int splits = 1 + (rows_each <= 64 ? sms : sms / 2) / std::max(1, (rows_each + 127) / 128) / a.b;
+    const int splits = 1 + (rows_each <= MLA_SINGLE_SM_ROWS ? sms : sms / 2) / std::max(1, (rows_each + 127) / 128) / a.b;
     const int64_t wave = (int64_t)sms * 3 * COMBINE_WARPS;         // warps
     const int wpr = splits >= 16 && rows <= 2 * sms ? 8 : splits >= 8 && rows * 4 <= wave ? 4 : splits >= 4 && rows * 2 <= wave ? 2 : 1;
     const int rows_per_cta = COMBINE_WARPS / wpr;

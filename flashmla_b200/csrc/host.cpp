@@ -259,7 +259,7 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     sa.num_sm_parts = api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_q, (int)h_kv, (int)s_q);
     if (sa.num_sm_parts <= 0) check(1, "mla_num_sm_parts");
     sa.seqlens_k = ptr<int32_t>(seqlens); sa.stream = stream;
-    const int pair_parts = s_q * (h_q / h_kv) <= 64 ? api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_kv * 128, (int)h_kv, 1) : sa.num_sm_parts;
+    const int pair_parts = s_q * (h_q / h_kv) <= MLA_SINGLE_SM_ROWS ? api.num_sm_parts(device.index(), MLA_MODE_DENSE_DECODE, (int)h_kv * 128, (int)h_kv, 1) : sa.num_sm_parts;
     // A table of two blocks a request: as many partitions as there are SMs cut requests of two blocks in two when b of them cost
     // less than that many (two blocks and the overhead each), half as many leave them whole from half that cost on, and nothing is
     // left to combine.  us, 15 requests of 68 / 100 tokens: 33 to 64 rows 16.6 / 15.9 -> 15.7 / 14.9; up to 32 rows lose nothing.
@@ -380,7 +380,7 @@ PyObject* sparse_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     sa.b = (int32_t)b; sa.s_q = (int32_t)s_q; sa.topk = (int32_t)topk; sa.extra_topk = (int32_t)extra_topk;
     sa.topk_length = ptr<int32_t>(topk_length); sa.extra_topk_length = ptr<int32_t>(extra_topk_length);
     sa.num_sm_parts = count_parts(h_q); sa.stream = stream;
-    const Sched sched = schedule(args[5], args[6], sa, h_q <= 64 ? count_parts(128) : sa.num_sm_parts, false, device);
+    const Sched sched = schedule(args[5], args[6], sa, h_q <= MLA_SINGLE_SM_ROWS ? count_parts(128) : sa.num_sm_parts, false, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);

@@ -6,7 +6,8 @@
 // A warp takes a token; lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is one coalesced
 // 512-byte store.  1152 bytes read + 656 bytes written per token.  The quotients x / s only need the correctly rounded reciprocal
 // of s, once per group, and three instructions each (Markstein's theorem; quotient16 below), two values per instruction.  66 K
-// tokens take 23.3 us (5.1 TB/s), 256 K 87 us (5.3 TB/s).  Registers count: with two tokens per warp (75 of them in the place of 47)
+// tokens take 23.3 us (5.1 TB/s), 256 K 87 us (5.3 TB/s), back to back on one input; with inputs that change 66 K take 26.2 (28.7 with
+// two tokens per warp and scalar instructions).  Registers count: with two tokens per warp (75 of them in the place of 47)
 // 26.6 and 96.7 us; with the scalar instructions, two / one token per warp, 27.3 / 26.8 and 98.2 / 99.2.  A persistent grid that
 // loads a token ahead is no faster (27.3).
 //

@@ -59,8 +59,12 @@ const char* mla_last_error(void);
 #define MLA_ABI_VERSION 2
 int mla_abi_version(void);
 
+/* Query rows (query tokens x heads of a kv head) that one SM serves by itself: up to this many, decode has a partition per SM
+ * in the place of one per pair of SMs. */
+#define MLA_SINGLE_SM_ROWS 64
+
 /* Number of SM partitions the decode kernels of `mode` use on `device` for a
- * launch with these head counts / query length.  Stands in for the expression in
+ * launch with these head counts / query length (the kernels take any other number of a schedule too).  Stands in for the expression in
  * csrc/api/dense_decode.h:78 and DecodeImplBase::get_meta
  * (csrc/api/sparse_decode.h:92-99,126-133).  Returns <= 0 on error. */
 int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q);

@@ -180,3 +180,20 @@ def test_uniform_partition_count_never_straddles_requests():
                 assert ns.tolist() == list(range(b + 1))
                 assert meta[:, 0].tolist() == list(range(b)) and meta[:, 1].tolist() == list(range(b))
                 assert not meta[:, 5].any() and not meta[:, 6].any()
+
+
+@pytest.mark.parametrize("h_q", [16, 64])
+def test_uniform_partition_count_with_a_partition_per_sm(h_q):
+    """The same with up to 64 heads, which have a partition per SM."""
+    from flashmla_b200 import _capi
+    lib = _capi.lib()
+    general = lib.mla_num_sm_parts(0, _capi.MLA_MODE_SPARSE_DECODE, h_q, 1, 1)
+    assert general >= 2 * lib.mla_num_sm_parts(0, _capi.MLA_MODE_SPARSE_DECODE, 128, 1, 1)
+    for b in (1, 74, 75, 147, 148, 149):
+        for blocks in (1, 8, 9, 48):
+            P = lib.mla_num_sm_parts_uniform(0, _capi.MLA_MODE_SPARSE_DECODE, h_q, 1, 1, b, blocks)
+            assert P in (b, general), (b, blocks, P)
+            if P == b:
+                meta, ns = _run_meta(b, P, 64, 5, topk=blocks * 64)
+                assert ns.tolist() == list(range(b + 1))
+                assert meta[:, 0].tolist() == list(range(b)) and meta[:, 1].tolist() == list(range(b))
