@@ -39,8 +39,8 @@ def test_dense_row_counts(s_q, h_q, h_kv, dtype):
 
 @pytest.mark.parametrize("h_q", [16, 32, 64])
 def test_dense_scores_that_grow(h_q):
-    """Every tile raises the running maximum by more than the rescale threshold: the RoPE part of K (not part of V) grows with the
-    token's position."""
+    """The RoPE part of K (not part of V) grows with the token's position.  (With a partition per SM a CTA walks one block here: scores far
+    apart are combined.  test_dense_maxima_that_move_on_later_tiles has the tiles behind one another.)"""
     q, k, bt, sl = _dense_inputs(1, h_q, 1, [1500, 129, 700], seed=5)
     for b in range(3):
         for j, page in enumerate(bt[b, :(int(sl[b]) + 63) // 64].tolist()):
