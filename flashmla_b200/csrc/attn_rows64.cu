@@ -24,12 +24,13 @@
 // are exact up to rounding.  Sums stay per thread until the end of a request.
 //
 // What bounds it: one tile is in flight, so a tile's period is the chain  fill -> Q K^T (36 MMAs) -> softmax -> P V (32 MMAs); an
-// MMA of 128 x NH x 16 takes 56 SM cycles for every NH up to 64.  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
+// MMA of 128 x NH x 16 takes what its operands take to be read, 40 SM cycles (NH = 16) to 49 (64).  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
 // fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
 // Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
 // and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape -> now, inputs changing from call to call, clocks settled:
 //   dense, 4 requests of 64..512, 16 heads     18.3 ->  13.1    dense fp16, 61 x 4096, 16 heads     95.9 ->  64.4
 //   FP8, 2 x 2 x 2048, 64 heads, schedule too  26.2 ->  21.7    prefill 512-wide, 117 tokens, ragged 38.8 ->  30.6
+// and with the issuing thread elected (elect_one, sm100_ptx.cuh) 13.4 -> 12.6, 63.7 -> 62.1, 22.1 -> 21.7 and 30.6 -> 24.4,
 // and one input in short runs:
 //   dense, 30 x 2048, 8 heads                  32.8 ->  23.7    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 68.7 / 78.0
 //   FP8, 64 x 2048, 16 heads                   93.3 ->  54.7    FP8, 74 x 2048, 64 heads            95.9 ->  82.2
@@ -280,7 +281,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer -----------------------------------------------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = make_idesc_ab(128, NH, false, false, FP16), idesc_o = make_idesc_ab(128, NH, true, true, FP16);
             // pairs: 64-dim chunks interleaved in every 8-token group (2 KB); RoPE and P: plain rows of 128 bytes
             constexpr uint32_t hi_pair = sw128_desc_hi(2048), hi_row = sw128_desc_hi(1024);
@@ -748,7 +749,7 @@ wind_down:
     if (__syncthreads_or((int)*reinterpret_cast<volatile uint32_t*>(&sm.aborted))) {
         // A bounded wait ran out; every thread has left its role and issues nothing more.  Wait - bounded again - for what is
         // still in flight: the MMAs and the TMA loads.
-        if (warp == 1 && lane == 0) {
+        if (warp == 1 && elect_one()) {
             tc_commit(smem_addr(&sm.drain));
             mbar_wait_bounded(smem_addr(&sm.drain), 0, DRAIN_LIMIT);
         }

@@ -386,7 +386,7 @@ attn_sm100_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer -----------------------------------------------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t g = 0, ks = 0, nreq = 0;
             if (cta_rank == 0) {
                 constexpr uint32_t idesc = make_idesc_16(ROWS, 128, false, FP16);
@@ -1215,7 +1215,7 @@ wind_down:
         // A bounded wait ran out in this CTA or in its peer; every thread of this CTA has left its role and issues
         // nothing more.  Wait - bounded again - for what this CTA still has in flight: its MMAs (they read shared memory
         // and write tensor memory) and the TMA loads into its rings.
-        if (warp == 1 && lane == 0) {
+        if (warp == 1 && elect_one()) {
             tc_commit(smem_addr(&sm.drain));
             mbar_wait_bounded(smem_addr(&sm.drain), 0, DRAIN_LIMIT);
         }

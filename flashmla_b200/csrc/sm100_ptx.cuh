@@ -29,6 +29,16 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 
+// True in one lane of the warp, which executes this together.  The MMA issuing thread is chosen with it: behind any other
+// condition (lane == 0) the compiler does not know that a single thread runs the branch and wraps every MMA in a loop over the
+// active lanes.  Cycles per MMA in a chain of them, lane == 0 -> elected: 128 x 16 x 16 50 -> 39.5, 128 x 64 x 16 50 -> 48.7,
+// 128 x 128 x 16 65.1 -> 65.0.  What is left is shared-memory bandwidth: both operands at 128 bytes a cycle.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // ---- mbarrier -------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
