@@ -37,6 +37,7 @@ struct Params {
     float* lse_accum; float* o_accum;
     int* status;
     int row_blocks;
+    int q_unit;                            // pairs of SMs: rows of Q a box brings (64 rows per CTA)
     // token-sparse prefill: one "request" is one query token, its keys are gathered by index
     const int* indices; int64_t idx_ss; int topk; const int* topk_len; int s_kv;
     const __nv_bfloat16* kv; int64_t kv_ss;

@@ -202,9 +202,9 @@ int mla_sparse_decode_fwd(const mla_sparse_decode_args_t* a) {
     if (a->impl == 2) {
         if (!sparse_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_decode_fwd: the tcgen05 kernel does not support this shape");
-        return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_sm100(*a);
+        return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_pair(*a);
     }
-    if (a->impl == 0 && sparse_decode_sm100_supports(*a)) return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_sm100(*a);
+    if (a->impl == 0 && sparse_decode_sm100_supports(*a)) return rows64 ? launch_sparse_decode_rows64(*a) : launch_sparse_decode_pair(*a);
     return launch_sparse_decode_portable(*a);
 }
 
