@@ -1,5 +1,5 @@
 // MLA attention for up to 128 query rows on a PAIR of SMs whose MMAs span both (sm_100a, tcgen05 with cta_group::2).  Serves sparse FP8
-// decode with 65 to 128 heads; attn_sm100.cu has the other modes of that size, attn_rows64.cu up to 64 rows on one SM.
+// decode with 65 to 128 heads and token-sparse prefill; attn_sm100.cu has dense decode of that size, attn_rows64.cu up to 64 rows on one SM.
 //
 // Each CTA holds 64 of the 128 rows.  With M = 128 over two CTAs both score and output accumulators split by rows:
 //   S = Q K^T   64 x 128 per CTA in 64 columns    A = Q (chunks 0..5 in tensor memory, the others in shared memory)
@@ -27,14 +27,17 @@
 // What bounds FP8 decode: 5200 cycles a tile, the feeding warps' conversion (six slots' worth, 64 x 128 values each, 450-600 cycles
 // apiece) and the chain conversion -> Q K^T -> softmax -> P V behind a ring of two and a half tiles.  One copy of every converted
 // value would save a third of it but the exchange costs more: by 16-byte asynchronous stores into the other SM 93 us, by
-// bulk copies 75.5, converting the half of the other page again 57.0 (below).  us a call, one input per call, back to back, score and
-// value CTAs -> now:
-//   64 x 2048 keys, 128 heads                    91.1 -> 57.0    74 x (512 + 1024) ragged, 512-wide     78.2 -> 52.1
+// bulk copies 75.5, converting the half of the other page again 57.0 (below).  Prefill: 3700 cycles a tile, of which the tensor core
+// works 2250 and the copies (208 instructions an SM, 14.5 cycles each at best) 3000 or more; back to back the power limit (1.55 GHz).
+// us a call, one input per call, back to back, score and value CTAs -> now:
+//   FP8, 64 x 2048 keys, 128 heads              91.2 -> 56.2    FP8, 74 x (512 + 1024) ragged, 512-wide     78.2 -> 51.0
+//   prefill, 4096 x 2048 keys, 128 heads        2740 -> 2284    prefill, 1 x 64 keys, 128 heads             16.3 ->  9.9
 //
 // Bounded waits and the wind-down are those of attn_sm100.cu (attn_shared.cuh).
 //
 // Behavioural reference: csrc/sm90/decode/dense/splitkv_mla.cuh:959-1272 (masking, split / direct epilogue, empty rows),
-// csrc/sm100/decode/head64/kernel.cuh:19-849 (FP8 records, validity, attn_sink) of deepseek-ai/FlashMLA.
+// csrc/sm100/decode/head64/kernel.cuh:19-849 (FP8 records, validity, attn_sink) and
+// csrc/sm100/prefill/sparse/fwd/head128/phase1.cuh:65-614 (prefill outputs) of deepseek-ai/FlashMLA.
 #include "attn_shared.cuh"
 
 namespace mla {
@@ -73,11 +76,12 @@ constexpr int DATA_BYTES = AT_TAB + NTAB * ROWS * 16;
 
 struct Smem {
     uint8_t data[DATA_BYTES];
-    // (those that only the issuing thread waits on live in CTA 0)
-    uint64_t full[NSLOT], empty[NSLOT], r_full[NROPE], r_empty[NROPE], p_full[2], k_done[2], f_tail, q_staged, q_taken, q_full, q_ready, s_full, s_empty,
+    // (those that only the issuing thread waits on live in CTA 0)  full[s]: the two slots from s on, behind a tile's second two its RoPE chunk too
+    uint64_t full[NSLOT], empty[NSLOT], r_empty[NROPE], p_full[2], k_done[2], f_tail, q_staged, q_taken, q_full, q_ready, s_full, s_empty,
         pv_done, o_empty, drain;
     uint32_t tmem_base, aborted;
     uint64_t tab_full[NTAB], tab_empty[NTAB];
+    uint64_t l_full[NSLOT], lf_full[2];     // prefill: this CTA's copies (as full) / of the other page have landed
     uint32_t mask[2 * NTAB][4];                   // gather modes: validity bits of a tile's tokens
 };
 static_assert(sizeof(Smem) <= 232448, "shared memory budget");
@@ -193,12 +197,16 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         return;                                            // both CTAs of the pair take this branch
     }
     if (threadIdx.x == 0) {
-        // a slot is filled by TMA (one arrival and bytes) or by the feeding warps of both CTAs
-        const uint32_t fill = DENSE ? 1 : 2 * W::FEED;
+        // a slot is filled by TMA (one arrival and bytes), by both CTAs' copies (one relaying thread each), or by both CTAs' feeding warps
+        const uint32_t fill = DENSE ? 1 : PREFILL ? 2 : 2 * W::FEED;
         for (int i = 0; i < NSLOT; ++i) { mbar_init(smem_addr(&sm.full[i]), fill); mbar_init(smem_addr(&sm.empty[i]), 1); }
-        for (int i = 0; i < NROPE; ++i) { mbar_init(smem_addr(&sm.r_full[i]), fill); mbar_init(smem_addr(&sm.r_empty[i]), 1); }
+        for (int i = 0; i < NROPE; ++i) mbar_init(smem_addr(&sm.r_empty[i]), 1);
         for (int i = 0; i < 2; ++i) { mbar_init(smem_addr(&sm.p_full[i]), 2 + fill); mbar_init(smem_addr(&sm.k_done[i]), 1); }
         mbar_init(smem_addr(&sm.f_tail), 1);
+        if (PREFILL) {
+            for (int i = 0; i < NSLOT; ++i) mbar_init(smem_addr(&sm.l_full[i]), 32 * W::FEED);
+            for (int i = 0; i < 2; ++i) mbar_init(smem_addr(&sm.lf_full[i]), 32 * W::FEED);
+        }
         for (int i = 0; i < NTAB; ++i) { mbar_init(smem_addr(&sm.tab_full[i]), 32); mbar_init(smem_addr(&sm.tab_empty[i]), W::FEED > 0 ? W::FEED : 1); }
         mbar_init(smem_addr(&sm.q_staged), 1);
         mbar_init(smem_addr(&sm.q_taken), 1);
@@ -234,7 +242,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             RingPos<NROPE> rope;
             uint32_t nq = 0;
             const int chunk0 = hk * p.head_chunks;
-            const uint32_t full0 = lead(sm.full[0]), r_full0 = lead(sm.r_full[0]);
+            const uint32_t full0 = lead(sm.full[0]);
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
                 const Work w = wk.get();
                 if (w.ntiles == 0) continue;
@@ -269,15 +277,18 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     for (int i = 0; i < w.ntiles; ++i) {
                         const int page = nxt;
                         if (i + 1 < w.ntiles) nxt = page_of(w.blk_begin + 2 * (i + 1) + rank);
+                        uint32_t bar = 0;
 #pragma unroll 1
                         for (int q = 0; q < 4; ++q, ring.next()) {
                             WAIT_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 1);
-                            if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.full[ring.slot]), 2 * SLOT);
-                            tma2_load_5d(smem_addr(sm.data) + ring.slot * SLOT, &kmap, full0 + ring.slot * 8, 0, 0, chunk0 + 2 * q, 0, page);
+                            if (!(q & 1)) {
+                                bar = ring.slot;
+                                if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.full[bar]), 4 * SLOT + (q ? 2 * CHUNK : 0));
+                            }
+                            tma2_load_5d(smem_addr(sm.data) + ring.slot * SLOT, &kmap, full0 + bar * 8, 0, 0, chunk0 + 2 * q, 0, page);
                         }
                         WAIT_OR_LEAVE(wt, false, &sm.r_empty[rope.slot], rope.par ^ 1, 2);
-                        if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.r_full[rope.slot]), 2 * CHUNK);
-                        tma2_load_5d(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK, &rmap, r_full0 + rope.slot * 8, 0, 0, chunk0 + 8, 0, page);
+                        tma2_load_5d(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK, &rmap, full0 + bar * 8, 0, 0, chunk0 + 8, 0, page);
                         rope.next();
                     }
                 } else {
@@ -297,6 +308,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             const uint32_t r_lo = sw128_desc_lo(smem_addr(sm.data) + AT_ROPE, 16), q_lo = sw128_desc_lo(smem_addr(sm.data) + AT_Q, 16);
             const uint32_t p_lo = sw128_desc_lo(smem_addr(sm.data) + AT_P, 16);
             constexpr uint32_t d_s = tmem + TM_S, d_o = tmem + TM_O, a_q = tmem + TM_Q;
+            const uint32_t full0 = smem_addr(&sm.full[0]), empty0 = smem_addr(&sm.empty[0]);
+            const uint32_t p_full0 = smem_addr(&sm.p_full[0]), s_empty = smem_addr(&sm.s_empty), o_empty = smem_addr(&sm.o_empty);
             RingPos<NSLOT> ring;
             RingPos<NROPE> rope;
             uint32_t g = 0, nq = 0, full_par = 0;          // full_par: bit s is the parity of slot s's next fill with K
@@ -308,20 +321,49 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     WAIT_OR_LEAVE(wt, false, &sm.q_full, nq & 1, 3);
                 }
                 WAIT_OR_LEAVE(wt, false, &sm.q_ready, nq & 1, 4);
-                // Two streams of work, whichever is ready: Q K^T of tile qi in stages (four slots, RoPE chunk) as they are filled, P V of
-                // tile pi - first, where both are: it frees ring slots.
-                auto is = [&](uint64_t& bar, uint32_t par) { return mbar_test_wait(smem_addr(&bar), par & 1); };
+                // Two streams of work: Q K^T of tile qi in two stages (two slots each, the second with the RoPE chunk) as they are filled, and
+                // where the next stage is not there, P V of tile pi.  A probe of a barrier costs this thread 150 to 300 cycles beside the
+                // other roles' traffic, eight MMAs of Q K^T 270 of the tensor core: with few probes it keeps ahead.  (4096 tokens, 576-wide
+                // prefill: all barriers probed at every step 2620 us, one stage per slot 2320.)
                 RingPos<NSLOT> pv = ring;
                 int qi = 0, pi = 0, stage = 0;
+                auto is = [&](uint32_t bar, uint32_t par) { return mbar_test_wait(bar, par & 1); };
                 uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
                 while (pi < w.ntiles) {
                     const uint32_t gp = g + pi, gq = g + qi;
-                    bool scored = false;                   // the tile's Q K^T is complete
-                    // (all probes at once: one after the other, each would cost its latency)
-                    const bool slot_full = stage < 4 ? is(sm.full[ring.slot], full_par >> ring.slot) : WIDE && is(sm.r_full[rope.slot], rope.par);
-                    const bool p_there = is(sm.p_full[gp & 1], gp >> 1), s_free = is(sm.s_empty, gq + 1);
-                    if (pi < qi && p_there && (pi > 0 || is(sm.o_empty, nq + 1))) {
+                    if (qi < w.ntiles && qi <= pi + 1 && (stage > 0 || is(s_empty, gq + 1)) && is(full0 + ring.slot * 8, full_par >> ring.slot)) {
+                        full_par ^= 1u << ring.slot;
+                        tc_fence_after();
+                        uint32_t b_lo = k_lo + ring.slot * (SLOT >> 4);
+                        ring.next();
+                        // (the first two 64-dim chunks of the stage)
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            mma2_ts_lohi(d_s, a_q + stage * 128 + k * 8, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, (stage | k) ? 1u : 0u);
+                        b_lo = k_lo + ring.slot * (SLOT >> 4);
+                        ring.next();
+                        if (stage == 0) {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                mma2_ts_lohi(d_s, a_q + 64 + k * 8, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, 1u);
+                            stage = 1;
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                mma2_ss_lohi(d_s, q_lo + (k >> 2) * (CHUNK >> 4) + (k & 3) * 2, hi_row, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, 1u);
+                            if (WIDE) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k)
+                                    mma2_ss_lohi(d_s, q_lo + 2 * (CHUNK >> 4) + k * 2, hi_row, r_lo + rope.slot * (CHUNK >> 4) + k * 2, hi_row, idesc_s, 1u);
+                            }
+                            tc_commit2(smem_addr(&sm.s_full));
+                            tc_commit2(smem_addr(&sm.k_done[gq & 1]));
+                            if (WIDE) { tc_commit2(smem_addr(&sm.r_empty[0]) + rope.slot * 8); rope.next(); }
+                            stage = 0;
+                            ++qi;
+                        }
+                    } else if (pi < qi && is(p_full0 + (gp & 1) * 8, gp >> 1) && (pi > 0 || is(o_empty, nq + 1))) {
                         tc_fence_after();
 #pragma unroll 1
                         for (int h = 0; h < 2; ++h)
@@ -332,43 +374,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                                 for (int kt = 0; kt < 4; ++kt)
                                     mma2_ss_lohi(d_o + n * 128, a_lo + kt * 2, hi_row, b_lo + kt * (4096 >> 4), hi_slot, idesc_o,
                                                  (pi > 0 || h > 0 || kt > 0) ? 1u : 0u);
-                                tc_commit2(smem_addr(&sm.empty[0]) + pv.slot * 8);
+                                tc_commit2(empty0 + pv.slot * 8);
                             }
                         tc_commit2(smem_addr(&sm.pv_done));
                         ++pi;
-                    } else if (stage < 4 && slot_full && qi < w.ntiles && qi <= pi + 1 && (stage > 0 || s_free)) {
-                        full_par ^= 1u << ring.slot;
-                        tc_fence_after();
-                        const uint32_t b_lo = k_lo + ring.slot * (SLOT >> 4);
-                        if (stage < QT / 2) {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                mma2_ts_lohi(d_s, a_q + stage * 64 + k * 8, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, (stage | k) ? 1u : 0u);
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                mma2_ss_lohi(d_s, q_lo + (k >> 2) * (CHUNK >> 4) + (k & 3) * 2, hi_row, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, 1u);
-                        }
-                        ring.next();
-                        ++stage;
-                        scored = !WIDE && stage == 4;
-                    } else if (WIDE && stage == 4 && slot_full) {
-                        tc_fence_after();
-                        const uint32_t b_lo = r_lo + rope.slot * (CHUNK >> 4);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            mma2_ss_lohi(d_s, q_lo + 2 * (CHUNK >> 4) + k * 2, hi_row, b_lo + k * 2, hi_row, idesc_s, 1u);
-                        scored = true;
                     } else {
                         if (clock_units<WAIT_UNIT_LOG2>() - t0 > wt.limit) { wt.code = 6; goto wind_down; }
                         continue;
-                    }
-                    if (scored) {
-                        tc_commit2(smem_addr(&sm.s_full));
-                        tc_commit2(smem_addr(&sm.k_done[gq & 1]));
-                        if (WIDE) { tc_commit2(smem_addr(&sm.r_empty[rope.slot])); rope.next(); }
-                        stage = 0;
-                        ++qi;
                     }
                     t0 = clock_units<WAIT_UNIT_LOG2>();
                 }
@@ -378,7 +390,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         }
     } else if (warp == 2) {
         // ---------------- this CTA's half of the dims of the other CTA's page, over chunks that Q K^T has read ----------
-        if ((DENSE || p.q_tma) && elect_one()) {
+        if ((!SPARSE || p.q_tma) && elect_one()) {
             RingPos<NSLOT> ring;
             uint32_t g = 0;
             const int chunk0 = hk * p.head_chunks;
@@ -405,6 +417,11 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     const int page = nxt, blk0 = w.blk_begin + 2 * i;
                     if (DENSE && i + 1 < w.ntiles) nxt = page_of(blk0 + 2 + (1 - (int)rank));
                     WAIT_OR_LEAVE(wt, false, &sm.k_done[g & 1], (g >> 1) & 1, 21);
+                    if (PREFILL) {
+                        WAIT_OR_LEAVE(wt, false, &sm.lf_full[g & 1], (g >> 1) & 1, 22);
+                        fence_proxy_async_smem();          // the copies of this CTA's warps -> visible to its tensor core
+                        mbar_arrive_remote_cta(p_full0 + (g & 1) * 8);
+                    }
                     if (!DENSE) continue;
                     // a page that the sequence ends in: its rows beyond the end are zeroed by the softmax warps when it has landed
                     auto ends_in = [&](int blk) { return blk < w.blk_end && w.seqlen < (blk + 1) * PAGE; };
@@ -461,7 +478,95 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 mbar_arrive(smem_addr(&sm.tab_full[g % NTAB]));
             }
         }
+    } else if (PREFILL && elect_one()) {
+        // ---------------- prefill: copies have landed -> CTA 0's barriers -----------------------------------------------
+        RingPos<NSLOT> ring;
+        uint32_t par = 0;                                  // bit s is the parity of barrier s's next phase
+        const uint32_t full0 = lead(sm.full[0]);
+        for (WalkerT wk(p, part); wk.valid(); wk.next()) {
+            const int ntiles = wk.get().ntiles;
+            if (ntiles == 0) continue;
+            if (p.q_tma) ring.skip(Q_SLOTS);
+            for (int i = 0; i < 2 * ntiles; ++i, ring.skip(2)) {
+                WAIT_OR_LEAVE(wt, false, &sm.l_full[ring.slot], (par >> ring.slot) & 1, 24);
+                par ^= 1u << ring.slot;
+                fence_proxy_async_smem();
+                mbar_arrive_remote_cta(full0 + ring.slot * 8);
+            }
+        }
     }
+    } else if (PREFILL && warp >= W::FIRST_FEED) {
+        regs_dec<W::FEEDING>();
+        // ---------------- prefill: rows by index, eight tokens of a page per warp -----------------------------------------
+        // One cp.async instruction of the warp copies 256 bytes of two rows (a slot's share); invalid tokens get zeros.  A barrier of this
+        // CTA counts one arrival per thread, made by the copy engine when that thread's copies have landed; warps 2 and 3 pass it on.
+        const int fw = warp - W::FIRST_FEED;
+        const int other = (lane >> 3) & 1, page_of_lane = other ? 1 - (int)rank : (int)rank;       // lanes 0..7 look up the own page's tokens, 8..15 the other's
+        const int tok = page_of_lane * PAGE + fw * 8 + (lane & 7);
+        const uint32_t group = smem_addr(sm.data) + fw * 2048 + ((lane >> 3) & 1) * 1024;
+        RingPos<NSLOT> ring;
+        uint32_t g = 0;
+        // this CTA's copy of slot-wide pieces (dims 128 q ..) of the eight rows that lanes l0 .. l0 + 7 looked up
+        auto copy_slot = [&](uint32_t slot, int q, int row_id, int l0) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int tk = 2 * u + (lane >> 4);
+                const int rid = __shfl_sync(0xffffffffu, row_id, l0 + tk);
+                const __nv_bfloat16* src = p.kv + (int64_t)(rid < 0 ? 0 : rid) * p.kv_ss + q * 128 + (lane & 15) * 8;
+                cp_async16_zfill(group + slot * SLOT + tk * 128 + (((lane & 7) ^ tk) << 4), src, rid < 0 ? 0u : 16u);
+            }
+        };
+        for (WalkerT wk(p, part); wk.valid(); wk.next()) {
+            const Work w = wk.get();
+            if (w.ntiles == 0) continue;
+            if (p.q_tma) ring.skip(Q_SLOTS);
+            const int* idx = p.indices + (int64_t)w.req * p.idx_ss;
+            int id_next = tok < w.seqlen ? __ldg(idx + tok) : -1;      // (a tile ahead)
+            int row_id = -1;
+#pragma unroll 1
+            for (int i = 0; i <= w.ntiles; ++i) {
+                const int before = row_id;                             // tile i - 1
+                const bool here = i < w.ntiles;
+                if (here) {
+                    row_id = id_next >= 0 && id_next < p.s_kv ? id_next : -1;
+                    const uint32_t bal = __ballot_sync(0xffffffffu, row_id >= 0);
+                    // token 32 w + l of the tile is bit l of word w
+                    if (lane < 2) { reinterpret_cast<uint8_t*>(sm.mask[(g + i) % (2 * NTAB)])[(lane ? 1 - rank : rank) * 8 + fw] = (uint8_t)(bal >> (8 * lane)); __threadfence_block(); }
+                    // (issued after the fence, which would otherwise wait for it)
+                    { const int posn = (i + 1) * 2 * PAGE + tok; id_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
+                    uint32_t bar = 0;
+#pragma unroll 1
+                    for (int q = 0; q < 4; ++q, ring.next()) {
+                        WAIT_WARP_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 201);
+                        copy_slot(ring.slot, q, row_id, 0);
+                        if (!(q & 1)) bar = ring.slot;
+                        if (q == 1 || (!WIDE && q == 3)) cp_async_arrive_noinc(smem_addr(&sm.l_full[bar]));
+                    }
+                    if (WIDE) {
+                        const uint32_t rs = (g + i) % NROPE;
+                        WAIT_WARP_OR_LEAVE(wt, false, &sm.r_empty[rs], (((g + i) / NROPE) & 1) ^ 1, 202);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int tk = 4 * u + (lane >> 3);
+                            const int rid = __shfl_sync(0xffffffffu, row_id, tk);
+                            const __nv_bfloat16* src = p.kv + (int64_t)(rid < 0 ? 0 : rid) * p.kv_ss + 512 + (lane & 7) * 8;
+                            cp_async16_zfill(smem_addr(sm.data) + AT_ROPE + rs * CHUNK + fw * 1024 + tk * 128 + (((lane & 7) ^ tk) << 4), src, rid < 0 ? 0u : 16u);
+                        }
+                        cp_async_arrive_noinc(smem_addr(&sm.l_full[bar]));
+                    }
+                }
+                if (i > 0) {
+                    // the other page of tile i - 1, over slots that its Q K^T has read
+                    const uint32_t gp = g + i - 1;
+                    WAIT_WARP_OR_LEAVE(wt, false, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
+                    const uint32_t back = (here ? 8 : 4) - (rank == 0 ? 2 : 0);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) copy_slot((ring.slot + NSLOT - back + k) % NSLOT, 2 * rank + k, before, 8);
+                    cp_async_arrive_noinc(smem_addr(&sm.lf_full[gp & 1]));
+                }
+            }
+            g += w.ntiles;
+        }
     } else if (SPARSE && warp >= W::FIRST_FEED) {
         regs_dec<W::FEEDING>();
         // ---------------- FP8 decode: records by address, four tokens of a page per warp ------------------------------------
@@ -512,13 +617,17 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     own = e.x; own_sc = e.y;
                 }
                 if (here) {
+                    uint32_t bar = 0;
 #pragma unroll
                     for (int q = 0; q < 4; ++q, ring.next()) {
                         WAIT_WARP_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 201);
                         store_share(ring.slot, q, raw[q], rope_raw, M1 ? sc[q & 2] : sc[q]);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_remote_cta(lead0 + ring.slot * 8);
+                        if (!(q & 1)) bar = lead0 + ring.slot * 8;
+                        if (q == 1 || (!WIDE && q == 3)) {
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_remote_cta(bar);
+                        }
                         raw[q] = load_share(own, q, rope_raw);
                     }
                     if (WIDE) {
@@ -526,7 +635,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         st_shared_v4(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK + r * 128 + (((ch * 4 + piece) ^ (r & 7)) << 4), rope_raw);
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_remote_cta(lead_at(sm.r_full[rope.slot]));
+                        if (lane == 0) mbar_arrive_remote_cta(bar);
                         rope.next();
                     }
                 } else if (i < 0) {
@@ -803,6 +912,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     }
 
 wind_down:
+    if (PREFILL && warp >= W::FIRST_FEED) cp_async_wait_all();      // this thread's own copies have landed
     if (wt.expired()) report_expired_wait(p.status, &sm.aborted, map_to_cta(smem_addr(&sm.aborted), rank ^ 1u), wt.code);
     tc_fence_before();
     if (__syncthreads_or((int)*reinterpret_cast<volatile uint32_t*>(&sm.aborted))) {
@@ -848,6 +958,23 @@ int launch_sparse_decode_pair(const mla_sparse_decode_args_t& a) {
     const dim3 grid(2, a.s_q, a.num_sm_parts);
     return a.d_qk == 512 ? pair::launch<MODE_SPARSE_DECODE, true>(grid, unused, unused, qmap, p, a.stream)
                          : pair::launch<MODE_SPARSE_DECODE, false>(grid, unused, unused, qmap, p, a.stream);
+}
+
+int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a) {
+    using namespace sm100;
+    Params p = prefill_params(a);
+    p.row_blocks = (p.rows + pair::ROWS - 1) / pair::ROWS;
+    CUtensorMap unused, qmap;
+    memset(&unused, 0, sizeof(unused));
+    memset(&qmap, 0, sizeof(qmap));
+    p.q_unit = pair::HALF;
+    p.q_tma = encode_q_map(&qmap, a.q, 1, a.s_q, a.h_q, 0, a.q_stride_s, a.q_stride_h, pair::HALF, 1, &p.q_box_bytes, false, a.d_qk) ? 1 : 0;
+    int pairs = current_device_num_sms() / 2 / p.row_blocks;
+    if (pairs < 1) pairs = 1;
+    if (pairs > a.s_q) pairs = a.s_q;
+    const dim3 grid(2, p.row_blocks, pairs);
+    return a.d_qk == 512 ? pair::launch<MODE_PREFILL, true>(grid, unused, unused, qmap, p, a.stream)
+                         : pair::launch<MODE_PREFILL, false>(grid, unused, unused, qmap, p, a.stream);
 }
 
 }  // namespace mla

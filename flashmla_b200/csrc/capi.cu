@@ -66,27 +66,22 @@ using namespace mla;
 // MLA_SINGLE_SM_ROWS: the kernel for that many rows on one SM (attn_rows64.cu) has measured both sides of the line.  Q of 96 rows
 // and a tile would not fit shared memory (108 + 144 KB), O^T and the scores tensor memory from 103 rows on.
 
-// Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens (one per SM, or one per pair) takes
-// about 5 : 3 as long on single SMs.  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 444, 512 tokens: 56 / 81,
-// 98 / 82, 141 / 159, 189 / 158, 283 / 235, 336 / 314; with 512 keys, up to 444 tokens: 24 / 28, 37 / 29, 51 / 52, 66 / 53, 93 / 77.
-//   Even counts (three waves against five, 297 to 370 tokens): 80 / 72 with 512 keys, 135 / 125 with 1024; with more keys the fuller
-// SMs lose, 2048 keys 220 / 231 for 297 tokens, 229.5 / 230.8 for 326, 235 / 231 for 370, 4096 keys 416 to 432 / 441.
-//   Lists with lengths of their own: the fullest CTA sets the time, and a pair, with two lists for one, varies less.  us, lists from
-// a quarter full to full, pair / one SM, up to three seeds: 75 tokens x 2048 keys 59 / 80, 223 x 2048 125 / 156, 310 to 350 x 2048 3 to
-// 20 % longer on single SMs, 520 x 2048 8 to 14 %, 75 and 223 x 1024 1 to 23 %; but 90 x 2048 up to 15 % shorter, 240 x 1024
-// 6 to 12 %, 76 to 84 x 640 3 to 14 %, 256 keys 7 to 25 % everywhere.  Lists that are full after all gain as above, so single SMs are given up
-// only where their last wave is less than 60 % full (more than 1024 keys, fewer than eight waves) or hardly more than half (more than
-// 512 keys, one or two waves).  Left: up to 8 % on some seeds, 740 x 2048 for one, and 12 % at 310 x 1024.
+// Prefill with at most 64 heads: one SM per query token, or a pair of SMs?  A wave of tokens takes 0.56 times as long on pairs, one token
+// per pair, as on single SMs, one per SM (0.6 times with up to 256 keys).  us with 2048 keys, pair / one SM, for 74, 148, 200, 296, 330,
+// 444, 518, 592 tokens: 37 / 59, 67 / 60, 96 / 115, 126 / 115, 155 / 170, 187 / 170, 216 / 226, 251 / 226; 512 keys the same within 5 %.
+//   Lists with lengths of their own: the fullest CTA sets the time, and a pair, with two lists for one, varies less.  Where one SM has
+// the better wave count it still takes a last wave that is filled: pair / one SM, 2048 keys, 75, 80, 100, 148 tokens 0.70, 1.01, 1.08,
+// 1.09; 223, 260, 296 tokens 0.89, 0.94, 1.03; 371, 444 tokens 0.89, 1.05; 640 keys, 75, 80, 223, 260 tokens 0.87, 1.07, 1.02, 1.05.
+// (Two seeds of one distribution, from a quarter full to full.)
 static bool prefill_rows64(const mla_sparse_prefill_args_t& a) {
     const int sms = current_device_num_sms();
     if (a.h_q > MLA_SINGLE_SM_ROWS || sms < 2) return false;
     const int64_t waves = (a.s_q + sms - 1) / sms, pair_waves = (a.s_q + sms / 2 - 1) / (sms / 2);
-    if (5 * waves > 3 * pair_waves) return false;
+    if (a.topk <= 256) return 5 * waves <= 3 * pair_waves;
+    if (25 * waves >= 14 * pair_waves) return false;
+    if (!a.topk_length || waves >= 6) return true;
     const int64_t last = a.s_q - (waves - 1) * sms;                // tokens of the last wave
-    if (a.topk_length && a.topk > 1024) return waves >= 8 || 5 * last >= 3 * sms;
-    if (a.topk_length) return a.topk <= 512 || waves > 2 || last >= sms / 2 + 2;
-    if (5 * waves == 3 * pair_waves) return a.topk <= 1024 || (a.topk <= 2048 && 6 * last >= sms);
-    return true;
+    return a.topk <= 1024 || waves == 1 ? last >= sms / 2 + 6 : 3 * last >= 2 * sms;
 }
 
 extern "C" {
@@ -223,9 +218,9 @@ int mla_sparse_prefill_fwd(const mla_sparse_prefill_args_t* a) {
     if (a->impl == 2) {
         if (!sparse_prefill_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_prefill_fwd: the tcgen05 kernel does not support this shape");
-        return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_sm100(*a);
+        return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_pair(*a);
     }
-    if (a->impl == 0 && sparse_prefill_sm100_supports(*a)) return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_sm100(*a);
+    if (a->impl == 0 && sparse_prefill_sm100_supports(*a)) return rows64 ? launch_sparse_prefill_rows64(*a) : launch_sparse_prefill_pair(*a);
     return launch_sparse_prefill_portable(*a);
 }
 

@@ -50,3 +50,29 @@ def test_sparse_decode_more_requests_than_partitions(width, h_q, most):
         assert requests >= 3 and (tiles >= 4 if most > 128 else tiles == 1)
         assert_out_close("out", out, ref_out)
         assert_lse_close("lse", lse, ref_lse)
+
+
+@pytest.mark.parametrize("width", [576, 512])
+@pytest.mark.parametrize("s_q,h_q,topk", [(1, 128, 64), (160, 65, 64), (160, 128, 192), (90, 200, 320), (3, 64, 704)])
+def test_sparse_prefill(width, s_q, h_q, topk):
+    """One and several query tokens per pair, of one tile and of more; more heads than a pair has rows, half a pair of them."""
+    small.test_sparse_prefill(width, s_q, h_q, topk)
+
+
+@pytest.mark.parametrize("width", [576, 512])
+def test_sparse_prefill_maxima_and_shared_query(width):
+    """Maxima that move on every tile (the true maximum is a result too); heads that share their query: Q that is no tensor map."""
+    import flashmla_b200 as fm
+    s_q, h_q, topk, gen = 90, 128, 640, torch.Generator().manual_seed(width)
+    q, kv = torch.randn(s_q, h_q, width, generator=gen).bfloat16(), torch.randn(1024, 1, width, generator=gen).bfloat16()
+    small._growing(q, kv, torch.arange(1024))
+    idx = torch.stack([torch.randperm(1024, generator=gen)[:topk].sort().values for _ in range(s_q)]).view(s_q, 1, topk).to(torch.int32)
+    small._assert_maxima_move(q, kv[:, 0], width ** -0.5, [(i, idx[i, 0]) for i in range(s_q)])
+    for rows, rows_dev in ((q, q.to(DEV)), (q[:, :1].expand(-1, h_q, -1), q[:, :1].to(DEV).expand(-1, h_q, -1))):
+        ref = attention.sparse_prefill(rows.contiguous(), kv, idx, width ** -0.5, 512)
+        got = fm.flash_mla_sparse_fwd(rows_dev, kv.to(DEV), idx.to(DEV), width ** -0.5, 512)
+        torch.cuda.synchronize()
+        fm.check_status()
+        assert_out_close("out", got[0], ref[0])
+        assert_lse_close("max_logits", got[1], ref[1])
+        assert_lse_close("lse", got[2], ref[2])
