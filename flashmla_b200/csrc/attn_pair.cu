@@ -944,7 +944,60 @@ static int launch(dim3 grid, const CUtensorMap& kmap, const CUtensorMap& rmap, c
 
 }  // namespace pair
 
+struct PairMaps {
+    const void* k_cache = nullptr;
+    int64_t sb = 0, sr = 0, sh = 0;
+    int num_blocks = 0, h_kv = 0, fp16 = 0;
+    CUtensorMap kmap, rmap;
+};
+
 }  // namespace sm100
+
+int launch_dense_decode_pair(const mla_dense_decode_args_t& a) {
+    using namespace sm100;
+    EncodeTiledFn encode = get_encode_fn();
+    if (!encode) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    const bool fp16 = a.dtype == MLA_DTYPE_FP16;
+    const int head_chunks = a.h_kv > 1 ? (int)(a.k_stride_head / 64) : 9;
+    static thread_local PairMaps cm;
+    if (cm.k_cache != a.k_cache || cm.sb != a.k_stride_block || cm.sr != a.k_stride_row || cm.sh != a.k_stride_head ||
+        cm.num_blocks != a.num_blocks || cm.h_kv != a.h_kv || cm.fp16 != (int)fp16) {
+        cm.k_cache = nullptr;
+        const CUtensorMapDataType dt = fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+        cuuint64_t dims[5] = {64, 8, (cuuint64_t)((a.h_kv - 1) * head_chunks + 9), 8, (cuuint64_t)a.num_blocks};
+        cuuint64_t strides[4] = {(cuuint64_t)a.k_stride_row * 2, 128, (cuuint64_t)a.k_stride_row * 16, (cuuint64_t)a.k_stride_block * 2};
+        cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        cuuint32_t kbox[5] = {64, 8, 2, 8, 1}, rbox[5] = {64, 8, 1, 8, 1};
+        CUresult r = encode(&cm.kmap, dt, 5, const_cast<void*>(a.k_cache), dims, strides, kbox, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r == CUDA_SUCCESS)
+            r = encode(&cm.rmap, dt, 5, const_cast<void*>(a.k_cache), dims, strides, rbox, estr,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+        cm.k_cache = a.k_cache; cm.sb = a.k_stride_block; cm.sr = a.k_stride_row; cm.sh = a.k_stride_head;
+        cm.num_blocks = a.num_blocks; cm.h_kv = a.h_kv; cm.fp16 = (int)fp16;
+    }
+    Params p = dense_params(a, head_chunks);
+    p.row_blocks = (p.rows + pair::ROWS - 1) / pair::ROWS;
+    CUtensorMap qmap;
+    memset(&qmap, 0, sizeof(qmap));
+    // boxes of q_unit rows: all 64 of a CTA where they are heads of one token or whole tokens, otherwise pieces that divide a
+    // token's heads
+    int unit = 64, box_h = 64, box_t = 1;
+    if (a.s_q > 1) {
+        while (p.g % unit) unit >>= 1;
+        box_h = unit;
+        if (unit == p.g) { box_t = 64 / unit; unit = 64; }
+    }
+    p.q_unit = unit;
+    if (unit >= 8)                                         // (a swizzle atom)
+        p.q_tma = encode_q_map(&qmap, a.q, a.b, a.s_q, a.h_q, a.q_stride_b, a.q_stride_s, a.q_stride_h, box_h, box_t, &p.q_box_bytes, fp16) ? 1 : 0;
+    const dim3 grid(2, p.row_blocks * a.h_kv, a.num_sm_parts);
+    return fp16 ? pair::launch<MODE_DENSE, true>(grid, cm.kmap, cm.rmap, qmap, p, a.stream)
+                : pair::launch<MODE_DENSE, false>(grid, cm.kmap, cm.rmap, qmap, p, a.stream);
+}
 
 int launch_sparse_decode_pair(const mla_sparse_decode_args_t& a) {
     using namespace sm100;

@@ -161,9 +161,9 @@ int mla_dense_decode_fwd(const mla_dense_decode_args_t* a) {
     if (a->impl == 2) {
         if (!dense_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: the tcgen05 kernel does not support this shape");
-        return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_sm100(*a);
+        return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_pair(*a);
     }
-    if (a->impl == 0 && dense_decode_sm100_supports(*a)) return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_sm100(*a);
+    if (a->impl == 0 && dense_decode_sm100_supports(*a)) return rows64 ? launch_dense_decode_rows64(*a) : launch_dense_decode_pair(*a);
     if (a->dtype != MLA_DTYPE_BF16)
         return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: fp16 is served by the tcgen05 kernel only, which does not support this shape");
     return launch_dense_decode_portable(*a);

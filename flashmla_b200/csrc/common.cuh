@@ -49,6 +49,7 @@ int launch_sparse_prefill_sm100(const mla_sparse_prefill_args_t& a);
 bool sparse_decode_sm100_supports(const mla_sparse_decode_args_t& a);
 int launch_sparse_decode_sm100(const mla_sparse_decode_args_t& a);
 int launch_sparse_decode_pair(const mla_sparse_decode_args_t& a);
+int launch_dense_decode_pair(const mla_dense_decode_args_t& a);
 int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a);
 // The kernel for up to 64 query rows on one SM (attn_rows64.cu); what it takes is what the kernel for 128 rows supports.
 int launch_dense_decode_rows64(const mla_dense_decode_args_t& a);

@@ -76,3 +76,42 @@ def test_sparse_prefill_maxima_and_shared_query(width):
         assert_out_close("out", got[0], ref[0])
         assert_lse_close("max_logits", got[1], ref[1])
         assert_lse_close("lse", got[2], ref[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("s_q,h_q,h_kv", [(1, 65, 1), (1, 96, 1), (2, 48, 1), (2, 96, 1), (3, 72, 1), (2, 35, 1), (1, 200, 1), (2, 256, 2)])
+def test_dense_row_counts(s_q, h_q, h_kv, dtype):
+    """Heads that are one box of Q per CTA, several, and none (their number shares no 8 with the rows)."""
+    small.test_dense_row_counts(s_q, h_q, h_kv, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("parts", [1, 3])
+@pytest.mark.parametrize("s_q,h_q", [(1, 128), (2, 64), (2, 41)])
+def test_dense_several_tiles_and_requests_per_pair(s_q, h_q, parts, dtype):
+    small.test_dense_several_tiles_and_requests_per_cta(s_q, h_q, parts, dtype)
+
+
+@pytest.mark.parametrize("parts", [1, 4])
+def test_dense_requests_of_a_single_tile(parts):
+    """Every request one tile (or none): a request's Q is staged behind the last one's before that has been multiplied."""
+    lengths = [1, 128, 64, 0, 65, 127, 128, 3, 0, 0, 100, 128, 64, 90]
+    q, k, bt, sl = small._dense_inputs(1, 128, 1, lengths, seed=parts)
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, True)
+    out, lse, sched = small._dense_parts(q, k, bt, sl, True, parts)
+    assert_out_close("out", out, ref_out)
+    assert_lse_close("lse", lse, ref_lse)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dense_maxima_that_move_on_later_tiles(dtype):
+    small.test_dense_maxima_that_move_on_later_tiles(128, dtype)
+
+
+def test_dense_heads_that_share_their_query():
+    q, k, bt, sl = small._dense_inputs(1, 1, 1, small.LENGTHS, seed=6)
+    q = q.to(DEV).expand(-1, -1, 100, -1)
+    ref_out, ref_lse = attention.dense_decode(q.cpu().contiguous(), k, bt, sl, 512, False)
+    out, lse = small._dense(q, k, bt, sl, False)
+    assert_out_close("out", out, ref_out)
+    assert_lse_close("lse", lse, ref_lse)
