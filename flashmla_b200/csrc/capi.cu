@@ -126,9 +126,15 @@ int mla_num_sm_parts_uniform(int device, int mode, int h_q, int h_kv, int s_q, i
     // (budget = blocks + 2 * overhead per partition, a request costs blocks + overhead: one fits, two do not): no
     // partition walks two requests (one Q load and one epilogue each instead of two), no request is split and nothing
     // is left to combine.  That leaves p - b partitions idle; take it when the extra blocks per partition cost less
-    // than the boundary they save (about 8 blocks of 64 tokens, measured on pairs of SMs, not again with up to 64 heads on single
-    // SMs: lists of at most 512 keys are never split there either).  (For a multiple k > 1 of b the cuts
+    // than the boundary they save (about 8 blocks of 64 tokens, measured with many requests).  (For a multiple k > 1 of b the cuts
     // drift off the request boundaries - the scheduler's budget rounds up - so only k = 1 is offered.)
+    //   Where few requests leave most SMs idle, cutting them pays from shorter lists on: the kernels take 3 to 4 us a tile of two blocks, the
+    // combine launch costs 1 to 4.  us, whole / cut, at most an eighth of the partitions' number of requests (10 to 20 % less
+    // up to twice as many): 64 heads, 2, 3, 4, 6, 8 blocks 14.0 / 15.4, 17.5 / 15.6, 18.1 / 15.6, 22.4 / 16, 26.3 / 16.5; 16 heads, 4, 6, 8
+    // blocks 12.7 / 12.3, 16.0 / 12.5, 18.8 / 12.9; 128 heads, 6, 8 blocks 16.4 / 16.4, 19.0 / 16.6.  A quarter: 64 and 16 heads, 6, 8
+    // blocks 22.7 / 21.9, 26.8 / 22.7 and 16.3 / 16.6, 19.1 / 17.3; 128 heads lose.
+    const int idle = p / b, blocks = blocks_per_request;
+    if (h_q <= MLA_SINGLE_SM_ROWS ? (idle >= 7 && blocks >= (h_q <= 16 ? 6 : 3)) || (idle >= 4 && blocks >= 8) : idle >= 7 && blocks >= 8) return p;
     const double blocks_greedy = (double)blocks_per_request * b / p;
     return ((double)blocks_per_request - blocks_greedy) < 8.0 ? b : p;
 }

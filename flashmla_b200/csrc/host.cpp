@@ -164,14 +164,16 @@ void check_sched(const Sched& s, int num_sm_parts, int64_t b, const at::Device& 
     require_cuda("num_splits", s.num_splits, &device);
 }
 
-// The stored schedule, or a new one.  A stored one may also have `pair_parts` partitions: a schedule made when every shape ran
-// on pairs of SMs stays usable (the kernels take any number of partitions).  `new_with_pair_parts`: a new one has that many.
-Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, int pair_parts, bool new_with_pair_parts, const at::Device& device) {
+// The stored schedule, or a new one.  A stored one may also have `pair_parts` or `whole_parts` partitions: a schedule made when every
+// shape ran on pairs of SMs, or when fewer requests were cut, stays usable (the kernels take any number of partitions).
+// `new_with_pair_parts`: a new one has that many.
+Sched schedule(PyObject* meta, PyObject* num_splits, mla_sched_meta_args_t a, int pair_parts, int whole_parts, bool new_with_pair_parts, const at::Device& device) {
     Sched s;
     if (meta != Py_None) {
         s.meta = tensor(meta, "tile_scheduler_metadata");
         s.num_splits = tensor(num_splits, "num_splits");
-        if (has_shape(s.meta, {pair_parts, META_INTS})) a.num_sm_parts = pair_parts;
+        for (int n : {pair_parts, whole_parts})
+            if (has_shape(s.meta, {n, META_INTS})) a.num_sm_parts = n;
         check_sched(s, a.num_sm_parts, a.b, device);
         s.parts = a.num_sm_parts;
         return s;
@@ -265,7 +267,7 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // left to combine.  us, 15 requests of 68 / 100 tokens: 33 to 64 rows 16.6 / 15.9 -> 15.7 / 14.9; up to 32 rows lose nothing.
     const int64_t cost = b * (2 + FIXED_OVERHEAD_NUM_BLOCKS);
     const bool whole = s_q * (h_q / h_kv) > 32 && table.size(1) == 2 && pair_parts <= cost && cost < sa.num_sm_parts;
-    const Sched sched = schedule(args[7], args[8], sa, pair_parts, whole, device);
+    const Sched sched = schedule(args[7], args[8], sa, pair_parts, pair_parts, whole, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);
@@ -368,19 +370,23 @@ PyObject* sparse_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const c10::cuda::CUDAGuard guard(device);
     void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     const bool uniform = !topk_length && !extra_topk_length;
-    const auto count_parts = [&](int64_t heads) {
-        // every request costs the same number of KV blocks: let the partition count follow the batch size
-        const int64_t blocks = (topk + 63) / 64 + (extra_topk + 63) / 64;
-        const int n = uniform ? api.num_sm_parts_uniform(device.index(), MLA_MODE_SPARSE_DECODE, (int)heads, 1, (int)s_q, (int)b, (int)blocks)
-                              : api.num_sm_parts(device.index(), MLA_MODE_SPARSE_DECODE, (int)heads, 1, (int)s_q);
+    // (every request costs the same number of KV blocks: the partition count follows the batch size)
+    const int64_t blocks = (topk + 63) / 64 + (extra_topk + 63) / 64;
+    const auto general_parts = [&](int64_t heads) {
+        const int n = api.num_sm_parts(device.index(), MLA_MODE_SPARSE_DECODE, (int)heads, 1, (int)s_q);
         if (n <= 0) check(1, "mla_num_sm_parts");
         return n;
     };
+    // the count that stored schedules may have: one partition per request where that adds less than eight blocks to each
+    const auto whole_parts = [&](int n) { return uniform && b <= n && (double)blocks - (double)blocks * b / n < 8.0 ? (int)b : n; };
     mla_sched_meta_args_t sa = {};
     sa.b = (int32_t)b; sa.s_q = (int32_t)s_q; sa.topk = (int32_t)topk; sa.extra_topk = (int32_t)extra_topk;
     sa.topk_length = ptr<int32_t>(topk_length); sa.extra_topk_length = ptr<int32_t>(extra_topk_length);
-    sa.num_sm_parts = count_parts(h_q); sa.stream = stream;
-    const Sched sched = schedule(args[5], args[6], sa, h_q <= MLA_SINGLE_SM_ROWS ? count_parts(128) : sa.num_sm_parts, false, device);
+    const int general = general_parts(h_q);
+    sa.num_sm_parts = uniform ? api.num_sm_parts_uniform(device.index(), MLA_MODE_SPARSE_DECODE, (int)h_q, 1, (int)s_q, (int)b, (int)blocks) : general;
+    if (sa.num_sm_parts <= 0) check(1, "mla_num_sm_parts");
+    sa.stream = stream;
+    const Sched sched = schedule(args[5], args[6], sa, whole_parts(h_q <= MLA_SINGLE_SM_ROWS ? general_parts(128) : general), whole_parts(general), false, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);

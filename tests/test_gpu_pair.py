@@ -115,3 +115,24 @@ def test_dense_heads_that_share_their_query():
     out, lse = small._dense(q, k, bt, sl, False)
     assert_out_close("out", out, ref_out)
     assert_lse_close("lse", lse, ref_lse)
+
+
+@pytest.mark.parametrize("h_q,topk,b,cut", [(16, 320, 4, False), (16, 384, 4, True), (64, 128, 4, False), (64, 192, 21, True), (64, 512, 37, True),
+                                            (128, 448, 10, False), (128, 512, 10, True), (128, 512, 11, False)])
+def test_few_requests_are_cut(h_q, topk, b, cut):
+    """Few requests of equal cost (148 SMs): lists long enough are cut over all partitions, shorter ones stay whole; a stored schedule of
+    the other kind, one partition per request, is still taken."""
+    import flashmla_b200 as fm
+    from flashmla_b200.flash_mla_interface import _make_sched_meta
+    q, kv, deq, idx = small._cache(576, b, 700, topk, 1, h_q, seed=h_q + topk)
+    ref_out, ref_lse = attention.sparse_decode(q, deq, idx, 576 ** -0.5, 512, None, None)
+    meta, kv = fm.get_mla_metadata()[0], kv.to(DEV).contiguous()
+    for stored in (False, True):
+        if stored:
+            meta.tile_scheduler_metadata, meta.num_splits = _make_sched_meta(b, 1, b, torch.device(DEV), topk=topk)
+        out, lse = fm.flash_mla_with_kvcache(q.to(DEV), kv, None, None, 512, meta, None, 576 ** -0.5, False, True, idx.to(DEV))
+        torch.cuda.synchronize()
+        fm.check_status()
+        assert meta.tile_scheduler_metadata.size(0) == (b if stored or not cut else 148 if h_q <= 64 else 74)
+        assert_out_close("out", out, ref_out)
+        assert_lse_close("lse", lse, ref_lse)
