@@ -1,13 +1,17 @@
-// MLA attention for up to 128 query rows on a PAIR of SMs whose MMAs span both (sm_100a, tcgen05 with cta_group::2).  Serves sparse FP8
-// decode with 65 to 128 heads and token-sparse prefill; attn_sm100.cu has dense decode of that size, attn_rows64.cu up to 64 rows on one SM.
+// MLA attention for up to 128 query rows on a PAIR of SMs whose MMAs span both (sm_100a, tcgen05 with cta_group::2).  One kernel template:
+//   MODE_DENSE          dense BF16 / FP16 paged decode, fed by TMA loads of 64-token KV pages through the block table
+//   MODE_PREFILL        token-sparse prefill, KV rows gathered by index with cp.async
+//   MODE_SPARSE_DECODE  sparse FP8 decode, token records gathered by address, converted in registers
+// Up to 64 rows: attn_rows64.cu (on one SM), or for short prefills this one.
 //
 // Each CTA holds 64 of the 128 rows.  With M = 128 over two CTAs both score and output accumulators split by rows:
 //   S = Q K^T   64 x 128 per CTA in 64 columns    A = Q (chunks 0..5 in tensor memory, the others in shared memory)
 //                                                 B = K, 128 tokens split by N: every CTA brings ITS page of the tile, 576 dims
 //   O += P V    64 x 512 per CTA in 256 columns   A = P of the CTA's own rows (never leaves the SM)
 //                                                 B = V, the dims split by N: every CTA brings BOTH pages, 256 dims
-// so 64 x 576 + 64 x 256 values enter an SM per tile of 128 tokens, where score and value CTAs (attn_sm100.cu) take 128 x 576 and
-// 128 x 512; softmax, P and epilogue are divided evenly, and no CTA waits for the other's P.
+// so 64 x 576 + 64 x 256 values enter an SM per tile of 128 tokens; softmax, P and epilogue are divided evenly, and no CTA waits for the
+// other's P.  (The kernel before this one split the products: a score CTA took 128 x 576 values a tile, a value CTA 128 x 512, P went from
+// one to the other, and one of them ran each epilogue.  Its times are the left-hand figures below.)
 //
 // One instruction's descriptors name the same offsets in both CTAs.  A tile takes four slots of a ring, slot q holding chunks 2 q and
 // 2 q + 1 of the CTA's own page.  CTA 0 serves the dims of slots 0 and 1, CTA 1 those of 2 and 3.  P V of page h reads slots 2 h and
@@ -24,16 +28,30 @@
 // barriers order inside the arriving CTA only (mbar_arrive_remote_cta): what they announce is read by that CTA's own tensor core.
 // With cluster-wide releases a tile of dense decode took 5350 cycles in the place of 4110.
 //
-// What bounds FP8 decode: 5200 cycles a tile, the feeding warps' conversion (six slots' worth, 64 x 128 values each, 450-600 cycles
-// apiece) and the chain conversion -> Q K^T -> softmax -> P V behind a ring of two and a half tiles.  One copy of every converted
-// value would save a third of it but the exchange costs more: by 16-byte asynchronous stores into the other SM 93 us, by
-// bulk copies 75.5, converting the half of the other page again 57.0 (below).  Prefill: 3700 cycles a tile, of which the tensor core
-// works 2250 and the copies (208 instructions an SM, 14.5 cycles each at best) 3000 or more; back to back the power limit (1.55 GHz).
-// us a call, one input per call, back to back, score and value CTAs -> now:
-//   FP8, 64 x 2048 keys, 128 heads              91.2 -> 56.2    FP8, 74 x (512 + 1024) ragged, 512-wide     78.2 -> 51.0
-//   prefill, 4096 x 2048 keys, 128 heads        2740 -> 2284    prefill, 1 x 64 keys, 128 heads             16.3 ->  9.9
+// What bounds it.  Dense decode, 128 requests of about 4096 tokens: 2700 to 3300 cycles a tile, of which the tensor core works 2250 (60 % of
+// the launch); DRAM at 4.9 TB/s in a launch by itself (136 us at 1.63 GHz), back to back the power limit (1.34 GHz).  A tile's loads wait for
+// P V two tiles before, 2000 to 2900 cycles before they have landed.  Prefill: 3700 cycles a tile, the tensor core 2250, the copies (208
+// instructions an SM, 14.5 cycles each at best) 3000 or more; back to back the power limit (1.55 GHz).  FP8 decode: 5200 cycles a tile,
+// the feeding warps' conversion (six slots' worth, 64 x 128 values each, 450-600 cycles apiece) and the chain conversion -> Q K^T ->
+// softmax -> P V behind a ring of two and a half tiles.  One copy of every converted value would save a third of the conversion but the
+// exchange costs more: by 16-byte asynchronous stores into the other SM 93 us, by bulk copies 75.5, converting the half of the
+// other page again 57.0 (first line below).  us a call, back to back, score and value CTAs -> now:
+//   one input per call                                          inputs changing from call to call, clocks settled
+//   FP8, 64 x 2048 keys, 128 heads              91.2 -> 56.2      92.4 -> 60.8
+//   FP8, 74 x (512 + 1024) ragged, 512-wide     78.2 -> 51.0      77.8 -> 50.6
+//   prefill, 4096 x 2048 keys, 128 heads        2740 -> 2284      2809 -> 2339
+//   prefill, 1 x 64 keys, 128 heads             16.3 ->  9.9
+//   dense, 128 x ~4096 tokens                    185 ->  172       189 ->  173
+//   dense, two query tokens                      314 ->  294       325 ->  300
+//   dense, one request of 100003 tokens                           54.9 -> 47.8
+// (914 calls of dense and FP8 decode and prefill with 64 to 128 heads: between 1.04 and 2.0 times as fast, none slower.)
 //
-// Bounded waits and the wind-down are those of attn_sm100.cu (attn_shared.cuh).
+// Every mbarrier wait is bounded (Params::wait_limit SM cycles, about a second by default).  A thread whose wait ran out LEAVES its role -
+// it issues no further arrival, MMA or copy -, records a code in the status words and raises the `aborted` flag of both CTAs.
+// Single-thread roles leave at once; warps leave together (a vote after every wait, because tcgen05.ld/st are warp-collective); the softmax
+// warpgroups, which meet at a named barrier every tile, carry the flag through that barrier (bar.red.or) and leave behind it.  Threads that
+// depend on the one that left run into their own limit.  The wind-down then waits - again bounded - for the MMAs, meets the peer
+// CTA, gives loads still under way time to land, and only then frees tensor memory; both CTAs leave together.
 //
 // Behavioural reference: csrc/sm90/decode/dense/splitkv_mla.cuh:959-1272 (masking, split / direct epilogue, empty rows),
 // csrc/sm100/decode/head64/kernel.cuh:19-849 (FP8 records, validity, attn_sink) and
@@ -944,6 +962,25 @@ static int launch(dim3 grid, const CUtensorMap& kmap, const CUtensorMap& rmap, c
 
 }  // namespace pair
 
+// ---- self-test of the bounded wait: one CTA, one barrier nobody arrives on ---------------------------------
+// Uses the same Waiter and the same reporting as the attention kernels, with nothing in flight (no TMA, no MMA, no
+// cluster): the wait runs into its limit, the status words are written, the kernel returns normally.
+__global__ void bounded_wait_selftest_kernel(int* status, uint32_t limit, int code, int* flag_out) {
+    __shared__ uint64_t bar;
+    __shared__ uint32_t flag;
+    if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); flag = 0; fence_mbar_init(); }
+    __syncthreads();
+    Waiter w(limit);
+    bool ok = threadIdx.x < 32 ? w.wait<false>(&bar, 0, code) : w.wait_warp<false>(&bar, 0, code);
+    // a second wait by the same thread returns at once
+    if (threadIdx.x < 32) ok = w.wait<false>(&bar, 0, code + 1) || ok;
+    if (w.expired()) report_expired_wait(status, &flag, 0u, w.code);
+    __syncthreads();
+    if (threadIdx.x == 0 && flag_out) { flag_out[0] = (int)flag; flag_out[1] = ok ? 1 : 0; }
+}
+
+// The two cache tensor maps of a dense launch depend only on the cache tensor (pointer, strides, pages, heads, type): a decode loop
+// calls with the same cache every step, so the last encoding is kept per host thread.
 struct PairMaps {
     const void* k_cache = nullptr;
     int64_t sb = 0, sr = 0, sh = 0;
@@ -952,6 +989,48 @@ struct PairMaps {
 };
 
 }  // namespace sm100
+
+int launch_bounded_wait_selftest(long long limit_cycles, int code, int* status, int* flag_out, void* stream) {
+    MLA_CHECK_ARG(limit_cycles > 0 && limit_cycles <= 2000000000LL, "mla_selftest_bounded_wait: limit_cycles must be in (0, 2e9]");
+    MLA_CHECK_ARG(status != nullptr, "mla_selftest_bounded_wait: status must not be null");
+    sm100::bounded_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status, wait_units(limit_cycles), code, flag_out);
+    MLA_CHECK_CUDA(cudaGetLastError());
+    return MLA_OK;
+}
+
+bool dense_decode_sm100_supports(const mla_dense_decode_args_t& a) {
+    if (a.d_qk != 576 || a.d_v != 512 || a.page_block_size != 64) return false;
+    if (a.h_kv <= 0 || a.h_q % a.h_kv != 0) return false;
+    // TMA: strides in bytes must be multiples of 16 and below 2^40
+    const int64_t lim = (int64_t)1 << 39;
+    if (a.k_stride_block <= 0 || a.k_stride_row <= 0 || a.k_stride_head <= 0) return false;
+    if (a.k_stride_block >= lim || a.k_stride_row >= lim || a.k_stride_head >= lim) return false;
+    if (a.k_stride_block % 8 || a.k_stride_row % 8 || a.k_stride_head % 8) return false;
+    // the kv heads of a row are addressed as 64-column chunks of one tensor-map dimension
+    if (a.h_kv > 1 && a.k_stride_head % 64) return false;
+    const int rows = a.s_q * (a.h_q / a.h_kv);
+    const int64_t row_blocks = (rows + 127) / 128;
+    if (row_blocks * a.h_kv > 65535 || a.num_sm_parts > 65535) return false;
+    if (!(a.softmax_scale > 0.f)) return false;       // the row maximum is taken before scaling
+    if (reinterpret_cast<uintptr_t>(a.o_accum) & 31) return false;      // split partials leave with 256-bit stores
+    return true;
+}
+
+bool sparse_prefill_sm100_supports(const mla_sparse_prefill_args_t& a) {
+    if ((a.d_qk != 576 && a.d_qk != 512) || a.d_v != 512 || a.h_kv != 1) return false;
+    if (a.kv_stride_s <= 0 || a.kv_stride_s % 8 || a.kv_stride_s >= ((int64_t)1 << 39)) return false;
+    if (!(a.sm_scale > 0.f)) return false;
+    if (a.h_q > 128 * 65535) return false;
+    return true;
+}
+
+bool sparse_decode_sm100_supports(const mla_sparse_decode_args_t& a) {
+    if ((a.d_qk != 576 && a.d_qk != 512) || a.d_v != 512) return false;
+    if (a.h_q > 128 || a.s_q > 65535 || a.num_sm_parts > 65535) return false;
+    if (!(a.sm_scale > 0.f)) return false;
+    if (reinterpret_cast<uintptr_t>(a.o_accum) & 31) return false;      // split partials leave with 256-bit stores
+    return true;
+}
 
 int launch_dense_decode_pair(const mla_dense_decode_args_t& a) {
     using namespace sm100;

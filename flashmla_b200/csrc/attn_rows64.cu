@@ -8,8 +8,8 @@
 //   O^T = V^T P^T [512 dims x NH]     A = the same bytes read along the dims      B = P (one row of NH values per token,
 //                                     (MN-major), 4 blocks of 128 dims            MN-major)
 // Both keep M = 128, O^T takes 4 x NH columns of tensor memory, and a KV tile enters the SM once and serves both products.
-// The kernel for 128 rows (attn_sm100.cu) needs a pair of SMs, because O[128 x 512] fills one SM's tensor memory, brings every
-// tile into both of them and hands P from one to the other.
+// The kernel for 128 rows (attn_pair.cu) needs a pair of SMs, because O[128 x 512] fills one SM's tensor memory, and brings
+// 1.44 times a tile's bytes into the two of them.
 //
 // A tile is 128 tokens (two pages): four PAIRS of 64-dim chunks (dims 128 p .. 128 p + 127) in a ring of NP slots, and the
 // RoPE chunk (576-wide rows) in a slot of its own.  Layout of a pair: [8-token group][chunk][8 rows x 128 B], 128-byte swizzle.
@@ -27,7 +27,7 @@
 // MMA of 128 x NH x 16 takes what its operands take to be read, 40 SM cycles (NH = 16) to 49 (64).  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
 // fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
 // Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
-// and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape -> now, inputs changing from call to call, clocks settled:
+// and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape (score and value CTAs, no longer here) -> now, inputs changing from call to call, clocks settled:
 //   dense, 4 requests of 64..512, 16 heads     18.3 ->  13.1    dense fp16, 61 x 4096, 16 heads     95.9 ->  64.4
 //   FP8, 2 x 2 x 2048, 64 heads, schedule too  26.2 ->  21.7    prefill 512-wide, 117 tokens, ragged 38.8 ->  30.6
 // and with the issuing thread elected (elect_one, sm100_ptx.cuh) 13.4 -> 12.6, 63.7 -> 62.1, 22.1 -> 21.7 and 30.6 -> 24.4,
@@ -45,7 +45,7 @@
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert
 // every record.
 //
-// Bounded waits and the wind-down are those of attn_sm100.cu (attn_shared.cuh).
+// Bounded waits and the wind-down are those of attn_pair.cu (attn_shared.cuh).
 //
 // Behavioural reference: csrc/sm90/decode/dense/splitkv_mla.cuh:959-1272 (masking, split / direct epilogue, empty rows),
 // csrc/sm100/decode/head64/kernel.cuh:19-849 (FP8 records, validity, attn_sink) and

@@ -1,4 +1,4 @@
-// What the two tcgen05 attention kernels (attn_sm100.cu: up to 128 query rows on a pair of SMs; attn_rows64.cu: up to 64 on
+// What the two tcgen05 attention kernels (attn_pair.cu: up to 128 query rows on a pair of SMs; attn_rows64.cu: up to 64 on
 // one) have in common: their parameters, the walk over a partition's work, bounded waits, conversions, the host's
 // tensor map over Q.
 #pragma once
@@ -29,7 +29,7 @@ struct Params {
     float scale_log2;
     uint32_t wait_limit;                   // units of 2^WAIT_UNIT_LOG2 SM cycles after which a barrier wait gives up
     const __nv_bfloat16* q; int64_t q_sb, q_ss, q_sh;
-    int q_tma, q_box_bytes;                // a request's Q comes as TMA boxes of q_box_bytes: 9 through the empty K ring (128 rows), 8 or 9 into a buffer of its own (64)
+    int q_tma, q_box_bytes;                // a request's Q comes as TMA boxes of q_box_bytes: pairs of SMs: six through the ring on their way to tensor memory, the others into a buffer of their own, which takes all of them on one SM
     __nv_bfloat16* out; int64_t o_sb, o_ss, o_sh;
     float* lse; int64_t l_sb, l_ss, l_sh;
     const int* block_table; int64_t bt_sb; const int* seqlens;

@@ -43,11 +43,8 @@ int launch_dense_decode_portable(const mla_dense_decode_args_t& a);
 int launch_sparse_decode_portable(const mla_sparse_decode_args_t& a);
 int launch_sparse_prefill_portable(const mla_sparse_prefill_args_t& a);
 bool dense_decode_sm100_supports(const mla_dense_decode_args_t& a);
-int launch_dense_decode_sm100(const mla_dense_decode_args_t& a);
 bool sparse_prefill_sm100_supports(const mla_sparse_prefill_args_t& a);
-int launch_sparse_prefill_sm100(const mla_sparse_prefill_args_t& a);
 bool sparse_decode_sm100_supports(const mla_sparse_decode_args_t& a);
-int launch_sparse_decode_sm100(const mla_sparse_decode_args_t& a);
 int launch_sparse_decode_pair(const mla_sparse_decode_args_t& a);
 int launch_dense_decode_pair(const mla_dense_decode_args_t& a);
 int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a);

@@ -51,16 +51,6 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Arrive on a barrier that lives in another CTA of the cluster (address from map_to_cta).
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-
-// Remote arrive without ordering of this thread's earlier memory operations: a pure "go ahead" signal
-// (the release form waits for everything the thread has in flight and costs over a microsecond).
-__device__ __forceinline__ void mbar_arrive_remote_relaxed(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
 
 // Remote arrive that orders this thread's earlier operations inside its own CTA only: for data that stays in this CTA and is
 // read by its tensor core when CTA 0 of the pair issues an MMA for both (1300 cycles less than the cluster-wide release).
@@ -87,7 +77,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Same, with acquire semantics at cluster scope (the arrival came from the other CTA of the pair).
+// try_wait with acquire semantics at cluster scope (the arrival came from another CTA).
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -131,9 +121,7 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- proxies / fences ------------------------------------------------------------------------------
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 
 // ---- TMA ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
@@ -155,19 +143,6 @@ __device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* m, int c0, in
     asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global.tile [%0, {%1, %2, %3, %4, %5}];"
                  ::"l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-
-// Row gather: four rows (given by their row coordinates) of a 2-D tensor, `box` columns starting at column c0, land
-// consecutively in shared memory (row coordinates outside the tensor read the fill value, zero).
-__device__ __forceinline__ void tma_gather4_2d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int r0, int r1, int r2, int r3) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
-}
 
 // Per-thread asynchronous 16-byte copy global -> shared; src_bytes = 0 writes zeros without reading.
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
@@ -175,62 +150,12 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 }
 // Arrive on `bar` (counted among its expected arrivals) once all cp.async copies this thread issued so far have landed.
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Waits until at most N of this thread's committed cp.async groups are still in flight.
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // Waits until every cp.async copy this thread has issued has landed.
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Fire-and-forget prefetch of `bytes` (multiple of 16, 16-byte aligned address) from global memory into L2.
-__device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-// L2 eviction-priority policies for loads that should stay in (or get out of) L2.
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-__device__ __forceinline__ void tma_gather4_2d_hint(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int r0, int r1, int r2, int r3,
-                                                    uint64_t policy) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
-        ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "l"(policy) : "memory");
-}
-__device__ __forceinline__ uint4 ldg_evict_first(const uint4* p, uint64_t policy) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy));
-    return v;
-}
-
-// Bulk copy from this CTA's shared memory into another CTA of the cluster; the bytes are counted on a
-// barrier of the destination CTA.  Addresses and size are multiples of 16 bytes.
-// Bulk store shared -> global (16-byte aligned addresses, size a multiple of 16), tracked by the thread's bulk groups
-__device__ __forceinline__ void bulk_store_to_global(void* dst, uint32_t src_local, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_local), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// this thread's bulk stores have read their shared-memory source / have completed
-__device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_local, uint32_t bytes, uint32_t bar_cluster) {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst_cluster), "r"(src_local), "r"(bytes), "r"(bar_cluster) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx_remote(uint32_t cluster_bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -251,12 +176,6 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
 }
 
 // ---- shared-memory stores into the other CTA of the cluster ---------------------------------------------
-__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
-}
 __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
@@ -282,47 +201,11 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Shared-memory matrix descriptor, 128-byte swizzle, tile base 1024-byte aligned.
-//   K-major operand : rows of 64 bf16 (128 B), 8-row groups `sbo` bytes apart (lbo unused).
-//   MN-major operand: 64 contiguous bf16 along M/N per row, 8-row (K) groups `sbo` bytes apart,
-//                     the next 64 M/N elements `lbo` bytes away.
-__device__ __forceinline__ uint64_t make_sw128_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-    d |= 1ull << 46;      // descriptor version of this architecture
-    d |= 2ull << 61;      // SWIZZLE_128B
-    return d;
-}
-
-// Instruction descriptor of tcgen05.mma.kind::f16 with bf16 inputs and fp32 accumulation.
-// A is K-major (or in tensor memory); b_mn_major selects the layout of B.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn_major) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
-           ((uint32_t)(M >> 4) << 24);
-}
-// The same with the 16-bit input type chosen: bf16 (format code 1 for A and B) or fp16 (format code 0).
+// Instruction descriptor of tcgen05.mma.kind::f16 with fp32 accumulation and bf16 (format code 1 for A and B) or fp16 (format code 0)
+// inputs.  A is K-major (or in tensor memory); b_mn_major selects the layout of B.
 __host__ __device__ constexpr uint32_t make_idesc_16(int M, int N, bool b_mn_major, bool fp16) {
     return (1u << 4) | ((fp16 ? 0u : 1u) << 7) | ((fp16 ? 0u : 1u) << 10) | ((b_mn_major ? 1u : 0u) << 16) |
            ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // Both operands' majorness chosen: MN-major A is the transpose of a K-major tile, likewise B.
@@ -330,9 +213,11 @@ __host__ __device__ constexpr uint32_t make_idesc_ab(int M, int N, bool a_mn_maj
     return make_idesc_16(M, N, b_mn_major, fp16) | ((a_mn_major ? 1u : 0u) << 15);
 }
 
-// The same two instructions with the descriptors given as (low, high) 32-bit halves: the high half of a
-// 128-byte-swizzle descriptor is constant for a given operand layout and the low half advances with the
-// address, so an issue loop only does 32-bit adds.
+// Shared-memory matrix descriptor, 128-byte swizzle, tile base 1024-byte aligned.
+//   K-major operand : rows of 64 16-bit values (128 B), 8-row groups `sbo` bytes apart (lbo unused).
+//   MN-major operand: 64 contiguous values along M/N per row, 8-row (K) groups `sbo` bytes apart, the next 64 M/N elements `lbo` bytes away.
+// Given as (low, high) 32-bit halves: the high half is constant for a given operand layout (with the descriptor version of
+// this architecture and the swizzle mode) and the low half advances with the address, so an issue loop only does 32-bit adds.
 __host__ __device__ constexpr uint32_t sw128_desc_hi(uint32_t sbo_bytes) {
     return ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) | (2u << 29);
 }
@@ -348,15 +233,6 @@ __device__ __forceinline__ void mma_ss_lohi(uint32_t d_tmem, uint32_t a_lo, uint
         "mov.b64 bd, {%3, %4};\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], ad, bd, %5, p;\n\t}"
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mma_ts_lohi(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // ---- tcgen05 on a pair of CTAs (cta_group::2) ------------------------------------------------------------

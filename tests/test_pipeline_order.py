@@ -1,7 +1,7 @@
-"""CPU: the happens-before order that protects the small rings in shared memory (gather modes of csrc/attn_sm100.cu, score CTA, and of
-csrc/attn_rows64.cu): the tokens' validity bits, written by the copy warps and read by the softmax warps, and in FP8 decode
-on pairs of SMs the tokens' scales, read by the converting warps.  Nobody arrives on a barrier of their own for these rings, so an entry may
-only be overwritten where the chain of the other barriers already orders its last reader before the writer.
+"""CPU: the happens-before order that protects the small rings in shared memory (gather modes of csrc/attn_pair.cu and of
+csrc/attn_rows64.cu): the tokens' validity bits, written by the copy or look-up warps and read by the softmax warps, and in FP8 decode
+on pairs of SMs the tokens' addresses, read by the converting warps.  Nobody arrives on a barrier of their own for the validity bits, so an
+entry may only be overwritten where the chain of the other barriers already orders its last reader before the writer.
 
 The roles' program order and the barriers between them are written down as a graph; the ring depths, and on which side of
 the arrival that gives the S accumulator back the softmax warps read the mask, come from the source."""
@@ -10,22 +10,19 @@ import re
 
 import pytest
 
-SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashmla_b200", "csrc", "attn_sm100.cu")
+SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashmla_b200", "csrc", "attn_pair.cu")
 
 
 def _plan():
     text = open(SOURCE).read()
-    narrow = {name: int(re.search(name + r" = WIDE \? \d+ : (\d+);", text).group(1)) for name in ("NKS", "S_BUFS")}
-    masks = [int(m) + 1 for m in re.findall(r"kmask\)?\[\(g & (\d)\)", text)] + [int(m) + 1 for m in re.findall(r"SC_MASK\) \+ \(g & (\d)\)", text)]
-    scales = [int(m) + 1 for m in re.findall(r"SC_SCALES\)\[\(g & (\d)\)", text)]
-    assert len(masks) == 3 and len(set(masks)) == 1 and len(scales) == 2 and len(set(scales)) == 1, (masks, scales)
-    read = re.search(r"m0 = km\[0\]", text).start()
-    give_back = text.index("mbar_arrive(smem_addr(&sm.s_empty[sb]))")
-    return narrow["NKS"], narrow["S_BUFS"], masks[0], scales[0], read < give_back
+    slots, tables = (int(re.search(r"\b" + name + r" = (\d+)[,;]", text).group(1)) for name in ("NSLOT", "NTAB"))
+    assert "uint32_t mask[2 * NTAB][4];" in text and len(re.findall(r"sm\.mask\[\(?g(?: \+ i\))? % \(2 \* NTAB\)\]", text)) == 3
+    read = text.index("sm.mask[g % (2 * NTAB)][quarter]")
+    return slots, 2 * tables, tables, read < text.index("mbar_arrive_remote_cta(s_empty)")
 
 
-def _graph(tiles, nks, s_bufs, convert, read_first):
-    """edges[event] = the events that directly precede it; events are (role, what, tile, group)."""
+def _graph(tiles, slots, tables, convert, read_first):
+    """edges[event] = the events that directly precede it; events are (role, what, tile, slot of the tile)."""
     edges = {}
 
     def program(role, steps):
@@ -34,26 +31,36 @@ def _graph(tiles, nks, s_bufs, convert, read_first):
             if i:
                 edges[(role,) + step].append((role,) + steps[i - 1])
 
-    groups = range(3)
-    program("copy", [s for g in range(tiles) for s in [("meta", g, 0)] + [("fill", g, j) for j in groups]])
-    program("mma", [s for g in range(tiles) for s in [("start", g, 0)] + [("group", g, j) for j in groups]])
-    softmax = lambda g: [("mask", g, 0), ("give", g, 0)] if read_first else [("give", g, 0), ("mask", g, 0)]
-    program("softmax", [s for g in range(tiles) for s in [("scores", g, 0)] + softmax(g)])
+    four = range(4)
     if convert:
-        program("convert", [("group", g, j) for g in range(tiles) for j in groups])
+        program("look-up", [("meta", g, 0) for g in range(tiles)])
+    # a tile's own page, then the other page of the tile before
+    meta = lambda g: [("own", g, 0)] if convert else [("meta", g, 0)]
+    feed = [s for g in range(tiles) for s in meta(g) + [("fill", g, q) for q in four] + ([("other", g - 1, 0)] if g else []) + [("done", g, 0)]]
+    program("feed", feed)
+    # (Q K^T of a tile may come before or behind P V of the one before, not earlier)
+    program("scores", [("scores", g, q) for g in range(tiles) for q in four])
+    program("values", [("values", g, q) for g in range(tiles) for q in four])
+    softmax = lambda g: [("mask", g, 0), ("give", g, 0)] if read_first else [("give", g, 0), ("mask", g, 0)]
+    program("softmax", [s for g in range(tiles) for s in [("start", g, 0)] + softmax(g) + [("p", g, 0)]])
     for g in range(tiles):
-        for j in groups:
-            fill = 3 * g + j
-            if fill >= nks:                                                                     # kv_empty: MMAs that read the slot
-                edges["copy", "fill", g, j].append(("mma", "group", (fill - nks) // 3, (fill - nks) % 3))
-            landed = ("copy", "fill", g, j)
-            if convert:                                                                         # raw_full, then kv_full
-                edges["convert", "group", g, j].append(landed)
-                landed = ("convert", "group", g, j)
-            edges["mma", "group", g, j].append(landed)
-        if g >= s_bufs:
-            edges["mma", "start", g, 0].append(("softmax", "give", g - s_bufs, 0))              # s_empty
-        edges["softmax", "scores", g, 0].append(("mma", "group", g, 2))                         # s_full
+        for q in four:
+            f = 4 * g + q
+            if f >= slots:                                                                      # empty: P V that read the slot
+                edges["feed", "fill", g, q].append(("values", "values", (f - slots) // 4, (f - slots) % 4))
+            edges["scores", "scores", g, q].append(("feed", "fill", g, q))                      # full
+            edges["values", "values", g, q] += [("softmax", "p", g, 0)] + ([("feed", "other", g, 0)] if g + 1 < tiles else [])    # p_full
+            edges["values", "values", g, q].append(("scores", "scores", g, 3))
+        if g >= 1:
+            edges["scores", "scores", g, 0].append(("softmax", "give", g - 1, 0))               # s_empty
+            edges["feed", "other", g - 1, 0].append(("scores", "scores", g - 1, 3))             # k_done
+        if g >= 2:
+            edges["scores", "scores", g, 0].append(("values", "values", g - 2, 3))              # the issuing thread's order
+        edges["softmax", "start", g, 0].append(("scores", "scores", g, 3))                      # s_full
+        if convert:
+            edges["feed", "own", g, 0].append(("look-up", "meta", g, 0))                        # tab_full
+            if g >= tables:
+                edges["look-up", "meta", g, 0].append(("feed", "done", g - tables, 0))          # tab_empty
     return edges
 
 
@@ -130,23 +137,23 @@ def _before(edges, first, then):
 
 @pytest.mark.parametrize("convert", [False, True])          # prefill, FP8 decode
 def test_ring_entries_are_read_before_they_are_overwritten(convert):
-    nks, s_bufs, masks, scales, read_first = _plan()
+    slots, masks, tables, read_first = _plan()
     tiles = masks + 8
-    edges = _graph(tiles, nks, s_bufs, convert, read_first)
+    edges = _graph(tiles, slots, tables, convert, read_first)
+    writer = "look-up" if convert else "feed"
     for g in range(tiles - masks):
-        assert _before(edges, ("copy", "meta", g, 0), ("softmax", "mask", g, 0)), "a mask is read after it was written"
-        assert _before(edges, ("softmax", "mask", g, 0), ("copy", "meta", g + masks, 0)), "... and before its entry is written again"
+        assert _before(edges, (writer, "meta", g, 0), ("softmax", "mask", g, 0)), "a mask is read after it was written"
+        assert _before(edges, ("softmax", "mask", g, 0), (writer, "meta", g + masks, 0)), "... and before its entry is written again"
     if convert:
-        for g in range(tiles - scales):
-            assert _before(edges, ("copy", "meta", g, 0), ("convert", "group", g, 0))
-            assert _before(edges, ("convert", "group", g, 0), ("copy", "meta", g + scales, 0))
+        for g in range(tiles - tables):
+            assert _before(edges, ("look-up", "meta", g, 0), ("feed", "own", g, 0))
+            assert _before(edges, ("feed", "done", g, 0), ("look-up", "meta", g + tables, 0))
 
 
 def test_the_check_sees_a_missing_order():
-    """The same graph with the mask read behind the arrival, and with rings of half the depth, has no such order."""
-    nks, s_bufs, masks, scales, _ = _plan()
-    late = _graph(masks + 8, nks, s_bufs, True, False)
-    assert not _before(late, ("softmax", "mask", 3, 0), ("copy", "meta", 3 + masks, 0))
-    good = _graph(masks + 8, nks, s_bufs, True, True)
-    assert not _before(good, ("softmax", "mask", 3, 0), ("copy", "meta", 3 + masks // 2, 0))
-    assert not _before(good, ("convert", "group", 3, 0), ("copy", "meta", 3 + scales // 2, 0))
+    """The same graph has no such order with rings of half the depth, nor for the table's entries where a mask of that depth would do."""
+    slots, masks, tables, _ = _plan()
+    good = _graph(masks + 8, slots, tables, True, True)
+    assert not _before(good, ("softmax", "mask", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
+    assert not _before(good, ("feed", "done", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
+    assert not _before(_graph(masks + 8, slots, tables, False, True), ("softmax", "mask", 3, 0), ("feed", "meta", 3 + 2, 0))
