@@ -136,3 +136,18 @@ def test_few_requests_are_cut(h_q, topk, b, cut):
         assert meta.tile_scheduler_metadata.size(0) == (b if stored or not cut else 148 if h_q <= 64 else 74)
         assert_out_close("out", out, ref_out)
         assert_lse_close("lse", lse, ref_lse)
+
+
+def test_schedules_of_few_long_requests():
+    """Requests of many partitions each, whose starts the scheduler writes a request at a time, and both sides of that line; counts above
+    the rows it makes at once."""
+    from flashmla_b200.flash_mla_interface import _make_sched_meta
+    from oracle import sched_meta
+    gen = torch.Generator().manual_seed(0)
+    for parts in (1, 2, 33, 74, 148, 255, 256, 257):
+        for lengths in ([100003], [1], [64 * parts], [64 * 9 * parts + 1], [7000, 0, 1, 9000], [64, 640000], [3000] * 9,
+                        torch.randint(0, 60000, (5,), generator=gen).tolist(), torch.randint(1, 4000, (12,), generator=gen).tolist()):
+            got, splits = _make_sched_meta(len(lengths), 1, parts, torch.device(DEV), seqlens_k=torch.tensor(lengths, dtype=torch.int32, device=DEV))
+            ref, ref_splits = sched_meta.get_sched_meta(len(lengths), parts, 64, 5, seqlens_k=lengths)
+            assert torch.equal(got.cpu(), torch.as_tensor(ref, dtype=torch.int32)), (parts, lengths)
+            assert splits.tolist() == list(ref_splits), (parts, lengths)
