@@ -24,7 +24,8 @@
 // are exact up to rounding.  Sums stay per thread until the end of a request.
 //
 // What bounds it: one tile is in flight, so a tile's period is the chain  fill -> Q K^T (36 MMAs) -> softmax -> P V (32 MMAs); an
-// MMA of 128 x NH x 16 takes what its operands take to be read, 40 SM cycles (NH = 16) to 49 (64).  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
+// MMA of 128 x NH x 16 takes what its operands take to be read, 40 SM cycles (NH = 16) to 49 (64).
+// (Cycles a tile, measured when the issuing thread made it 56:)  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
 // fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
 // Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
 // and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape (score and value CTAs, no longer here) -> now, inputs changing from call to call, clocks settled:
@@ -41,7 +42,7 @@
 // requests as well (64 x 200 27.8 -> 21.4), and the lengths are known on the device only, so no rule of the host tells them apart.
 // (Two blocks at most: see csrc/host.cpp.)
 // Registers: at the launch bound of the FP8 variants 36 to 76 bytes are spilled (576-wide 64 / 16 heads 76 / 56, 512-wide 64 heads 36,
-// 16 none), of prefill 8 (576-wide); where they are reloaded has not been established.  Dense: none.
+// 16 none); where they are reloaded has not been established.  Dense and prefill: none.
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert
 // every record.
 //
