@@ -40,7 +40,7 @@
 // nearly the same, short length.  One input, us, pairs -> now, with 64 heads: 45 x 200 tokens 17.5 -> 21.2, 64 x 300 20.0 -> 24.7,
 // 64 x 400 21.9 -> 24.7, 56 x 800 26.8 -> 28.8, 70 x 1000 32.3 -> 35.4, 64 x 2048 56.0 -> 54.5.  With lengths spread by 30 % pairs cut
 // requests as well (64 x 200 27.8 -> 21.4), and the lengths are known on the device only, so no rule of the host tells them apart.
-// (Two blocks at most: see csrc/host.cpp.)
+// (Where the block table says that few tokens are to be read, 33 to 64 rows run on pairs of SMs: see csrc/host.cpp.)
 // Registers: at the launch bound of the FP8 variants 36 to 76 bytes are spilled (576-wide 64 / 16 heads 76 / 56, 512-wide 64 heads 36,
 // 16 none); where they are reloaded has not been established.  Dense and prefill: none.
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert

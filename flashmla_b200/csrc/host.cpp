@@ -267,7 +267,14 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // left to combine.  us, 15 requests of 68 / 100 tokens: 33 to 64 rows 16.6 / 15.9 -> 15.7 / 14.9; up to 32 rows lose nothing.
     const int64_t cost = b * (2 + FIXED_OVERHEAD_NUM_BLOCKS);
     const bool whole = s_q * (h_q / h_kv) > 32 && table.size(1) == 2 && pair_parts <= cost && cost < sa.num_sm_parts;
-    const Sched sched = schedule(args[7], args[8], sa, pair_parts, pair_parts, whole, device);
+    // 33 to 64 rows: a pair of SMs per partition (csrc/attn_pair.cu, half of its rows empty) where the table says that few tokens are to be
+    // read.  A pair takes a tile about as fast as two single SMs two of them, with half the partials and a shorter first tile, but
+    // more power.  us, 64 heads, single SMs / pairs: 1 x 9000 tokens 25.3 / 19.7, 4 x 1000 16.1 / 14.5, 37 x 200 21.4 / 14.3, 64 x 1000 33.5 / 31.9,
+    // 4 x 30000 46.9 / 40.4; alone behind a cold L2 the same up to 37 x 4000 (65.5 / 65.5), then 64 x 3000 73.7 / 80.  Tables of up to three
+    // blocks, either way by 10 to 30 %, keep the rule above, and more requests than pairs theirs up to seven (100 x 250 22.4 / 24.5); several kv
+    // heads have not been measured.  A table wider than its requests are long keeps single SMs.
+    const bool on_pairs = h_kv == 1 && s_q * h_q > 32 && s_q * h_q <= MLA_SINGLE_SM_ROWS && table.size(1) >= (b <= pair_parts ? 4 : 8) && b * table.size(1) <= 3000;
+    const Sched sched = schedule(args[7], args[8], sa, pair_parts, pair_parts, whole || on_pairs, device);
     const int parts = sched.parts;
 
     const at::Tensor out = empty({b, s_q, h_q, d_v}, q.scalar_type(), device);

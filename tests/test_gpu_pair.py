@@ -151,3 +151,22 @@ def test_schedules_of_few_long_requests():
             ref, ref_splits = sched_meta.get_sched_meta(len(lengths), parts, 64, 5, seqlens_k=lengths)
             assert torch.equal(got.cpu(), torch.as_tensor(ref, dtype=torch.int32)), (parts, lengths)
             assert splits.tolist() == list(ref_splits), (parts, lengths)
+
+
+@pytest.mark.parametrize("s_q,h_q,lengths,parts", [(1, 64, [200] * 40, 74), (2, 20, [1, 900, 65, 0, 300], 74), (1, 64, [40000, 1, 300], 74), (1, 32, [900] * 4, 148),
+                                                   (1, 33, [700] * 450, 148)])
+def test_dense_33_to_64_rows(s_q, h_q, lengths, parts):
+    """On pairs of SMs up to three thousand blocks of the table, on single SMs beyond and up to 32 rows (148 SMs); either stored schedule."""
+    import flashmla_b200 as fm
+    from flashmla_b200.flash_mla_interface import _make_sched_meta
+    q, k, bt, sl = small._dense_inputs(s_q, h_q, 1, lengths, seed=h_q)
+    bt = bt[:, :(max(lengths) + 63) // 64].contiguous()
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, True)
+    meta = fm.get_mla_metadata()[0]
+    for other in (False, True):
+        if other:
+            meta.tile_scheduler_metadata, meta.num_splits = _make_sched_meta(len(lengths), s_q, 222 - parts, torch.device(DEV), seqlens_k=sl.to(DEV))
+        out, lse = small._dense(q, k, bt, sl, True, meta)
+        assert meta.tile_scheduler_metadata.size(0) == (222 - parts if other else parts)
+        assert_out_close("out", out, ref_out)
+        assert_lse_close("lse", lse, ref_lse)
