@@ -2,7 +2,7 @@
 //   MODE_DENSE          dense BF16 / FP16 paged decode, fed by TMA loads of 64-token KV pages through the block table
 //   MODE_PREFILL        token-sparse prefill, KV rows gathered by index with cp.async
 //   MODE_SPARSE_DECODE  sparse FP8 decode, token records gathered by address, converted in registers
-// Up to 64 rows: attn_rows64.cu (on one SM), or for short prefills this one.
+// Up to 64 rows: attn_rows64.cu (on one SM), or, for short prefills and dense batches of few tokens, this one.
 //
 // Each CTA holds 64 of the 128 rows.  With M = 128 over two CTAs both score and output accumulators split by rows:
 //   S = Q K^T   64 x 128 per CTA in 64 columns    A = Q (chunks 0..5 in tensor memory, the others in shared memory)
