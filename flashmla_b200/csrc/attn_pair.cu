@@ -757,8 +757,9 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             if (pending) {
                 // ---- epilogue -----------------------------------------------------------------------------------------
                 const bool has_tiles = w.ntiles > 0;
-                if (has_tiles) WAIT_WARP_OR_LEAVE(wt, false, &sm.pv_done, (g - 1) & 1, 32);
+                if (has_tiles) wt.template wait<false>(&sm.pv_done, (g - 1) & 1, 32);
                 tc_fence_after();
+                const bool stores = row_ok && !wt.expired();              // (the flag of an expired wait goes on to the next barrier)
                 const bool empty = !(l_run > 0.f) || !has_tiles;         // also catches NaN
                 float scale = empty ? 0.f : 1.f / l_run;
                 if (!DENSE && !w.is_split && p.attn_sink && !empty && row_ok)
@@ -770,8 +771,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 unsigned long long to = 0;                               // where this thread's row goes
                 if (w.is_split) {
                     const int64_t arow = ((int64_t)w.slot * p.s_q + t) * p.h_q + hd;
-                    if (row_ok) to = reinterpret_cast<unsigned long long>(p.o_accum + arow * D_V + dim0);
-                    if (row_ok && quarter == 0) p.lse_accum[arow] = empty ? -INFINITY : log2f(l_run) + m_run;
+                    if (stores) to = reinterpret_cast<unsigned long long>(p.o_accum + arow * D_V + dim0);
+                    if (stores && quarter == 0) p.lse_accum[arow] = empty ? -INFINITY : log2f(l_run) + m_run;
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         uint32_t v[32];
@@ -787,8 +788,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     }
                 } else {
                     const int64_t orow = PREFILL ? ((int64_t)w.req * p.h_q + hd) * D_V : (int64_t)w.req * p.o_sb + (int64_t)t * p.o_ss + (int64_t)hd * p.o_sh;
-                    if (row_ok) to = reinterpret_cast<unsigned long long>(p.out + orow + dim0);
-                    if (row_ok && quarter == 0) {
+                    if (stores) to = reinterpret_cast<unsigned long long>(p.out + orow + dim0);
+                    if (stores && quarter == 0) {
                         const float lse_nat = empty ? INFINITY : (log2f(l_run) + m_run) * kLn2;
                         if (PREFILL) {
                             p.lse[(int64_t)w.req * p.h_q + hd] = lse_nat;
@@ -814,7 +815,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (has_tiles && lane == 0) mbar_arrive_remote_cta(o_empty);
+                if (has_tiles && lane == 0 && !wt.expired()) mbar_arrive_remote_cta(o_empty);
             }
             if (!wk.valid()) break;
             w = wk.get();

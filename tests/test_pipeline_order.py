@@ -157,3 +157,35 @@ def test_the_check_sees_a_missing_order():
     assert not _before(good, ("softmax", "mask", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
     assert not _before(good, ("feed", "done", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
     assert not _before(_graph(masks + 8, slots, tables, False, True), ("softmax", "mask", 3, 0), ("feed", "meta", 3 + 2, 0))
+
+
+# ---- bounded waits in the warps that meet at a named barrier ----------------------------------------------------------
+def _softmax_steps(path):
+    """What the softmax role of a kernel does in program order: ("wait", text), ("leave", text): a thread or warp leaves the role by itself,
+    ("barrier", all leave): the 256 threads meet, and leave together where one says so."""
+    text = open(path).read()
+    start = max(m.start() for m in re.finditer(r"// -+ softmax", text))
+    role = re.sub(r"//[^\n]*", "", text[start:text.index("wind_down:", start)])
+    steps = []
+    for m in re.finditer(r"BAR_OR_LEAVE\(wt\.expired\(\)\)|named_bar_red_or\(1, 256, [^;]*;|named_bar_sync\(1, 256\)|"
+                         r"WAIT_(?:WARP_)?OR_LEAVE\([^;]*;|wt\.template wait\w*<\w+>\([^;]*;|goto wind_down", role):
+        step = m.group()
+        if "bar" in step.lower().split("(")[0]:
+            steps.append(("barrier", "BAR_OR_LEAVE" in step or "goto wind_down" in step))
+        elif step == "goto wind_down":
+            steps.append(("leave", step))
+        else:
+            steps += [("wait", step)] + [("leave", step)] * step.startswith("WAIT_")
+    return steps
+
+
+@pytest.mark.parametrize("path", [SOURCE, ROWS64])
+def test_softmax_threads_leave_together(path):
+    """The 256 softmax threads meet at a named barrier that has no limit of its own.  So a thread whose wait ran out, while another one's
+    did not, must walk on to the next barrier that tells them all."""
+    steps = _softmax_steps(path)
+    waits = [i for i, step in enumerate(steps) if step[0] == "wait"]
+    assert len(waits) == (5 if path == SOURCE else 2)
+    for i in waits:
+        after = [step for step in (steps + steps)[i + 1:] if step != ("barrier", False)]          # (the role is a loop)
+        assert after[0][0] == "wait" or after[0] == ("barrier", True), (steps[i], after[0])
