@@ -95,7 +95,7 @@ constexpr int DATA_BYTES = AT_TAB + NTAB * ROWS * 16;
 struct Smem {
     uint8_t data[DATA_BYTES];
     // (those that only the issuing thread waits on live in CTA 0)  full[s]: the two slots from s on, behind a tile's second two its RoPE chunk too
-    uint64_t full[NSLOT], empty[NSLOT], r_empty[NROPE], p_full[2], k_done[2], f_tail, q_staged, q_taken, q_full, q_ready, s_full, s_empty,
+    uint64_t full[NSLOT], empty[NSLOT], r_empty[NROPE], p_full[2], k_done[2], f_tail, q_staged, q_taken, q_next, q_free, q_full, q_ready, s_full, s_empty,
         pv_done, o_empty, drain;
     uint32_t tmem_base, aborted;
     uint64_t tab_full[NTAB], tab_empty[NTAB];
@@ -109,6 +109,7 @@ template <int N>
 struct RingPos {
     uint32_t slot = 0, par = 0;
     __device__ __forceinline__ void skip(uint32_t n) { slot += n; while (slot >= (uint32_t)N) { slot -= N; par ^= 1; } }
+    __device__ __forceinline__ void skip_many(uint32_t n) { slot += n; par ^= slot / N & 1; slot %= N; }
     __device__ __forceinline__ void next() { if (++slot == (uint32_t)N) { slot = 0; par ^= 1; } }
 };
 
@@ -228,6 +229,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         for (int i = 0; i < NTAB; ++i) { mbar_init(smem_addr(&sm.tab_full[i]), 32); mbar_init(smem_addr(&sm.tab_empty[i]), W::FEED > 0 ? W::FEED : 1); }
         mbar_init(smem_addr(&sm.q_staged), 1);
         mbar_init(smem_addr(&sm.q_taken), 1);
+        mbar_init(smem_addr(&sm.q_next), 1);
+        mbar_init(smem_addr(&sm.q_free), 1);
         mbar_init(smem_addr(&sm.q_full), 1);
         mbar_init(smem_addr(&sm.q_ready), 2);              // one thread of each CTA
         mbar_init(smem_addr(&sm.s_full), 1);
@@ -258,13 +261,19 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         if (elect_one()) {
             RingPos<NSLOT> ring;
             RingPos<NROPE> rope;
-            uint32_t nq = 0;
+            uint32_t nq = 0, n_next = 0;
+            int tiles_before = 0;
             const int chunk0 = hk * p.head_chunks;
             const uint32_t full0 = lead(sm.full[0]);
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
                 const Work w = wk.get();
                 if (w.ntiles == 0) continue;
                 if (p.q_tma) {
+                    // A parity wait only means what it says to a thread for which the barrier's phase before is known to be over, and which
+                    // the phase behind waits for.  In the gather modes this thread does not see the ring's fills: the last Q K^T but one of
+                    // the request before (where it has a single tile, q_taken) says that all but the last releases of these slots are past.
+                    if (!DENSE && tiles_before > 1) { WAIT_OR_LEAVE(wt, false, &sm.q_next, n_next & 1, 12); ++n_next; }
+                    tiles_before = w.ntiles;
                     if (nq > 0) WAIT_OR_LEAVE(wt, false, &sm.q_taken, (nq - 1) & 1, 13);      // q_staged's previous phase is over
                     ++nq;
                     const uint32_t bar = smem_addr(&sm.q_staged);
@@ -310,10 +319,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         rope.next();
                     }
                 } else {
-                    // the feeding warps fill the ring.  A parity wait only means what it says to a thread that has seen every earlier
-                    // phase of the barrier, so this thread follows the ring fill by fill.
-                    for (int i = 0; p.q_tma && i < 4 * w.ntiles; ++i, ring.next())
-                        WAIT_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 12);
+                    ring.skip_many(4 * w.ntiles);
                 }
             }
         }
@@ -377,6 +383,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                             }
                             tc_commit2(smem_addr(&sm.s_full));
                             tc_commit2(smem_addr(&sm.k_done[gq & 1]));
+                            if (!DENSE && qi + 2 == w.ntiles) tc_commit2(smem_addr(&sm.q_next));
+                            if (SPARSE && qi + 1 == w.ntiles) tc_commit2(smem_addr(&sm.q_free));
                             if (WIDE) { tc_commit2(smem_addr(&sm.r_empty[0]) + rope.slot * 8); rope.next(); }
                             stage = 0;
                             ++qi;
@@ -410,7 +418,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         // ---------------- this CTA's half of the dims of the other CTA's page, over chunks that Q K^T has read ----------
         if ((!SPARSE || p.q_tma) && elect_one()) {
             RingPos<NSLOT> ring;
-            uint32_t g = 0;
+            uint32_t g = 0, nq = 0;
             const int chunk0 = hk * p.head_chunks;
             const uint32_t p_full0 = lead(sm.p_full[0]), q_full = lead(sm.q_full);
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
@@ -418,7 +426,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (w.ntiles == 0) continue;
                 if (p.q_tma) {
                     ring.skip(Q_SLOTS);
-                    // (this thread has seen k_done of the previous request's last tile: nothing reads its Q any more)
+                    // nothing reads the previous request's Q any more (otherwise this thread has seen k_done of its last tile)
+                    if (SPARSE && nq++ > 0) WAIT_OR_LEAVE(wt, false, &sm.q_free, nq & 1, 23);
                     if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.q_full), 2 * (CHUNKS - QT) * CHUNK);
 #pragma unroll 1
                     for (int c = QT; c < CHUNKS; ++c)
@@ -428,6 +437,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                                          SPARSE ? (int)blockIdx.y : PREFILL ? w.req : row / p.g, PREFILL ? 0 : w.req);
                         }
                 }
+                if (SPARSE) continue;
                 const int* bt = p.block_table + (int64_t)w.req * p.bt_sb;
                 auto page_of = [&](int blk) -> int { return (blk < w.blk_end && blk < p.max_blocks) ? __ldg(bt + blk) : p.num_blocks; };
                 int nxt = DENSE ? page_of(w.blk_begin + (1 - (int)rank)) : 0;

@@ -159,6 +159,118 @@ def test_the_check_sees_a_missing_order():
     assert not _before(_graph(masks + 8, slots, tables, False, True), ("softmax", "mask", 3, 0), ("feed", "meta", 3 + 2, 0))
 
 
+# ---- the pair kernel's ring across requests: parity waits -------------------------------------------------------------
+# A request takes three slots of the ring for its Q (filled by a thread of warp 0, given back by the softmax warps) and four a tile (filled by
+# the feeding warps, given back behind P V).  A wait for the release of a slot's fill, by parity, is right if the release before
+# that one is ordered before the wait, and the wait before the release behind.
+
+def _request_plan():
+    """Whether warp 0's thread follows the releases of the feeding warps' fills itself, and whether warp 2's (FP8 decode) follows k_done."""
+    text = open(SOURCE).read()
+    loads = text[text.index("own page of every tile"):text.index("MMA issuer (CTA 0")]
+    gather = loads[loads.index("} else {", loads.index("if (DENSE) {")):]
+    other = text[text.index("half of the dims of the other CTA's page"):text.index("FP8 decode: index ->")]
+    loop = other[:other.index("k_done[g & 1]")]
+    return "sm.empty[" in gather, "if (SPARSE) continue;" not in loop
+
+
+def _request_graph(requests, slots, follow, follow_k):
+    """(edges, waits): waits = (the step before the wait, the wait, what must be past when it begins, what must not be past when it ends)."""
+    edges, waits, before = {}, [], {}
+
+    def program(role, steps):
+        for i, step in enumerate(steps):
+            before[(role,) + step] = (role,) + steps[i - 1] if i else None
+            edges[(role,) + step] = [(role,) + steps[i - 1]] if i else []
+
+    q_slots = 3
+    owner, at, first, g = [], 0, [], 0                        # fill -> what gives it back; a request's first fill and first tile
+    for n, t in enumerate(requests):
+        first.append((at, g))
+        owner += [("softmax", "take", n)] * q_slots + [("issue", "values", g + i) for i in range(t) for _ in range(4)]
+        at, g = at + q_slots + 4 * t, g + t
+    release = lambda f: owner[f] if f >= 0 else None
+    load, feed, issue, soft, copy = [], [], [], [], []
+    for n, t in enumerate(requests):
+        f0, g0 = first[n]
+        if n:
+            load += [("next", n)] * (not follow and requests[n - 1] > 1) + [("taken", n)]
+            copy += [("free", n)] * (not follow_k)
+        load += [("q wait", f0 + k) for k in range(q_slots)] + [("q load", n)] + [("follow", f) for f in range(f0 + q_slots, f0 + q_slots + 4 * t)] * follow
+        copy += [("q rest", n)] + [("k_done", i) for i in range(g0, g0 + t)] * follow_k
+        for i in range(t):
+            f = f0 + q_slots + 4 * i
+            feed += [("wait", f + k) for k in range(4)] + [("filled", g0 + i)]
+            soft += [("start", g0 + i), ("p", g0 + i)]
+        soft = soft[:len(soft) - 2 * t] + [("take", n)] + soft[len(soft) - 2 * t:]
+        issue += [("begin", n)] + [("scores", g0)] + [x for i in range(1, t) for x in (("scores", g0 + i), ("values", g0 + i - 1))] + [("values", g0 + t - 1)]
+    for role, steps in (("load", load), ("feed", feed), ("softmax", soft), ("copy", copy)):
+        program(role, steps)
+    # Q K^T of a tile comes before or behind P V of the one before: two chains, joined where the issuing thread takes a request
+    for i, (what, x) in enumerate(issue):
+        edges.setdefault(("issue", what, x), [])
+        if what == "begin" and i:
+            edges["issue", what, x].append(("issue",) + issue[i - 1])
+    for n, t in enumerate(requests):
+        f0, g0 = first[n]
+        edges["issue", "begin", n] += [("softmax", "take", n), ("copy", "q rest", n)]                   # q_ready, q_full
+        edges["softmax", "take", n].append(("load", "q load", n))                                       # q_staged
+        if n:
+            edges["load", "taken", n].append(("softmax", "take", n - 1))
+            if not follow and requests[n - 1] > 1:
+                edges["load", "next", n].append(("issue", "scores", first[n - 1][1] + requests[n - 1] - 2))
+            if not follow_k:
+                edges["copy", "free", n].append(("issue", "scores", g0 - 1))
+        for k in range(q_slots):
+            if release(f0 + k - slots):
+                edges["load", "q wait", f0 + k].append(release(f0 + k - slots))
+        for i in range(g0, g0 + t):
+            f = f0 + q_slots + 4 * (i - g0)
+            edges["issue", "scores", i] += [("issue", "begin", n), ("feed", "filled", i)]               # full
+            edges["issue", "values", i] += [("issue", "scores", i), ("softmax", "p", i)]                # p_full
+            edges["softmax", "start", i].append(("issue", "scores", i))                                 # s_full
+            if i > g0:
+                edges["issue", "scores", i] += [("issue", "scores", i - 1), ("softmax", "start", i - 1)]    # s_empty
+                edges["issue", "values", i].append(("issue", "values", i - 1))
+            if i > g0 + 1:
+                edges["issue", "scores", i].append(("issue", "values", i - 2))                          # at most one tile ahead
+            for k in range(4):
+                if release(f + k - slots):
+                    edges["feed", "wait", f + k].append(release(f + k - slots))
+                    if follow:
+                        edges["load", "follow", f + k].append(release(f + k - slots))
+            if follow_k:
+                edges["copy", "k_done", i].append(("issue", "scores", i))
+    for role, what, f in [e for e in edges if e[1] in ("q wait", "wait", "follow")]:
+        waits.append((before[role, what, f], (role, what, f), release(f - 2 * slots), release(f) if release(f - slots) else None))
+    total = sum(requests)
+    for role, what, i in [e for e in edges if e[1] == "k_done"]:                                        # (two barriers, tiles in turn)
+        waits.append((before[role, what, i], (role, what, i), ("issue", "scores", i - 2) if i >= 2 else None, ("issue", "scores", i + 2) if i + 2 < total else None))
+    return edges, waits
+
+
+def _misread(requests, follow, follow_k, slots=None):
+    edges, waits = _request_graph(requests, slots or _plan()[0], follow, follow_k)
+    return [w for step, w, past, behind in waits
+            if (past and not (step and _before(edges, past, step))) or (behind and not _before(edges, w, behind))]
+
+
+MANY = [[1] * 9, [2] * 8, [3] * 7, [1, 2] * 4, [2, 1, 1, 3, 1, 2, 2, 1], [6, 1, 2, 1, 5], [1, 4, 1, 1, 4, 2], [2, 2, 1, 2, 3, 2, 2], [9, 2, 2, 9]]
+
+
+@pytest.mark.parametrize("convert", [False, True])          # prefill, FP8 decode
+def test_parity_waits_of_the_ring_across_requests(convert):
+    follow, follow_k = _request_plan()
+    for requests in MANY:
+        assert not _misread(requests, follow, follow_k and convert), requests
+
+
+def test_the_check_sees_a_parity_that_may_be_misread():
+    """A thread that watches every phase without anybody waiting for it may see one two phases late."""
+    assert _misread([3] * 7, True, False) and _misread([6], False, True)
+    assert _misread([2] * 8, False, False, slots=4)             # ... and a thread that skips phases nobody has ordered for it
+
+
 # ---- bounded waits in the warps that meet at a named barrier ----------------------------------------------------------
 def _softmax_steps(path):
     """What the softmax role of a kernel does in program order: ("wait", text), ("leave", text): a thread or warp leaves the role by itself,
