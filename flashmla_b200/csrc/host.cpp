@@ -267,13 +267,21 @@ PyObject* dense_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // left to combine.  us, 15 requests of 68 / 100 tokens: 33 to 64 rows 16.6 / 15.9 -> 15.7 / 14.9; up to 32 rows lose nothing.
     const int64_t cost = b * (2 + FIXED_OVERHEAD_NUM_BLOCKS);
     const bool whole = s_q * (h_q / h_kv) > 32 && table.size(1) == 2 && pair_parts <= cost && cost < sa.num_sm_parts;
-    // 33 to 64 rows: a pair of SMs per partition (csrc/attn_pair.cu, half of its rows empty) where the table says that few tokens are to be
-    // read.  A pair takes a tile about as fast as two single SMs two of them, with half the partials and a shorter first tile, but
-    // more power.  us, 64 heads, single SMs / pairs: 1 x 9000 tokens 25.3 / 19.7, 4 x 1000 16.1 / 14.5, 37 x 200 21.4 / 14.3, 64 x 1000 33.5 / 31.9,
-    // 4 x 30000 46.9 / 40.4; alone behind a cold L2 the same up to 37 x 4000 (65.5 / 65.5), then 64 x 3000 73.7 / 80.  Tables of up to three
-    // blocks, either way by 10 to 30 %, keep the rule above, and more requests than pairs theirs up to seven (100 x 250 22.4 / 24.5); several kv
-    // heads have not been measured.  A table wider than its requests are long keeps single SMs.
-    const bool on_pairs = h_kv == 1 && s_q * h_q > 32 && s_q * h_q <= MLA_SINGLE_SM_ROWS && table.size(1) >= (b <= pair_parts ? 4 : 8) && b * table.size(1) <= 3000;
+    // 33 to 64 rows: a pair of SMs per partition (csrc/attn_pair.cu, half of its rows empty), which takes a tile about as fast as two single
+    // SMs two of them, with half the partials and a shorter first tile, but more power.  us, 64 heads, single SMs / pairs: 1 x 9000 tokens
+    // 23.7 / 19.6, 4 x 1000 15.5 / 14.1, 56 x 190 17.4 / 13.1, 4 x 30000 46.4 / 39.5; alone behind a cold L2 the same up to 37 x 4000 (65.5 / 65.5),
+    // then 64 x 3000 73.7 / 80: up to 3000 blocks of the table.
+    //   How long the requests are is known on the device only, and the table may be wider.  So pairs are taken for the batch sizes at which they
+    // hardly lose whatever the lengths are: the two ways to cut a batch differ in how evenly they divide, which follows from the requests per
+    // pair.  Pairs / single SMs over 89 batch sizes x lengths of 30 to 30000 tokens (equal, 1 : 3, lognormal), mean and worst with a stored schedule,
+    // worst with the schedule's time: 1 to 34 requests (74 pairs) 0.87, 1.07, 1.02; 50 to 62 0.83, 1.08, 1.01; 160 to 192 0.93, 1.03, 0.96.
+    // 35 to 49: 0.84, but 1.15 and 1.04 with equal requests of 500 to 1500 tokens, hence tables of up to seven blocks (0.73, 0.91, 0.85).  63 to
+    // 74: 0.88, but 1.36 and 1.22 with requests of one or two blocks; 75 to 148: 1.00, 1.40, 1.20; 193 to 375: 0.98, 1.31, 1.16.
+    //   (Tables of up to three blocks keep the rule above, and more requests than pairs theirs up to seven.  Several kv heads have not been
+    // measured here.)
+    const int64_t width = table.size(1), load = 100 * b / pair_parts;
+    const bool even = load < 47 || (load < 67 && width <= 7) || (load >= 67 && load < 84) || (load >= 216 && load < 260);
+    const bool on_pairs = h_kv == 1 && s_q * h_q > 32 && s_q * h_q <= MLA_SINGLE_SM_ROWS && even && width >= (b <= pair_parts ? 4 : 8) && b * width <= 3000;
     const Sched sched = schedule(args[7], args[8], sa, pair_parts, pair_parts, whole || on_pairs, device);
     const int parts = sched.parts;
 

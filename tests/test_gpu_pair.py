@@ -170,3 +170,19 @@ def test_dense_33_to_64_rows(s_q, h_q, lengths, parts):
         assert meta.tile_scheduler_metadata.size(0) == (222 - parts if other else parts)
         assert_out_close("out", out, ref_out)
         assert_lse_close("lse", lse, ref_lse)
+
+
+@pytest.mark.parametrize("b,width,pairs", [(34, 10, True), (35, 7, True), (35, 8, False), (49, 7, True), (49, 10, False), (50, 8, True), (62, 10, True),
+                                           (63, 6, False), (74, 16, False), (80, 16, False), (128, 8, False), (160, 10, True), (192, 8, True), (193, 10, False)])
+def test_dense_33_to_64_rows_in_wide_tables(b, width, pairs):
+    """A table may be wider than its requests are long: one that holds short requests for which a pair of SMs per partition is slower keeps
+    a partition per SM (148 SMs; 80 requests of 128 tokens in a table 16 wide took 20 us in the place of 14.5)."""
+    import flashmla_b200 as fm
+    lengths = [128 - i % 70 for i in range(b)]
+    q, k, bt, sl = small._dense_inputs(1, 33, 1, lengths, seed=b)
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, False)
+    meta = fm.get_mla_metadata()[0]
+    out, lse = small._dense(q, k, torch.nn.functional.pad(bt[:, :2], (0, width - 2)), sl, False, meta)
+    assert meta.tile_scheduler_metadata.size(0) == (74 if pairs else 148)
+    assert_out_close("out", out, ref_out)
+    assert_lse_close("lse", lse, ref_lse)
