@@ -2,7 +2,6 @@
 // Declarations and the reference interfaces they replace: include/flashmla_b200.h.
 #include "common.cuh"
 
-#include <algorithm>
 #include <mutex>
 #include <string.h>
 
@@ -164,10 +163,11 @@ int mla_dense_decode_fwd(const mla_dense_decode_args_t* a) {
     MLA_CHECK_ARG(a->num_blocks > 0, "mla_dense_decode_fwd: num_blocks must be positive");
     MLA_CHECK_ARG(is_aligned16(a->k_cache) && a->k_stride_block % 8 == 0 && a->k_stride_row % 8 == 0 && a->k_stride_head % 8 == 0,
                   "mla_dense_decode_fwd: k_cache must be 16-byte aligned with strides that are multiples of 8 elements");
-    // 33 to 64 rows run on pairs of SMs where the schedule has no more partitions than there are pairs (the host's choice, see
-    // csrc/host.cpp; us with 74 partitions, single SMs / pairs: 16 requests of 100 tokens 15.3 / 11.7)
+    // 33 to 64 rows run on pairs of SMs where the schedule has no more partitions than there are pairs for every kv head (the host's choice,
+    // see csrc/host.cpp; us with 74 partitions, single SMs / pairs: 16 requests of 100 tokens 15.3 / 11.7, with 37 and two kv heads 8 x 70
+    // 15.8 / 11.7).  More kv heads than pairs have one partition either way and stay on single SMs: 75 of 34 rows, 2 x 128 tokens 21.5 / 28.5.
     const int rows = a->s_q * (a->h_q / a->h_kv);
-    const bool rows64 = rows <= 32 || (rows <= MLA_SINGLE_SM_ROWS && a->num_sm_parts > std::max(1, current_device_num_sms() / 2 / a->h_kv));
+    const bool rows64 = rows <= 32 || (rows <= MLA_SINGLE_SM_ROWS && a->num_sm_parts > current_device_num_sms() / 2 / a->h_kv);
     if (a->impl == 2) {
         if (!dense_decode_sm100_supports(*a))
             return set_error(MLA_ERR_UNSUPPORTED, "mla_dense_decode_fwd: the tcgen05 kernel does not support this shape");

@@ -186,3 +186,25 @@ def test_dense_33_to_64_rows_in_wide_tables(b, width, pairs):
     assert meta.tile_scheduler_metadata.size(0) == (74 if pairs else 148)
     assert_out_close("out", out, ref_out)
     assert_lse_close("lse", lse, ref_lse)
+
+
+def _kernels(call):
+    """Names of the attention kernels that a call launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        call()
+        torch.cuda.synchronize()
+    return {name for e in prof.events() for name in ("attn_pair_kernel", "attn_rows64_kernel", "attn_portable_kernel") if name in e.name}
+
+
+@pytest.mark.parametrize("h_kv,g,lengths,kernel", [(75, 34, [128, 60], "attn_rows64_kernel"), (74, 34, [128, 60], "attn_rows64_kernel"),
+                                                   (2, 64, [70] * 8, "attn_pair_kernel"), (2, 64, [130] * 8, "attn_rows64_kernel")])
+def test_dense_33_to_64_rows_with_several_kv_heads(h_kv, g, lengths, kernel):
+    """As many kv heads as there are pairs and more (148 SMs) have one partition whatever the kernel, and stay on single SMs; fewer are
+    on pairs where the rule for tables of two blocks says so."""
+    q, k, bt, sl = small._dense_inputs(1, h_kv * g, h_kv, lengths, seed=h_kv)
+    bt = bt[:, :(max(lengths) + 63) // 64].contiguous()
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, False)
+    got = []
+    assert _kernels(lambda: got.append(small._dense(q, k, bt, sl, False))) == {kernel}
+    assert_out_close("out", got[0][0], ref_out)
+    assert_lse_close("lse", got[0][1], ref_lse)
