@@ -22,9 +22,12 @@
 //                     b 4          b 32         b 64         b 128        b 1000
 //    74 partitions    6.6 / 5.3    7.0 / 5.8    7.0 / 5.9    7.2 / 6.1    10.8 / 9.3
 //   148 partitions   11.1 / 8.2   11.4 / 8.7   11.8 / 9.0   12.1 / 9.3    15.7 / 12.6
-// Where requests span more than eight partitions each on average, their ends alone are walked, 570 cycles a request: 1, 2, 4, 9 requests of up to
-// 8000 tokens 2.3 / 4.9 / 5.2 / 5.5 -> 2.6 / 3.1 / 3.9 / 5.5 us with 74 partitions, 2.5 / 6.3 / 8.2 / 7.8 -> 2.7 / 3.1 / 3.9 / 5.8 with 148; one
-// of 100003 tokens decoded with 128 heads, schedule included, 48.9 -> 46.3.  (With fewer partitions to a request the chain above is shorter.)
+// Where requests span more than eight partitions each on average, their ends alone are walked, 400 cycles a request, in loops that are
+// not unrolled (a launch fetches its instructions anew: unrolled the walk takes 0.1 to 0.5 us more, and the chain 0.05).  us, the chain / now, requests
+// of one length:              1 x 30     1 x 400    1 x 8000   4 x 1000   4 x 8000   9 x 200    9 x 8000   16 x 1000
+//    74 partitions           2.2 / 2.2  2.4 / 2.5  4.8 / 2.4  3.6 / 3.7  5.0 / 3.5  3.2 / 3.2  5.4 / 5.5  5.1 / 5.2
+//   148 partitions           2.4 / 2.4  2.6 / 2.7  7.6 / 2.5  5.1 / 3.7  7.8 / 3.5  4.0 / 4.1  8.6 / 5.2  6.6 / 6.7
+// (The test that chooses costs every schedule 0.03 to 0.07.)  One of 100003 tokens decoded with 128 heads, schedule included, 48.9 -> 46.3.
 // (A serial walk over the requests by one thread: 6.9, 8.4, 9.8, 12.2, 32 with 148 partitions.  A branch that steps inside a
 // request without the reduction: 6.4, 7.7, 8.8, 10.2, 15.4, but slower than votes and shuffles where requests are short.)
 #include "common.cuh"
@@ -117,22 +120,28 @@ sched_meta_kernel(const mla_sched_meta_args_t a) {
         // the serial chain: where partitions p0 .. begin, and where the last of them ends
         if (threadIdx.x < 32) {
             const int n_all = min(SCHED_THREADS, P - p0);
-            if (P <= SCHED_THREADS && total - (int64_t)b * F > 8 * (int64_t)b * own) {
+            // (either way finds the same starts: the line between them may be rounded)
+            if (P <= SCHED_THREADS && (float)(total - b * F) > 8.f * (float)b * (float)own) {
                 // Requests of more than eight partitions each: as long as no request ends inside the budget the starts lie budget - F
                 // apart, so all of these are written at once and only the requests' ends stand in the chain.
                 int p = 0, r = 0;
+#pragma unroll 1
                 while (p < P && x < total) {
+#pragma unroll 1
                     while (C[r + 1] <= x) ++r;
                     const int gap = C[r + 1] - budget - x, n = gap > 0 ? min((gap + own - 1) / own, P - p) : 0;
+#pragma unroll 1
                     for (int j = lane; j <= n; j += 32) starts[p + j] = x + j * own;
                     p += n;
                     x += n * own;
                     if (p < P) {
+#pragma unroll 1
                         while (r < b && C[r + 1] <= x + budget) ++r;
                         x = min(max(C[r], x + own), total);
                         ++p;
                     }
                 }
+#pragma unroll 1
                 for (int j = p + lane; j <= P; j += 32) starts[j] = x;
             } else
             for (int g0 = 0; g0 < n_all; g0 += 32) {
