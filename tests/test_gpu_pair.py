@@ -188,14 +188,6 @@ def test_dense_33_to_64_rows_in_wide_tables(b, width, pairs):
     assert_lse_close("lse", lse, ref_lse)
 
 
-def _kernels(call):
-    """Names of the attention kernels that a call launches."""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
-        call()
-        torch.cuda.synchronize()
-    return {name for e in prof.events() for name in ("attn_pair_kernel", "attn_rows64_kernel", "attn_portable_kernel") if name in e.name}
-
-
 @pytest.mark.parametrize("h_kv,g,lengths,kernel", [(75, 34, [128, 60], "attn_rows64_kernel"), (74, 34, [128, 60], "attn_rows64_kernel"),
                                                    (2, 64, [70] * 8, "attn_pair_kernel"), (2, 64, [130] * 8, "attn_rows64_kernel")])
 def test_dense_33_to_64_rows_with_several_kv_heads(h_kv, g, lengths, kernel):
@@ -205,6 +197,6 @@ def test_dense_33_to_64_rows_with_several_kv_heads(h_kv, g, lengths, kernel):
     bt = bt[:, :(max(lengths) + 63) // 64].contiguous()
     ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, False)
     got = []
-    assert _kernels(lambda: got.append(small._dense(q, k, bt, sl, False))) == {kernel}
+    assert small.kernels(lambda: got.append(small._dense(q, k, bt, sl, False))) == {kernel}
     assert_out_close("out", got[0][0], ref_out)
     assert_lse_close("lse", got[0][1], ref_lse)

@@ -1,6 +1,8 @@
 """GPU: the kernel for up to 64 query rows on one SM (csrc/attn_rows64.cu) at the sizes where it can go wrong: rows at the edges
 of its variants (16 / 32 / 64), tiles of 128 tokens and their remainders, scores that keep growing, Q that TMA cannot address,
-schedules with another number of partitions.  Against the CPU oracle, within the bounds of tests/helpers.py (element-wise
+schedules with another number of partitions.  (Dense calls with 33 to 64 rows run on pairs of SMs, csrc/attn_pair.cu, where the
+schedule has no more partitions than there are pairs: the tests with one to three partitions or few requests among them; those of
+the kernel on one SM with that many rows ask for a partition per SM.)  Against the CPU oracle, within the bounds of tests/helpers.py (element-wise
 rounding of P and of the output to 16 bits; fp32 sums)."""
 import pytest
 import torch
@@ -116,6 +118,53 @@ def test_dense_maxima_that_move_on_later_tiles(h_q, dtype):
         assert _most_tiles(sched, [(n + 63) // 64 for n in lengths])[1] >= 6
         assert_out_close("out", out, ref_out)
         assert_lse_close("lse", lse, ref_lse)
+
+
+def kernels(call):
+    """Names of the attention kernels that a call launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        call()
+        torch.cuda.synchronize()
+    return {name for e in prof.events() for name in ("attn_pair_kernel", "attn_rows64_kernel", "attn_portable_kernel") if name in e.name}
+
+
+def _dense_on_single_sms(q, k, bt, sl, causal, lengths):
+    """With a partition per SM (148): every CTA that walks the most requests has at least three, the longest request at least five tiles."""
+    got = []
+    assert kernels(lambda: got.append(_dense_parts(q, k, bt, sl, causal, 148))) == {"attn_rows64_kernel"}
+    out, lse, sched = got[0]
+    requests, tiles = _most_tiles(sched, [max(1, (n + 63) // 64) for n in lengths])
+    assert requests >= 3 and tiles >= 5
+    return out, lse
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("s_q,h_q", [(1, 64), (2, 32), (1, 41), (1, 33)])
+def test_dense_33_to_64_rows_several_tiles_and_requests_per_sm(s_q, h_q, dtype):
+    lengths = SEVERAL * 45
+    q, k, bt, sl = _dense_inputs(s_q, h_q, 1, lengths, seed=h_q, dtype=dtype)
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, True)
+    out, lse = _dense_on_single_sms(q, k, bt, sl, True, lengths)
+    assert_out_close("out", out, ref_out)
+    assert_lse_close("lse", lse, ref_lse)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dense_64_rows_maxima_that_move_on_later_tiles(dtype):
+    """As test_dense_maxima_that_move_on_later_tiles, with a partition per SM and requests enough for each to walk whole ones."""
+    lengths = [1500, 129, 700] * 90
+    q, k, bt, sl = _dense_inputs(1, 64, 1, lengths, seed=5, dtype=dtype)
+    # (an output is nearly one key's value: below 4 a step of bf16 is 2^-6, within the bound of 2e-2; from 4 on it is 2^-5, and
+    # 8.8 million values of N(0, 1) hold some)
+    k[..., :512] *= 0.5
+    for b, n in enumerate(lengths):
+        for j, page in enumerate(bt[b, :(n + 63) // 64].tolist()):
+            k[page, :, :, 512:] *= 1.0 + 6.0 * j
+    assert k[..., :512].nan_to_num(0.0).abs().max() < 4
+    ref_out, ref_lse = attention.dense_decode(q, k, bt, sl, 512, False)
+    out, lse = _dense_on_single_sms(q, k, bt, sl, False, lengths)
+    assert_out_close("out", out, ref_out)
+    assert_lse_close("lse", lse, ref_lse)
 
 
 def test_dense_heads_that_share_their_query():
