@@ -842,7 +842,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 tc_fence_after();
                 uint32_t s[32];
                 tmem_ld32(tlane + TM_S + wg * 32, s);
-                const uint32_t valid = DENSE ? 0xffffffffu : sm.mask[g % (2 * NTAB)][quarter];      // (before s_empty: it is what keeps the entry)
+                const uint32_t valid = DENSE ? 0xffffffffu : sm.mask[g % (2 * NTAB)][quarter];      // (P needs it, and P V gives the tile's slots back: that keeps the entry)
                 tmem_wait_ld();
                 tc_fence_before();
                 if (lane == 0 && !wt.expired()) mbar_arrive_remote_cta(s_empty);          // S may be overwritten

@@ -3,8 +3,9 @@ csrc/attn_rows64.cu): the tokens' validity bits, written by the copy or look-up 
 on pairs of SMs the tokens' addresses, read by the converting warps.  Nobody arrives on a barrier of their own for the validity bits, so an
 entry may only be overwritten where the chain of the other barriers already orders its last reader before the writer.
 
-The roles' program order and the barriers between them are written down as a graph; the ring depths, and on which side of
-the arrival that gives the S accumulator back the softmax warps read the mask, come from the source."""
+The roles' program order and the barriers between them are written down as a graph; the ring depths, and in attn_rows64.cu on which
+side of P's arrival the softmax warps read the mask, come from the source.  (In attn_pair.cu the mask is needed for P, and P V of a tile
+gives its slots back: that alone keeps the entry.)"""
 import os
 import re
 
@@ -17,11 +18,11 @@ def _plan():
     text = open(SOURCE).read()
     slots, tables = (int(re.search(r"\b" + name + r" = (\d+)[,;]", text).group(1)) for name in ("NSLOT", "NTAB"))
     assert "uint32_t mask[2 * NTAB][4];" in text and len(re.findall(r"sm\.mask\[\(?g(?: \+ i\))? % \(2 \* NTAB\)\]", text)) == 3
-    read = text.index("sm.mask[g % (2 * NTAB)][quarter]")
-    return slots, 2 * tables, tables, read < text.index("mbar_arrive_remote_cta(s_empty)")
+    assert text.index("sm.mask[g % (2 * NTAB)][quarter]") < text.index("mbar_arrive_remote_cta(p_full0", text.index("float* xmax"))
+    return slots, 2 * tables, tables
 
 
-def _graph(tiles, slots, tables, convert, read_first):
+def _graph(tiles, slots, tables, convert):
     """edges[event] = the events that directly precede it; events are (role, what, tile, slot of the tile)."""
     edges = {}
 
@@ -41,8 +42,7 @@ def _graph(tiles, slots, tables, convert, read_first):
     # (Q K^T of a tile may come before or behind P V of the one before, not earlier)
     program("scores", [("scores", g, q) for g in range(tiles) for q in four])
     program("values", [("values", g, q) for g in range(tiles) for q in four])
-    softmax = lambda g: [("mask", g, 0), ("give", g, 0)] if read_first else [("give", g, 0), ("mask", g, 0)]
-    program("softmax", [s for g in range(tiles) for s in [("start", g, 0)] + softmax(g) + [("p", g, 0)]])
+    program("softmax", [(what, g, 0) for g in range(tiles) for what in ("start", "give", "mask", "p")])
     for g in range(tiles):
         for q in four:
             f = 4 * g + q
@@ -137,9 +137,9 @@ def _before(edges, first, then):
 
 @pytest.mark.parametrize("convert", [False, True])          # prefill, FP8 decode
 def test_ring_entries_are_read_before_they_are_overwritten(convert):
-    slots, masks, tables, read_first = _plan()
+    slots, masks, tables = _plan()
     tiles = masks + 8
-    edges = _graph(tiles, slots, tables, convert, read_first)
+    edges = _graph(tiles, slots, tables, convert)
     writer = "look-up" if convert else "feed"
     for g in range(tiles - masks):
         assert _before(edges, (writer, "meta", g, 0), ("softmax", "mask", g, 0)), "a mask is read after it was written"
@@ -151,12 +151,17 @@ def test_ring_entries_are_read_before_they_are_overwritten(convert):
 
 
 def test_the_check_sees_a_missing_order():
-    """The same graph has no such order with rings of half the depth, nor for the table's entries where a mask of that depth would do."""
-    slots, masks, tables, _ = _plan()
-    good = _graph(masks + 8, slots, tables, True, True)
+    """The same graph has no such order with rings of half the depth, nor for the table's entries where a mask of that depth would do;
+    nor for a mask that is still read when P has been handed over."""
+    slots, masks, tables = _plan()
+    good = _graph(masks + 8, slots, tables, True)
     assert not _before(good, ("softmax", "mask", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
     assert not _before(good, ("feed", "done", 3, 0), ("look-up", "meta", 3 + tables // 2, 0))
-    assert not _before(_graph(masks + 8, slots, tables, False, True), ("softmax", "mask", 3, 0), ("feed", "meta", 3 + 2, 0))
+    assert not _before(_graph(masks + 8, slots, tables, False), ("softmax", "mask", 3, 0), ("feed", "meta", 3 + 2, 0))
+    for convert in (False, True):
+        late = _graph(masks + 8, slots, tables, convert)
+        late["softmax", "p", 3, 0] = [("softmax", "give", 3, 0)]
+        assert not _before(late, ("softmax", "mask", 3, 0), ("look-up" if convert else "feed", "meta", 3 + masks, 0))
 
 
 # ---- the pair kernel's ring across requests: parity waits -------------------------------------------------------------
