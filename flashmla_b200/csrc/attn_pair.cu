@@ -272,15 +272,15 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     // A parity wait only means what it says to a thread for which the barrier's phase before is known to be over, and which
                     // the phase behind waits for.  In the gather modes this thread does not see the ring's fills: the last Q K^T but one of
                     // the request before (where it has a single tile, q_taken) says that all but the last releases of these slots are past.
-                    if (!DENSE && tiles_before > 1) { WAIT_OR_LEAVE(wt, false, &sm.q_next, n_next & 1, 12); ++n_next; }
+                    if (!DENSE && tiles_before > 1) { WAIT_OR_LEAVE(wt, &sm.q_next, n_next & 1, 12); ++n_next; }
                     tiles_before = w.ntiles;
-                    if (nq > 0) WAIT_OR_LEAVE(wt, false, &sm.q_taken, (nq - 1) & 1, 13);      // q_staged's previous phase is over
+                    if (nq > 0) WAIT_OR_LEAVE(wt, &sm.q_taken, (nq - 1) & 1, 13);      // q_staged's previous phase is over
                     ++nq;
                     const uint32_t bar = smem_addr(&sm.q_staged);
                     uint32_t slots[Q_SLOTS];
 #pragma unroll
                     for (int k = 0; k < Q_SLOTS; ++k) {
-                        WAIT_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 11);
+                        WAIT_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 11);
                         slots[k] = ring.slot;
                         ring.next();
                     }
@@ -307,14 +307,14 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         uint32_t bar = 0;
 #pragma unroll 1
                         for (int q = 0; q < 4; ++q, ring.next()) {
-                            WAIT_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 1);
+                            WAIT_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 1);
                             if (!(q & 1)) {
                                 bar = ring.slot;
                                 if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.full[bar]), 4 * SLOT + (q ? 2 * CHUNK : 0));
                             }
                             tma2_load_5d(smem_addr(sm.data) + ring.slot * SLOT, &kmap, full0 + bar * 8, 0, 0, chunk0 + 2 * q, 0, page);
                         }
-                        WAIT_OR_LEAVE(wt, false, &sm.r_empty[rope.slot], rope.par ^ 1, 2);
+                        WAIT_OR_LEAVE(wt, &sm.r_empty[rope.slot], rope.par ^ 1, 2);
                         tma2_load_5d(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK, &rmap, full0 + bar * 8, 0, 0, chunk0 + 8, 0, page);
                         rope.next();
                     }
@@ -342,9 +342,9 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (w.ntiles == 0) continue;
                 if (p.q_tma) {
                     ring.skip(Q_SLOTS);
-                    WAIT_OR_LEAVE(wt, false, &sm.q_full, nq & 1, 3);
+                    WAIT_OR_LEAVE(wt, &sm.q_full, nq & 1, 3);
                 }
-                WAIT_OR_LEAVE(wt, false, &sm.q_ready, nq & 1, 4);
+                WAIT_OR_LEAVE(wt, &sm.q_ready, nq & 1, 4);
                 // Two streams of work: Q K^T of tile qi in two stages (two slots each, the second with the RoPE chunk) as they are filled, and
                 // where the next stage is not there, P V of tile pi.  A probe of a barrier costs this thread 150 to 300 cycles beside the
                 // other roles' traffic, eight MMAs of Q K^T 270 of the tensor core: with few probes it keeps ahead.  (4096 tokens, 576-wide
@@ -427,7 +427,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (p.q_tma) {
                     ring.skip(Q_SLOTS);
                     // nothing reads the previous request's Q any more (otherwise this thread has seen k_done of its last tile)
-                    if (SPARSE && nq++ > 0) WAIT_OR_LEAVE(wt, false, &sm.q_free, nq & 1, 23);
+                    if (SPARSE && nq++ > 0) WAIT_OR_LEAVE(wt, &sm.q_free, nq & 1, 23);
                     if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.q_full), 2 * (CHUNKS - QT) * CHUNK);
 #pragma unroll 1
                     for (int c = QT; c < CHUNKS; ++c)
@@ -444,9 +444,9 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 for (int i = 0; i < w.ntiles; ++i, ++g) {
                     const int page = nxt, blk0 = w.blk_begin + 2 * i;
                     if (DENSE && i + 1 < w.ntiles) nxt = page_of(blk0 + 2 + (1 - (int)rank));
-                    WAIT_OR_LEAVE(wt, false, &sm.k_done[g & 1], (g >> 1) & 1, 21);
+                    WAIT_OR_LEAVE(wt, &sm.k_done[g & 1], (g >> 1) & 1, 21);
                     if (PREFILL) {
-                        WAIT_OR_LEAVE(wt, false, &sm.lf_full[g & 1], (g >> 1) & 1, 22);
+                        WAIT_OR_LEAVE(wt, &sm.lf_full[g & 1], (g >> 1) & 1, 22);
                         fence_proxy_async_smem();          // the copies of this CTA's warps -> visible to its tensor core
                         mbar_arrive_remote_cta(p_full0 + (g & 1) * 8);
                     }
@@ -486,7 +486,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             for (int k = 0; k < 4; ++k) id[k] = w.ntiles > 0 ? load_id(w.blk_begin + (k >> 1), (k & 1) * 32 + lane) : -1;
 #pragma unroll 1
             for (int i = 0; i < w.ntiles; ++i, ++g) {
-                WAIT_WARP_OR_LEAVE(wt, false, &sm.tab_empty[g % NTAB], ((g / NTAB) & 1) ^ 1, 205);
+                WAIT_WARP_OR_LEAVE(wt, &sm.tab_empty[g % NTAB], ((g / NTAB) & 1) ^ 1, 205);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int blk = w.blk_begin + 2 * i + (k >> 1), scope = blk >= w.nblk0 ? 1 : 0, pbs = p.pbs[scope];
@@ -516,7 +516,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             if (ntiles == 0) continue;
             if (p.q_tma) ring.skip(Q_SLOTS);
             for (int i = 0; i < 2 * ntiles; ++i, ring.skip(2)) {
-                WAIT_OR_LEAVE(wt, false, &sm.l_full[ring.slot], (par >> ring.slot) & 1, 24);
+                WAIT_OR_LEAVE(wt, &sm.l_full[ring.slot], (par >> ring.slot) & 1, 24);
                 par ^= 1u << ring.slot;
                 fence_proxy_async_smem();
                 mbar_arrive_remote_cta(full0 + ring.slot * 8);
@@ -565,14 +565,14 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     uint32_t bar = 0;
 #pragma unroll 1
                     for (int q = 0; q < 4; ++q, ring.next()) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 201);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 201);
                         copy_slot(ring.slot, q, row_id, 0);
                         if (!(q & 1)) bar = ring.slot;
                         if (q == 1 || (!WIDE && q == 3)) cp_async_arrive_noinc(smem_addr(&sm.l_full[bar]));
                     }
                     if (WIDE) {
                         const uint32_t rs = (g + i) % NROPE;
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.r_empty[rs], (((g + i) / NROPE) & 1) ^ 1, 202);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty[rs], (((g + i) / NROPE) & 1) ^ 1, 202);
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int tk = 4 * u + (lane >> 3);
@@ -586,7 +586,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (i > 0) {
                     // the other page of tile i - 1, over slots that its Q K^T has read
                     const uint32_t gp = g + i - 1;
-                    WAIT_WARP_OR_LEAVE(wt, false, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
+                    WAIT_WARP_OR_LEAVE(wt, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
                     const uint32_t back = (here ? 8 : 4) - (rank == 0 ? 2 : 0);
 #pragma unroll
                     for (int k = 0; k < 2; ++k) copy_slot((ring.slot + NSLOT - back + k) % NSLOT, 2 * rank + k, before, 8);
@@ -640,7 +640,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 const bool here = i >= 0 && i < ntiles;
                 unsigned long long own = 0, own_sc = 0;
                 if (i + 1 < ntiles) {
-                    WAIT_WARP_OR_LEAVE(wt, false, &sm.tab_full[g % NTAB], (g / NTAB) & 1, 204);
+                    WAIT_WARP_OR_LEAVE(wt, &sm.tab_full[g % NTAB], (g / NTAB) & 1, 204);
                     const ulonglong2 e = tab[g % NTAB * ROWS + rank * PAGE];
                     own = e.x; own_sc = e.y;
                 }
@@ -648,7 +648,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     uint32_t bar = 0;
 #pragma unroll
                     for (int q = 0; q < 4; ++q, ring.next()) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.empty[ring.slot], ring.par ^ 1, 201);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 201);
                         store_share(ring.slot, q, raw[q], rope_raw, M1 ? sc[q & 2] : sc[q]);
                         if (!(q & 1)) bar = lead0 + ring.slot * 8;
                         if (q == 1 || (!WIDE && q == 3)) {
@@ -659,7 +659,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         raw[q] = load_share(own, q, rope_raw);
                     }
                     if (WIDE) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.r_empty[rope.slot], rope.par ^ 1, 202);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty[rope.slot], rope.par ^ 1, 202);
                         st_shared_v4(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK + r * 128 + (((ch * 4 + piece) ^ (r & 7)) << 4), rope_raw);
                         fence_proxy_async_smem();
                         __syncwarp();
@@ -678,7 +678,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (i > 0) {
                     // the other page of tile i - 1 (= g - 2), over slots that its Q K^T has read
                     const uint32_t gp = g - 2;
-                    WAIT_WARP_OR_LEAVE(wt, false, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
+                    WAIT_WARP_OR_LEAVE(wt, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
                     const uint32_t back = (here ? 8 : 4) - (rank == 0 ? 2 : 0);
 #pragma unroll
                     for (int k = 0; k < 2; ++k) store_share((ring.slot + NSLOT - back + k) % NSLOT, 2 * rank + k, raw_o[k], rope_o, sc_o[k]);
@@ -733,7 +733,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (v.ntiles == 0) continue;
                 // (every MMA that read the previous request's Q has completed: this thread saw s_full of its last tile)
                 if (p.q_tma) {
-                    wt.template wait<false>(&sm.q_staged, nq & 1, 31);
+                    wt.wait(&sm.q_staged, nq & 1, 31);
 #pragma unroll 1
                     for (int c = wg * 3; c < wg * 3 + 3; ++c) {
                         const uint8_t* src = sm.data + (q_ring.slot + c / 2) % NSLOT * SLOT + (c & 1) * CHUNK + r * 128;
@@ -767,7 +767,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             if (pending) {
                 // ---- epilogue -----------------------------------------------------------------------------------------
                 const bool has_tiles = w.ntiles > 0;
-                if (has_tiles) wt.template wait<false>(&sm.pv_done, (g - 1) & 1, 32);
+                if (has_tiles) wt.wait(&sm.pv_done, (g - 1) & 1, 32);
                 tc_fence_after();
                 const bool stores = row_ok && !wt.expired();              // (the flag of an expired wait goes on to the next barrier)
                 const bool empty = !(l_run > 0.f) || !has_tiles;         // also catches NaN
@@ -838,7 +838,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             const int limit = min(p.causal ? w.seqlen - (p.s_q - 1 - t) : w.seqlen, w.blk_end * PAGE);
             m_run = -INFINITY; l_run = 0.f; m_true = -INFINITY;
             for (int i = 0; i < w.ntiles; ++i, ++g) {
-                wt.template wait<false>(&sm.s_full, g & 1, 33);
+                wt.wait(&sm.s_full, g & 1, 33);
                 tc_fence_after();
                 uint32_t s[32];
                 tmem_ld32(tlane + TM_S + wg * 32, s);
@@ -888,7 +888,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         }
                     }
                     // P's buffer is free, and O may be touched, when the previous tile's P V has finished
-                    if (pass == 0 && g > 0) wt.template wait<false>(&sm.pv_done, (g - 1) & 1, 34);
+                    if (pass == 0 && g > 0) wt.wait(&sm.pv_done, (g - 1) & 1, 34);
                     if (make && !wt.expired()) {
 #pragma unroll
                         for (int ch = 0; ch < 4; ++ch)
@@ -901,7 +901,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         for (int h = 0; h < 2; ++h) {
                             const int blk = w.blk_begin + 2 * i + h;
                             if (blk < w.blk_end && w.seqlen < (blk + 1) * PAGE) {
-                                if (h != (int)rank) { wt.template wait<false>(&sm.f_tail, ntail & 1, 35); ++ntail; }
+                                if (h != (int)rank) { wt.wait(&sm.f_tail, ntail & 1, 35); ++ntail; }
                                 if (!wt.expired())
                                     for (int n = 0; n < 2; ++n) zero_rows(sm.data + (ring.slot + 2 * h + n) % NSLOT * SLOT, max(w.seqlen - blk * PAGE, 0));
                             }
@@ -982,9 +982,9 @@ __global__ void bounded_wait_selftest_kernel(int* status, uint32_t limit, int co
     if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); flag = 0; fence_mbar_init(); }
     __syncthreads();
     Waiter w(limit);
-    bool ok = threadIdx.x < 32 ? w.wait<false>(&bar, 0, code) : w.wait_warp<false>(&bar, 0, code);
+    bool ok = threadIdx.x < 32 ? w.wait(&bar, 0, code) : w.wait_warp(&bar, 0, code);
     // a second wait by the same thread returns at once
-    if (threadIdx.x < 32) ok = w.wait<false>(&bar, 0, code + 1) || ok;
+    if (threadIdx.x < 32) ok = w.wait(&bar, 0, code + 1) || ok;
     if (w.expired()) report_expired_wait(status, &flag, 0u, w.code);
     __syncthreads();
     if (threadIdx.x == 0 && flag_out) { flag_out[0] = (int)flag; flag_out[1] = ok ? 1 : 0; }

@@ -231,7 +231,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                 if (p.q_tma) {
                     // coordinates: (column, head, query token, request); prefill: a "request" is a query token of the only batch
                     const int c1 = DENSE ? hk * p.g : row0, c2 = DENSE ? 0 : PREFILL ? w.req : (int)blockIdx.y, c3 = PREFILL ? 0 : w.req;
-                    if (nq > 0) WAIT_OR_LEAVE(wt, false, &sm.q_empty, (nq - 1) & 1, 13);
+                    if (nq > 0) WAIT_OR_LEAVE(wt, &sm.q_empty, (nq - 1) & 1, 13);
                     const uint32_t bar = smem_addr(&sm.q_full);
                     mbar_arrive_expect_tx(bar, L::CHUNKS * (uint32_t)p.q_box_bytes);
                     q_armed = ++nq;
@@ -252,7 +252,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                         }
 #pragma unroll 1
                         for (int q = 0; q < 4; ++q, ring.next()) {
-                            WAIT_OR_LEAVE(wt, false, &sm.k_empty[ring.slot], ring.par ^ 1, 1);
+                            WAIT_OR_LEAVE(wt, &sm.k_empty[ring.slot], ring.par ^ 1, 1);
                             const uint32_t bar = smem_addr(&sm.k_full[ring.slot]);
                             mbar_arrive_expect_tx(bar, PAIR_BYTES);
                             ++fills_armed;
@@ -260,7 +260,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                             tma_load_5d(dst, &kmap, bar, 0, 0, chunk0 + 2 * q, 0, page0);
                             tma_load_5d(dst + PAIR_BYTES / 2, &kmap, bar, 0, 0, chunk0 + 2 * q, 0, page1);
                         }
-                        WAIT_OR_LEAVE(wt, false, &sm.r_empty, (nr & 1) ^ 1, 2);
+                        WAIT_OR_LEAVE(wt, &sm.r_empty, (nr & 1) ^ 1, 2);
                         const uint32_t bar = smem_addr(&sm.r_full);
                         mbar_arrive_expect_tx(bar, ROPE_BYTES);
                         ropes_armed = ++nr;
@@ -306,7 +306,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
                 const Work w = wk.get();
                 if (w.ntiles == 0) continue;
-                WAIT_OR_LEAVE(wt, false, &sm.q_full, nq & 1, 3);
+                WAIT_OR_LEAVE(wt, &sm.q_full, nq & 1, 3);
                 ++nq;
                 bool begun = false;                        // the tile's first pair has been done already
                 for (int i = 0; i < w.ntiles; ++i, ++g) {
@@ -315,11 +315,11 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     if (begun) ring.next();
 #pragma unroll 1
                     for (int q = begun ? 1 : 0; q < 4; ++q, ring.next()) {
-                        WAIT_OR_LEAVE(wt, false, &sm.k_full[ring.slot], ring.par, 4);
+                        WAIT_OR_LEAVE(wt, &sm.k_full[ring.slot], ring.par, 4);
                         scores_of_pair(s_tmem, q, ring.slot);
                     }
                     if (WIDE) {
-                        WAIT_OR_LEAVE(wt, false, &sm.r_full, g & 1, 5);
+                        WAIT_OR_LEAVE(wt, &sm.r_full, g & 1, 5);
                         if (!DENSE) fence_proxy_async_smem();      // the feeding warps' stores and copies -> visible to the tensor core
                         tc_fence_after();
 #pragma unroll
@@ -332,7 +332,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     // While the softmax runs: the next tile's first pair, where the ring holds one more than a tile and it is there.
                     begun = EARLY && i + 1 < w.ntiles && mbar_try_wait(smem_addr(&sm.k_full[ring.slot]), ring.par);
                     if (begun) scores_of_pair(tmem + TM_S + ((g + 1) & 1) * NH, 0, ring.slot);
-                    WAIT_OR_LEAVE(wt, false, &sm.p_full, g & 1, 6);
+                    WAIT_OR_LEAVE(wt, &sm.p_full, g & 1, 6);
                     tc_fence_after();
 #pragma unroll 1
                     for (int m = 0; m < 4; ++m, pv.next()) {
@@ -354,7 +354,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         for (WalkerT wk(p, part); wk.valid(); wk.next()) {
             const Work w = wk.get();
             if (w.ntiles == 0) continue;
-            if (nq > 0) WAIT_OR_LEAVE(wt, false, &sm.q_empty, (nq - 1) & 1, 14);
+            if (nq > 0) WAIT_OR_LEAVE(wt, &sm.q_empty, (nq - 1) & 1, 14);
             ++nq;
             for (int k = threadIdx.x - 64; k < rows * L::CHUNKS * 8; k += 64) {
                 const int r = k / (L::CHUNKS * 8), piece = k - r * (L::CHUNKS * 8), c = piece >> 3, u = piece & 7;
@@ -390,7 +390,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     { const int posn = (i + 1) * TILE + tok; id_next = posn < w.seqlen ? __ldg(idx + posn) : -1; }
 #pragma unroll 1
                     for (int q = 0; q < 4; ++q, ring.next()) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.k_empty[ring.slot], ring.par ^ 1, 201);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.k_empty[ring.slot], ring.par ^ 1, 201);
                         if (q == 0 && lane == 0) { reinterpret_cast<uint16_t*>(sm.mask[g & 1])[fw] = (uint16_t)bal; __threadfence_block(); }
                         const uint32_t dst0 = ring0 + ring.slot * PAIR_BYTES;
 #pragma unroll
@@ -403,7 +403,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                         cp_async_arrive_noinc(smem_addr(&sm.k_full[ring.slot]));
                     }
                     if (WIDE) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.r_empty, (g & 1) ^ 1, 202);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty, (g & 1) ^ 1, 202);
                         const uint32_t dst0 = smem_addr(sm.data + L::ROPE) + tok0 * 128;
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
@@ -479,7 +479,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     id_next = load_id(blk0 + 2 * (i + 2));
 #pragma unroll
                     for (int q = 0; q < 4; ++q, ring.next()) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.k_empty[ring.slot], ring.par ^ 1, 201);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.k_empty[ring.slot], ring.par ^ 1, 201);
                         if (q == 0 && lane == 0) {
                             uint32_t bits = 0;
 #pragma unroll
@@ -501,7 +501,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                         load_pair(rec, q);
                     }
                     if (WIDE) {
-                        WAIT_WARP_OR_LEAVE(wt, false, &sm.r_empty, (g & 1) ^ 1, 202);
+                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty, (g & 1) ^ 1, 202);
 #pragma unroll
                         for (int u = 0; u < 2; ++u)
                             st_shared_v4(smem_addr(sm.data + L::ROPE) + tok * 128 + (((2 * piece + u) ^ tl) << 4), rope[u]);
@@ -536,7 +536,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
 #pragma unroll
             for (int c = 0; c < HC; ++c) { l[c] = 0.f; if (PREFILL) top[c] = -INFINITY; }
             for (int i = 0; i < w.ntiles; ++i, ++g) {
-                wt.template wait<false>(&sm.s_full, g & 1, 7);
+                wt.wait(&sm.s_full, g & 1, 7);
                 tc_fence_after();
                 const int blk = w.blk_begin + 2 * i + (tok >> 6), pos = blk * PAGE + (tok & 63);
                 const bool ok = DENSE ? pos < limit : (sm.mask[g & 1][wq] >> lane) & 1u;
@@ -677,7 +677,7 @@ each([&](int c0, uint32_t (&s)[CW]) {
                 }
             }
             const bool has_tiles = w.ntiles > 0;
-            if (has_tiles) { wt.template wait<false>(&sm.o_full, nreq & 1, 8); ++nreq; }
+            if (has_tiles) { wt.wait(&sm.o_full, nreq & 1, 8); ++nreq; }
             if (named_bar_red_or(1, 256, wt.expired())) goto wind_down;
             tc_fence_after();
             if (tid < rows) {

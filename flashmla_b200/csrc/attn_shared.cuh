@@ -50,7 +50,6 @@ struct Params {
 // One unit of work of a partition: a request and the range of its 64-token blocks walked here.
 struct Work {
     int req, blk_begin, blk_end, ntiles, seqlen, is_split, slot;
-    int last;                   // dense decode: the partition's last request (nothing is loaded into the V ring after it)
     int len0, len1, nblk0;      // sparse decode: valid positions of the two index scopes, blocks of the first scope
 };
 
@@ -75,7 +74,6 @@ struct Walker<MODE_DENSE> {
         w.ntiles = (w.blk_end - w.blk_begin + 1) / 2;
         w.is_split = req == m.begin_req_idx ? m.is_first_req_splitted : (req == m.end_req_idx ? m.is_last_req_splitted : 0);
         w.slot = p.num_splits[req] + (req == m.begin_req_idx ? m.begin_split_idx : 0);
-        w.last = req == m.end_req_idx;
         return w;
     }
     __device__ void next() { ++req; }
@@ -139,33 +137,31 @@ template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setm
 // ---- bounded waits -------------------------------------------------------------------------------------------
 // A wait is a loop of probes (the hardware holds a thread for a while before it answers one) and clock reads, compared in 32
 // bits and units of 2^8 cycles.  All roles of a CTA share one instruction cache, and there are some thirty wait sites in
-// their loops: with 64-bit comparisons and the report at every site, 4096-token prefill takes 2870 us in the place of 2800,
-// FP8 decode of 64 requests 95.7 (94.4), of 512-wide records 84.7 (81.6), dense decode the same (back to back, kernels
-// otherwise equal).  Counted in cycles, prefill (2774 against 2790) and dense decode (192.2 against 193.1 for the serving
-// batch) are 0.5 % faster, but limits above 2^32 cycles are lost;
-// waiting for those in several 32-bit spans costs every site a few instructions more: 2920, and FP8 decode 93.6 -> 105.2.
+// their loops.  Measured with the kernel of score and value CTAs that was here before attn_pair.cu (back to back, otherwise equal):
+// with 64-bit comparisons and the report at every site, 4096-token prefill took 2870 us in the place of 2800, FP8 decode of 64
+// requests 95.7 (94.4), of 512-wide records 84.7 (81.6), dense decode the same.  Counted in cycles, prefill (2774 against 2790) and
+// dense decode (192.2 against 193.1 for the serving batch) were 0.5 % faster, but limits above 2^32 cycles are lost; waiting for
+// those in several 32-bit spans cost every site a few instructions more: 2920, and FP8 decode 93.6 -> 105.2.
 // A thread whose wait ran out only keeps the site's code; it reports when it has left its role.
 //
-// wait() / wait_warp() return false when the wait ran out now or earlier: the caller leaves its role.  CLUSTER: the
-// arrivals come from the other CTA of the pair.
+// wait() / wait_warp() return false when the wait ran out now or earlier: the caller leaves its role.  Arrivals of the other CTA of a
+// pair are waited for at CTA scope too: what they announce is not read by the waiting thread (mbar_arrive_remote_cta, sm100_ptx.cuh).
 struct Waiter {
     uint32_t limit;                      // units of 2^WAIT_UNIT_LOG2 SM cycles
     int code = 0;
     __device__ explicit Waiter(uint32_t limit_) : limit(limit_) {}
     __device__ __forceinline__ bool expired() const { return code != 0; }
-    template <bool CLUSTER>
     __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int site) {
         if (expired()) return false;
         const uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
-        while (!(CLUSTER ? mbar_try_wait_cluster(smem_addr(bar), parity) : mbar_try_wait(smem_addr(bar), parity)))
+        while (!mbar_try_wait(smem_addr(bar), parity))
             if (clock_units<WAIT_UNIT_LOG2>() - t0 > limit) { code = site; break; }
         return !expired();
     }
     // whole warps (all 32 lanes execute this): the same answer for every lane
-    template <bool CLUSTER>
     __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, int site) {
-        wait<CLUSTER>(bar, parity, site);
+        wait(bar, parity, site);
         return !__any_sync(0xffffffffu, expired());
     }
 };
@@ -177,10 +173,9 @@ static __device__ __noinline__ void report_expired_wait(int* status, uint32_t* f
 }
 
 // single-thread roles: leave at once
-#define WAIT_OR_LEAVE(W, CL, bar, par, code) do { if (!(W).template wait<CL>(bar, par, code)) goto wind_down; } while (0)
+#define WAIT_OR_LEAVE(W, bar, par, code) do { if (!(W).wait(bar, par, code)) goto wind_down; } while (0)
 // whole warps (all 32 lanes execute this): leave together, tcgen05.ld/st and shuffles are warp-collective
-#define WAIT_WARP_OR_LEAVE(W, CL, bar, par, code) \
-    do { if (!(W).template wait_warp<CL>(bar, par, code)) goto wind_down; } while (0)
+#define WAIT_WARP_OR_LEAVE(W, bar, par, code) do { if (!(W).wait_warp(bar, par, code)) goto wind_down; } while (0)
 
 __device__ __forceinline__ float ex2(float x) {
     float y;

@@ -30,8 +30,8 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 
 // True in one lane of the warp, which executes this together.  The MMA issuing thread is chosen with it: behind any other
-// condition (lane == 0) the compiler does not know that a single thread runs the branch and wraps every MMA in a loop over the
-// active lanes.  Cycles per MMA in a chain of them, lane == 0 -> elected: 128 x 16 x 16 50 -> 39.5, 128 x 64 x 16 50 -> 48.7,
+// condition (lane == 0) the compiler is not told that a single thread runs the branch, and an MMA takes 50 cycles at least,
+// whatever its size.  Cycles per MMA in a chain of them, lane == 0 -> elected: 128 x 16 x 16 50 -> 39.5, 128 x 64 x 16 50 -> 48.7,
 // 128 x 128 x 16 65.1 -> 65.0.  What is left is shared-memory bandwidth: both operands at 128 bytes a cycle.
 __device__ __forceinline__ bool elect_one() {
     uint32_t r;
@@ -54,6 +54,9 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 
 // Remote arrive that orders this thread's earlier operations inside its own CTA only: for data that stays in this CTA and is
 // read by its tensor core when CTA 0 of the pair issues an MMA for both (1300 cycles less than the cluster-wide release).
+// That this is enough is an argument about the hardware - the data is read where it was written, after the proxy fence of the
+// thread that wrote it - and not about the PTX memory model, which orders it for a thread of CTA 0, and what that issues, with
+// cluster scope on both sides only.
 __device__ __forceinline__ void mbar_arrive_remote_cta(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
@@ -73,16 +76,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// try_wait with acquire semantics at cluster scope (the arrival came from another CTA).
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
@@ -148,10 +141,9 @@ __device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* m, int c0, in
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
-// Arrive on `bar` (counted among its expected arrivals) once all cp.async copies this thread issued so far have landed.
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Waits until every cp.async copy this thread has issued has landed.
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Arrive on `bar` (counted among its expected arrivals) once all cp.async copies this thread issued so far have landed.
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }

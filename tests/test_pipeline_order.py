@@ -78,7 +78,7 @@ def _plan64():
     read = text.index("(sm.mask[g & 1][wq] >> lane)")
     for write in re.finditer(r"sm\.mask\[g & 1\]\)\[fw\] = ", text):
         guard = text.rindex("if (q == 0 && lane == 0)", 0, write.start())
-        wait = text.rindex("WAIT_WARP_OR_LEAVE(wt, false, &sm.k_empty[ring.slot]", 0, guard)
+        wait = text.rindex("WAIT_WARP_OR_LEAVE(wt, &sm.k_empty[ring.slot]", 0, guard)
         assert "for (int q = 0; q < 4; ++q" in text[wait - 120:wait]
     return slots, masks.pop(), read < text.index("mbar_arrive(smem_addr(&sm.p_full))")
 
@@ -285,7 +285,7 @@ def _softmax_steps(path):
     role = re.sub(r"//[^\n]*", "", text[start:text.index("wind_down:", start)])
     steps = []
     for m in re.finditer(r"BAR_OR_LEAVE\(wt\.expired\(\)\)|named_bar_red_or\(1, 256, [^;]*;|named_bar_sync\(1, 256\)|"
-                         r"WAIT_(?:WARP_)?OR_LEAVE\([^;]*;|wt\.template wait\w*<\w+>\([^;]*;|goto wind_down", role):
+                         r"WAIT_(?:WARP_)?OR_LEAVE\([^;]*;|wt\.wait\w*\([^;]*;|goto wind_down", role):
         step = m.group()
         if "bar" in step.lower().split("(")[0]:
             steps.append(("barrier", "BAR_OR_LEAVE" in step or "goto wind_down" in step))
