@@ -25,25 +25,24 @@
 //
 // What bounds it: one tile is in flight, so a tile's period is the chain  fill -> Q K^T (36 MMAs) -> softmax -> P V (32 MMAs); an
 // MMA of 128 x NH x 16 takes what its operands take to be read, 40 SM cycles (NH = 16) to 49 (64).
-// (Cycles a tile, measured when the issuing thread made it 56:)  Dense decode with up to 32 / 64 rows: 5200-5800 / 6600 cycles a tile, the
-// fills behind P V (the next tile's pages are prefetched into L2 while this one is worked on: with 64 rows 8500 cycles without).
-// Prefill, 64 heads: 8500 cycles, of which the copies 3000 and P V slowed by them 2500.  FP8 decode, 64 heads: 8500-10000, conversion
-// and its loads 4500-6000 of them.  us a call, pairs of SMs for every shape (score and value CTAs, no longer here) -> now, inputs changing from call to call, clocks settled:
+// us a tile on all SMs at once (148 lists of two lengths, short runs of one input): dense, 16 / 32 / 64 rows 3.2 / 3.2 / 3.5, of which
+// DRAM's rate asks for 3.3 (the fills come behind P V; the next tile's pages are prefetched into L2 while this one is worked on: a
+// third longer with 64 rows without); prefill, 64 heads 3.35 (576-wide) and 2.95, copies and P V slowed by them; FP8, 64 heads 6.0 and
+// 4.9, 16 heads 4.8 and 3.6, conversion and its loads two thirds of them.
+// us a call, pairs of SMs for every shape (score and value CTAs, no longer here) -> now, inputs changing from call to call, clocks settled:
 //   dense, 4 requests of 64..512, 16 heads     18.3 ->  13.1    dense fp16, 61 x 4096, 16 heads     95.9 ->  64.4
 //   FP8, 2 x 2 x 2048, 64 heads, schedule too  26.2 ->  21.7    prefill 512-wide, 117 tokens, ragged 38.8 ->  30.6
-// and with the issuing thread elected (elect_one, sm100_ptx.cuh) 13.4 -> 12.6, 63.7 -> 62.1, 22.1 -> 21.7 and 30.6 -> 24.4,
+// and with the issuing thread elected (elect_one, sm100_ptx.cuh) 13.4 -> 12.6, 63.8 -> 62.1, 22.1 -> 21.7 and
+// 30.6 -> 24.4,
 // and one input in short runs:
 //   dense, 30 x 2048, 8 heads                  32.8 ->  23.7    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 68.7 / 78.0
 //   FP8, 64 x 2048, 16 heads                   93.3 ->  54.7    FP8, 74 x 2048, 64 heads            95.9 ->  82.2
 //   prefill, 512 x 2048, 64 heads               333 ->   308    prefill, 2000 x 1024, 64 heads       677 ->   564
-// What loses: dense decode with 33 to 64 rows where as many pairs of SMs as requests left every request whole - 37 to 74 requests of
-// nearly the same, short length.  One input, us, pairs -> now, with 64 heads: 45 x 200 tokens 17.5 -> 21.2, 64 x 300 20.0 -> 24.7,
-// 64 x 400 21.9 -> 24.7, 56 x 800 26.8 -> 28.8, 70 x 1000 32.3 -> 35.4, 64 x 2048 56.0 -> 54.5.  With lengths spread by 30 % pairs cut
-// requests as well (64 x 200 27.8 -> 21.4), and the lengths are known on the device only, so no rule of the host tells them apart.
-// (Where the block table says that few tokens are to be read, 33 to 64 rows run on pairs of SMs: see csrc/host.cpp.)
+// Dense decode with 33 to 64 rows runs on pairs of SMs (attn_pair.cu) for batch sizes at which that hardly loses whatever the lengths are, where the block
+// table says that few tokens are to be read: see csrc/host.cpp.
 // Registers: at the launch bound of the FP8 variants 36 to 76 bytes are spilled (576-wide 64 / 16 heads 76 / 56, 512-wide 64 heads 36,
 // 16 none); where they are reloaded has not been established.  Dense and prefill: none.
-// FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101 against 91.5), since both CTAs convert
+// FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101, pairs 56), since both CTAs convert
 // every record.
 //
 // Bounded waits and the wind-down are those of attn_pair.cu (attn_shared.cuh).

@@ -99,7 +99,8 @@ int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q) {
     }
     if (mode == MLA_MODE_DENSE_DECODE) {
         // A partition is walked, for every block of 128 query rows of every kv head, by a pair of CTAs on two
-        // SMs (the tcgen05 kernel's or the portable kernel's two 64-row CTAs); up to 64 rows take one CTA.
+        // SMs (the tcgen05 kernel's or the portable kernel's two 64-row CTAs); up to 64 rows take one CTA (33 to 64 a pair where a
+        // schedule has been made with half of this count, see mla_dense_decode_fwd).
         const int rows = s_q * (h_q / h_kv);
         const int row_blocks = (rows + 127) / 128;
         int p = (rows <= MLA_SINGLE_SM_ROWS ? sms : sms / 2) / h_kv / row_blocks;

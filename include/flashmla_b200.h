@@ -64,7 +64,9 @@ int mla_abi_version(void);
 #define MLA_SINGLE_SM_ROWS 64
 
 /* Number of SM partitions the decode kernels of `mode` use on `device` for a
- * launch with these head counts / query length (the kernels take any other number of a schedule too).  Stands in for the expression in
+ * launch with these head counts / query length (the kernels take any other number of a schedule too).  For dense decode with 33 to 64
+ * rows the number of a schedule also chooses the kernel: up to (SMs / 2) / h_kv of them run on pairs of SMs, more, and h_kv above
+ * SMs / 2, on single ones.  This function returns the count for single SMs.  Stands in for the expression in
  * csrc/api/dense_decode.h:78 and DecodeImplBase::get_meta
  * (csrc/api/sparse_decode.h:92-99,126-133).  Returns <= 0 on error. */
 int mla_num_sm_parts(int device, int mode, int h_q, int h_kv, int s_q);
@@ -125,7 +127,7 @@ typedef struct {
 
     const mla_sched_meta_t* meta;     /* [num_sm_parts]                                        */
     const int32_t* num_splits;        /* [b + 1]                                               */
-    int32_t num_sm_parts;
+    int32_t num_sm_parts;             /* chooses the kernel for 33 to 64 rows, see mla_num_sm_parts */
 
     float* lse_accum;                 /* scratch fp32 [b + num_sm_parts, s_q, h_q]   (base-2 LSE of each split) */
     float* o_accum;                   /* scratch fp32 [b + num_sm_parts, s_q, h_q, d_v]        */
