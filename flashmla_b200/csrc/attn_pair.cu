@@ -1,6 +1,6 @@
 // MLA attention for up to 128 query rows on a PAIR of SMs whose MMAs span both (sm_100a, tcgen05 with cta_group::2).  One kernel template:
 //   MODE_DENSE          dense BF16 / FP16 paged decode, fed by TMA loads of 64-token KV pages through the block table
-//   MODE_PREFILL        token-sparse prefill, KV rows gathered by index with cp.async
+//   MODE_PREFILL        token-sparse prefill, KV rows gathered by index: the own page's with cp.async, the other page's with TMA
 //   MODE_SPARSE_DECODE  sparse FP8 decode, token records gathered by address, converted in registers
 // Up to 64 rows: attn_rows64.cu (on one SM), or, for short prefills and dense batches of few tokens, this one.
 //
@@ -16,12 +16,17 @@
 // One instruction's descriptors name the same offsets in both CTAs.  A tile takes four slots of a ring, slot q holding chunks 2 q and
 // 2 q + 1 of the CTA's own page.  CTA 0 serves the dims of slots 0 and 1, CTA 1 those of 2 and 3.  P V of page h reads slots 2 h and
 // 2 h + 1: in CTA h that is its own page's half of the dims, in place since Q K^T; in the other CTA those slots held dims it does
-// not serve, which Q K^T alone needed - behind it they are filled again with page h's dims that it serves.
+// not serve, which Q K^T alone needed - behind it they are filled again with page h's dims that it serves.  CTA 1's are in Q K^T's first
+// half (k_half), CTA 0's in the second (k_done), and P V is issued page by page: page 0, whose other part is there first, gives the
+// slots back that the tile after next waits for while page 1 is still on its way.
+//
+// The RoPE chunks have two buffers of their own, and nobody waits for those: a tile's last two slots are given back by P V of page 0 of
+// the tile before last or later, or by the hand-over of a Q behind that tile, and its Q K^T is older than either.
 //
 // Softmax: warps 4..11, a thread = one row, one page, half of the page's tokens.  P is made with the maximum in use on the guess that no
-// row has outgrown it by 2^6; the named barrier behind P's stores carries the votes, and where the guess was wrong (and on a
-// request's first tile) the maxima are exchanged, O is rescaled and P is made again.  P, the row sums and O always refer to the
-// same maximum, so results are exact up to rounding.
+// row has outgrown it by 2^6.  The warps vote on that before they make P, on an mbarrier, so that the answer is there when P is; every warp
+// hands its part of P over by itself.  Where the guess was wrong (and on a request's first tile) all meet, the maxima are exchanged, O is
+// rescaled and P is made again.  P, the row sums and O always refer to the same maximum, so results are exact up to rounding.
 //
 // CTA 0's issuing thread takes whatever is ready: Q K^T of the next tile slot by slot, or P V of the last one.  It is chosen with
 // elect_one (sm100_ptx.cuh).  A chain of these MMAs takes 33 cycles per 128 x 128 x 16 and 65 per 128 x 256 x 16.  Arrivals on CTA 0's
@@ -30,8 +35,9 @@
 //
 // What bounds it.  Dense decode, 128 requests of about 4096 tokens: 2700 to 3300 cycles a tile, of which the tensor core works 2250 (60 % of
 // the launch); DRAM at 4.9 TB/s in a launch by itself (136 us at 1.63 GHz), back to back the power limit (1.34 GHz).  A tile's loads wait for
-// P V two tiles before, 2000 to 2900 cycles before they have landed.  Prefill: 3700 cycles a tile, the tensor core 2250, the copies (208
-// instructions an SM, 14.5 cycles each at best) 3000 or more; back to back the power limit (1.55 GHz).  FP8 decode: 5200 cycles a tile,
+// P V two tiles before, 2000 to 2900 cycles before they have landed.  Prefill: 3700 cycles a tile, the tensor core 2250, the own page's copies
+// (144 instructions an SM, 14.5 cycles each at best) and the other page's row gathers (64 of TMA, 20 each) beside each other; back to back the
+// power limit (1.6 GHz).  FP8 decode: 5200 cycles a tile,
 // the feeding warps' conversion (six slots' worth, 64 x 128 values each, 450-600 cycles apiece) and the chain conversion -> Q K^T ->
 // softmax -> P V behind a ring of two and a half tiles.  One copy of every converted value would save a third of the conversion but the
 // exchange costs more: by 16-byte asynchronous stores into the other SM 93 us, by bulk copies 75.5, converting the half of the
@@ -44,13 +50,15 @@
 //   dense, 128 x ~4096 tokens                    185 ->  172       189 ->  173
 //   dense, two query tokens                      314 ->  294       325 ->  300
 //   dense, one request of 100003 tokens                           54.9 -> 47.8
+// and with P V page by page, the vote on an mbarrier and no wait for the RoPE buffers (inputs changing): FP8 60.5 -> 58.3, prefill 2324 -> 2242,
+// dense 180.4 -> 178.3, two query tokens 306 -> 302, 128 requests of lognormal lengths 536 -> 522.
 // (914 calls of dense and FP8 decode and prefill with 64 to 128 heads: between 1.04 and 2.0 times as fast, none slower.)
 // Registers: both FP8 forms spill 12 bytes a thread (24 reloaded), the others none.
 //
 // Every mbarrier wait is bounded (Params::wait_limit SM cycles, about a second by default).  A thread whose wait ran out LEAVES its role -
 // it issues no further arrival, MMA or copy -, records a code in the status words and raises the `aborted` flag of both CTAs.
 // Single-thread roles leave at once; warps leave together (a vote after every wait, because tcgen05.ld/st are warp-collective); the softmax
-// warpgroups, which meet at a named barrier every tile, carry the flag through that barrier (bar.red.or) and leave behind it.  Threads that
+// warpgroups vote against the guess, meet at a named barrier that carries the flag (bar.red.or) and leave behind it.  Threads that
 // depend on the one that left run into their own limit.  The wind-down then waits - again bounded - for the MMAs, meets the peer
 // CTA, gives loads still under way time to land, and only then frees tensor memory; both CTAs leave together.
 //
@@ -96,11 +104,11 @@ constexpr int DATA_BYTES = AT_TAB + NTAB * ROWS * 16;
 struct Smem {
     uint8_t data[DATA_BYTES];
     // (those that only the issuing thread waits on live in CTA 0)  full[s]: the two slots from s on, behind a tile's second two its RoPE chunk too
-    uint64_t full[NSLOT], empty[NSLOT], r_empty[NROPE], p_full[2], k_done[2], f_tail, q_staged, q_taken, q_next, q_free, q_full, q_ready, s_full, s_empty,
-        pv_done, o_empty, drain;
-    uint32_t tmem_base, aborted;
+    uint64_t full[NSLOT], empty[NSLOT], p_full[2][2], k_done[2], k_half[2], f_tail, q_staged, q_taken, q_next, q_free, q_full, q_ready, s_full, s_empty,
+        pv_done, o_empty, vote[2], drain;
+    uint32_t tmem_base, aborted, outgrown[2];
     uint64_t tab_full[NTAB], tab_empty[NTAB];
-    uint64_t l_full[NSLOT], lf_full[2];     // prefill: this CTA's copies (as full) / of the other page have landed
+    uint64_t l_full[NSLOT];                       // prefill: this CTA's copies (as full) have landed
     uint32_t mask[2 * NTAB][4];                   // gather modes: validity bits of a tile's tokens
 };
 static_assert(sizeof(Smem) <= 232448, "shared memory budget");
@@ -114,6 +122,8 @@ struct RingPos {
     __device__ __forceinline__ void next() { if (++slot == (uint32_t)N) { slot = 0; par ^= 1; } }
 };
 
+// (a barrier that is ready costs a probe and a vote)
+#define READY_OR_WAIT(W, bar, par, code) do { if (!__all_sync(0xffffffffu, mbar_try_wait(smem_addr(bar), par))) WAIT_WARP_OR_LEAVE(W, bar, par, code); } while (0)
 // the softmax warpgroups' named barrier carries the flag of an expired wait
 #define BAR_OR_LEAVE(flag) do { if (named_bar_red_or(1, 256, flag)) goto wind_down; } while (0)
 
@@ -220,12 +230,12 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         // a slot is filled by TMA (one arrival and bytes), by both CTAs' copies (one relaying thread each), or by both CTAs' feeding warps
         const uint32_t fill = DENSE ? 1 : PREFILL ? 2 : 2 * W::FEED;
         for (int i = 0; i < NSLOT; ++i) { mbar_init(smem_addr(&sm.full[i]), fill); mbar_init(smem_addr(&sm.empty[i]), 1); }
-        for (int i = 0; i < NROPE; ++i) mbar_init(smem_addr(&sm.r_empty[i]), 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(smem_addr(&sm.p_full[i]), 2 + fill); mbar_init(smem_addr(&sm.k_done[i]), 1); }
+        for (int i = 0; i < 4; ++i) mbar_init(smem_addr(&sm.p_full[i >> 1][i & 1]), SPARSE ? 8 + W::FEED : PREFILL ? 8 : 9);
+        for (int i = 0; i < 2; ++i) mbar_init(smem_addr(&sm.vote[i]), 8);
+        for (int i = 0; i < 2; ++i) { mbar_init(smem_addr(&sm.k_done[i]), 1); mbar_init(smem_addr(&sm.k_half[i]), 1); }
         mbar_init(smem_addr(&sm.f_tail), 1);
         if (PREFILL) {
             for (int i = 0; i < NSLOT; ++i) mbar_init(smem_addr(&sm.l_full[i]), 32 * W::FEED);
-            for (int i = 0; i < 2; ++i) mbar_init(smem_addr(&sm.lf_full[i]), 32 * W::FEED);
         }
         for (int i = 0; i < NTAB; ++i) { mbar_init(smem_addr(&sm.tab_full[i]), 32); mbar_init(smem_addr(&sm.tab_empty[i]), W::FEED > 0 ? W::FEED : 1); }
         mbar_init(smem_addr(&sm.q_staged), 1);
@@ -240,8 +250,10 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         mbar_init(smem_addr(&sm.o_empty), 16);
         mbar_init(smem_addr(&sm.drain), 1);
         sm.aborted = 0;
+        sm.outgrown[0] = sm.outgrown[1] = 0;
         fence_mbar_init();
-        if (DENSE) { prefetch_tensormap(&kmap); prefetch_tensormap(&rmap); }
+        if (!SPARSE) prefetch_tensormap(&kmap);
+        if (DENSE) prefetch_tensormap(&rmap);
         if (p.q_tma) prefetch_tensormap(&qmap);
     }
     if (warp == 1) { tmem_alloc2(smem_addr(&sm.tmem_base), 512); tmem_relinquish2(); }
@@ -315,7 +327,6 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                             }
                             tma2_load_5d(smem_addr(sm.data) + ring.slot * SLOT, &kmap, full0 + bar * 8, 0, 0, chunk0 + 2 * q, 0, page);
                         }
-                        WAIT_OR_LEAVE(wt, &sm.r_empty[rope.slot], rope.par ^ 1, 2);
                         tma2_load_5d(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK, &rmap, full0 + bar * 8, 0, 0, chunk0 + 8, 0, page);
                         rope.next();
                     }
@@ -334,7 +345,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             const uint32_t p_lo = sw128_desc_lo(smem_addr(sm.data) + AT_P, 16);
             constexpr uint32_t d_s = tmem + TM_S, d_o = tmem + TM_O, a_q = tmem + TM_Q;
             const uint32_t full0 = smem_addr(&sm.full[0]), empty0 = smem_addr(&sm.empty[0]);
-            const uint32_t p_full0 = smem_addr(&sm.p_full[0]), s_empty = smem_addr(&sm.s_empty), o_empty = smem_addr(&sm.o_empty);
+            const uint32_t p_full0 = smem_addr(&sm.p_full[0][0]), s_empty = smem_addr(&sm.s_empty), o_empty = smem_addr(&sm.o_empty);
             RingPos<NSLOT> ring;
             RingPos<NROPE> rope;
             uint32_t g = 0, nq = 0, full_par = 0;          // full_par: bit s is the parity of slot s's next fill with K
@@ -351,7 +362,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 // other roles' traffic, eight MMAs of Q K^T 270 of the tensor core: with few probes it keeps ahead.  (4096 tokens, 576-wide
                 // prefill: all barriers probed at every step 2620 us, one stage per slot 2320.)
                 RingPos<NSLOT> pv = ring;
-                int qi = 0, pi = 0, stage = 0;
+                int qi = 0, pi = 0, stage = 0, half = 0;
                 auto is = [&](uint32_t bar, uint32_t par) { return mbar_test_wait(bar, par & 1); };
                 uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
@@ -372,6 +383,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
 #pragma unroll
                             for (int k = 0; k < 8; ++k)
                                 mma2_ts_lohi(d_s, a_q + 64 + k * 8, b_lo + (k >> 2) * (1024 >> 4) + (k & 3) * 2, hi_slot, idesc_s, 1u);
+                            tc_commit2(smem_addr(&sm.k_half[gq & 1]));
                             stage = 1;
                         } else {
 #pragma unroll
@@ -385,26 +397,24 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                             tc_commit2(smem_addr(&sm.s_full));
                             tc_commit2(smem_addr(&sm.k_done[gq & 1]));
                             if (!DENSE && qi + 2 == w.ntiles) tc_commit2(smem_addr(&sm.q_next));
-                            if (SPARSE && qi + 1 == w.ntiles) tc_commit2(smem_addr(&sm.q_free));
-                            if (WIDE) { tc_commit2(smem_addr(&sm.r_empty[0]) + rope.slot * 8); rope.next(); }
+                            if (qi + 1 == w.ntiles) tc_commit2(smem_addr(&sm.q_free));
+                            if (WIDE) rope.next();
                             stage = 0;
                             ++qi;
                         }
-                    } else if (pi < qi && is(p_full0 + (gp & 1) * 8, gp >> 1) && (pi > 0 || is(o_empty, nq + 1))) {
+                    } else if (pi < qi && is(p_full0 + (gp & 1) * 16 + half * 8, gp >> 1) && (pi > 0 || half > 0 || is(o_empty, nq + 1))) {
                         tc_fence_after();
-#pragma unroll 1
-                        for (int h = 0; h < 2; ++h)
 #pragma unroll
-                            for (int n = 0; n < 2; ++n, pv.next()) {
-                                const uint32_t b_lo = v_lo + pv.slot * (SLOT >> 4), a_lo = p_lo + h * (CHUNK >> 4);
+                        for (int n = 0; n < 2; ++n, pv.next()) {
+                            const uint32_t b_lo = v_lo + pv.slot * (SLOT >> 4), a_lo = p_lo + half * (CHUNK >> 4);
 #pragma unroll
-                                for (int kt = 0; kt < 4; ++kt)
-                                    mma2_ss_lohi(d_o + n * 128, a_lo + kt * 2, hi_row, b_lo + kt * (4096 >> 4), hi_slot, idesc_o,
-                                                 (pi > 0 || h > 0 || kt > 0) ? 1u : 0u);
-                                tc_commit2(empty0 + pv.slot * 8);
-                            }
-                        tc_commit2(smem_addr(&sm.pv_done));
-                        ++pi;
+                            for (int kt = 0; kt < 4; ++kt)
+                                mma2_ss_lohi(d_o + n * 128, a_lo + kt * 2, hi_row, b_lo + kt * (4096 >> 4), hi_slot, idesc_o,
+                                             (pi > 0 || half > 0 || kt > 0) ? 1u : 0u);
+                            tc_commit2(empty0 + pv.slot * 8);
+                        }
+                        if (half) { tc_commit2(smem_addr(&sm.pv_done)); ++pi; }
+                        half ^= 1;
                     } else {
                         if (clock_units<WAIT_UNIT_LOG2>() - t0 > wt.limit) { wt.code = 6; goto wind_down; }
                         continue;
@@ -417,18 +427,18 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         }
     } else if (warp == 2) {
         // ---------------- this CTA's half of the dims of the other CTA's page, over chunks that Q K^T has read ----------
-        if ((!SPARSE || p.q_tma) && elect_one()) {
+        if ((DENSE || p.q_tma) && elect_one()) {
             RingPos<NSLOT> ring;
             uint32_t g = 0, nq = 0;
             const int chunk0 = hk * p.head_chunks;
-            const uint32_t p_full0 = lead(sm.p_full[0]), q_full = lead(sm.q_full);
+            const uint32_t p_full0 = lead(sm.p_full[0][0]), q_full = lead(sm.q_full);
             for (WalkerT wk(p, part); wk.valid(); wk.next()) {
                 const Work w = wk.get();
                 if (w.ntiles == 0) continue;
                 if (p.q_tma) {
                     ring.skip(Q_SLOTS);
                     // nothing reads the previous request's Q any more (otherwise this thread has seen k_done of its last tile)
-                    if (SPARSE && nq++ > 0) WAIT_OR_LEAVE(wt, &sm.q_free, nq & 1, 23);
+                    if (nq++ > 0) WAIT_OR_LEAVE(wt, &sm.q_free, nq & 1, 23);
                     if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.q_full), 2 * (CHUNKS - QT) * CHUNK);
 #pragma unroll 1
                     for (int c = QT; c < CHUNKS; ++c)
@@ -438,23 +448,20 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                                          SPARSE ? (int)blockIdx.y : PREFILL ? w.req : row / p.g, PREFILL ? 0 : w.req);
                         }
                 }
-                if (SPARSE) continue;
+                if (!DENSE) continue;
                 const int* bt = p.block_table + (int64_t)w.req * p.bt_sb;
                 auto page_of = [&](int blk) -> int { return (blk < w.blk_end && blk < p.max_blocks) ? __ldg(bt + blk) : p.num_blocks; };
-                int nxt = DENSE ? page_of(w.blk_begin + (1 - (int)rank)) : 0;
+                int nxt = page_of(w.blk_begin + (1 - (int)rank));
                 for (int i = 0; i < w.ntiles; ++i, ++g) {
                     const int page = nxt, blk0 = w.blk_begin + 2 * i;
-                    if (DENSE && i + 1 < w.ntiles) nxt = page_of(blk0 + 2 + (1 - (int)rank));
-                    WAIT_OR_LEAVE(wt, &sm.k_done[g & 1], (g >> 1) & 1, 21);
-                    if (PREFILL) {
-                        WAIT_OR_LEAVE(wt, &sm.lf_full[g & 1], (g >> 1) & 1, 22);
-                        fence_proxy_async_smem();          // the copies of this CTA's warps -> visible to its tensor core
-                        mbar_arrive_remote_cta(p_full0 + (g & 1) * 8);
-                    }
-                    if (!DENSE) continue;
+                    if (i + 1 < w.ntiles) nxt = page_of(blk0 + 2 + (1 - (int)rank));
+                    WAIT_OR_LEAVE(wt, rank == 0 ? &sm.k_done[g & 1] : &sm.k_half[g & 1], (g >> 1) & 1, 21);
                     // a page that the sequence ends in: its rows beyond the end are zeroed by the softmax warps when it has landed
                     auto ends_in = [&](int blk) { return blk < w.blk_end && w.seqlen < (blk + 1) * PAGE; };
-                    if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.p_full[g & 1]), 2 * SLOT * (uint32_t)(!ends_in(blk0) + !ends_in(blk0 + 1)));
+                    if (rank == 0) {
+                        mbar_arrive_expect_tx(smem_addr(&sm.p_full[g & 1][0]), ends_in(blk0) ? 0 : 2 * SLOT);
+                        mbar_arrive_expect_tx(smem_addr(&sm.p_full[g & 1][1]), ends_in(blk0 + 1) ? 0 : 2 * SLOT);
+                    }
                     const bool tail = ends_in(blk0 + (1 - (int)rank));
                     if (tail) mbar_arrive_expect_tx(smem_addr(&sm.f_tail), 2 * SLOT);
 #pragma unroll 1
@@ -462,7 +469,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         if ((q >> 1) == (int)rank) continue;           // (slots of this CTA's own half)
                         const uint32_t dst = smem_addr(sm.data) + ring.slot * SLOT;
                         if (tail) tma_load_5d(dst, &kmap, smem_addr(&sm.f_tail), 0, 0, chunk0 + 4 * rank + 2 * (q & 1), 0, page);
-                        else tma2_load_5d(dst, &kmap, p_full0 + (g & 1) * 8, 0, 0, chunk0 + 4 * rank + 2 * (q & 1), 0, page);
+                        else tma2_load_5d(dst, &kmap, p_full0 + (g & 1) * 16 + (1 - rank) * 8, 0, 0, chunk0 + 4 * rank + 2 * (q & 1), 0, page);
                     }
                 }
             }
@@ -533,6 +540,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         const int other = (lane >> 3) & 1, page_of_lane = other ? 1 - (int)rank : (int)rank;       // lanes 0..7 look up the own page's tokens, 8..15 the other's
         const int tok = page_of_lane * PAGE + fw * 8 + (lane & 7);
         const uint32_t group = smem_addr(sm.data) + fw * 2048 + ((lane >> 3) & 1) * 1024;
+        const uint32_t p_full0 = lead(sm.p_full[0][0]);
         RingPos<NSLOT> ring;
         uint32_t g = 0;
         // this CTA's copy of slot-wide pieces (dims 128 q ..) of the eight rows that lanes l0 .. l0 + 7 looked up
@@ -566,14 +574,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     uint32_t bar = 0;
 #pragma unroll 1
                     for (int q = 0; q < 4; ++q, ring.next()) {
-                        WAIT_WARP_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 201);
+                        READY_OR_WAIT(wt, &sm.empty[ring.slot], ring.par ^ 1, 201);
                         copy_slot(ring.slot, q, row_id, 0);
                         if (!(q & 1)) bar = ring.slot;
                         if (q == 1 || (!WIDE && q == 3)) cp_async_arrive_noinc(smem_addr(&sm.l_full[bar]));
                     }
                     if (WIDE) {
                         const uint32_t rs = (g + i) % NROPE;
-                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty[rs], (((g + i) / NROPE) & 1) ^ 1, 202);
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int tk = 4 * u + (lane >> 3);
@@ -587,11 +594,22 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (i > 0) {
                     // the other page of tile i - 1, over slots that its Q K^T has read
                     const uint32_t gp = g + i - 1;
-                    WAIT_WARP_OR_LEAVE(wt, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
+                    READY_OR_WAIT(wt, rank == 0 ? &sm.k_done[gp & 1] : &sm.k_half[gp & 1], (gp >> 1) & 1, 203);
                     const uint32_t back = (here ? 8 : 4) - (rank == 0 ? 2 : 0);
+                    int rid[8];                                        // (a row behind the tensor's last one reads zeros)
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) copy_slot((ring.slot + NSLOT - back + k) % NSLOT, 2 * rank + k, before, 8);
-                    cp_async_arrive_noinc(smem_addr(&sm.lf_full[gp & 1]));
+                    for (int k = 0; k < 8; ++k) { rid[k] = __shfl_sync(0xffffffffu, before, 8 + k); rid[k] = rid[k] < 0 ? p.s_kv : rid[k]; }
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const uint32_t dst = smem_addr(sm.data) + (ring.slot + NSLOT - back + k) % NSLOT * SLOT + fw * 2048;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                                tma2_gather4(dst + u * 512, &kmap, p_full0 + (gp & 1) * 16 + (1 - rank) * 8, (2 * rank + k) * 128 + (u >> 1) * 64,
+                                             rid[(u & 1) * 4], rid[(u & 1) * 4 + 1], rid[(u & 1) * 4 + 2], rid[(u & 1) * 4 + 3]);
+                        }
+                    }
+                    __syncwarp();
                 }
             }
             g += w.ntiles;
@@ -660,7 +678,6 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         raw[q] = load_share(own, q, rope_raw);
                     }
                     if (WIDE) {
-                        WAIT_WARP_OR_LEAVE(wt, &sm.r_empty[rope.slot], rope.par ^ 1, 202);
                         st_shared_v4(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK + r * 128 + (((ch * 4 + piece) ^ (r & 7)) << 4), rope_raw);
                         fence_proxy_async_smem();
                         __syncwarp();
@@ -679,13 +696,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (i > 0) {
                     // the other page of tile i - 1 (= g - 2), over slots that its Q K^T has read
                     const uint32_t gp = g - 2;
-                    WAIT_WARP_OR_LEAVE(wt, &sm.k_done[gp & 1], (gp >> 1) & 1, 203);
+                    WAIT_WARP_OR_LEAVE(wt, rank == 0 ? &sm.k_done[gp & 1] : &sm.k_half[gp & 1], (gp >> 1) & 1, 203);
                     const uint32_t back = (here ? 8 : 4) - (rank == 0 ? 2 : 0);
 #pragma unroll
                     for (int k = 0; k < 2; ++k) store_share((ring.slot + NSLOT - back + k) % NSLOT, 2 * rank + k, raw_o[k], rope_o, sc_o[k]);
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote_cta(lead_at(sm.p_full[gp & 1]));
+                    if (lane == 0) mbar_arrive_remote_cta(lead_at(sm.p_full[gp & 1][1 - rank]));
                 }
                 if (here) {
                     const uint32_t gi = g - 1;
@@ -716,7 +733,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         const int hd = SPARSE ? (row_ok ? row : 0) : hk * p.g + (row_ok ? row - t * p.g : 0);
         float* xmax = reinterpret_cast<float*>(sm.data + AT_XMAX);
         const uint32_t prow = smem_addr(sm.data) + AT_P + page * CHUNK + r * 128;
-        const uint32_t s_empty = lead(sm.s_empty), p_full0 = lead(sm.p_full[0]), o_empty = lead(sm.o_empty), q_ready = lead(sm.q_ready);
+        const uint32_t s_empty = lead(sm.s_empty), p_full0 = lead(sm.p_full[0][0]), o_empty = lead(sm.o_empty), q_ready = lead(sm.q_ready);
         const bool wide_out = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 &&
                               (PREFILL || ((p.o_sb | p.o_ss | p.o_sh) & 15) == 0);
         RingPos<NSLOT> ring, q_ring;
@@ -725,8 +742,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         WalkerT qw(p, part), wk(p, part);
         Work w;
         float m_run = -INFINITY, l_run = 0.f, m_true = -INFINITY;
-        // These 256 threads meet at a named barrier every tile, so none of them may leave alone: a thread whose wait ran out keeps
-        // walking (it arrives nowhere and stores nothing) until the next such barrier, which carries the flag to everyone.
+        // These 256 threads meet at a named barrier at every request and where the guess was wrong, so none of them may leave alone: a warp
+        // with an expired wait votes against the guess, stores nothing and announces nothing more until the barrier that carries the flag.
         while (true) {
             // ---- Q of the next request that has tiles, before this one's epilogue: its first Q K^T runs meanwhile
             for (; !have_q && qw.valid(); qw.next()) {
@@ -869,48 +886,37 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 }
                 const float mx = fmaxf(mx0, mx1) * p.scale_log2;   // scale > 0: max commutes with scaling
                 m_true = fmaxf(m_true, mx);
-                // P with the maximum in use, on the guess that no row of this CTA outgrows it; the barrier behind P's stores tells.
+                // P with the maximum in use, on the guess that no row of this CTA outgrows it: the warps vote on it while P is made.
                 // Otherwise (and on a request's first tile) the rows' maxima are exchanged and P is made again.
-                const bool grow = mx > m_run + RESCALE_THRESHOLD;
-                bool make = !__any_sync(0xffffffffu, grow);
-                float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll 1
-                for (int pass = 0; pass < 2; ++pass) {
-                    uint32_t pk[16];
-                    if (make) {
-                        const float neg_m = m_run == -INFINITY ? 0.f : -m_run;
-                        sum0 = 0.f; sum1 = 0.f;
+                const uint32_t vote = smem_addr(&sm.vote[g & 1]);
+                volatile uint32_t& outgrown = sm.outgrown[g & 1];
+                if (__any_sync(0xffffffffu, mx > m_run + RESCALE_THRESHOLD || wt.expired()) && lane == 0) outgrown = g + 1;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(vote);
+                uint32_t pk[16];
+                float sum0, sum1;
+                auto make = [&] {
+                    const float neg_m = m_run == -INFINITY ? 0.f : -m_run;
+                    sum0 = 0.f; sum1 = 0.f;
 #pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            const float e0 = ex2(fmaf(__uint_as_float(s[c]), p.scale_log2, neg_m));
-                            const float e1 = ex2(fmaf(__uint_as_float(s[c + 1]), p.scale_log2, neg_m));
-                            sum0 += e0; sum1 += e1;
-                            pk[c >> 1] = pack16<FP16>(e0, e1);
-                        }
+                    for (int c = 0; c < 32; c += 2) {
+                        const float e0 = ex2(fmaf(__uint_as_float(s[c]), p.scale_log2, neg_m));
+                        const float e1 = ex2(fmaf(__uint_as_float(s[c + 1]), p.scale_log2, neg_m));
+                        sum0 += e0; sum1 += e1;
+                        pk[c >> 1] = pack16<FP16>(e0, e1);
                     }
-                    // P's buffer is free, and O may be touched, when the previous tile's P V has finished
-                    if (pass == 0 && g > 0) wt.wait(&sm.pv_done, (g - 1) & 1, 34);
-                    if (make && !wt.expired()) {
+                };
+                auto store = [&] {
 #pragma unroll
-                        for (int ch = 0; ch < 4; ++ch)
-                            st_shared_v4(prow + (((wg * 4 + ch) ^ (r & 7)) << 4), make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]));
-                    }
-                    if (DENSE && pass == 0) {
-                        // Tokens at or beyond the sequence length may hold anything (NaN included) in a real page: their probabilities
-                        // are zero, so their V rows are zeroed to keep 0 * NaN out of O (Q K^T has read them).
-#pragma unroll 1
-                        for (int h = 0; h < 2; ++h) {
-                            const int blk = w.blk_begin + 2 * i + h;
-                            if (blk < w.blk_end && w.seqlen < (blk + 1) * PAGE) {
-                                if (h != (int)rank) { wt.wait(&sm.f_tail, ntail & 1, 35); ++ntail; }
-                                if (!wt.expired())
-                                    for (int n = 0; n < 2; ++n) zero_rows(sm.data + (ring.slot + 2 * h + n) % NSLOT * SLOT, max(w.seqlen - blk * PAGE, 0));
-                            }
-                        }
-                    }
-                    fence_proxy_async_smem();                          // P and zeroed rows are read by the tensor core
-                    tc_fence_before();
-                    if (!named_bar_red_or(1, 256, pass == 0 && (grow || wt.expired()))) break;
+                    for (int ch = 0; ch < 4; ++ch)
+                        st_shared_v4(prow + (((wg * 4 + ch) ^ (r & 7)) << 4), make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]));
+                };
+                make();
+                // P's buffer is free, and O may be touched, when the previous tile's P V has finished
+                if (g > 0) wt.wait(&sm.pv_done, (g - 1) & 1, 34);
+                wt.wait(&sm.vote[g & 1], (g >> 1) & 1, 36);
+                bool together = false;                         // something of this tile that all warps have a hand in
+                if (__any_sync(0xffffffffu, outgrown == g + 1 || wt.expired())) {
                     // ---- some row has outgrown its maximum (or a wait ran out)
                     xmax[quarter * HALF + r] = mx;
                     BAR_OR_LEAVE(wt.expired());
@@ -925,11 +931,34 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         tc_fence_after();
                         rescale_o(tlane + TM_O + wg * 128, factor);
                     }
-                    make = true;
+                    make();
+                    together = true;
                 }
+                store();
                 l_run += sum0 + sum1;
+                if (DENSE) {
+                    // Tokens at or beyond the sequence length may hold anything (NaN included) in a real page: their probabilities
+                    // are zero, so their V rows are zeroed to keep 0 * NaN out of O (Q K^T has read them).
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        const int blk = w.blk_begin + 2 * i + h;
+                        if (blk < w.blk_end && w.seqlen < (blk + 1) * PAGE) {
+                            if (h != (int)rank) { wt.wait(&sm.f_tail, ntail & 1, 35); ++ntail; }
+                            if (!wt.expired())
+                                for (int n = 0; n < 2; ++n) zero_rows(sm.data + (ring.slot + 2 * h + n) % NSLOT * SLOT, max(w.seqlen - blk * PAGE, 0));
+                            together = true;
+                        }
+                    }
+                }
                 ring.skip(4);
-                if (threadIdx.x == 128) mbar_arrive_remote_cta(p_full0 + (g & 1) * 8);
+                fence_proxy_async_smem();                      // P and zeroed rows are read by the tensor core
+                tc_fence_before();
+                if (together) BAR_OR_LEAVE(wt.expired());
+                __syncwarp();
+                if (lane == 0 && !wt.expired()) {              // (prefill: CTA 0 adds the bytes that complete the barrier)
+                    if (PREFILL && rank == 0 && (warp == 4 || warp == 6)) mbar_arrive_expect_tx(smem_addr(&sm.p_full[g & 1][page]), 2 * SLOT);
+                    else mbar_arrive_remote_cta(p_full0 + (g & 1) * 16 + page * 8);
+                }
             }
             // the row's sum (and true maximum) over its four quarters (the barrier of the next request's Q comes before the next use
             // of the buffers)
@@ -1108,7 +1137,15 @@ int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a) {
     using namespace sm100;
     Params p = prefill_params(a);
     p.row_blocks = (p.rows + pair::ROWS - 1) / pair::ROWS;
-    CUtensorMap unused, qmap;
+    EncodeTiledFn encode = get_encode_fn();
+    if (!encode) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    // the keys as rows for TMA's gathers of four of them, 64 columns a box
+    CUtensorMap kmap, unused, qmap;
+    cuuint64_t dims[2] = {(cuuint64_t)a.d_qk, (cuuint64_t)a.s_kv}, strides[1] = {(cuuint64_t)a.kv_stride_s * 2};
+    cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
+    const CUresult r = encode(&kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     memset(&unused, 0, sizeof(unused));
     memset(&qmap, 0, sizeof(qmap));
     p.q_unit = pair::HALF;
@@ -1117,8 +1154,8 @@ int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a) {
     if (pairs < 1) pairs = 1;
     if (pairs > a.s_q) pairs = a.s_q;
     const dim3 grid(2, p.row_blocks, pairs);
-    return a.d_qk == 512 ? pair::launch<MODE_PREFILL, true>(grid, unused, unused, qmap, p, a.stream)
-                         : pair::launch<MODE_PREFILL, false>(grid, unused, unused, qmap, p, a.stream);
+    return a.d_qk == 512 ? pair::launch<MODE_PREFILL, true>(grid, kmap, unused, qmap, p, a.stream)
+                         : pair::launch<MODE_PREFILL, false>(grid, kmap, unused, qmap, p, a.stream);
 }
 
 }  // namespace mla

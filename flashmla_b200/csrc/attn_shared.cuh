@@ -153,6 +153,7 @@ struct Waiter {
     __device__ __forceinline__ bool expired() const { return code != 0; }
     __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, int site) {
         if (expired()) return false;
+        if (mbar_try_wait(smem_addr(bar), parity)) return true;
         const uint32_t t0 = clock_units<WAIT_UNIT_LOG2>();
 #pragma unroll 1
         while (!mbar_try_wait(smem_addr(bar), parity))

@@ -275,6 +275,13 @@ __device__ __forceinline__ void tma2_load_5d(uint32_t dst, const CUtensorMap* m,
         ::"r"(dst), "l"(m), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
 
+// Rows r0 .. r3 of a 2-D tensor, a box's columns from c on, one after the other (rows outside the tensor: zeros).
+__device__ __forceinline__ void tma2_gather4(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int c, int r0, int r1, int r2, int r3) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(dst), "l"(m), "r"(bar_cluster), "r"(c), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+
 // 32 lanes x 32 columns of 32-bit: thread i of the warp gets lane (32*(warp%4) + i), register j column j.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(

@@ -22,8 +22,10 @@ def _plan():
     return slots, 2 * tables, tables
 
 
-def _graph(tiles, slots, tables, convert):
-    """edges[event] = the events that directly precede it; events are (role, what, tile, slot of the tile)."""
+def _graph(tiles, slots, tables, convert, rank=0):
+    """edges[event] = the events that directly precede it; events are (role, what, tile, slot of the tile), those of CTA `rank` of the pair
+    and the issuing thread's.  P V of page h (slots 2 h and 2 h + 1) waits for the other page's part of CTA 1 - h, which may be brought in
+    when Q K^T has read the slots that it goes to: CTA 1's first half of them, CTA 0's second."""
     edges = {}
 
     def program(role, steps):
@@ -49,11 +51,13 @@ def _graph(tiles, slots, tables, convert):
             if f >= slots:                                                                      # empty: P V that read the slot
                 edges["feed", "fill", g, q].append(("values", "values", (f - slots) // 4, (f - slots) % 4))
             edges["scores", "scores", g, q].append(("feed", "fill", g, q))                      # full
-            edges["values", "values", g, q] += [("softmax", "p", g, 0)] + ([("feed", "other", g, 0)] if g + 1 < tiles else [])    # p_full
+            edges["values", "values", g, q].append(("softmax", "p", g, 0))                       # p_full
+            if g + 1 < tiles and q // 2 == 1 - rank:
+                edges["values", "values", g, q].append(("feed", "other", g, 0))
             edges["values", "values", g, q].append(("scores", "scores", g, 3))
         if g >= 1:
             edges["scores", "scores", g, 0].append(("softmax", "give", g - 1, 0))               # s_empty
-            edges["feed", "other", g - 1, 0].append(("scores", "scores", g - 1, 3))             # k_done
+            edges["feed", "other", g - 1, 0].append(("scores", "scores", g - 1, 1 if rank else 3))    # k_half, k_done
         if g >= 2:
             edges["scores", "scores", g, 0].append(("values", "values", g - 2, 3))              # the issuing thread's order
         edges["softmax", "start", g, 0].append(("scores", "scores", g, 3))                      # s_full
@@ -135,11 +139,12 @@ def _before(edges, first, then):
     return False
 
 
+@pytest.mark.parametrize("rank", [0, 1])
 @pytest.mark.parametrize("convert", [False, True])          # prefill, FP8 decode
-def test_ring_entries_are_read_before_they_are_overwritten(convert):
+def test_ring_entries_are_read_before_they_are_overwritten(convert, rank):
     slots, masks, tables = _plan()
     tiles = masks + 8
-    edges = _graph(tiles, slots, tables, convert)
+    edges = _graph(tiles, slots, tables, convert, rank)
     writer = "look-up" if convert else "feed"
     for g in range(tiles - masks):
         assert _before(edges, (writer, "meta", g, 0), ("softmax", "mask", g, 0)), "a mask is read after it was written"
@@ -166,17 +171,17 @@ def test_the_check_sees_a_missing_order():
 
 # ---- the pair kernel's ring across requests: parity waits -------------------------------------------------------------
 # A request takes three slots of the ring for its Q (filled by a thread of warp 0, given back by the softmax warps) and four a tile (filled by
-# the feeding warps, given back behind P V).  A wait for the release of a slot's fill, by parity, is right if the release before
+# the feeding warps, given back behind P V of page 0, which reads the first two, and of page 1).  A wait for the release of a slot's fill, by parity, is right if the release before
 # that one is ordered before the wait, and the wait before the release behind.
 
 def _request_plan():
-    """Whether warp 0's thread follows the releases of the feeding warps' fills itself, and whether warp 2's (FP8 decode) follows k_done."""
+    """Whether warp 0's thread follows the releases of the feeding warps' fills itself, and whether warp 2's follows k_done in the gather modes."""
     text = open(SOURCE).read()
     loads = text[text.index("own page of every tile"):text.index("MMA issuer (CTA 0")]
     gather = loads[loads.index("} else {", loads.index("if (DENSE) {")):]
     other = text[text.index("half of the dims of the other CTA's page"):text.index("FP8 decode: index ->")]
     loop = other[:other.index("k_done[g & 1]")]
-    return "sm.empty[" in gather, "if (SPARSE) continue;" not in loop
+    return "sm.empty[" in gather, "if (!DENSE) continue;" not in loop
 
 
 def _request_graph(requests, slots, follow, follow_k):
@@ -192,7 +197,7 @@ def _request_graph(requests, slots, follow, follow_k):
     owner, at, first, g = [], 0, [], 0                        # fill -> what gives it back; a request's first fill and first tile
     for n, t in enumerate(requests):
         first.append((at, g))
-        owner += [("softmax", "take", n)] * q_slots + [("issue", "values", g + i) for i in range(t) for _ in range(4)]
+        owner += [("softmax", "take", n)] * q_slots + [("issue", "values", g + i if k >= 2 else ("half", g + i)) for i in range(t) for k in range(4)]
         at, g = at + q_slots + 4 * t, g + t
     release = lambda f: owner[f] if f >= 0 else None
     load, feed, issue, soft, copy = [], [], [], [], []
@@ -232,11 +237,12 @@ def _request_graph(requests, slots, follow, follow_k):
         for i in range(g0, g0 + t):
             f = f0 + q_slots + 4 * (i - g0)
             edges["issue", "scores", i] += [("issue", "begin", n), ("feed", "filled", i)]               # full
-            edges["issue", "values", i] += [("issue", "scores", i), ("softmax", "p", i)]                # p_full
+            edges["issue", "values", ("half", i)] = [("issue", "scores", i), ("softmax", "p", i)]       # p_full of page 0 (page 1: below)
+            edges["issue", "values", i] += [("issue", "values", ("half", i)), ("softmax", "p", i)]
             edges["softmax", "start", i].append(("issue", "scores", i))                                 # s_full
             if i > g0:
                 edges["issue", "scores", i] += [("issue", "scores", i - 1), ("softmax", "start", i - 1)]    # s_empty
-                edges["issue", "values", i].append(("issue", "values", i - 1))
+                edges["issue", "values", ("half", i)].append(("issue", "values", i - 1))
             if i > g0 + 1:
                 edges["issue", "scores", i].append(("issue", "values", i - 2))                          # at most one tile ahead
             for k in range(4):
@@ -268,6 +274,20 @@ def test_parity_waits_of_the_ring_across_requests(convert):
     follow, follow_k = _request_plan()
     for requests in MANY:
         assert not _misread(requests, follow, follow_k and convert), requests
+
+
+def test_rope_chunks_need_no_wait():
+    """A tile's RoPE chunk goes to the buffer of the tile before last's without a wait of its own: Q K^T of that tile is past when the last two
+    slots of this one have been given back."""
+    text = open(SOURCE).read()
+    assert int(re.search(r"\bNROPE = (\d+);", text).group(1)) == 2 and "r_empty" not in text
+    for requests in MANY:
+        for follow in (False, True):
+            edges, _ = _request_graph(requests, _plan()[0], follow, False)
+            for g in range(2, sum(requests)):
+                assert _before(edges, ("issue", "scores", g - 2), ("feed", "filled", g)), (requests, g)
+    edges, _ = _request_graph([9], 16, False, False)            # the check sees a ring that would be too deep for that
+    assert not _before(edges, ("issue", "scores", 5), ("feed", "filled", 7))
 
 
 def test_the_check_sees_a_parity_that_may_be_misread():
@@ -302,7 +322,7 @@ def test_softmax_threads_leave_together(path):
     did not, must walk on to the next barrier that tells them all."""
     steps = _softmax_steps(path)
     waits = [i for i, step in enumerate(steps) if step[0] == "wait"]
-    assert len(waits) == (5 if path == SOURCE else 2)
+    assert len(waits) == (6 if path == SOURCE else 2)
     for i in waits:
         after = [step for step in (steps + steps)[i + 1:] if step != ("barrier", False)]          # (the role is a loop)
         assert after[0][0] == "wait" or after[0] == ("barrier", True), (steps[i], after[0])
