@@ -37,9 +37,10 @@
 // the launch); DRAM at 4.9 TB/s in a launch by itself (136 us at 1.63 GHz), back to back the power limit (1.34 GHz).  A tile's loads wait for
 // P V two tiles before, 2000 to 2900 cycles before they have landed.  Prefill: 3700 cycles a tile, the tensor core 2250, the own page's copies
 // (144 instructions an SM, 14.5 cycles each at best) and the other page's row gathers (64 of TMA, 20 each) beside each other; back to back the
-// power limit (1.6 GHz).  FP8 decode: 5200 cycles a tile,
-// the feeding warps' conversion (six slots' worth, 64 x 128 values each, 450-600 cycles apiece) and the chain conversion -> Q K^T ->
-// softmax -> P V behind a ring of two and a half tiles.  One copy of every converted value would save a third of the conversion but the
+// power limit (1.6 GHz).  FP8 decode: 4300 to 4800 cycles a tile; 64 x 2048
+// keys take 54 us, without the records' loads 47, without their conversion 52, without both 43 (512-wide 48.5, 46.6, 41.6, 38.9; shares of
+// other values in their place): the chain conversion -> Q K^T -> softmax -> P V behind a ring of two and a half tiles, the loads' way
+// through the little that is left of L1, and the conversion.  One copy of every converted value would save a third of the conversion but the
 // exchange costs more: by 16-byte asynchronous stores into the other SM 93 us, by bulk copies 75.5, converting the half of the
 // other page again 57.0 (first line below).  us a call, back to back, score and value CTAs -> now:
 //   one input per call                                          inputs changing from call to call, clocks settled
@@ -50,10 +51,11 @@
 //   dense, 128 x ~4096 tokens                    185 ->  172       189 ->  173
 //   dense, two query tokens                      314 ->  294       325 ->  300
 //   dense, one request of 100003 tokens                           54.9 -> 47.8
-// and with P V page by page, the vote on an mbarrier and no wait for the RoPE buffers (inputs changing): FP8 60.5 -> 58.3, prefill 2324 -> 2242,
-// dense 180.4 -> 178.3, two query tokens 306 -> 302, 128 requests of lognormal lengths 536 -> 522.
+// and with P V page by page, the vote on an mbarrier and no wait for the RoPE buffers (inputs changing): FP8 60.3 -> 57.7, prefill 2328 -> 2247,
+// dense 180.4 -> 178.9, two query tokens 306 -> 304, 128 requests of lognormal lengths 530 -> 526; 512-wide records, whose exponent bytes
+// are converted in pairs, whose loads have no condition and are preceded by L2 prefetches, 50.7 -> 47.3.
 // (914 calls of dense and FP8 decode and prefill with 64 to 128 heads: between 1.04 and 2.0 times as fast, none slower.)
-// Registers: both FP8 forms spill 12 bytes a thread (24 reloaded), the others none.
+// Registers: both FP8 forms spill 4 bytes a thread, the others none.
 //
 // Every mbarrier wait is bounded (Params::wait_limit SM cycles, about a second by default).  A thread whose wait ran out LEAVES its role -
 // it issues no further arrival, MMA or copy -, records a code in the status words and raises the `aborted` flag of both CTAs.
@@ -201,6 +203,10 @@ __device__ __noinline__ void load_q_by_threads(Smem& sm, const __nv_bfloat16* qr
         }
     }
 }
+
+// FP8 decode of 512-wide records: the record and the scales of list entries that are no token (loads without a condition: 49.1 -> 47.4 us for
+// 74 x (512 + 1024), 128 heads; 576-wide records lose, 52.9 -> 54.8 for 64 x 2048)
+__device__ __align__(128) uint8_t no_record[576];
 
 template <int MODE, bool ALT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Warps<MODE>::THREADS, 1)
@@ -497,14 +503,22 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 WAIT_WARP_OR_LEAVE(wt, &sm.tab_empty[g % NTAB], ((g / NTAB) & 1) ^ 1, 205);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const int blk = w.blk_begin + 2 * i + (k >> 1), scope = blk >= w.nblk0 ? 1 : 0, pbs = p.pbs[scope];
-                    const bool ok = id[k] >= 0 && (int64_t)id[k] < (int64_t)p.nblocks[scope] * pbs;
+                    const int blk = w.blk_begin + 2 * i + (k >> 1), scope = blk >= w.nblk0 ? 1 : 0;
+                    const bool ok = (uint32_t)id[k] < p.tokens[scope];
                     ulonglong2 e = make_ulonglong2(0, 0);
+                    if (M1) e.x = e.y = reinterpret_cast<unsigned long long>(no_record);
                     if (ok) {
-                        const int off = id[k] % pbs;
-                        const uint8_t* block = p.kvb[scope] + (int64_t)(id[k] / pbs) * p.kvb_sblock[scope];
-                        e.x = reinterpret_cast<unsigned long long>(block + (int64_t)off * (M1 ? 576 : 656));
-                        e.y = M1 ? reinterpret_cast<unsigned long long>(block + (int64_t)pbs * 576 + (int64_t)off * 8) : e.x + 512;
+                        uint32_t off;
+                        const uint8_t* block = p.kvb[scope] + page_of_token(p, scope, id[k], off) * p.kvb_sblock[scope];
+                        e.x = reinterpret_cast<unsigned long long>(block + (uint64_t)off * (M1 ? 576 : 656));
+                        e.y = M1 ? reinterpret_cast<unsigned long long>(block + (int64_t)p.pbs[scope] * 576 + (uint64_t)off * 8) : e.x + 512;
+                    }
+                    // the own page's records into L2, tiles ahead of the loads, which keep L1's few free lines (what is left of 256 KB) busy as
+                    // long as they are under way (512-wide records only: of 576-wide ones, 64 x 2048, 53.2 -> 57.9 us)
+                    if (M1 && ok && (k >> 1) == (int)rank) {
+#pragma unroll
+                        for (int at = 0; at < 576; at += 128) prefetch_l2(e.x + at);
+                        prefetch_l2(e.y);
                     }
                     reinterpret_cast<ulonglong2*>(sm.data + AT_TAB)[g % NTAB * ROWS + k * 32 + lane] = e;
                     const uint32_t bits = __ballot_sync(0xffffffffu, ok);
@@ -631,7 +645,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         RingPos<NSLOT> ring;
         RingPos<NROPE> rope;
         uint32_t g = 0;
-        auto load16 = [&](unsigned long long rec, int off) { return rec ? __ldg(reinterpret_cast<const uint4*>(rec + off)) : make_uint4(0, 0, 0, 0); };
+        auto load16 = [&](unsigned long long rec, int off) { return M1 || rec ? __ldg(reinterpret_cast<const uint4*>(rec + off)) : make_uint4(0, 0, 0, 0); };
         // slot q's share of a record: 16 e4m3 (512-wide form, chunk 7: 32 bytes of RoPE, the second half in `more`)
         auto is_rope = [&](int q) { return M1 && q == 3 && ch == 1; };
         auto load_share = [&](unsigned long long rec, int q, uint4& more) {
@@ -641,7 +655,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         // (a scale word: fp32, or four exponent bytes of the 512-wide form)
         auto store_share = [&](uint32_t slot, int q, const uint4& raw, const uint4& more, uint32_t word) {
             uint4 lo = raw, hi = more;
-            const float scale = M1 ? e8m0_to_float((word >> (8 * ((2 * q + ch) & 3))) & 0xffu) : __uint_as_float(word);
+            const float scale = M1 ? e8m0_of(word, 2 * (q & 1) + ch) : __uint_as_float(word);
             if (!is_rope(q)) dequant16(raw, scale, lo, hi);
             st_shared_v4(row_at + slot * SLOT, lo);
             st_shared_v4((row_at + slot * SLOT) ^ 16, hi);
@@ -663,34 +677,56 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     const ulonglong2 e = tab[g % NTAB * ROWS + rank * PAGE];
                     own = e.x; own_sc = e.y;
                 }
-                if (here) {
+                if (M1 && i < ntiles) {
+                    // (two slots at a time: with a RoPE chunk to store, 576-wide records are faster by single slots, 53.3 us against 55.4)
+#pragma unroll
+                    for (int q = 0; q < 4; q += 2) {
+                        if (here) {
+                            const uint32_t s0 = ring.slot, par0 = ring.par ^ 1;
+                            ring.next();
+                            const uint32_t s1 = ring.slot, par1 = ring.par ^ 1;
+                            ring.next();
+                            if (!__all_sync(0xffffffffu, mbar_try_wait(smem_addr(&sm.empty[s0]), par0, smem_addr(&sm.empty[s1]), par1))) {
+                                WAIT_WARP_OR_LEAVE(wt, &sm.empty[s0], par0, 201);
+                                WAIT_WARP_OR_LEAVE(wt, &sm.empty[s1], par1, 201);
+                            }
+                            store_share(s0, q, raw[q], rope_raw, sc[q]);
+                            store_share(s1, q + 1, raw[q + 1], rope_raw, sc[q]);
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_remote_cta(lead0 + s0 * 8);
+                        }
+                        if (i + 1 < ntiles) {
+                            raw[q] = load_share(own, q, rope_raw);
+                            raw[q + 1] = load_share(own, q + 1, rope_raw);
+                        }
+                    }
+                } else if (here) {
                     uint32_t bar = 0;
 #pragma unroll
                     for (int q = 0; q < 4; ++q, ring.next()) {
                         WAIT_WARP_OR_LEAVE(wt, &sm.empty[ring.slot], ring.par ^ 1, 201);
-                        store_share(ring.slot, q, raw[q], rope_raw, M1 ? sc[q & 2] : sc[q]);
+                        store_share(ring.slot, q, raw[q], rope_raw, sc[q]);
                         if (!(q & 1)) bar = lead0 + ring.slot * 8;
-                        if (q == 1 || (!WIDE && q == 3)) {
+                        if (q == 1) {
                             fence_proxy_async_smem();
                             __syncwarp();
                             if (lane == 0) mbar_arrive_remote_cta(bar);
                         }
                         raw[q] = load_share(own, q, rope_raw);
                     }
-                    if (WIDE) {
-                        st_shared_v4(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK + r * 128 + (((ch * 4 + piece) ^ (r & 7)) << 4), rope_raw);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_remote_cta(bar);
-                        rope.next();
-                    }
+                    st_shared_v4(smem_addr(sm.data) + AT_ROPE + rope.slot * CHUNK + r * 128 + (((ch * 4 + piece) ^ (r & 7)) << 4), rope_raw);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote_cta(bar);
+                    rope.next();
                 } else if (i < 0) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) raw[q] = load_share(own, q, rope_raw);
                 }
                 if (i + 1 < ntiles) {
                     if (WIDE) rope_raw = load16(own, 528 + (ch * 4 + piece) * 16);
-                    if (M1) { const uint2 e = own_sc ? __ldg(reinterpret_cast<const uint2*>(own_sc)) : make_uint2(0, 0); sc[0] = e.x; sc[2] = e.y; }
+                    if (M1) { const uint2 e = __ldg(reinterpret_cast<const uint2*>(own_sc)); sc[0] = e.x; sc[2] = e.y; }
                     else { const uint4 e = load16(own_sc, 0); sc[0] = e.x; sc[1] = e.y; sc[2] = e.z; sc[3] = e.w; }
                 }
                 if (i > 0) {
@@ -709,7 +745,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     const ulonglong2 e = tab[gi % NTAB * ROWS + (1 - rank) * PAGE];
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_addr(&sm.tab_empty[gi % NTAB]));
-                    if (M1) { sc_o[0] = sc_o[1] = e.y ? __ldg(reinterpret_cast<const uint32_t*>(e.y) + rank) : 0u; }
+                    if (M1) { sc_o[0] = sc_o[1] = __ldg(reinterpret_cast<const uint32_t*>(e.y) + rank); }
                     else { const uint2 x = e.y ? __ldg(reinterpret_cast<const uint2*>(e.y) + rank) : make_uint2(0, 0); sc_o[0] = x.x; sc_o[1] = x.y; }
 #pragma unroll
                     for (int k = 0; k < 2; ++k) raw_o[k] = load_share(e.x, 2 * rank + k, rope_o);
@@ -887,12 +923,12 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 const float mx = fmaxf(mx0, mx1) * p.scale_log2;   // scale > 0: max commutes with scaling
                 m_true = fmaxf(m_true, mx);
                 // P with the maximum in use, on the guess that no row of this CTA outgrows it: the warps vote on it while P is made.
-                // Otherwise (and on a request's first tile) the rows' maxima are exchanged and P is made again.
-                const uint32_t vote = smem_addr(&sm.vote[g & 1]);
+                // Otherwise the rows' maxima are exchanged and P is made again; on a request's first tile that is always so, and nothing is
+                // made on the guess (3 x 100 tokens 14.2 -> 13.7 us; the votes are cast all the same, so that their phases follow the tiles).
                 volatile uint32_t& outgrown = sm.outgrown[g & 1];
                 if (__any_sync(0xffffffffu, mx > m_run + RESCALE_THRESHOLD || wt.expired()) && lane == 0) outgrown = g + 1;
                 __syncwarp();
-                if (lane == 0) mbar_arrive(vote);
+                if (lane == 0) mbar_arrive(smem_addr(&sm.vote[g & 1]));
                 uint32_t pk[16];
                 float sum0, sum1;
                 auto make = [&] {
@@ -911,12 +947,13 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     for (int ch = 0; ch < 4; ++ch)
                         st_shared_v4(prow + (((wg * 4 + ch) ^ (r & 7)) << 4), make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]));
                 };
-                make();
+                if (i > 0) make();
                 // P's buffer is free, and O may be touched, when the previous tile's P V has finished
                 if (g > 0) wt.wait(&sm.pv_done, (g - 1) & 1, 34);
-                wt.wait(&sm.vote[g & 1], (g >> 1) & 1, 36);
-                bool together = false;                         // something of this tile that all warps have a hand in
-                if (__any_sync(0xffffffffu, outgrown == g + 1 || wt.expired())) {
+                if (i > 0) wt.wait(&sm.vote[g & 1], (g >> 1) & 1, 36);
+                // something of this tile that all warps have a hand in
+                bool together = i == 0 || __any_sync(0xffffffffu, outgrown == g + 1 || wt.expired());
+                if (together) {
                     // ---- some row has outgrown its maximum (or a wait ran out)
                     xmax[quarter * HALF + r] = mx;
                     BAR_OR_LEAVE(wt.expired());
@@ -932,7 +969,6 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         rescale_o(tlane + TM_O + wg * 128, factor);
                     }
                     make();
-                    together = true;
                 }
                 store();
                 l_run += sum0 + sum1;

@@ -442,7 +442,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     const int scope = blk >= w.nblk0 ? 1 : 0;
                     const int pbs = p.pbs[scope];
                     sc = make_uint4(0, 0, 0, 0);
-                    if (id < 0 || (int64_t)id >= (int64_t)p.nblocks[scope] * pbs) return nullptr;
+                    if ((uint32_t)id >= p.tokens[scope]) return nullptr;
                     const uint8_t* block = p.kvb[scope] + (int64_t)(id / pbs) * p.kvb_sblock[scope];
                     const int off = id % pbs;
                     if (M1) {
@@ -489,7 +489,7 @@ attn_rows64_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const uint32_t word = M1 ? (q < 2 ? sc.x : sc.y) : q == 0 ? sc.x : q == 1 ? sc.y : q == 2 ? sc.z : sc.w;
-                            const float scale = M1 ? e8m0_to_float((word >> (8 * ((2 * q + u) & 3))) & 0xffu) : __uint_as_float(word);
+                            const float scale = M1 ? e8m0_of(word, (2 * q + u) & 3) : __uint_as_float(word);
                             uint4 lo = raw[q][u], hi = rope[0];
                             if (!(M1 && q == 3 && u == 1)) dequant16(raw[q][u], scale, lo, hi);
                             st_shared_v4(dst0 + u * 1024 + (((2 * piece) ^ tl) << 4), lo);

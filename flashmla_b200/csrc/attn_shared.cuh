@@ -7,6 +7,7 @@
 #include "wait_limit.h"
 #include <cuda_fp16.h>
 #include <string.h>
+#include <algorithm>
 #include <stdlib.h>
 #include <mutex>
 
@@ -42,10 +43,18 @@ struct Params {
     const int* indices; int64_t idx_ss; int topk; const int* topk_len; int s_kv;
     const __nv_bfloat16* kv; int64_t kv_ss;
     // sparse FP8 decode: two index scopes (main cache, optional extra cache) of 656-byte token records
-    const uint8_t* kvb[2]; int64_t kvb_sblock[2]; int pbs[2]; int nblocks[2];
+    const uint8_t* kvb[2]; int64_t kvb_sblock[2]; int pbs[2]; uint32_t pbs_mul[2]; int pbs_shift[2];      // (a token's page: times mul, shifted)
+    uint32_t tokens[2];                    // of the cache: indices below are valid
     const int* sidx[2]; int64_t sidx_sb[2], sidx_ss[2]; int stopk[2]; const int* stopk_len[2];
     const float* attn_sink; float* max_logits;
 };
+
+// The page of token `id` of scope `scope` (id < p.tokens[scope]) and its place there.
+__device__ __forceinline__ uint32_t page_of_token(const Params& p, int scope, uint32_t id, uint32_t& off) {
+    const uint32_t page = (uint32_t)(((uint64_t)id * p.pbs_mul[scope]) >> p.pbs_shift[scope]);
+    off = id - page * (uint32_t)p.pbs[scope];
+    return page;
+}
 
 // One unit of work of a partition: a request and the range of its 64-token blocks walked here.
 struct Work {
@@ -198,6 +207,13 @@ __device__ __forceinline__ float e8m0_to_float(uint32_t e) {
     return __uint_as_float(e == 0 ? 0x00400000u : e == 255 ? 0x7fc00000u : e << 23);
 }
 
+// The same of byte `k` of a word (through bf16, which has all of these values).
+__device__ __forceinline__ float e8m0_of(uint32_t word, int k) {
+    uint32_t r;
+    asm("{\n\t.reg .b16 x, y;\n\tmov.b32 {x, y}, %1;\n\tcvt.rn.bf16x2.ue8m0x2 %0, x;\n\t}" : "=r"(r) : "r"(__byte_perm(word, 0, 0x4440 | k)));
+    return __uint_as_float(r << 16);
+}
+
 // two fp32 products in one instruction
 __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
     float2 r;
@@ -329,6 +345,16 @@ static Params prefill_params(const mla_sparse_prefill_args_t& a) {
     return p;
 }
 
+// n / d = n * mul >> shift for 0 <= n < 2^31, d >= 1: with 2^l >= d, mul = floor(2^(31 + l) / d) + 1 is off by at most d / 2^(31 + l), so the
+// product by less than 1 / d of the quotient (T. Granlund, P. L. Montgomery, "Division by invariant integers using multiplication",
+// PLDI 1994).
+static void reciprocal(int d, uint32_t& mul, int& shift) {
+    int l = 0;
+    while (((int64_t)1 << l) < d) ++l;
+    mul = (uint32_t)(((uint64_t)1 << (31 + l)) / (uint64_t)d + 1);
+    shift = 31 + l;
+}
+
 static Params sparse_decode_params(const mla_sparse_decode_args_t& a) {
     Params p = {};
     p.b = a.b; p.s_q = a.s_q; p.h_q = a.h_q; p.h_kv = 1; p.g = a.h_q; p.rows = a.h_q;
@@ -341,13 +367,18 @@ static Params sparse_decode_params(const mla_sparse_decode_args_t& a) {
     p.attn_sink = a.attn_sink;
     p.meta = a.meta; p.num_splits = a.num_splits; p.lse_accum = a.lse_accum; p.o_accum = a.o_accum;
     p.status = a.status;
-    p.kvb[0] = (const uint8_t*)a.kv; p.kvb_sblock[0] = a.kv_stride_block_bytes; p.pbs[0] = a.page_block_size; p.nblocks[0] = a.num_blocks;
+    p.kvb[0] = (const uint8_t*)a.kv; p.kvb_sblock[0] = a.kv_stride_block_bytes; p.pbs[0] = a.page_block_size;
     p.sidx[0] = a.indices; p.sidx_sb[0] = a.indices_stride_b; p.sidx_ss[0] = a.indices_stride_s; p.stopk[0] = a.topk;
     p.stopk_len[0] = a.topk_length;
     p.kvb[1] = (const uint8_t*)a.extra_kv; p.kvb_sblock[1] = a.extra_kv_stride_block_bytes;
-    p.pbs[1] = a.extra_page_block_size > 0 ? a.extra_page_block_size : 1; p.nblocks[1] = a.extra_num_blocks;
+    p.pbs[1] = a.extra_page_block_size > 0 ? a.extra_page_block_size : 1;
     p.sidx[1] = a.extra_indices; p.sidx_sb[1] = a.extra_indices_stride_b; p.sidx_ss[1] = a.extra_indices_stride_s;
     p.stopk[1] = a.extra_kv ? a.extra_topk : 0; p.stopk_len[1] = a.extra_topk_length;
+    const int nblocks[2] = {a.num_blocks, a.extra_num_blocks};
+    for (int i = 0; i < 2; ++i) {
+        p.tokens[i] = (uint32_t)std::min((int64_t)std::max(nblocks[i], 0) * p.pbs[i], (int64_t)1 << 31);
+        reciprocal(p.pbs[i], p.pbs_mul[i], p.pbs_shift[i]);
+    }
     return p;
 }
 

@@ -70,6 +70,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// Two barriers at once: a probe's way to shared memory and back is most of what it costs.
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "and.pred p, p, q;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar0), "r"(par0), "r"(bar1), "r"(par1) : "memory");
+    return ok != 0;
+}
 // A probe that answers at once (try_wait may hold the thread for a while).
 __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -136,6 +148,8 @@ __device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* m, int c0, in
     asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global.tile [%0, {%1, %2, %3, %4, %5}];"
                  ::"l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
+
+__device__ __forceinline__ void prefetch_l2(unsigned long long global) { asm volatile("prefetch.global.L2 [%0];" ::"l"(global)); }
 
 // Per-thread asynchronous 16-byte copy global -> shared; src_bytes = 0 writes zeros without reading.
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
