@@ -1173,15 +1173,8 @@ int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a) {
     using namespace sm100;
     Params p = prefill_params(a);
     p.row_blocks = (p.rows + pair::ROWS - 1) / pair::ROWS;
-    EncodeTiledFn encode = get_encode_fn();
-    if (!encode) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    // the keys as rows for TMA's gathers of four of them, 64 columns a box
     CUtensorMap kmap, unused, qmap;
-    cuuint64_t dims[2] = {(cuuint64_t)a.d_qk, (cuuint64_t)a.s_kv}, strides[1] = {(cuuint64_t)a.kv_stride_s * 2};
-    cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
-    const CUresult r = encode(&kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(MLA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+    if (!encode_kv_rows_map(&kmap, a)) return a.impl == 2 ? set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_prefill_fwd: no tensor map over these keys") : launch_sparse_prefill_portable(a);
     memset(&unused, 0, sizeof(unused));
     memset(&qmap, 0, sizeof(qmap));
     p.q_unit = pair::HALF;

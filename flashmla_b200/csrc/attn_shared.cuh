@@ -310,6 +310,17 @@ static bool encode_q_map(CUtensorMap* qmap, const void* q, int b, int s_q, int h
     return true;
 }
 
+// Tensor map over the prefill's keys as rows (d_qk columns, s_kv rows) for gathers of four rows by index, 64 columns at a time.  Returns false
+// where the driver rejects it (rows that overlap).
+static bool encode_kv_rows_map(CUtensorMap* kmap, const mla_sparse_prefill_args_t& a) {
+    EncodeTiledFn encode = get_encode_fn();
+    if (!encode) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)a.d_qk, (cuuint64_t)a.s_kv}, strides[1] = {(cuuint64_t)(a.s_kv > 1 ? a.kv_stride_s : 576) * 2};
+    cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
+    return encode(kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.kv), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // ---- the kernels' parameters from a call's arguments -----------------------------------------------------------
 static Params dense_params(const mla_dense_decode_args_t& a, int head_chunks) {
     Params p = {};
