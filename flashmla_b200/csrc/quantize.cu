@@ -6,8 +6,8 @@
 // A warp takes a token; lane l holds values 16l .. 16l+15 (8 lanes per scale group), so the record's e4m3 part is one coalesced
 // 512-byte store.  1152 bytes read + 656 bytes written per token.  The quotients x / s only need the correctly rounded reciprocal
 // of s, once per group, and three instructions each (Markstein's theorem; quotient16 below), two values per instruction.  66 K
-// tokens take 23.3 us (5.1 TB/s), 256 K 87 us (5.3 TB/s), back to back on one input; with inputs that change 66 K take 26.2 (28.7 with
-// two tokens per warp and scalar instructions).  Registers count: with two tokens per warp (75 of them in the place of 47)
+// tokens take 23.3 us (5.1 TB/s), 256 K 87 us (5.3 TB/s), back to back on one input; with inputs that change 66 K took 26.2 (28.7 with
+// two tokens per warp and scalar instructions) and take 23.7 in the launch chain below.  Registers count: with two tokens per warp (75 of them in the place of 47)
 // 26.6 and 96.7 us; with the scalar instructions, two / one token per warp, 27.3 / 26.8 and 98.2 / 99.2.  A persistent grid that
 // loads a token ahead is no faster (27.3).
 //
@@ -106,12 +106,20 @@ __device__ __forceinline__ void block_of(int64_t tok, int64_t ntok, int block_si
     row = tok - blk * block_size;
 }
 
+// The writers are launched as dependents of what is before them in the stream, and let their own dependents start when all their CTAs
+// have: back to back, the next call's CTAs are there when this one's last wave ends (66 K tokens 26.5 -> 23.7 us, inputs changing).
+__device__ __forceinline__ void join_chain() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __global__ void __launch_bounds__(256)
 quantize_fp8_kernel(const mla_quantize_args_t a) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
+    join_chain();
     for (int64_t tok = warp; tok < ntok; tok += nwarps) {
         int64_t blk, row;
         block_of(tok, ntok, a.block_size, blk, row);
@@ -143,6 +151,7 @@ quantize_fp8_model1_kernel(const mla_quantize_args_t a, const int pad_bytes) {
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
+    join_chain();
     if (pad_bytes)
 #pragma unroll 1
         for (int64_t blk = warp; blk < a.num_blocks; blk += nwarps)
@@ -199,9 +208,11 @@ int launch_quantize_fp8(const mla_quantize_args_t& a, bool zero_padding) {
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
     const int per_warp = a.layout && ntok > MODEL1_TWO_FROM ? 2 : 1, per_block = 8 * per_warp;         // tokens
     const int64_t blocks = min((ntok + per_block - 1) / per_block, (int64_t)1 << 24);
-    if (a.layout && per_warp == 2) quantize_fp8_model1_kernel<2><<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
-    else if (a.layout) quantize_fp8_model1_kernel<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a, (int)pad_bytes);
-    else quantize_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)a.stream>>>(a);
+    const cudaStream_t stream = (cudaStream_t)a.stream;
+    const dim3 grid((unsigned)blocks), block(256);
+    MLA_CHECK_CUDA(!a.layout       ? launch_dependent(quantize_fp8_kernel, grid, block, 0, stream, a)
+                   : per_warp == 2 ? launch_dependent(quantize_fp8_model1_kernel<2>, grid, block, 0, stream, a, (int)pad_bytes)
+                                   : launch_dependent(quantize_fp8_model1_kernel<1>, grid, block, 0, stream, a, (int)pad_bytes));
     MLA_CHECK_CUDA(cudaGetLastError());
     return MLA_OK;
 }
