@@ -25,8 +25,8 @@ combine_kernel(const mla_combine_args_t a) {
     // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
     // kernel set itself up from here on costs more than it hides: its CTAs take whole SMs while this grid still needs them;
     // dense decode with 2 query tokens 346 -> 351 us a step.  Every CTA does so when it has its sums: 4 requests of 64..512 tokens, 16 heads
-    // 12.4 -> 12.05 us a step, 128 requests of lognormal lengths 488.6 -> 484.2.  Not with eight warps a row, whose CTAs
-    // come in a single wave: one request of 100003 tokens, with its schedule, 44.8 -> 45.1.)
+    // 12.4 -> 12.05 us a step, 128 requests of lognormal lengths 488.6 -> 484.2.  With eight warps a row when they are in shared memory:
+    // one request of 100003 tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int ROWS = COMBINE_WARPS / WPR;            // heads per CTA
     constexpr int UNROLL = WPR == 8 ? 4 : 2;             // splits in flight per warp
@@ -140,6 +140,7 @@ combine_kernel(const mla_combine_args_t a) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) mine[i * 32] = acc[i];
         __syncthreads();
+        if (WPR == 8) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         // every warp of the row adds up and writes 512 / WPR columns
         if (!head_ok) return;
         const float4* row = reinterpret_cast<const float4*>(part) + (warp - sub) * 128;
