@@ -8,7 +8,8 @@
 // Per (request, query token, head) it reads n_splits * 2 KiB and writes 1 KiB: HBM-bound where there are many rows, bound
 // by its chain of memory latencies (split counts -> log-sum-exps -> partials -> output) where there are few.  A row is served
 // by WPR warps of a CTA, each taking every WPR-th split with 16 output columns per lane (4 x float4 per split: 512 coalesced
-// bytes per warp instruction); with WPR > 1 their sums meet in shared memory.  The first partials are requested together
+// bytes per warp instruction); with WPR > 1 their sums meet in shared memory.  Where there are hardly any rows, PARTS CTAs share
+// a row's columns.  The first partials are requested together
 // with the log-sum-exps, so that a row of up to WPR * UNROLL splits costs two round trips instead of three.  There is no
 // limit on the number of splits.
 #include "common.cuh"
@@ -19,7 +20,7 @@ namespace mla {
 
 constexpr int COMBINE_WARPS = 8;
 
-template <int WPR>
+template <int WPR, int PARTS>
 __global__ void __launch_bounds__(COMBINE_WARPS * 32, WPR == 8 ? 2 : WPR == 1 ? 4 : 3)
 combine_kernel(const mla_combine_args_t a) {
     // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
@@ -29,8 +30,10 @@ combine_kernel(const mla_combine_args_t a) {
     // one request of 100003 tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int ROWS = COMBINE_WARPS / WPR;            // heads per CTA
-    constexpr int UNROLL = WPR == 8 ? 4 : 2;             // splits in flight per warp
-    __shared__ float part[WPR > 1 ? COMBINE_WARPS * 512 : 1];
+    constexpr int NV = 4 / PARTS;                        // float4s of a split per lane
+    constexpr int UNROLL = (WPR == 8 ? 4 : 2) * PARTS;   // splits in flight per warp
+    __shared__ float part[WPR > 1 ? COMBINE_WARPS * 512 / PARTS : 1];
+    const int col0 = PARTS > 1 ? (int)blockIdx.z * (512 / PARTS) : 0;      // this CTA's columns
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = warp % WPR;
     const int bs_idx = blockIdx.x;                       // request * s_q + query token
@@ -43,17 +46,17 @@ combine_kernel(const mla_combine_args_t a) {
 
     const int64_t row_stride = (int64_t)a.s_q * a.h_q;   // rows per split slot
     const float* lse_acc = a.lse_accum + (int64_t)s0 * row_stride + (int64_t)t * a.h_q + head;
-    const float4* o_acc = reinterpret_cast<const float4*>(a.o_accum + ((int64_t)s0 * row_stride + (int64_t)t * a.h_q + head) * 512) + lane;
+    const float4* o_acc = reinterpret_cast<const float4*>(a.o_accum + ((int64_t)s0 * row_stride + (int64_t)t * a.h_q + head) * 512 + col0) + lane;
     const int64_t o_step = row_stride * 128;             // float4s from one split to the next
 
     // the first partials of this warp; their weights are not known yet
-    float4 v[UNROLL][4];
+    float4 v[UNROLL][NV];
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
         const int s = sub + u * WPR;
         if (s < n) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
+            for (int i = 0; i < NV; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
         }
     }
 
@@ -71,7 +74,7 @@ combine_kernel(const mla_combine_args_t a) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     float g = (sum == 0.f || sum != sum) ? INFINITY : log2f(sum) + mx;
-    if (lane == 0 && sub == 0 && head_ok)
+    if (lane == 0 && sub == 0 && head_ok && col0 == 0)
         a.lse[req * a.lse_stride_b + t * a.lse_stride_s + head * a.lse_stride_h] = g * kLn2;
     if (a.attn_sink) {
         const float sink = a.attn_sink[head];
@@ -80,9 +83,9 @@ combine_kernel(const mla_combine_args_t a) {
     }
 
     // pass 2: weighted sum of this warp's splits.  Lane l holds columns 4 l .. 4 l + 3 of every 128.
-    float4 acc[4];
+    float4 acc[NV];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     float w_block = exp2f(l_first - g);                  // weights of splits block .. block + 31, one per lane
     int block = 0;
 #pragma unroll 1
@@ -93,7 +96,7 @@ combine_kernel(const mla_combine_args_t a) {
                 const int s = base + u * WPR;
                 if (s < n) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
+                    for (int i = 0; i < NV; ++i) v[u][i] = __ldcs(o_acc + s * o_step + i * 32);
                 }
             }
         }
@@ -107,7 +110,7 @@ combine_kernel(const mla_combine_args_t a) {
                 }
                 const float w = __shfl_sync(0xffffffffu, w_block, s & 31);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < NV; ++i) {
                     acc[i].x += w * v[u][i].x; acc[i].y += w * v[u][i].y; acc[i].z += w * v[u][i].z; acc[i].w += w * v[u][i].w;
                 }
             }
@@ -115,7 +118,7 @@ combine_kernel(const mla_combine_args_t a) {
     }
     if (WPR < 8) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // out is bf16 or fp16: both are 2 bytes wide
-    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + req * a.o_stride_b + t * a.o_stride_s + head * a.o_stride_h;
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + req * a.o_stride_b + t * a.o_stride_s + head * a.o_stride_h + col0;
     auto store4 = [&](int col, float4 x) {
         uint2 packed;
         if (a.dtype == MLA_DTYPE_FP16) {
@@ -134,21 +137,22 @@ combine_kernel(const mla_combine_args_t a) {
     if (WPR == 1) {
         if (!head_ok) return;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) store4((lane + i * 32) * 4, acc[i]);
+        for (int i = 0; i < NV; ++i) store4((lane + i * 32) * 4, acc[i]);
     } else {
-        float4* mine = reinterpret_cast<float4*>(part) + warp * 128 + lane;
+        constexpr int ROW = 128 / PARTS;                  // float4s of a row
+        float4* mine = reinterpret_cast<float4*>(part) + warp * ROW + lane;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mine[i * 32] = acc[i];
+        for (int i = 0; i < NV; ++i) mine[i * 32] = acc[i];
         __syncthreads();
         if (WPR == 8) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         // every warp of the row adds up and writes 512 / WPR columns
         if (!head_ok) return;
-        const float4* row = reinterpret_cast<const float4*>(part) + (warp - sub) * 128;
-        for (int c = sub * (128 / WPR) + lane; c < (sub + 1) * (128 / WPR); c += 32) {
+        const float4* row = reinterpret_cast<const float4*>(part) + (warp - sub) * ROW;
+        for (int c = sub * (ROW / WPR) + lane; c < (sub + 1) * (ROW / WPR); c += 32) {
             float4 x = row[c];
 #pragma unroll
             for (int k = 1; k < WPR; ++k) {
-                const float4 y = row[k * 128 + c];
+                const float4 y = row[k * ROW + c];
                 x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
             }
             store4(c * 4, x);
@@ -183,12 +187,17 @@ int launch_combine(const mla_combine_args_t& a) {
     const int64_t wave = (int64_t)sms * 3 * COMBINE_WARPS;         // warps
     const int wpr = splits >= 16 && rows <= 2 * sms ? 8 : splits >= 8 && rows * 4 <= wave ? 4 : splits >= 4 && rows * 2 <= wave ? 2 : 1;
     const int rows_per_cta = COMBINE_WARPS / wpr;
-    const dim3 grid(a.b * a.s_q, (a.h_q + rows_per_cta - 1) / rows_per_cta), block(COMBINE_WARPS * 32);
+    // One to three requests: a row's columns in two CTAs, twice as many splits in flight each.  us a step, one request: 20000 tokens, 128 heads 21.2 ->
+    // 19.8, 100000, 64 heads 40.0 -> 38.9, 50000, two query tokens of 16 heads 31.5 -> 29.4; two requests of 2048 keys, 64 heads 17.1 -> 16.5.  Four requests
+    // of 64..512 tokens, whose splits are fewer than estimated, 12.3 -> 12.45.
+    const int parts = wpr == 8 && splits >= 48 && rows <= sms ? 2 : 1;
+    const dim3 grid(a.b * a.s_q, (a.h_q + rows_per_cta - 1) / rows_per_cta, parts), block(COMBINE_WARPS * 32);
     const cudaStream_t stream = (cudaStream_t)a.stream;
-    MLA_CHECK_CUDA(wpr == 8   ? launch_dependent(combine_kernel<8>, grid, block, 0, stream, a)
-                   : wpr == 4 ? launch_dependent(combine_kernel<4>, grid, block, 0, stream, a)
-                   : wpr == 2 ? launch_dependent(combine_kernel<2>, grid, block, 0, stream, a)
-                              : launch_dependent(combine_kernel<1>, grid, block, 0, stream, a));
+    MLA_CHECK_CUDA(parts == 2 ? launch_dependent(combine_kernel<8, 2>, grid, block, 0, stream, a)
+                   : wpr == 8 ? launch_dependent(combine_kernel<8, 1>, grid, block, 0, stream, a)
+                   : wpr == 4 ? launch_dependent(combine_kernel<4, 1>, grid, block, 0, stream, a)
+                   : wpr == 2 ? launch_dependent(combine_kernel<2, 1>, grid, block, 0, stream, a)
+                              : launch_dependent(combine_kernel<1, 1>, grid, block, 0, stream, a));
     return MLA_OK;
 }
 

@@ -40,6 +40,14 @@ def test_combine_warps_per_row(h_q, counts):
     assert torch.allclose(lse.cpu(), ref_lse, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("h_q,counts", [
+    (1, [2]), (16, [64, 1, 3]), (49, [65, 63, 8]),    # a row's columns in two CTAs; 64 splits are in flight at once
+    (148, [65]), (149, [64]),                         # ... up to a row per SM
+])
+def test_combine_columns_in_two_ctas(h_q, counts):
+    test_combine_warps_per_row(h_q, counts)
+
+
 @pytest.mark.parametrize("b", [1, 31, 32, 33, 64, 255, 256, 257, 1000])
 @pytest.mark.parametrize("parts", [1, 74, 300])
 def test_schedule_window_edges(b, parts):
