@@ -37,11 +37,12 @@
 // and one input in short runs:
 //   dense, 30 x 2048, 8 heads                  32.8 ->  23.7    dense, 61 x 4096, 32 / 64 heads     77 / 79.3 -> 68.7 / 78.0
 //   FP8, 64 x 2048, 16 heads                   93.3 ->  54.7    FP8, 74 x 2048, 64 heads            95.9 ->  82.2
+//   (these two since: 52.5 and 75.9)
 //   prefill, 512 x 2048, 64 heads               333 ->   308    prefill, 2000 x 1024, 64 heads       677 ->   564
 // Dense decode with 33 to 64 rows runs on pairs of SMs (attn_pair.cu) for batch sizes at which that hardly loses whatever the lengths are, where the block
 // table says that few tokens are to be read: see csrc/host.cpp.
-// Registers: at the launch bound of the FP8 variants 36 to 76 bytes are spilled (576-wide 64 / 16 heads 76 / 56, 512-wide 64 heads 36,
-// 16 none); where they are reloaded has not been established.  Dense and prefill: none.
+// Registers: at the launch bound of the FP8 variants 12 to 68 bytes are spilled (576-wide 64 / 16 heads 68 / 40, 512-wide 44 / 12);
+// where they are reloaded has not been established.  Dense and prefill: none.
 // FP8 decode with 128 heads as two CTAs of 64 is slower than a pair of SMs (64 x 2048: 101, pairs 56), since both CTAs convert
 // every record.
 //

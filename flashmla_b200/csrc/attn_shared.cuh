@@ -202,12 +202,8 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return pack16<false>(lo, hi); }
 
-// e8m0 scale byte -> fp32: 2^(e - 127); 0 is the subnormal 2^-127, 255 is NaN (as the format defines it)
-__device__ __forceinline__ float e8m0_to_float(uint32_t e) {
-    return __uint_as_float(e == 0 ? 0x00400000u : e == 255 ? 0x7fc00000u : e << 23);
-}
-
-// The same of byte `k` of a word (through bf16, which has all of these values).
+// e8m0 scale byte `k` of a word -> fp32: 2^(e - 127), 255 is NaN (as the format defines it).  Through bf16, which has all of these values, the
+// subnormal 2^-127 of byte 0 included.
 __device__ __forceinline__ float e8m0_of(uint32_t word, int k) {
     uint32_t r;
     asm("{\n\t.reg .b16 x, y;\n\tmov.b32 {x, y}, %1;\n\tcvt.rn.bf16x2.ue8m0x2 %0, x;\n\t}" : "=r"(r) : "r"(__byte_perm(word, 0, 0x4440 | k)));
