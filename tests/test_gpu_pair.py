@@ -60,6 +60,30 @@ def test_sparse_prefill(width, s_q, h_q, topk):
 
 
 @pytest.mark.parametrize("width", [576, 512])
+@pytest.mark.parametrize("rows,stride", [(200, 640), (200, 576), (200, 72), (1, 576), (1, 8)])
+def test_sparse_prefill_keys_in_rows_of_other_strides(width, rows, stride):
+    """The row gathers' tensor map: padded rows (NaN between and behind them), rows that overlap, a single row.  Entries that are no key read zeros,
+    not what lies behind the last row.  Against the same keys in rows of their own."""
+    import flashmla_b200 as fm
+    gen = torch.Generator().manual_seed(rows + stride)
+    memory = torch.full((rows * max(stride, width) + 4 * 640,), float("nan"))
+    index = (torch.arange(rows).view(-1, 1) * stride + torch.arange(width)).view(-1)
+    memory[index] = torch.randn(rows * width, generator=gen)
+    memory = memory.bfloat16().to(DEV)
+    kv = memory.as_strided((rows, 1, width), (stride, width, 1))
+    idx = torch.randint(-3, rows + 40, (90, 1, 320), generator=gen, dtype=torch.int32)
+    idx[7], idx[8, :, 128:] = -1, rows
+    q = torch.randn(90, 128, width, generator=gen).bfloat16().to(DEV)
+    out, top, lse = fm.flash_mla_sparse_fwd(q, kv, idx.to(DEV), width ** -0.5, 512)
+    ref_out, ref_top, ref_lse = fm.flash_mla_sparse_fwd(q, kv.clone(memory_format=torch.contiguous_format), idx.to(DEV), width ** -0.5, 512)
+    fm.check_status()
+    assert not torch.isnan(out.float()).any()
+    assert_out_close("out", out.cpu(), ref_out.cpu())
+    assert_lse_close("lse", lse.cpu(), ref_lse.cpu())
+    assert torch.allclose(top.cpu(), ref_top.cpu(), rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("width", [576, 512])
 def test_sparse_prefill_maxima_and_shared_query(width):
     """Maxima that move on every tile (the true maximum is a result too); heads that share their query: Q that is no tensor map."""
     import flashmla_b200 as fm
