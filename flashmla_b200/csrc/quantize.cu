@@ -14,8 +14,9 @@
 // Layout 1 is the 512-wide "MODEL1" form (tests/quant.py:55-75 of the reference): 448 values in groups of 64 with
 // power-of-two scales stored as e8m0 bytes, 64 bf16 RoPE values; a block is block_size x 576 value bytes followed by
 // block_size x 8 scale bytes (7 scales + 1 pad).  Lanes 0-27 hold the quantised values (4 lanes per group), lanes 28-31
-// the RoPE part.  A warp of a long call takes two tokens, whose loads are in flight together, with registers for four blocks per SM
-// (20 bytes of them spilled): 66 K tokens 27.2 us, 256 K 92.9 (one token per warp 27.2 and 101, scalar instructions 35.5 and
+// the RoPE part.  A warp of a long call takes two tokens, whose loads are in flight together, with registers for 32 warps per SM
+// (20 bytes of them spilled), in blocks of four warps (of eight: 45 K tokens 17.7 us, four 17.1; 66 K 25.3, 24.6; 256 K 91.5, 89.5; the 656-byte
+// form loses, 23.7, 24.3).  Before that and the launch chain: 66 K tokens 27.2 us, 256 K 92.9 (one token per warp 27.2 and 101, scalar instructions 35.5 and
 // 131.7).  A short call is bound by its own latency and takes one (MODEL1_TWO_FROM).  The first warps also zero
 // the `pad_bytes` behind every block, where the caller owns them (one warp a block; with the last token's stores, inside the
 // loop, 66 K tokens took 36.9 us instead of 34.9, on the scalar kernel).
@@ -145,7 +146,7 @@ quantize_fp8_kernel(const mla_quantize_args_t a) {
 
 // TOKENS: tokens per warp, in flight together
 template <int TOKENS>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(128, 8)
 quantize_fp8_model1_kernel(const mla_quantize_args_t a, const int pad_bytes) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -206,10 +207,10 @@ int launch_quantize_fp8(const mla_quantize_args_t& a, bool zero_padding) {
     const int64_t pad_bytes = zero_padding && a.layout ? a.out_stride_block_bytes - (int64_t)a.block_size * rec : 0;
     MLA_CHECK_ARG(pad_bytes <= 0x7fffff00, "mla_quantize_fp8_kvcache_padded: more than 2 GB of padding behind a block");
     const int64_t ntok = (int64_t)a.num_blocks * a.block_size;
-    const int per_warp = a.layout && ntok > MODEL1_TWO_FROM ? 2 : 1, per_block = 8 * per_warp;         // tokens
+    const int per_warp = a.layout && ntok > MODEL1_TWO_FROM ? 2 : 1, warps = a.layout ? 4 : 8, per_block = warps * per_warp;      // tokens
     const int64_t blocks = min((ntok + per_block - 1) / per_block, (int64_t)1 << 24);
     const cudaStream_t stream = (cudaStream_t)a.stream;
-    const dim3 grid((unsigned)blocks), block(256);
+    const dim3 grid((unsigned)blocks), block(32 * warps);
     MLA_CHECK_CUDA(!a.layout       ? launch_dependent(quantize_fp8_kernel, grid, block, 0, stream, a)
                    : per_warp == 2 ? launch_dependent(quantize_fp8_model1_kernel<2>, grid, block, 0, stream, a, (int)pad_bytes)
                                    : launch_dependent(quantize_fp8_model1_kernel<1>, grid, block, 0, stream, a, (int)pad_bytes));
