@@ -1174,6 +1174,7 @@ int launch_sparse_prefill_pair(const mla_sparse_prefill_args_t& a) {
     Params p = prefill_params(a);
     p.row_blocks = (p.rows + pair::ROWS - 1) / pair::ROWS;
     CUtensorMap kmap, unused, qmap;
+    // (a driver that refuses rows that overlap: the kernel for all shapes)
     if (!encode_kv_rows_map(&kmap, a)) return a.impl == 2 ? set_error(MLA_ERR_UNSUPPORTED, "mla_sparse_prefill_fwd: no tensor map over these keys") : launch_sparse_prefill_portable(a);
     memset(&unused, 0, sizeof(unused));
     memset(&qmap, 0, sizeof(qmap));

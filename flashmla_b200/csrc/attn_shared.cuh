@@ -307,7 +307,7 @@ static bool encode_q_map(CUtensorMap* qmap, const void* q, int b, int s_q, int h
 }
 
 // Tensor map over the prefill's keys as rows (d_qk columns, s_kv rows) for gathers of four rows by index, 64 columns at a time.  Returns false
-// where the driver rejects it (rows that overlap).
+// where the driver makes none; driver 580 does for all keys that get here, padded rows and rows that overlap among them.
 static bool encode_kv_rows_map(CUtensorMap* kmap, const mla_sparse_prefill_args_t& a) {
     EncodeTiledFn encode = get_encode_fn();
     if (!encode) return false;

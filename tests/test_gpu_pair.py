@@ -83,6 +83,32 @@ def test_sparse_prefill_keys_in_rows_of_other_strides(width, rows, stride):
     assert torch.allclose(top.cpu(), ref_top.cpu(), rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("impl", [0, 2])
+@pytest.mark.parametrize("width,h_q,stride", [(576, 128, 640), (512, 128, 520), (576, 128, 576), (576, 128, 504), (512, 128, 72), (512, 100, 504), (576, 200, 8)])
+def test_sparse_prefill_keys_of_any_row_stride_run_on_pairs(width, h_q, stride, impl):
+    """The driver makes a tensor map over rows of their own, padded or not, and over rows that overlap: none of them leaves the pair kernel, and
+    overlapping rows give what the oracle gives for them."""
+    import flashmla_b200 as fm
+    rows, s_q, topk, gen = 300, 65, 320, torch.Generator().manual_seed(h_q + stride)
+    memory = torch.randn(rows * stride + width, generator=gen).bfloat16()
+    kv = memory.as_strided((rows, 1, width), (stride, width, 1))
+    idx = torch.randint(-3, rows + 40, (s_q, 1, topk), generator=gen, dtype=torch.int32)
+    idx[7], idx[8, :, 128:] = -1, rows
+    lengths = torch.randint(0, topk + 1, (s_q,), generator=gen, dtype=torch.int32)
+    q, sink = torch.randn(s_q, h_q, width, generator=gen).bfloat16(), torch.randn(h_q, generator=gen)
+    ref = attention.sparse_prefill(q, kv.contiguous(), torch.where(idx < rows, idx, -1), width ** -0.5, 512, sink, lengths)
+    kv_dev, got = memory.to(DEV).as_strided((rows, 1, width), (stride, width, 1)), []
+    fm.set_impl(impl)
+    try:
+        assert small.kernels(lambda: got.append(fm.flash_mla_sparse_fwd(q.to(DEV), kv_dev, idx.to(DEV), width ** -0.5, 512, sink.to(DEV), lengths.to(DEV)))) == {"attn_pair_kernel"}
+    finally:
+        fm.set_impl(0)
+    fm.check_status()
+    assert_out_close("out", got[0][0], ref[0])
+    assert_lse_close("max_logits", got[0][1], ref[1])
+    assert_lse_close("lse", got[0][2], ref[2])
+
+
 @pytest.mark.parametrize("width", [576, 512])
 def test_sparse_prefill_maxima_and_shared_query(width):
     """Maxima that move on every tile (the true maximum is a result too); heads that share their query: Q that is no tensor map."""
