@@ -213,3 +213,38 @@ def test_model1_block_padding_is_zero(block_size):
     whole = got.view(torch.uint8).as_strided((blocks, n), (n, 1))
     assert not whole[:, block_size * 584:].any()
     assert torch.equal(got.view(torch.uint8).cpu(), quant.quantize_model1(x.cpu()).view(torch.uint8))
+
+
+@pytest.mark.parametrize("impl", [1, 2])
+@pytest.mark.parametrize("h_q", [16, 64, 128])
+def test_exponent_bytes_at_their_ends(h_q, impl):
+    """Scale bytes 0 (2^-127, a subnormal), 1 and 2 in every place of a record: values are those of the format to 2^-7 (16-bit probabilities and
+    outputs: 2^-9 each; values of one sign).  Byte 255 is NaN: the request that has such a key gets no number (NaN, or the zeros of a request without
+    keys), the other nothing of it."""
+    import flashmla_b200 as fm
+    gen, tokens, topk = torch.Generator().manual_seed(h_q), 256, 128
+    kv = quant.quantize_model1(torch.randn(4, 64, 1, 512, generator=gen).bfloat16())
+    data = kv.contiguous().view(torch.uint8).reshape(4, -1)
+    values, scales = data[:, :64 * 576].view(4, 64, 576), data[:, 64 * 576:].view(4, 64, 8)
+    values[..., :448] = torch.randint(0x78, 0x7f, (4, 64, 448), generator=gen, dtype=torch.uint8)      # 256 .. 448
+    scales[..., :7] = torch.randint(0, 3, (4, 64, 7), generator=gen, dtype=torch.uint8)
+    e4m3 = values[..., :448].clone().view(torch.float8_e4m3fn).double().view(tokens, 7, 64)
+    keys = torch.cat([(e4m3 * torch.exp2(scales[..., :7].double().view(tokens, 7, 1) - 127)).view(tokens, 448),
+                      values[..., 448:].clone().view(torch.bfloat16).double().view(tokens, 64)], 1)
+    scales[3, 8, 3] = 255                                                   # token 200
+    idx = torch.stack([torch.randperm(200, generator=gen)[:topk], torch.randperm(256, generator=gen)[:topk]]).view(2, 1, topk).to(torch.int32)
+    idx[1, 0, 77] = 200
+    q = (torch.randn(2, 1, h_q, 512, generator=gen) * 0.1).bfloat16()
+    fm.set_impl(impl)
+    try:
+        out, lse = _decode(q.to(DEV), model1_cache_from_bytes(data.view(4, 64, 1, 584), quant.model1_block_bytes(64), DEV), idx.to(DEV), 512 ** -0.5)
+    finally:
+        fm.set_impl(0)
+    chosen = keys[idx[0, 0].long()]
+    score = q[0, 0].double() @ chosen.T * 512 ** -0.5
+    want = torch.softmax(score, -1) @ chosen
+    got = out[0, 0].cpu().double()
+    assert (want[:, :448] > 0).all() and ((got - want)[:, :448].abs() <= 2 ** -7 * want[:, :448]).all()
+    assert_out_close("RoPE columns", got[:, 448:], want[:, 448:])
+    assert_lse_close("lse", lse[0, :, 0], torch.logsumexp(score, -1))
+    assert (out[1].isnan() | (out[1] == 0)).all() and not lse[1].isfinite().any()
