@@ -326,3 +326,76 @@ def test_softmax_threads_leave_together(path):
     for i in waits:
         after = [step for step in (steps + steps)[i + 1:] if step != ("barrier", False)]          # (the role is a loop)
         assert after[0][0] == "wait" or after[0] == ("barrier", True), (steps[i], after[0])
+
+
+# ---- the pair kernel's softmax warps by page ---------------------------------------------------------------------------
+def _graph_by_page(tiles, slots, tables, convert, rank):
+    """`_graph` with the softmax warps of page 0 and of page 1 as roles of their own: each hands its part of P over by itself, and P V of a
+    page waits for that part alone.  (The vote, which holds every warp's P back until all have read their masks, is left out.)"""
+    edges = {e: list(p) for e, p in _graph(tiles, slots, tables, convert, rank).items() if e[0] != "softmax"}
+    for page in range(2):
+        steps = [(what, g, page) for g in range(tiles) for what in ("start", "give", "mask", "p")]
+        for i, step in enumerate(steps):
+            edges[("softmax",) + step] = [("softmax",) + steps[i - 1]] if i else []
+        for g in range(tiles):
+            edges["softmax", "start", g, page].append(("scores", "scores", g, 3))                  # s_full
+    for event, before in edges.items():
+        if event[0] == "values":
+            edges[event] = [("softmax", "p", e[2], event[3] // 2) if e[:2] == ("softmax", "p") else e for e in before]
+        elif event[0] == "scores":
+            edges[event] = [f for e in before for f in ([("softmax", "give", e[2], page) for page in range(2)] if e[0] == "softmax" else [e])]
+    return edges
+
+
+@pytest.mark.parametrize("rank", [0, 1])
+@pytest.mark.parametrize("convert", [False, True])          # prefill, FP8 decode
+def test_masks_are_read_by_both_pages_before_they_are_overwritten(convert, rank):
+    slots, masks, tables = _plan()
+    tiles, writer = masks + 8, "look-up" if convert else "feed"
+    edges = _graph_by_page(tiles, slots, tables, convert, rank)
+
+    def kept(edges, depth, page):
+        return all(_before(edges, ("softmax", "mask", g, page), (writer, "meta", g + depth, 0)) for g in range(tiles - masks))
+
+    for page in range(2):
+        assert all(_before(edges, (writer, "meta", g, 0), ("softmax", "mask", g, page)) for g in range(tiles))
+        assert kept(edges, masks, page)
+        assert not kept(edges, masks // 2 if convert else 2, page)      # the check sees a ring that is too shallow
+        late = dict(edges)                                  # ... and a mask that is read when this page's P has been handed over
+        late["softmax", "p", 3, page] = [("softmax", "give", 3, page)]
+        assert not _before(late, ("softmax", "mask", 3, page), (writer, "meta", 3 + masks, 0))
+
+
+# ---- the conditional barriers of the pair kernel's softmax warps -----------------------------------------------------------
+def _leaves_behind_every_wait(text):
+    """The barriers behind the waits of a tile stand under `if (together)`.  A warp with an expired wait must find that true, every warp must go there
+    where a tail was waited for, and P is stored behind the first of them."""
+    start = max(m.start() for m in re.finditer(r"// -+ softmax", text))
+    role = re.sub(r"//[^\n]*", "", text[start:text.index("wind_down:", start)])
+    tile = role[role.index("wt.wait(&sm.s_full"):]
+    decided = re.search(r"bool together = ([^;]*);", tile)
+    first = tile.index("BAR_OR_LEAVE(wt.expired());")
+    second = tile.index("if (together) BAR_OR_LEAVE(wt.expired());")
+    announced = tile.index("if (lane == 0 && !wt.expired())", second)
+    waits = [m.start() for m in re.finditer(r"wt\.wait\(", tile[:second])]
+    tails = [w for w in waits if w > first]
+    return (decided is not None and "wt.expired()" in decided.group(1) and all(w < decided.start() or w in tails for w in waits)
+            and tile.count("{", decided.end(), first) == 1 and "if (together) {" in tile[decided.end():first]
+            and re.search(r"__any_sync\(0xffffffffu, mx > m_run \+ RESCALE_THRESHOLD \|\| wt\.expired\(\)\)", tile[:decided.start()]) is not None
+            and first < tile.index("store();", decided.end()) < second < announced
+            and all("together = true;" in tile[w:tile.index("ring.skip(4);", w)] and "sm.f_tail" in tile[w:w + 40] for w in tails))
+
+
+def test_a_warp_with_an_expired_wait_reaches_the_conditional_barriers():
+    text = open(SOURCE).read()
+    assert _leaves_behind_every_wait(text)
+    for there, instead in ((" || wt.expired());\n                if (together) {", ");\n                if (together) {"),
+                           ("RESCALE_THRESHOLD || wt.expired())", "RESCALE_THRESHOLD)"),
+                           ("together = true;", ""),
+                           ("if (together) BAR_OR_LEAVE(wt.expired());", "")):
+        assert text.count(there) == 1
+        changed = text.replace(there, instead)
+        try:
+            assert not _leaves_behind_every_wait(changed), there
+        except ValueError:                                  # (a piece it looks for is gone)
+            pass
