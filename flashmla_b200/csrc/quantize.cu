@@ -26,8 +26,8 @@
 
 namespace mla {
 
-// Layout 1, more tokens than this: two per warp, up to it one.  us, one / two tokens per warp: 64 tokens 1.9 / 2.7, 4 K 2.9 / 3.7,
-// 33 K 12.0 / 12.5, 66 K 24.7 / 24.3, 131 K 51.5 / 48.0.
+// Layout 1, more tokens than this: two per warp, up to it one.  us, one / two tokens per warp, inputs changing: 64 tokens 1.55 / 2.15, 4 K 2.5 / 3.1,
+// 16 K 7.88 / 7.97, 26 K 11.26 / 11.20, 33 K 13.7 / 13.9, 40 K 16.3 / 16.6, 45 K 18.2 / 17.9, 66 K 25.7 / 25.0, 131 K 49.2 / 46.8, 256 K 94.2 / 88.6.
 constexpr int64_t MODEL1_TWO_FROM = 40000;
 
 __device__ __forceinline__ float pow2_ceil(float s) {
@@ -108,7 +108,9 @@ __device__ __forceinline__ void block_of(int64_t tok, int64_t ntok, int block_si
 }
 
 // The writers are launched as dependents of what is before them in the stream, and let their own dependents start when all their CTAs
-// have: back to back, the next call's CTAs are there when this one's last wave ends (66 K tokens 26.5 -> 23.7 us, inputs changing).
+// have: back to back, the next call's CTAs are there when this one's last wave ends (66 K tokens 26.5 -> 23.7 us, inputs changing).  What a single call
+// between two ordinary kernels adds to them, as a plain launch / now: 1 K tokens 3.0 / 2.2 us, 8 K 4.7 / 4.0, 66 K 23.6 / 22.75; 512-wide 2.6 / 1.9, 5.0 /
+// 4.1, 26.2 / 25.0 (the blocks of four warps among it).
 __device__ __forceinline__ void join_chain() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -207,3 +207,40 @@ def test_schedule_rows_in_groups_of_32_partitions(b, parts):
         meta, ns = _run_meta(b, parts, 64, 5, seqlens=seq)
         want_meta, want_ns = sched_meta.get_sched_meta(b, parts, 64, 5, seqlens_k=seq)
         assert np.array_equal(np.asarray(meta)[:, :7], want_meta[:, :7]) and np.array_equal(np.asarray(ns), want_ns)
+
+
+@pytest.mark.parametrize("width,pages,h_q", [(576, 3, 64), (576, 1031, 128), (512, 3, 128), (512, 700, 64)])
+def test_writer_in_a_captured_graph(width, pages, h_q):
+    """The writers as links of the launch chain: in a graph behind the kernel that makes their input and in front of the decode that reads the records,
+    which starts while they run.  Replayed with other inputs; bytes and results are those of single launches with the device idle between them."""
+    import flashmla_b200 as fm
+    from flashmla_b200.kvcache import quantize_fp8_kvcache, quantize_fp8_kvcache_model1
+    write = quantize_fp8_kvcache if width == 576 else quantize_fp8_kvcache_model1
+    gen = torch.Generator(device=DEV).manual_seed(pages)
+    new = lambda: torch.randn(pages, 64, 1, width, generator=gen, device=DEV).bfloat16()
+    q = torch.randn(2, 1, h_q, width, generator=gen, device=DEV).bfloat16()
+    # the last tokens that the writers write, and some of the others
+    idx = torch.randint(0, pages * 64, (2, 1, 192), generator=gen, device=DEV, dtype=torch.int32)
+    idx[..., :64] = torch.arange(pages * 64 - 64, pages * 64, device=DEV, dtype=torch.int32)
+    source, meta = new(), fm.get_mla_metadata()[0]
+
+    def step(wait):
+        made = source * 0.5
+        wait()
+        records = write(made)
+        wait()
+        return (records,) + fm.flash_mla_with_kvcache(q, records, None, None, 512, meta, None, width ** -0.5, False, True, idx)
+
+    step(torch.cuda.synchronize)                   # (makes the schedule, loads the kernels)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(lambda: None)
+    for _ in range(4):
+        source.copy_(new())
+        graph.replay()
+        torch.cuda.synchronize()
+        want = step(torch.cuda.synchronize)
+        torch.cuda.synchronize()
+        assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8))
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    fm.check_status()
