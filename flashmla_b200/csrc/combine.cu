@@ -19,22 +19,31 @@
 namespace mla {
 
 constexpr int COMBINE_WARPS = 8;
-// Rows whose columns two CTAs may share: with up to this many splits the first one takes them all and the second leaves.  us a step, one CTA a row / two
-// wherever they may / this rule: 16 heads, 1 to 3 requests of 100 tokens (2 splits each) 10.59, 10.65, 10.68 / 10.74, 10.86, 10.86 / 10.60, 10.68, 10.70;
-// of 300 (5) 10.42, 10.44, 10.60 / 10.58, 10.61, 10.76 / 10.42, 10.51, 10.58; of 900 (15) 12.19, 12.29, 12.49 / 12.17, 12.30, 12.39 / 12.12, 12.22, 12.39;
-// of 1200 (19) 10.96, 11.13, 11.44 / 10.85, 10.94, 11.12 / 10.89, 11.03, 11.19.  With 8 in the place of 16, 600 and 900 tokens take 0.1 to 0.2 more.
-constexpr int ONE_CTA_SPLITS = 16;
 
-// One CTA's rows: columns col0 .. col0 + 512 / PARTS - 1 of the sums of splits s0 .. s0 + n - 1 (n > 1).
 template <int WPR, int PARTS>
-__device__ __forceinline__ void combine_rows(const mla_combine_args_t& a, float* part, int req, int t, int s0, int n, int col0) {
+__global__ void __launch_bounds__(COMBINE_WARPS * 32, WPR == 8 ? 2 : WPR == 1 ? 4 : 3)
+combine_kernel(const mla_combine_args_t a) {
+    // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
+    // kernel set itself up from here on costs more than it hides: its CTAs take whole SMs while this grid still needs them;
+    // dense decode with 2 query tokens 346 -> 351 us a step.  Every CTA does so when it has its sums: 4 requests of 64..512 tokens, 16 heads
+    // 12.4 -> 12.05 us a step, 128 requests of lognormal lengths 488.6 -> 484.2.  With eight warps a row when they are in shared memory:
+    // one request of 100003 tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int ROWS = COMBINE_WARPS / WPR;            // heads per CTA
     constexpr int NV = 4 / PARTS;                        // float4s of a split per lane
     constexpr int UNROLL = (WPR == 8 ? 4 : 2) * PARTS;   // splits in flight per warp
+    __shared__ float part[WPR > 1 ? COMBINE_WARPS * 512 / PARTS : 1];
+    const int col0 = PARTS > 1 ? (int)blockIdx.z * (512 / PARTS) : 0;      // this CTA's columns
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = warp % WPR;
+    const int bs_idx = blockIdx.x;                       // request * s_q + query token
+    const int req = bs_idx / a.s_q, t = bs_idx - req * a.s_q;
     const int head = min((int)blockIdx.y * ROWS + warp / WPR, a.h_q - 1);
     const bool head_ok = blockIdx.y * ROWS + warp / WPR < a.h_q;
+    const int s0 = a.num_splits[req], s1 = a.num_splits[req + 1];
+    const int n = s1 - s0;
+    if (n <= 1) return;                                  // the decode kernel wrote the final result (whole CTA)
+
     const int64_t row_stride = (int64_t)a.s_q * a.h_q;   // rows per split slot
     const float* lse_acc = a.lse_accum + (int64_t)s0 * row_stride + (int64_t)t * a.h_q + head;
     const float4* o_acc = reinterpret_cast<const float4*>(a.o_accum + ((int64_t)s0 * row_stride + (int64_t)t * a.h_q + head) * 512 + col0) + lane;
@@ -151,25 +160,6 @@ __device__ __forceinline__ void combine_rows(const mla_combine_args_t& a, float*
     }
 }
 
-template <int WPR, int PARTS>
-__global__ void __launch_bounds__(COMBINE_WARPS * 32, WPR == 8 ? 2 : WPR == 1 ? 4 : 3)
-combine_kernel(const mla_combine_args_t a) {
-    // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
-    // kernel set itself up from here on costs more than it hides: its CTAs take whole SMs while this grid still needs them;
-    // dense decode with 2 query tokens 346 -> 351 us a step.  Every CTA does so when it has its sums: 4 requests of 64..512 tokens, 16 heads
-    // 12.4 -> 12.05 us a step, 128 requests of lognormal lengths 488.6 -> 484.2.  With eight warps a row when they are in shared memory:
-    // one request of 100003 tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    __shared__ float part[WPR > 1 ? COMBINE_WARPS * 512 : 1];
-    const int bs_idx = blockIdx.x;                       // request * s_q + query token
-    const int req = bs_idx / a.s_q, t = bs_idx - req * a.s_q;
-    const int s0 = a.num_splits[req], n = a.num_splits[req + 1] - s0;
-    if (n <= 1) return;                                  // the decode kernel wrote the final result (whole CTA)
-    if (PARTS == 1) combine_rows<WPR, 1>(a, part, req, t, s0, n, 0);
-    else if (n > ONE_CTA_SPLITS) combine_rows<WPR, PARTS>(a, part, req, t, s0, n, (int)blockIdx.z * (512 / PARTS));
-    else if (blockIdx.z == 0) combine_rows<WPR, 1>(a, part, req, t, s0, n, 0);
-}
-
 int launch_combine(const mla_combine_args_t& a) {
     MLA_CHECK_ARG(a.b > 0 && a.s_q > 0 && a.h_q > 0, "combine: b, s_q, h_q must be positive");
     MLA_CHECK_ARG(a.d_v == 512, "combine: only d_v == 512 is supported (got %d)", a.d_v);
@@ -197,10 +187,9 @@ int launch_combine(const mla_combine_args_t& a) {
     const int64_t wave = (int64_t)sms * 3 * COMBINE_WARPS;         // warps
     const int wpr = splits >= 16 && rows <= 2 * sms ? 8 : splits >= 8 && rows * 4 <= wave ? 4 : splits >= 4 && rows * 2 <= wave ? 2 : 1;
     const int rows_per_cta = COMBINE_WARPS / wpr;
-    // At most a row per SM and 48 splits by the estimate (one to three requests of up to 64 rows, one of up to 128): two CTAs for rows of many
-    // splits, each with half of the columns and twice as many splits in flight.  The estimate knows no lengths; how many splits there are decides on the
-    // device (ONE_CTA_SPLITS).  us a step, one CTA / two, one request: 20000 tokens, 128 heads 20.3 / 18.8, 64 heads 20.0 / 18.8, 16 heads 19.0 / 17.5; two
-    // requests of 2048 keys, 64 heads 16.5 / 16.1; 12000 tokens, two requests of 16 heads 17.0 / 15.6.
+    // One to three requests: a row's columns in two CTAs, twice as many splits in flight each.  us a step, one request: 20000 tokens, 128 heads 21.2 ->
+    // 19.8, 100000, 64 heads 40.0 -> 38.9, 50000, two query tokens of 16 heads 31.5 -> 29.4; two requests of 2048 keys, 64 heads 17.1 -> 16.5.  Four requests
+    // of 64..512 tokens, whose splits are fewer than estimated, 12.3 -> 12.45.
     const int parts = wpr == 8 && splits >= 48 && rows <= sms ? 2 : 1;
     const dim3 grid(a.b * a.s_q, (a.h_q + rows_per_cta - 1) / rows_per_cta, parts), block(COMBINE_WARPS * 32);
     const cudaStream_t stream = (cudaStream_t)a.stream;

@@ -48,21 +48,6 @@ def test_combine_columns_in_two_ctas(h_q, counts):
     test_combine_warps_per_row(h_q, counts)
 
 
-@pytest.mark.parametrize("h_q,counts", [
-    (16, [16, 17, 2]), (49, [17, 15, 64]),        # up to 16 splits the first CTA of a row takes all of its columns, the second leaves
-    (50, [65, 63, 8]), (128, [17]), (128, [16]),  # 150 rows: one CTA each; one request of 128 rows: two (148 SMs)
-])
-def test_combine_one_or_two_ctas_by_the_splits_there_are(h_q, counts):
-    test_combine_warps_per_row(h_q, counts)
-
-
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("with_sink", [False, True])
-@pytest.mark.parametrize("h_q,counts", [(24, [16, 50]), (8, [17, 3, 66])])
-def test_combine_columns_in_two_ctas_two_query_tokens(h_q, counts, dtype, with_sink):
-    test_combine_variants_two_query_tokens(h_q, counts, dtype, with_sink)
-
-
 @pytest.mark.parametrize("b", [1, 31, 32, 33, 64, 255, 256, 257, 1000])
 @pytest.mark.parametrize("parts", [1, 74, 300])
 def test_schedule_window_edges(b, parts):
