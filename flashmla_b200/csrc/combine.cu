@@ -187,9 +187,14 @@ int launch_combine(const mla_combine_args_t& a) {
     const int64_t wave = (int64_t)sms * 3 * COMBINE_WARPS;         // warps
     const int wpr = splits >= 16 && rows <= 2 * sms ? 8 : splits >= 8 && rows * 4 <= wave ? 4 : splits >= 4 && rows * 2 <= wave ? 2 : 1;
     const int rows_per_cta = COMBINE_WARPS / wpr;
-    // One to three requests: a row's columns in two CTAs, twice as many splits in flight each.  us a step, one request: 20000 tokens, 128 heads 21.2 ->
-    // 19.8, 100000, 64 heads 40.0 -> 38.9, 50000, two query tokens of 16 heads 31.5 -> 29.4; two requests of 2048 keys, 64 heads 17.1 -> 16.5.  Four requests
-    // of 64..512 tokens, whose splits are fewer than estimated, 12.3 -> 12.45.
+    // Up to a row per SM and 48 splits or more by the estimate (on 148 SMs one to three requests with 148 rows together, of more than 64 rows each
+    // one): a row's columns in two CTAs, twice as many splits in flight each.  us a step, one CTA / two, one request: 20000 tokens, 128 heads 20.2 /
+    // 18.9, 64 heads 20.0 / 18.8, 16 heads 18.7 / 17.1; two requests of 2048 keys, 64 heads 16.7 / 16.1; 2000 tokens, 1, 2, 3 requests of 16 heads 12.8,
+    // 12.8, 13.1 / 12.3, 12.4, 12.6.  The estimate knows no lengths.  Short requests have fewer splits and lose: 2 splits (100 tokens), 1, 2, 3 requests of 16
+    // heads 10.85, 10.77, 10.94 / 10.94, 10.94, 11.03, of 48 heads 13.85, 14.01, 14.02 / 14.02, 14.18, 14.21; 5 splits 0.1 or less; from 10 on both are equal or
+    // two CTAs ahead.  Four requests of 64..512 tokens lose (12.3 / 12.45) and stay with one.
+    //   Left to the device - up to 8 or 16 splits the first CTA takes all columns, the second leaves - 2 splits are as fast as with one CTA, but rows of other
+    // calls are slower by the longer code: 15 splits 12.3 -> 12.7, 105 splits 17.3 -> 17.7, four requests of 100 tokens 10.8 -> 11.1 (one source for both forms).
     const int parts = wpr == 8 && splits >= 48 && rows <= sms ? 2 : 1;
     const dim3 grid(a.b * a.s_q, (a.h_q + rows_per_cta - 1) / rows_per_cta, parts), block(COMBINE_WARPS * 32);
     const cudaStream_t stream = (cudaStream_t)a.stream;

@@ -48,6 +48,21 @@ def test_combine_columns_in_two_ctas(h_q, counts):
     test_combine_warps_per_row(h_q, counts)
 
 
+@pytest.mark.parametrize("h_q,counts", [
+    (49, [17, 15, 64]), (50, [65, 63, 8]),        # 147 and 150 rows: two CTAs a row up to a row per SM (148), one beyond
+    (128, [2]), (128, [65]), (16, [16, 17, 2]),   # one request of 128 rows; rows of few splits beside others
+])
+def test_combine_up_to_a_row_per_sm(h_q, counts):
+    test_combine_warps_per_row(h_q, counts)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("with_sink", [False, True])
+@pytest.mark.parametrize("h_q,counts", [(24, [16, 50]), (8, [17, 3, 66])])
+def test_combine_columns_in_two_ctas_two_query_tokens(h_q, counts, dtype, with_sink):
+    test_combine_variants_two_query_tokens(h_q, counts, dtype, with_sink)
+
+
 @pytest.mark.parametrize("b", [1, 31, 32, 33, 64, 255, 256, 257, 1000])
 @pytest.mark.parametrize("parts", [1, 74, 300])
 def test_schedule_window_edges(b, parts):
