@@ -34,7 +34,7 @@
 // With cluster-wide releases a tile of dense decode took 5350 cycles in the place of 4110.
 //
 // What bounds it.  Dense decode, 128 requests of about 4096 tokens: 2700 to 3300 cycles a tile, of which the tensor core works 2250 (60 % of
-// the launch); DRAM at 4.9 TB/s in a launch by itself (136 us at 1.63 GHz), back to back the power limit (1.34 GHz).  A tile's loads wait for
+// the launch); DRAM at 4.9 TB/s in a launch by itself (136 us at 1.63 GHz), back to back the power limit (1.32 to 1.39 GHz).  A tile's loads wait for
 // P V two tiles before, 2000 to 2900 cycles before they have landed.  Prefill: 3700 cycles a tile, the tensor core 2250, the own page's copies
 // (144 instructions an SM, 14.5 cycles each at best) and the other page's row gathers (64 of TMA, 20 each) beside each other; back to back the
 // power limit (1.6 GHz).  FP8 decode: 4300 to 4800 cycles a tile; 64 x 2048
@@ -51,10 +51,11 @@
 //   dense, 128 x ~4096 tokens                    185 ->  172       189 ->  173
 //   dense, two query tokens                      314 ->  294       325 ->  300
 //   dense, one request of 100003 tokens                           54.9 -> 47.8
-// and with P V page by page, the vote on an mbarrier and no wait for the RoPE buffers (inputs changing): FP8 60.3 -> 57.7, prefill 2328 -> 2247,
-// dense 180.4 -> 178.9, two query tokens 306 -> 304, 128 requests of lognormal lengths 530 -> 526; 512-wide records, whose exponent bytes
-// are converted in pairs, whose loads have no condition and are preceded by L2 prefetches, 50.7 -> 47.3.
-// (914 calls of dense and FP8 decode and prefill with 64 to 128 heads: between 1.04 and 2.0 times as fast, none slower.)
+// (914 calls of dense and FP8 decode and prefill with 64 to 128 heads: between 1.04 and 2.0 times as fast, none slower.)  From that state on, with
+// P V page by page, the vote on an mbarrier and no wait for the RoPE buffers (the table's calls with inputs changing, both in turn): FP8 60.5 -> 57.7,
+// prefill 2338 -> 2252; dense and two query tokens nothing to 1 % (181.7 -> 179.9, 309.0 -> 307.2), 128 requests of lognormal lengths nothing (534 ->
+// 533); 512-wide records, whose exponent bytes are converted by the instruction for them, whose loads have no condition and are preceded by L2
+// prefetches, 50.8 -> 47.5.
 // Registers: both FP8 forms spill 4 bytes a thread, the others none.
 //
 // Every mbarrier wait is bounded (Params::wait_limit SM cycles, about a second by default).  A thread whose wait ran out LEAVES its role -
@@ -443,7 +444,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 if (w.ntiles == 0) continue;
                 if (p.q_tma) {
                     ring.skip(Q_SLOTS);
-                    // nothing reads the previous request's Q any more (otherwise this thread has seen k_done of its last tile)
+                    // nothing reads the previous request's Q any more (in the gather modes this thread follows no tile, in CTA 1 only the first half of
+                    // each tile's Q K^T)
                     if (nq++ > 0) WAIT_OR_LEAVE(wt, &sm.q_free, nq & 1, 23);
                     if (rank == 0) mbar_arrive_expect_tx(smem_addr(&sm.q_full), 2 * (CHUNKS - QT) * CHUNK);
 #pragma unroll 1
@@ -549,7 +551,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         regs_dec<W::FEEDING>();
         // ---------------- prefill: rows by index, eight tokens of a page per warp -----------------------------------------
         // One cp.async instruction of the warp copies 256 bytes of two rows (a slot's share); invalid tokens get zeros.  A barrier of this
-        // CTA counts one arrival per thread, made by the copy engine when that thread's copies have landed; warps 2 and 3 pass it on.
+        // CTA counts one arrival per thread, made by the copy engine when that thread's copies have landed; a thread of warp 3 passes it on.
         const int fw = warp - W::FIRST_FEED;
         const int other = (lane >> 3) & 1, page_of_lane = other ? 1 - (int)rank : (int)rank;       // lanes 0..7 look up the own page's tokens, 8..15 the other's
         const int tok = page_of_lane * PAGE + fw * 8 + (lane & 7);

@@ -25,9 +25,10 @@ __global__ void __launch_bounds__(COMBINE_WARPS * 32, WPR == 8 ? 2 : WPR == 1 ? 
 combine_kernel(const mla_combine_args_t a) {
     // launched with programmatic stream serialization: the decode kernel before it may still be running.  (Letting the next
     // kernel set itself up from here on costs more than it hides: its CTAs take whole SMs while this grid still needs them;
-    // dense decode with 2 query tokens 346 -> 351 us a step.  Every CTA does so when it has its sums: 4 requests of 64..512 tokens, 16 heads
-    // 12.4 -> 12.05 us a step, 128 requests of lognormal lengths 488.6 -> 484.2.  With eight warps a row when they are in shared memory:
-    // one request of 100003 tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
+    // dense decode with 2 query tokens 346 -> 351 us a step.  Every CTA does so when it has its sums: 16 heads, 1, 4, 8, 16
+    // requests of 100 tokens 11.05, 11.12, 11.19, 11.39 -> 10.77, 10.79, 10.86, 10.95 us a step, of 8000 15.5, 18.6, 24.6, 38.6 -> 15.3, 18.3, 24.2, 38.0;
+    // 16 of 900 tokens, 64 heads 16.7 -> 17.0; the full batches nothing.  With eight warps a row when they are in shared memory: one request of 100003
+    // tokens, with its schedule, takes 44.8 as without, 45.1 otherwise.)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int ROWS = COMBINE_WARPS / WPR;            // heads per CTA
     constexpr int NV = 4 / PARTS;                        // float4s of a split per lane
